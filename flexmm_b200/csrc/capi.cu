@@ -264,41 +264,55 @@ struct fmm_plan {
   DevBuf<double> st_dip;    // Stokes stresslets: sigma_x, sigma_y, n_x, n_y, sorted ([4][n])
   bool has_st_dipoles = false;
   cudaStream_t side = nullptr;  // from the device's pool, not owned
-  cudaEvent_t ev_ready = nullptr, ev_near = nullptr, ev_far = nullptr;
+  cudaStream_t pass = nullptr;  // the pair's high-priority stream (PassStream)
+  cudaEvent_t ev_ready = nullptr, ev_near = nullptr, ev_far = nullptr, ev_pass = nullptr;
   bool ready_recorded = false;
   // mixed form: the split near field pauses during the M2L (SplitEval::hold)
   cudaEvent_t ev_m2l = nullptr;
   DevBuf<int> near_hold;
   bool hold_armed = false;
   ~fmm_plan() {
-    for (cudaEvent_t e : {ev_ready, ev_near, ev_far, ev_m2l})
+    for (cudaEvent_t e : {ev_ready, ev_near, ev_far, ev_m2l, ev_pass})
       if (e) cudaEventDestroy(e);
   }
 };
 
 namespace {
-// Side streams for the split evaluation: a few non-blocking streams per
-// device, handed to plans round-robin (created once, kept until exit).
+// Streams beside the caller's: a few pairs of non-blocking streams per device,
+// handed to plans round-robin (created once, kept until exit).  g_side runs
+// the split evaluation's near field at the lowest priority, g_pass the FP64
+// level passes at the highest: wherever a near-field block ends, a waiting
+// block of a level pass goes first, so the chain of levels is not held up by
+// the work it runs beside.
 constexpr int SIDE_STREAMS = 8;
 constexpr int SIDE_MAX_DEVICES = 64;
 std::mutex g_side_mu;
 cudaStream_t g_side[SIDE_MAX_DEVICES][SIDE_STREAMS] = {};
+cudaStream_t g_pass[SIDE_MAX_DEVICES][SIDE_STREAMS] = {};
 int g_side_next[SIDE_MAX_DEVICES] = {};
 
-cudaStream_t side_stream() {
+cudaStream_t side_stream(cudaStream_t *pass) {
   int dev = 0;
   FMMB_CUDA(cudaGetDevice(&dev));
   FMMB_CHECK(dev >= 0 && dev < SIDE_MAX_DEVICES, ERR_UNSUPPORTED, "device ordinal too large");
   std::lock_guard<std::mutex> g(g_side_mu);
   if (!g_side[dev][0])  // all at once: no plan after the first pays for a stream
-    for (int k = 0; k < SIDE_STREAMS; ++k)
-      FMMB_CUDA(cudaStreamCreateWithFlags(&g_side[dev][k], cudaStreamNonBlocking));
-  return g_side[dev][g_side_next[dev]++ % SIDE_STREAMS];
+  {
+    int least = 0, greatest = 0;
+    FMMB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    for (int k = 0; k < SIDE_STREAMS; ++k) {
+      FMMB_CUDA(cudaStreamCreateWithPriority(&g_pass[dev][k], cudaStreamNonBlocking, greatest));
+      FMMB_CUDA(cudaStreamCreateWithPriority(&g_side[dev][k], cudaStreamNonBlocking, least));
+    }
+  }
+  const int k = g_side_next[dev]++ % SIDE_STREAMS;
+  *pass = g_pass[dev][k];
+  return g_side[dev][k];
 }
 
 // Whether own-source evaluation runs split (near field beside the level
-// passes).  Measured at 1M clustered sources: the FP64 form gains ~0.6 ms
-// (its level passes are DMMA tiles that share SMs well); the mixed form,
+// passes).  Measured at 1M clustered sources: the FP64 form gains ~0.3 ms
+// (2.72 ms with its passes at high priority, 2.89 without); the mixed form,
 // whose near field pauses while the persistent tcgen05 M2L runs, gains
 // ~0.03 ms (1.39 -> 1.36 ms).  On for both by default;
 // FLEXMM_B200_SPLIT_EVAL=0 turns it off, =1 on.
@@ -318,10 +332,46 @@ bool split_enabled(int precision) {
 
 // the plan's split-evaluation events (created on first use) and side stream
 void split_prepare(fmm_plan *p) {
-  if (!p->side) p->side = side_stream();
-  for (cudaEvent_t *e : {&p->ev_ready, &p->ev_near, &p->ev_far, &p->ev_m2l})
+  if (!p->side) p->side = side_stream(&p->pass);
+  for (cudaEvent_t *e : {&p->ev_ready, &p->ev_near, &p->ev_far, &p->ev_m2l, &p->ev_pass})
     if (!*e) FMMB_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
 }
+
+// The stream of a plan's FP64 level passes: the high-priority one of its pair,
+// which waits for ev_ready and which the caller's stream waits for at join()
+// (at the latest when this object ends, so that buffers freed in the caller's
+// stream order are no longer read).  A stream that is being captured keeps
+// its passes: the pool's streams are shared with plans outside the capture.
+class PassStream {
+ public:
+  PassStream(fmm_plan *p, cudaStream_t s) : p_(p), s_(s), ps_(s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (!split_enabled(PREC_FP64) || cudaStreamIsCapturing(s, &st) != cudaSuccess ||
+        st != cudaStreamCaptureStatusNone) {
+      cudaGetLastError();
+      return;
+    }
+    FMMB_CUDA(cudaStreamWaitEvent(p->pass, p->ev_ready, 0));
+    ps_ = p->pass;
+  }
+  PassStream(const PassStream &) = delete;
+  PassStream &operator=(const PassStream &) = delete;
+  ~PassStream() {
+    if (ps_ != s_ && cudaEventRecord(p_->ev_pass, ps_) == cudaSuccess)
+      cudaStreamWaitEvent(s_, p_->ev_pass, 0);
+  }
+  cudaStream_t stream() const { return ps_; }
+  void join() {
+    if (ps_ == s_) return;
+    FMMB_CUDA(cudaEventRecord(p_->ev_pass, ps_));
+    ps_ = s_;
+    FMMB_CUDA(cudaStreamWaitEvent(s_, p_->ev_pass, 0));
+  }
+
+ private:
+  fmm_plan *p_;
+  cudaStream_t s_, ps_;
+};
 
 // Zeroes up to 8 device buffers in one launch (instead of one memset each:
 // at the start of build_expansions these sit between the tree and the first
@@ -1206,9 +1256,11 @@ static void build_expansions_impl(fmm_plan *p, const double *tau, void *stream) 
       FMMB_CUDA(cudaEventRecord(p->ev_ready, s));  // sorted charges: all the near field reads
       p->ready_recorded = true;
       t_prep.reset();
-      run_upward(a, p->tau_s.get(), p->mult.get(), s);
-      run_m2l(a, p->mult.get(), p->ple.get(), s);
-      run_downward(a, p->ple.get(), p->loc.get(), s);
+      PassStream ps(p, s);
+      run_upward(a, p->tau_s.get(), p->mult.get(), ps.stream());
+      run_m2l(a, p->mult.get(), p->ple.get(), ps.stream());
+      run_downward(a, p->ple.get(), p->loc.get(), ps.stream());
+      ps.join();
     }
     p->have_expansions = true;
   }
@@ -1601,7 +1653,7 @@ extern "C" int fmm_evaluate_noalloc(fmm_plan *p, const double *tx, const double 
     int *nch = (int *)carve(total * sizeof(int));
     int *choff = (int *)carve(total * sizeof(int));
     int4 *items = (int4 *)carve((total + m / EVAL_CHUNK + 1) * sizeof(int4));
-    int *n_items = (int *)carve(sizeof(int));
+    int *n_items = (int *)carve((1 + EVAL_COUNTERS) * sizeof(int));
     void *sort_tmp = carve(sort_bytes);
     void *scan_tmp = carve(scan_bytes);
     FMMB_CHECK(at <= NOALLOC_SCRATCH_BYTES, ERR_CAPACITY,

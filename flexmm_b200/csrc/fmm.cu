@@ -27,6 +27,7 @@
 #include "fmm.cuh"
 #include "gemm.cuh"
 #include "scan.cuh"
+#include "sweep.cuh"
 #include "timing.cuh"
 
 namespace fmmb {
@@ -35,11 +36,7 @@ namespace {
 constexpr int TN = 32;      // nodes per upward / downward tile
 constexpr int TM = 64;      // targets per M2L tile
 constexpr int NT = 256;     // threads per tile CTA
-constexpr int TCH = 128;    // targets per evaluation work item (= threads)
-// callers size the work-item array as total + m / EVAL_CHUNK + 1 entries
-static_assert(TCH == EVAL_CHUNK, "evaluation work items hold EVAL_CHUNK targets");
-constexpr int SMAX = 896;   // sources staged per evaluation pass (8 blocks of 128 per SM
-                            // with the log2 table beside them)
+constexpr int TCH = EVAL_CHUNK;  // targets per evaluation work item
 
 // the 27 offsets a target can see, by its parity class 2*(ix&1) + (iy&1)
 // (offset ids walk ox = -3..3 outer, oy = -3..3 inner, skipping (-1..1)^2)
@@ -87,15 +84,6 @@ __device__ __forceinline__ double kernel_at(const KF &K, double ax, double ay) {
 // sums one node's sources into its check potentials (lanes over check
 // points, the node's sources staged 32 at a time, four independent sums
 // per lane); C2E runs once for each level the tile holds.
-constexpr double INV_2PI = 1.0 / (2.0 * M_PI);
-
-// double-layer kernel of the Laplace kernel -log(r^2)/(4 pi): the field at
-// offset (ax, ay) = target - source of a dipole (dx, dy) = strength * normal,
-// (d . a) / (2 pi |a|^2) (Laplace_Both_Eval, examples/pure_kifmm_laplace_dipoles.py:31-40)
-__device__ __forceinline__ double dipole_at(double dx, double dy, double ax, double ay) {
-  return fma(dx, ax, dy * ay) / fma(ax, ax, ay * ay) * INV_2PI;
-}
-
 template <class KF, bool DIP = false>
 __global__ void __launch_bounds__(NT) k_s2m(KernelParams kp, int neq, int np, int L,
                                             const int *__restrict__ off,
@@ -527,9 +515,12 @@ __global__ void k_leaf_targets(int total, int L, const int *__restrict__ off,
 __global__ void k_make_items(int total, int L, const int *__restrict__ off, const int *__restrict__ tb,
                              const int *__restrict__ te, const int *__restrict__ nch,
                              const int *__restrict__ choff, int4 *__restrict__ items,
-                             int *__restrict__ n_items, int mark_multi) {
+                             int *__restrict__ n_items, int binned) {
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
-    if (g == total - 1) *n_items = choff[g] + nch[g];
+    if (g == total - 1) {
+      n_items[0] = choff[g] + nch[g];
+      for (int c = 1; c <= EVAL_COUNTERS; ++c) n_items[c] = 0;
+    }
     const int n = nch[g];
     if (n == 0) continue;
     int lo = 0, hi = L;
@@ -537,7 +528,8 @@ __global__ void k_make_items(int total, int L, const int *__restrict__ off, cons
       int mid = (lo + hi) >> 1;
       if (off[mid] <= g) lo = mid; else hi = mid;
     }
-    const int y = lo | (mark_multi && n > 1 ? EVAL_MULTI : 0);
+    const int y = lo | (binned && n > 1 ? EVAL_MULTI : 0) |
+                  (binned && te[g] - tb[g] > 32 ? EVAL_UNORDERED : 0);
     for (int c = 0; c < n; ++c) {
       const int t0 = tb[g] + c * TCH;
       items[choff[g] + c] = make_int4(g, y, t0, min(TCH, te[g] - t0));
@@ -545,204 +537,130 @@ __global__ void k_make_items(int total, int L, const int *__restrict__ off, cons
   }
 }
 
-// One work item = (leaf, up to 128 of its targets).  G = 128 / targets
-// (rounded down to a power of two) threads share a target: they split the
-// circle points of L2T and the colleague sources of P2P, then reduce with
-// warp shuffles (and shared memory when G > 32).
-// NOUT = 1: potential; NOUT = 3: potential and its gradient in the target
-// position (rows of out, stride ld_out).
+// KIFMM evaluation of an item: L2T (flexmm/flexmm2d/kifmm.py:106-120: the
+// leaf's equivalent sources on its large circle, swept like any other
+// sources) and P2P.
 // PART: EVAL_FULL (L2T + P2P), EVAL_NEAR (P2P only, into near[], caller's
 // point order) or EVAL_FAR (L2T only, plus near[]: out = far + near).
-// DIP: the sources also carry dipoles (dvx, dvy: strength * normal, sorted);
-// Laplace (table-driven functor), potential only.
-// CAT (near field only): a source whose category scat[] (sorted order)
-// equals the target's tcat[] (caller's order) is left out
-// (flexmm/flexmm2d/local_evaluator_category.py:33-38).
-template <class KF, int NOUT, int PART = EVAL_FULL, bool DIP = false, bool CAT = false>
-__global__ void __launch_bounds__(TCH) k_evaluate(KernelParams kp, int neq, int np,
-                                                  const int4 *__restrict__ items,
-                                                  const int *__restrict__ n_items_ptr,
-                                                  const int *__restrict__ coll,
-                                                  const int *__restrict__ bot,
-                                                  const int *__restrict__ top,
-                                                  const double *__restrict__ xmid,
-                                                  const double *__restrict__ ymid,
-                                                  const double *__restrict__ sx,
-                                                  const double *__restrict__ sy,
-                                                  const double *__restrict__ tau,
-                                                  const LevelOpsDev *__restrict__ ops,
-                                                  const double *__restrict__ loc,
-                                                  const double *__restrict__ txs,
-                                                  const double *__restrict__ tys,
-                                                  const int *__restrict__ tperm, int check,
-                                                  double *__restrict__ out, int64_t ld_out,
-                                                  double *__restrict__ near = nullptr,
-                                                  const double *__restrict__ dvx = nullptr,
-                                                  const double *__restrict__ dvy = nullptr,
-                                                  const int64_t *__restrict__ scat = nullptr,
-                                                  const int64_t *__restrict__ tcat = nullptr) {
+template <class KF, int NOUT, int PART, bool DIP = false, bool CAT = false>
+struct KIPolicy : ChargePolicy<KF, NOUT, DIP, CAT> {
+  using Base = ChargePolicy<KF, NOUT, DIP, CAT>;
   static_assert(PART == EVAL_FULL || NOUT == 1, "split evaluation: potential only");
-  static_assert(!CAT || (PART == EVAL_NEAR && !DIP), "categories: near field of charges only");
-  static_assert(!DIP || (KF::kLogTable && NOUT == 1), "dipoles: table Laplace, potential only");
-  __shared__ double Ls[64], lxs[64], lys[64];
-  __shared__ double ssx[SMAX], ssy[SMAX], stau[SMAX];
-  __shared__ double sdx[DIP ? SMAX : 1], sdy[DIP ? SMAX : 1];
-  __shared__ long long scs[CAT ? SMAX : 1];
-  __shared__ int rb[9], rs[10];  // colleague range begins and prefix sizes
-  __shared__ double red[NOUT][TCH / 32];
-  __shared__ FunctorSmem<KF> fsm;
-  KF K(kp);
-  fsm.bind(K);
-  // table-driven Laplace (potential only): the kernel's constant factor is
-  // folded into the staged locals and charges, the loops sum raw log2 values
-  constexpr bool kFolded = KF::kLogTable && NOUT == 1;
-  const double fold = fold_of<KF, kFolded>();
-  const int n_items = *n_items_ptr;
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const int4 it = items[item];
-    const int g = it.x, lev = it.y & EVAL_LEVEL_MASK, t0 = it.z, cnt = it.w;
-    int G = 1;
-    if (!(it.y & EVAL_MULTI))
-      while (2 * G * cnt <= TCH) G *= 2;
-    const int t = threadIdx.x / G, sub = threadIdx.x % G;
-    const bool valid = t < cnt;
-    const double x = valid ? txs[t0 + t] : 0.0, y = valid ? tys[t0 + t] : 0.0;
-    long long tc = 0;
-    if constexpr (CAT) tc = valid ? (long long)tcat[tperm[t0 + t]] : 0;
-    if (threadIdx.x < 9) {
-      const int cg = PART == EVAL_FAR ? -1 : coll[(size_t)g * 9 + threadIdx.x];
-      rb[threadIdx.x] = cg >= 0 ? bot[cg] : 0;
-      rs[threadIdx.x + 1] = cg >= 0 ? top[cg] - bot[cg] : 0;
-    }
-    if (threadIdx.x == 0) rs[0] = 0;
-    // L2T (flexmm/flexmm2d/kifmm.py:106-120); locals of levels 0-1 are zero
-    const bool l2t = lev >= 2 && PART != EVAL_NEAR;
-    if (l2t)
-      for (int k = threadIdx.x; k < neq; k += TCH) {
-        Ls[k] = loc[(size_t)g * np + k] * fold;
-        lxs[k] = ops[lev].lx[k];
-        lys[k] = ops[lev].ly[k];
+  static_assert(!CAT || PART == EVAL_NEAR, "categories: near field only");
+  static constexpr bool kNear = PART != EVAL_FAR, kFar = PART != EVAL_NEAR;
+  static constexpr int SMAX = Base::SMAX;
+  struct FarSmem {
+    double2 xy[64];
+    double q[64];
+    double cx, cy;
+  };
+  struct NoSmem {
+    FunctorSmem<KF> f;
+  };
+  struct Smem : std::conditional<kNear, typename Base::Smem, NoSmem>::type {
+    typename std::conditional<kFar, FarSmem, char>::type far;
+  };
+  int neq, np;
+  const double *xmid, *ymid, *loc;
+  const LevelOpsDev *ops;
+  double *near;
+
+  __device__ __forceinline__ void stage_far(Smem &sm, int g, int lev) const {
+    if constexpr (kFar) {
+      for (int k = threadIdx.x; k < neq; k += EV_THREADS) {
+        sm.far.q[k] = loc[(size_t)g * np + k] * Base::fold();
+        sm.far.xy[k] = make_double2(ops[lev].lx[k], ops[lev].ly[k]);
       }
-    __syncthreads();
-    if (threadIdx.x == 0)
-      for (int c = 1; c <= 9; ++c) rs[c] += rs[c - 1];
-    double u0 = 0.0, u1 = 0.0, u2 = 0.0, u3 = 0.0;
-    double gu = 0.0, gx = 0.0, gy = 0.0;  // NOUT = 3
-    if (l2t && valid) {
-      const double dx = x - xmid[g], dy = y - ymid[g];
-      if constexpr (NOUT == 1) {
-        auto kv = [&](int k) -> double {
-          if constexpr (kFolded)
-            return K.raw(dx - lxs[k], dy - lys[k]);
-          else
-            return K(lxs[k], lys[k], dx, dy);
-        };
-        int k = sub;
-        for (; k + 3 * G < neq; k += 4 * G) {
-          u0 = fma(kv(k), Ls[k], u0);
-          u1 = fma(kv(k + G), Ls[k + G], u1);
-          u2 = fma(kv(k + 2 * G), Ls[k + 2 * G], u2);
-          u3 = fma(kv(k + 3 * G), Ls[k + 3 * G], u3);
-        }
-        for (; k < neq; k += G) u0 = fma(kv(k), Ls[k], u0);
-      } else {
-        for (int k = sub; k < neq; k += G) K.grad(lxs[k], lys[k], dx, dy, Ls[k], gu, gx, gy);
+      if (threadIdx.x == 64) {
+        sm.far.cx = xmid[g];
+        sm.far.cy = ymid[g];
       }
     }
-    __syncthreads();
-    // P2P over the colleagues' sorted source ranges (flexmm/flexmm2d/helpers.py:152-194);
-    // a coincident pair is skipped when check is set (helpers.py:99-107)
-    auto pair = [&](int j) -> double {
-      const double qx = ssx[j], qy = ssy[j];
-      if constexpr (DIP) {  // single plus double layer; coincident pairs skipped when check
-        const double ax = x - qx, ay = y - qy;
-        if (check && ax == 0.0 && ay == 0.0) return 0.0;
-        return K.raw(ax, ay) * stau[j] + dipole_at(sdx[j], sdy[j], ax, ay);
-      } else if constexpr (CAT) {  // a source of the target's own category adds nothing
-        if (scs[j] == tc) return 0.0;
-        if constexpr (kFolded) {
-          return K.raw_checked(qx, qy, x, y, check) * stau[j];
-        } else {
-          const double v = K(qx, qy, x, y) * stau[j];
-          return (check && x - qx == 0.0 && y - qy == 0.0) ? 0.0 : v;
-        }
-      } else if constexpr (kFolded) {
-        return K.raw_checked(qx, qy, x, y, check) * stau[j];
-      } else {
-        const double v = K(qx, qy, x, y) * stau[j];
-        return (check && x - qx == 0.0 && y - qy == 0.0) ? 0.0 : v;
-      }
-    };
-    const int ns = rs[9];
-    for (int base = 0; base < ns; base += SMAX) {
-      const int nb = min(SMAX, ns - base);
-      for (int i = threadIdx.x; i < nb; i += TCH) {
-        const int idx = base + i;
-        int c = 0;
-        while (idx >= rs[c + 1]) ++c;
-        const int j = rb[c] + (idx - rs[c]);
-        ssx[i] = sx[j];
-        ssy[i] = sy[j];
-        stau[i] = tau[j] * fold;
-        if constexpr (DIP) {
-          sdx[i] = dvx[j];
-          sdy[i] = dvy[j];
-        }
-        if constexpr (CAT) scs[i] = (long long)scat[j];
-      }
-      __syncthreads();
-      if (valid) {
-        if constexpr (NOUT == 1) {
-          int j = sub;
-          for (; j + 3 * G < nb; j += 4 * G) {
-            u0 += pair(j);
-            u1 += pair(j + G);
-            u2 += pair(j + 2 * G);
-            u3 += pair(j + 3 * G);
-          }
-          for (; j < nb; j += G) u0 += pair(j);
-        } else {
-          for (int j = sub; j < nb; j += G) {
-            const double qx = ssx[j], qy = ssy[j];
-            if (!(check && x - qx == 0.0 && y - qy == 0.0)) K.grad(qx, qy, x, y, stau[j], gu, gx, gy);
-          }
-        }
-      }
-      __syncthreads();
-    }
-    // reduce over the G threads of each target
-    double r[NOUT];
-    if constexpr (NOUT == 1) {
-      r[0] = (u0 + u1) + (u2 + u3);
-    } else {
-      r[0] = gu;
-      r[1] = gx;
-      r[2] = gy;
-    }
-#pragma unroll
-    for (int o = 0; o < NOUT; ++o) {
-      double u = r[o];
-      for (int w = min(G, 32) >> 1; w >= 1; w >>= 1) u += __shfl_xor_sync(0xffffffffu, u, w);
-      if (G > 32) {
-        if ((threadIdx.x & 31) == 0) red[o][threadIdx.x >> 5] = u;
-        __syncthreads();
-        if (sub == 0) {
-          u = 0.0;
-          for (int w = 0; w < G / 32; ++w) u += red[o][(threadIdx.x >> 5) + w];
-        }
-      }
-      if (valid && sub == 0) {
-        const int i = tperm[t0 + t];
-        if constexpr (PART == EVAL_NEAR)
-          near[i] = u;
-        else if constexpr (PART == EVAL_FAR)
-          out[i] = u + near[i];
-        else
-          out[o * ld_out + i] = u;
-      }
-    }
-    __syncthreads();
   }
+  __device__ __forceinline__ void stage(Smem &sm, int i, int j) const {
+    if constexpr (kNear) Base::stage(sm, i, j);
+  }
+  template <int R>
+  __device__ __forceinline__ void sweep(const KF &K, const Smem &sm, const double (&x)[R],
+                                        const double (&y)[R],
+                                        const typename Base::template Tgt<R> &tg, int lo, int hi,
+                                        int G, double (&v)[R][Base::NV]) const {
+    if constexpr (kNear) Base::template sweep<R>(K, sm, x, y, tg, lo, hi, G, v);
+  }
+  template <int R>
+  __device__ __forceinline__ void far_field(const KF &K, const Smem &sm, int, int,
+                                            const double (&x)[R], const double (&y)[R], int warp,
+                                            int sub, int G, double (&v)[R][Base::NV]) const {
+    if constexpr (kFar) {
+      double dx[R], dy[R];
+      long long none[R] = {};
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        dx[r] = x[r] - sm.far.cx;
+        dy[r] = y[r] - sm.far.cy;
+      }
+      const int lo = (neq * warp) / EV_WARPS + sub, hi = (neq * (warp + 1)) / EV_WARPS;
+      if constexpr (NOUT == 1)
+        pot_sweep<KF, R, false, false>(K, sm.far.xy, sm.far.q, nullptr, nullptr, dx, dy, none, lo,
+                                       hi, G, 0, v);
+      else
+        grad_sweep<KF, R>(K, sm.far.xy, sm.far.q, dx, dy, lo, hi, G, 0, v);
+    }
+  }
+  __device__ __forceinline__ void store(int i, const double (&o)[NOUT]) const {
+    if constexpr (PART == EVAL_NEAR)
+      near[i] = o[0];
+    else if constexpr (PART == EVAL_FAR)
+      this->out[i] = o[0] + near[i];
+    else
+      Base::store(i, o);
+  }
+};
+
+// the policy's fields that every part has
+template <class Pol>
+Pol ki_policy(const PassArgs &a, const double *tau_s, const double *loc, int check, double *out,
+              int64_t ld_out, double *near) {
+  const TreeDev &td = *a.td;
+  Pol p{};
+  p.kp = a.kp;
+  p.sx = td.sx.get();
+  p.sy = td.sy.get();
+  p.tau = tau_s;
+  p.dvx = a.dvx;
+  p.dvy = a.dvy;
+  p.check = check;
+  p.out = out;
+  p.ld_out = ld_out;
+  p.neq = a.neq;
+  p.np = a.np;
+  p.xmid = td.xmid.get();
+  p.ymid = td.ymid.get();
+  p.loc = loc;
+  p.ops = a.ops_dev;
+  p.near = near;
+  return p;
+}
+
+ItemArgs item_args(const PassArgs &a, const int4 *items, int *n_items, int counter,
+                   const double *txs, const double *tys, const int *tperm) {
+  const TreeDev &td = *a.td;
+  return ItemArgs{items, n_items, n_items + 1 + counter, td.coll.get(), td.bot.get(),
+                  td.top.get(), txs, tys, tperm};
+}
+
+template <class T>
+struct TypeOf {
+  using type = T;
+};
+
+// resident blocks per SM the potential and gradient evaluations are built for
+constexpr int EVAL_BLOCKS = 8, EVAL_BLOCKS_GRAD = 6;
+
+template <class Pol, int BLOCKS>
+void launch_items(const Pol &pol, const ItemArgs &ia, int64_t units, int per_sm, cudaStream_t s) {
+  k_items<Pol, BLOCKS><<<work_grid(units, per_sm), EV_THREADS, 0, s>>>(pol, ia);
+  FMMB_CUDA(cudaGetLastError());
 }
 
 // FP64 direct sum (kernel_apply / kernel_apply_single_check,
@@ -970,7 +888,7 @@ void eval_items(const PassArgs &a, const uint64_t *tkeys, int64_t m, EvalItems &
   FMMB_CUDA(cudaGetLastError());
   prefix_sum<int, false>(it.nch.get(), it.choff.get(), total, td.sort_fail.get(), true, s);
   it.items.alloc(total + m / TCH + 1, s);
-  it.n_items.alloc(1, s);
+  it.n_items.alloc(1 + EVAL_COUNTERS, s);
   k_make_items<<<grid_for(total, 256), 256, 0, s>>>(total, th.L, td.dev_off.get(), it.tb.get(),
                                                     it.te.get(), it.nch.get(), it.choff.get(),
                                                     it.items.get(), it.n_items.get(), 0);
@@ -1008,7 +926,7 @@ void eval_items_binned(const PassArgs &a, const double *tx, const double *ty, in
   FMMB_CUDA(cudaGetLastError());
   prefix_sum<int, false>(it.nch.get(), it.choff.get(), total, td.sort_fail.get(), true, s);
   it.items.alloc(total + m / TCH + 1, s);
-  it.n_items.alloc(1, s);
+  it.n_items.alloc(1 + EVAL_COUNTERS, s);
   k_make_items<<<grid_for(total, 256), 256, 0, s>>>(total, th.L, td.dev_off.get(), it.tb.get(),
                                                     it.te.get(), it.nch.get(), it.choff.get(),
                                                     it.items.get(), it.n_items.get(), 1);
@@ -1020,31 +938,30 @@ template <class KF>
 void evaluate_impl(const PassArgs &a, const double *tau_s, const double *loc, const double *txs,
                    const double *tys, const uint64_t *tkeys, const int *tperm, int64_t m, int check,
                    int nout, double *out, int64_t ld_out, cudaStream_t s, const EvalItems *pre) {
-  const TreeDev &td = *a.td;
   EvalItems own;
   if (!pre) eval_items(a, tkeys, m, own, s);
   const EvalItems &it = pre ? *pre : own;
   const int64_t units = a.th->n_total() + m / TCH + 1;  // work items, upper bound
   PhaseTimer timer(PH_EVAL, s);
+  const ItemArgs ia = item_args(a, it.items.get(), it.n_items.get(), 0, txs, tys, tperm);
   if (a.dvx) {
     FMMB_CHECK(nout == 1, ERR_UNSUPPORTED, "dipole sources: potential only");
     if constexpr (std::is_same<KF, LaplaceF64T>::value) {
-      k_evaluate<KF, 1, EVAL_FULL, true><<<work_grid(units, 5), TCH, 0, s>>>(
-          a.kp, a.neq, a.np, it.items.get(), it.n_items.get(), td.coll.get(), td.bot.get(),
-          td.top.get(), td.xmid.get(), td.ymid.get(), td.sx.get(), td.sy.get(), tau_s, a.ops_dev,
-          loc, txs, tys, tperm, check, out, ld_out, nullptr, a.dvx, a.dvy);
+      using Pol = KIPolicy<KF, 1, EVAL_FULL, true>;
+      launch_items<Pol, EVAL_BLOCKS_GRAD>(
+          ki_policy<Pol>(a, tau_s, loc, check, out, ld_out, nullptr), ia, units, EVAL_BLOCKS_GRAD, s);
     } else {
       throw Error(ERR_UNSUPPORTED, "dipole sources: Laplace kernel only");
     }
+  } else if (nout == 3) {
+    using Pol = KIPolicy<KF, 3, EVAL_FULL>;
+    launch_items<Pol, EVAL_BLOCKS_GRAD>(ki_policy<Pol>(a, tau_s, loc, check, out, ld_out, nullptr),
+                                        ia, units, EVAL_BLOCKS_GRAD, s);
   } else {
-    auto kern = nout == 3 ? k_evaluate<KF, 3> : k_evaluate<KF, 1>;
-    kern<<<work_grid(units, 8), TCH, 0, s>>>(a.kp, a.neq, a.np, it.items.get(), it.n_items.get(),
-                                 td.coll.get(), td.bot.get(), td.top.get(), td.xmid.get(),
-                                 td.ymid.get(), td.sx.get(), td.sy.get(), tau_s, a.ops_dev, loc,
-                                 txs, tys, tperm, check, out, ld_out, nullptr, nullptr, nullptr,
-                                 nullptr, nullptr);
+    using Pol = KIPolicy<KF, 1, EVAL_FULL>;
+    launch_items<Pol, EVAL_BLOCKS>(ki_policy<Pol>(a, tau_s, loc, check, out, ld_out, nullptr), ia,
+                                   units, EVAL_BLOCKS, s);
   }
-  FMMB_CUDA(cudaGetLastError());
 }
 }  // namespace
 
@@ -1144,30 +1061,32 @@ void evaluate_split_impl(const PassArgs &a, const double *tau_s, const double *l
   {
     // the SMs keep their largest shared-memory carveout while near-field
     // blocks sit on them, so the level passes' CTAs still fit beside them
+    using Near = KIPolicy<KF, 1, EVAL_NEAR, DIP>;
     static const bool carveout_set = [] {
-      FMMB_CUDA(cudaFuncSetAttribute(k_evaluate<KF, 1, EVAL_NEAR, DIP>,
+      FMMB_CUDA(cudaFuncSetAttribute(k_items<Near, EVAL_BLOCKS>,
                                      cudaFuncAttributePreferredSharedMemoryCarveout,
                                      cudaSharedmemCarveoutMaxShared));
       return true;
     }();
     (void)carveout_set;
     PhaseTimer timer(PH_EVAL, se.side);
-    k_evaluate<KF, 1, EVAL_NEAR, DIP><<<work_grid(units, NEAR_BLOCKS_PER_SM), TCH, 0, se.side>>>(
-        a.kp, a.neq, a.np, it.items.get(), it.n_items.get(), td.coll.get(), td.bot.get(),
-        td.top.get(), td.xmid.get(), td.ymid.get(), td.sx.get(), td.sy.get(), tau_s, a.ops_dev,
-        loc, td.sx.get(), td.sy.get(), td.ordv.get(), check, out, 0, near.get(), a.dvx, a.dvy);
+    ItemArgs ia = item_args(a, it.items.get(), it.n_items.get(), 0, td.sx.get(), td.sy.get(),
+                            td.ordv.get());
+    ia.per_block = NEAR_ITEMS_PER_BLOCK;
+    const int blocks = int((units + NEAR_ITEMS_PER_BLOCK - 1) / NEAR_ITEMS_PER_BLOCK);
+    k_items<Near, EVAL_BLOCKS><<<blocks, EV_THREADS, 0, se.side>>>(
+        ki_policy<Near>(a, tau_s, loc, check, out, 0, near.get()), ia);
     FMMB_CUDA(cudaGetLastError());
   }
   FMMB_CUDA(cudaEventRecord(se.near_done, se.side));
   FMMB_CUDA(cudaStreamWaitEvent(s, se.near_done, 0));
   {
     PhaseTimer timer(PH_EVAL, s);
-    k_evaluate<KF, 1, EVAL_FAR><<<work_grid(units, 8), TCH, 0, s>>>(
-        a.kp, a.neq, a.np, it.items.get(), it.n_items.get(), td.coll.get(), td.bot.get(),
-        td.top.get(), td.xmid.get(), td.ymid.get(), td.sx.get(), td.sy.get(), tau_s, a.ops_dev,
-        loc, td.sx.get(), td.sy.get(), td.ordv.get(), check, out, 0, near.get(), nullptr,
-        nullptr);
-    FMMB_CUDA(cudaGetLastError());
+    using Far = KIPolicy<KF, 1, EVAL_FAR>;
+    launch_items<Far, EVAL_BLOCKS>(
+        ki_policy<Far>(a, tau_s, loc, check, out, 0, near.get()),
+        item_args(a, it.items.get(), it.n_items.get(), 1, td.sx.get(), td.sy.get(), td.ordv.get()),
+        units, EVAL_BLOCKS, s);
   }
   // the scratch (allocated on the side stream) is freed there once the plan
   // stream is done with it
@@ -1246,22 +1165,22 @@ template <class KF>
 void local_impl(const PassArgs &a, const double *tau_s, const double *txs, const double *tys,
                 const uint64_t *tkeys, const int *tperm, int64_t m, int check,
                 const int64_t *scat, const int64_t *tcat, double *out, cudaStream_t s) {
-  const TreeDev &td = *a.td;
   EvalItems it;
   eval_items(a, tkeys, m, it, s);
-  const int grid = work_grid(a.th->n_total() + m / TCH + 1, 8);
+  const int64_t units = a.th->n_total() + m / TCH + 1;
+  const ItemArgs ia = item_args(a, it.items.get(), it.n_items.get(), 0, txs, tys, tperm);
   PhaseTimer timer(PH_EVAL, s);
-  if (scat)
-    k_evaluate<KF, 1, EVAL_NEAR, false, true><<<grid, TCH, 0, s>>>(
-        a.kp, a.neq, a.np, it.items.get(), it.n_items.get(), td.coll.get(), td.bot.get(),
-        td.top.get(), td.xmid.get(), td.ymid.get(), td.sx.get(), td.sy.get(), tau_s, a.ops_dev,
-        nullptr, txs, tys, tperm, check, out, 0, out, nullptr, nullptr, scat, tcat);
-  else
-    k_evaluate<KF, 1, EVAL_NEAR><<<grid, TCH, 0, s>>>(
-        a.kp, a.neq, a.np, it.items.get(), it.n_items.get(), td.coll.get(), td.bot.get(),
-        td.top.get(), td.xmid.get(), td.ymid.get(), td.sx.get(), td.sy.get(), tau_s, a.ops_dev,
-        nullptr, txs, tys, tperm, check, out, 0, out, nullptr, nullptr, nullptr, nullptr);
-  FMMB_CUDA(cudaGetLastError());
+  if (scat) {
+    using Pol = KIPolicy<KF, 1, EVAL_NEAR, false, true>;
+    Pol pol = ki_policy<Pol>(a, tau_s, nullptr, check, nullptr, 0, out);
+    pol.scat = scat;
+    pol.tcat = tcat;
+    launch_items<Pol, EVAL_BLOCKS>(pol, ia, units, EVAL_BLOCKS, s);
+  } else {
+    using Pol = KIPolicy<KF, 1, EVAL_NEAR>;
+    launch_items<Pol, EVAL_BLOCKS>(ki_policy<Pol>(a, tau_s, nullptr, check, nullptr, 0, out), ia,
+                                   units, EVAL_BLOCKS, s);
+  }
 }
 }  // namespace
 
@@ -1337,20 +1256,18 @@ void run_evaluate_scratch(const PassArgs &a, const double *tau_s, const double *
                                                     items, n_items, 0);
   FMMB_CUDA(cudaGetLastError());
   PhaseTimer timer(PH_EVAL, s);
-  auto launch = [&](auto kern) {
-    kern<<<work_grid(total + m / TCH + 1, 8), TCH, 0, s>>>(a.kp, a.neq, a.np, items, n_items,
-                                                             td.coll.get(), td.bot.get(),
-                                 td.top.get(), td.xmid.get(), td.ymid.get(), td.sx.get(),
-                                 td.sy.get(), tau_s, a.ops_dev, loc, txs, tys, tperm, check, out, 0,
-                                 nullptr, nullptr, nullptr, nullptr, nullptr);
+  const ItemArgs ia = item_args(a, items, n_items, 0, txs, tys, tperm);
+  auto launch = [&](auto kf) {
+    using Pol = KIPolicy<typename decltype(kf)::type, 1, EVAL_FULL>;
+    launch_items<Pol, EVAL_BLOCKS>(ki_policy<Pol>(a, tau_s, loc, check, out, 0, nullptr), ia,
+                                   total + m / TCH + 1, EVAL_BLOCKS, s);
   };
   switch (a.kernel_id) {
-    case KERNEL_LAPLACE: launch(k_evaluate<LaplaceF64T, 1>); break;
-    case KERNEL_MOD_HELMHOLTZ: launch(k_evaluate<ModHelmholtzF64, 1>); break;
-    case KERNEL_RADIAL_TABLE: launch(k_evaluate<RadialTableF64, 1>); break;
+    case KERNEL_LAPLACE: launch(TypeOf<LaplaceF64T>{}); break;
+    case KERNEL_MOD_HELMHOLTZ: launch(TypeOf<ModHelmholtzF64>{}); break;
+    case KERNEL_RADIAL_TABLE: launch(TypeOf<RadialTableF64>{}); break;
     default: throw Error(ERR_UNSUPPORTED, "unknown kernel id");
   }
-  FMMB_CUDA(cudaGetLastError());
 }
 
 namespace {

@@ -127,15 +127,18 @@ struct SplitEval {
   int *hold = nullptr;
   cudaEvent_t m2l_done = nullptr;
 };
-// near-field blocks per SM, leaving room for the level passes: FP64 (28 KB of
-// shared memory each) beside the DMMA M2L tiles; mixed (17 KB each) beside
-// the upward pass until the M2L (which it leaves to the persistent tcgen05
-// CTAs), then beside the downward pass.  Mixed, measured at 1M (step ms,
+// FP64 near field beside the passes: items a block takes before it ends (its
+// place may then go to a level pass, which has the higher priority).  Step in
+// us at 1 / 2 / 4: 1M clustered points 2753 / 2717 / 2708, a 250k-point
+// product on a kept tree 843 / 835 / 832, 100k uniform 625 / 645 / 663; blocks
+// that stay to the end: 2890 / 890 / 643.
+constexpr int NEAR_ITEMS_PER_BLOCK = 2;
+// near-field blocks per SM of the mixed form (17 KB of shared memory each),
+// beside the upward pass until the M2L (which it leaves to the persistent
+// tcgen05 CTAs), then beside the downward pass.  Measured at 1M (step ms,
 // two runs each, one box): before / after the M2L 3/10 1.277-1.281, 2/10
 // 1.282-1.286, 6/10 1.253-1.262, 8/10 1.245-1.247, 12/10 1.287, 6/8
-// 1.247-1.249, 6/12 1.273-1.277.  FP64 (step ms, same way): 2 5.10, 3 3.86,
-// 4 3.350-3.351, 6 3.194, 8 3.197-3.204.
-constexpr int NEAR_BLOCKS_PER_SM = 6;
+// 1.247-1.249, 6/12 1.273-1.277.
 constexpr int NEAR_BLOCKS_PER_SM_MIXED = 8;
 constexpr int NEAR_BLOCKS_PER_SM_MIXED_RESUME = 10;  // after the M2L, beside the downward pass
 void run_evaluate_sources_split(const PassArgs &a, const double *tau_sorted, const double *loc,
@@ -179,14 +182,18 @@ void run_evaluate(const PassArgs &a, const double *tau_sorted, const double *loc
 // chunks of 128 targets; choff = exclusive scan of the chunk counts.
 struct EvalItems {
   DevBuf<int> tb, te, nch, choff;
-  DevBuf<int4> items;   // (leaf, level | EVAL_MULTI, first sorted target, count)
-  DevBuf<int> n_items;  // device count of items
+  DevBuf<int4> items;   // (leaf, level | flags, first sorted target, count)
+  DevBuf<int> n_items;  // [0] device count of items, [1 ..] zeroed hand-out counters
 };
+constexpr int EVAL_COUNTERS = 3;  // hand-out counters of an item list (one per launch over it)
 // item .y: the leaf's level, plus EVAL_MULTI when the leaf's targets fill more
 // than one item (targets placed in no particular order inside the leaf): then
 // every item of the leaf gives one thread per target (G = 1), so that a
 // target's arithmetic does not depend on which item holds it
 constexpr int EVAL_LEVEL_MASK = 0xFF, EVAL_MULTI = 0x100;
+// item .y: more than 32 targets in no particular order inside their leaf: the
+// FP64 evaluation then splits the sources of every target the same way
+constexpr int EVAL_UNORDERED = 0x200;
 constexpr int EVAL_CHUNK = 128;  // targets per evaluation work item
 // parts of an evaluation: both, the near field (P2P) alone, the far field (L2T) alone
 constexpr int EVAL_FULL = 0, EVAL_NEAR = 1, EVAL_FAR = 2;

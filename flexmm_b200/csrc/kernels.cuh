@@ -32,56 +32,71 @@ struct KernelParams {
 // ---------------------------------------------------------------------------
 // Table-driven FP64 log2, after P. T. P. Tang, "Table-driven implementation
 // of the logarithm function in IEEE floating-point arithmetic", ACM TOMS 16
-// (1990): d = 2^e m, m in [1, 2); F = 1 + j/256 is the table point nearest m,
-// so r = (m - F) / F has |r| <= 2^-9 and
-//   log2 d = e + log2 F + log2(1 + r),
-//   log2(1 + r) = r (c1 + r (c2 + r (c3 + r (c4 + r c5)))),  c_k = (-1)^(k+1) / (k ln 2),
-// the Taylor series of log(1 + r) / ln 2 cut after r^5 (the first dropped
-// term, r^6 / (6 ln 2), is below 1.3e-17).  m - F is exact; the table holds
-// 1/F (IEEE division) and log2 F (CUDA's log2) for j = 0..256, filled in
+// (1990): d = 2^e m, m in [1, 2); F = 1 + j/128 is the table point nearest m
+// and c = 1/F rounded, so r = m c - 1 (one fused multiply-add) has
+// |r| <= 2^-8 and
+//   log2 d = e - log2 c + log2(1 + r),  log2(1 + r) = r q(r),
+// q the degree-4 polynomial that takes log2(1 + r)/r's values at the five
+// Chebyshev nodes of [-2^-8, 2^-8] (error of r q(r): 5.4e-17).  The table
+// holds c (IEEE division) and -log2 c (CUDA's log2) for j = 0..128, filled in
 // shared memory by each block.  Absolute error about one ulp of the result
-// (~1e-16 relative to max(1, |log2 d|)): far inside the 1e-12 parity bar,
-// at about a third of the FP64 instructions of the library log.  Zero,
-// subnormal, infinite and NaN arguments take the library log2 instead.
-constexpr int LOG2_TAB_N = 256;
+// (~1e-16 relative to max(1, |log2 d|)): far inside the 1e-12 parity bar, in
+// 9 FP64 instructions.  Zero, subnormal, infinite and NaN arguments take the
+// library log2 instead.
+// A pair loop over it costs 11.8 clocks per 32 pairs and SM with two targets
+// a thread, 17.2 with the 257-point table and r = (m - F) / F before (the
+// FP64 instructions alone: 7.2); spreading the table over the banks (8
+// copies) gave 11.35 for 14 KB more per block.
+constexpr int LOG2_TAB_N = 128;
 struct Log2Table {
   double2 t[LOG2_TAB_N + 1];
   __device__ void fill() {
     for (int i = threadIdx.x; i <= LOG2_TAB_N; i += blockDim.x) {
-      const double F = 1.0 + i * (1.0 / LOG2_TAB_N);
-      t[i] = make_double2(1.0 / F, log2(F));
+      const double c = 1.0 / (1.0 + i * (1.0 / LOG2_TAB_N));
+      t[i] = make_double2(c, -log2(c));
     }
   }
 };
 
-// true for arguments outside the table path: zero, subnormal, negative,
-// infinite or NaN (one unsigned compare of the high word)
-__device__ __forceinline__ bool log2_tab_rare(double d) {
-  return (unsigned)(__double2hiint(d) - 0x00100000) >= 0x7FE00000u;
+// log2_rare_key(d) >= LOG2_RARE for arguments outside the table path: zero,
+// subnormal, negative, infinite or NaN (one unsigned compare; the largest key
+// of several arguments tests them together)
+constexpr unsigned LOG2_RARE = 0x7FE00000u;
+__device__ __forceinline__ unsigned log2_rare_key(double d) {
+  return (unsigned)(__double2hiint(d) - 0x00100000);
 }
+__device__ __forceinline__ bool log2_tab_rare(double d) { return log2_rare_key(d) >= LOG2_RARE; }
 
 // log2 of a positive normal finite d (callers route log2_tab_rare arguments
 // elsewhere)
 __device__ __forceinline__ double log2_tab(double d, const double2 *__restrict__ tab) {
-  constexpr double LN2 = 0.69314718055994530942;
-  constexpr double C1 = 1.0 / LN2, C2 = -1.0 / (2.0 * LN2), C3 = 1.0 / (3.0 * LN2),
-                   C4 = -1.0 / (4.0 * LN2), C5 = 1.0 / (5.0 * LN2);
+  constexpr double Q0 = 0x1.71547652b82fep+0, Q1 = -0x1.7154765291b6fp-1,
+                   Q2 = 0x1.ec709dc35e431p-2, Q3 = -0x1.7155aa1a01b8ap-2,
+                   Q4 = 0x1.2777ccebb940ap-2;
   const int hi = __double2hiint(d), lo = __double2loint(d);
   const int mh = hi & 0x000FFFFF;
-  const int j = (mh + (1 << 11)) >> 12;                           // nearest 1/256 step: 0..256
-  const double m = __hiloint2double(mh | 0x3FF00000, lo);         // [1, 2)
-  const double F = __hiloint2double(0x3FF00000 + (j << 12), 0);   // 1 + j/256 (j = 256: 2)
-  const double2 tj = tab[j];
-  const double r = (m - F) * tj.x;
-  // the exponent as a double without a conversion instruction:
-  // bits (0x43300000, e + 2^31) are 2^52 + 2^31 + e
-  const double e = __hiloint2double(0x43300000, ((hi >> 20) - 1023) ^ (int)0x80000000) -
-                   4503601774854144.0;
-  double q = fma(r, C5, C4);
-  q = fma(r, q, C3);
-  q = fma(r, q, C2);
-  q = fma(r, q, C1);
+  const double m = __hiloint2double(mh | 0x3FF00000, lo);  // [1, 2)
+  const double2 tj = tab[(mh + (1 << 12)) >> 13];          // nearest 1/128 step: 0..128
+  const double r = fma(m, tj.x, -1.0);
+  // the exponent as a double without a conversion instruction: the bits
+  // (0x43300000, n) are 2^52 + n
+  const double e = __hiloint2double(0x43300000, hi >> 20) - (4503599627370496.0 + 1023.0);
+  double q = fma(r, Q4, Q3);
+  q = fma(r, q, Q2);
+  q = fma(r, q, Q1);
+  q = fma(r, q, Q0);
   return fma(r, q, e + tj.y);
+}
+
+// 1/d for d in [2^-1022, 2^1021): the hardware's approximate reciprocal
+// (rcp.approx.ftz.f64, about 20 bits), refined by the third-order Newton step
+// y (1 + e + e^2), e = 1 - d y: error e^3, below the last bit
+constexpr unsigned RCP_RARE = 0x7FC00000u;  // log2_rare_key from here on: not for rcp_newton
+__device__ __forceinline__ double rcp_newton(double d) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  const double e = fma(-d, y, 1.0);
+  return fma(y, fma(e, e, e), y);
 }
 
 // Shared-memory state a functor needs inside a kernel (the log2 table of
@@ -114,34 +129,43 @@ struct LaplaceF64 {
 // The Laplace kernel of the FP64 passes: LaplaceF64 with the table-driven
 // log2 above.  raw(dx, dy) = log2(dx^2 + dy^2), so K = kFold * raw; the P2P
 // and L2T loops fold kFold into their staged charges / locals.
+// A table functor's pair loops split raw into arg() of the squared distance,
+// at() of an argument inside the table path, and raw_rare() for the others.
 struct LaplaceF64T {
   static constexpr bool kLogTable = true;
   static constexpr double kFold = -0.69314718055994530942 / (4.0 * M_PI);  // -ln2 / (4 pi)
   const double2 *lt = nullptr;  // the block's table (FunctorSmem::bind)
   __host__ __device__ explicit LaplaceF64T(const KernelParams &) {}
-  __device__ __forceinline__ double raw(double dx, double dy) const {
-    const double d2 = dx * dx + dy * dy;
-    return log2_tab_rare(d2) ? log2(d2) : log2_tab(d2, lt);
+  __device__ __forceinline__ double arg(double d2) const { return d2; }
+  __device__ __forceinline__ double at(double s) const { return log2_tab(s, lt); }
+  // a pair whose argument is outside the table path; 0 for a coincident pair
+  // when check is set (flexmm/flexmm2d/helpers.py:99-107)
+  __device__ __forceinline__ double raw_rare(double dx, double dy, int check) const {
+    return (check && dx == 0.0 && dy == 0.0) ? 0.0 : log2(dx * dx + dy * dy);
   }
-  // raw value of a P2P pair, 0 for a coincident pair when check is set
-  // (flexmm/flexmm2d/helpers.py:99-107): a coincident pair has d2 = 0, so
-  // the test only runs on the rare path
-  __device__ __forceinline__ double raw_checked(double sx, double sy, double tx, double ty,
-                                                int check) const {
-    const double dx = tx - sx, dy = ty - sy, d2 = dx * dx + dy * dy;
-    if (!log2_tab_rare(d2)) return log2_tab(d2, lt);
-    return (check && dx == 0.0 && dy == 0.0) ? 0.0 : log2(d2);
+  __device__ __forceinline__ double raw_checked(double dx, double dy, int check) const {
+    const double s = arg(fma(dy, dy, dx * dx));
+    return log2_tab_rare(s) ? raw_rare(dx, dy, check) : at(s);
   }
+  __device__ __forceinline__ double raw(double dx, double dy) const { return raw_checked(dx, dy, 0); }
   __device__ __forceinline__ double operator()(double sx, double sy, double tx, double ty) const {
     return kFold * raw(tx - sx, ty - sy);
   }
-  __device__ __forceinline__ void grad(double sx, double sy, double tx, double ty, double q,
-                                       double &u, double &ux, double &uy) const {
-    const double dx = tx - sx, dy = ty - sy, d2 = dx * dx + dy * dy;
-    const double s = -(1.0 / (2.0 * M_PI)) / d2 * q;
-    u += kFold * raw(dx, dy) * q;
-    ux += s * dx;
-    uy += s * dy;
+  // raw value and raw gradient factor of a pair inside the table path: the
+  // potential is kFold * v, its gradient in the target position
+  // kGradFold * w * (dx, dy) (Gradient_Eval, examples/pure_kifmm_laplace_gradient.py:32-55)
+  static constexpr double kGradFold = -1.0 / (2.0 * M_PI);
+  __device__ __forceinline__ void at_grad(double s, double &v, double &w) const {
+    v = at(s);
+    w = rcp_newton(s);
+  }
+  __device__ __forceinline__ void grad_rare(double dx, double dy, int check, double &v,
+                                            double &w) const {
+    v = w = 0.0;
+    if (check && dx == 0.0 && dy == 0.0) return;
+    const double d2 = dx * dx + dy * dy;
+    v = log2(d2);
+    w = 1.0 / d2;
   }
 };
 
