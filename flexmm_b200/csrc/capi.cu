@@ -78,37 +78,51 @@ void fmmb::smem_limit_impl(const void *kernel, size_t bytes) {
 
 namespace {
 
-// sqrt(x) e^x K_n(x), n = 0, 1, for x >= 1: trapezoidal rule on
+// h_0 = e^x K0(x), h_1 = e^x K1(x) / x for x >= 1: trapezoidal rule on
 // int_0^inf exp(-2x sinh^2(t/2)) cosh^n(t) dt (exponent without cancellation;
 // step below the integrand's width 1/sqrt(x); summed from the small terms up)
-double bessel_g_host(int n, double x) {
-  const double h = std::min(1.0 / 16.0, 0.2 / std::sqrt(x));
-  const int m = (int)std::ceil(std::acosh(1.0 + 60.0 / x) / h);
-  double s = 0.0;
+long double bessel_h_host(int n, long double x) {
+  const long double h = std::min(1.0L / 16.0L, 0.2L / std::sqrt(x));
+  const int m = (int)std::ceil(std::acosh(1.0L + 60.0L / x) / h);
+  long double s = 0.0L;
   for (int i = m; i >= 1; --i) {
-    const double t = i * h, sh = std::sinh(0.5 * t);
-    s += std::exp(-2.0 * x * sh * sh) * (n ? std::cosh(t) : 1.0);
+    const long double t = i * h, sh = std::sinh(0.5L * t);
+    s += std::exp(-2.0L * x * sh * sh) * (n ? std::cosh(t) : 1.0L);
   }
-  s += 0.5;  // t = 0
-  return std::sqrt(x) * h * s;
+  s += 0.5L;  // t = 0
+  return n ? h * s / x : h * s;
 }
 
-// Chebyshev coefficients of g_0, g_1 on the octaves [2^j, 2^(j+1)) (bessel.cuh)
+// the polynomials of h_0, h_1 on the eighths of the octaves (bessel.cuh):
+// interpolation at Chebyshev nodes, rewritten in powers of x - c
 const std::vector<double> &bessel_table_host() {
   static const std::vector<double> tab = [] {
-    std::vector<double> t(BESSEL_TABLE_DOUBLES);
-    const int N = BESSEL_NCHEB;
+    std::vector<double> t(BESSEL_TABLE_DOUBLES, 0.0);
+    constexpr int N = BESSEL_NCOEF;
+    const long double pi = std::acos(-1.0L);
     for (int n = 0; n < 2; ++n)
-      for (int j = 0; j < BESSEL_OCTAVES; ++j) {
-        const double a = std::ldexp(1.0, j);
-        double f[BESSEL_NCHEB];
-        for (int k = 0; k < N; ++k)
-          f[k] = bessel_g_host(n, 1.5 * a + 0.5 * a * std::cos(M_PI * (k + 0.5) / N));
+      for (int iv = 0; iv < BESSEL_INTERVALS; ++iv) {
+        const long double a = std::ldexp(1.0L, iv / BESSEL_PARTS), hw = a / (2 * BESSEL_PARTS);
+        const long double c = a + hw * (2 * (iv % BESSEL_PARTS) + 1);
+        long double f[N], cheb[N];
+        for (int k = 0; k < N; ++k) f[k] = bessel_h_host(n, c + hw * std::cos(pi * (k + 0.5L) / N));
         for (int i = 0; i < N; ++i) {
-          double c = 0.0;
-          for (int k = 0; k < N; ++k) c += f[k] * std::cos(M_PI * i * (k + 0.5) / N);
-          t[(n * BESSEL_OCTAVES + j) * N + i] = (i == 0 ? 1.0 : 2.0) * c / N;
+          long double v = 0.0L;
+          for (int k = 0; k < N; ++k) v += f[k] * std::cos(pi * i * (k + 0.5L) / N);
+          cheb[i] = (i == 0 ? 1.0L : 2.0L) * v / N;
         }
+        // sum_i cheb_i T_i(u), T_i in powers of u = (x - c) / hw
+        long double pow[N] = {}, t0[N] = {1.0L}, t1[N] = {0.0L, 1.0L};
+        for (int i = 0; i < N; ++i) {
+          for (int k = 0; k < N; ++k) pow[k] += cheb[i] * t0[k];
+          long double t2[N];
+          for (int k = 0; k < N; ++k) t2[k] = (k ? 2.0L * t1[k - 1] : 0.0L) - t0[k];
+          std::copy(t1, t1 + N, t0);
+          std::copy(t2, t2 + N, t1);
+        }
+        long double scale = 1.0L;
+        for (int k = 0; k < N; ++k, scale /= hw)
+          t[(n * BESSEL_INTERVALS + iv) * BESSEL_ROW + k] = double(pow[k] * scale);
       }
     return t;
   }();

@@ -971,7 +971,7 @@ void run_upward(const PassArgs &a, const double *tau_s, double *mult, cudaStream
   switch (a.kernel_id) {
     case KERNEL_LAPLACE: upward_impl<LaplaceF64T>(a, tau_s, mult, s, n_rhs, tstride, cstride); break;
     case KERNEL_MOD_HELMHOLTZ:
-      upward_impl<ModHelmholtzF64>(a, tau_s, mult, s, n_rhs, tstride, cstride);
+      upward_impl<ModHelmholtzF64T>(a, tau_s, mult, s, n_rhs, tstride, cstride);
       break;
     case KERNEL_RADIAL_TABLE:
       upward_impl<RadialTableF64>(a, tau_s, mult, s, n_rhs, tstride, cstride);
@@ -1034,7 +1034,7 @@ void run_evaluate(const PassArgs &a, const double *tau_s, const double *loc, con
                                  s, pre);
       break;
     case KERNEL_MOD_HELMHOLTZ:
-      evaluate_impl<ModHelmholtzF64>(a, tau_s, loc, txs, tys, tkeys, tperm, m, check, nout, out,
+      evaluate_impl<ModHelmholtzF64T>(a, tau_s, loc, txs, tys, tkeys, tperm, m, check, nout, out,
                                      ld_out, s, pre);
       break;
     case KERNEL_RADIAL_TABLE:
@@ -1127,7 +1127,7 @@ void run_evaluate_multi(const PassArgs &a, const double *tau_s, int64_t n_src, i
                                       tperm, m, check, out, ld_out, s);
       break;
     case KERNEL_MOD_HELMHOLTZ:
-      evaluate_multi_impl<ModHelmholtzF64>(a, tau_s, n_src, n_rhs, loc, col_stride, txs, tys, tkeys,
+      evaluate_multi_impl<ModHelmholtzF64T>(a, tau_s, n_src, n_rhs, loc, col_stride, txs, tys, tkeys,
                                            tperm, m, check, out, ld_out, s);
       break;
     case KERNEL_RADIAL_TABLE:
@@ -1150,7 +1150,7 @@ void run_evaluate_sources_split(const PassArgs &a, const double *tau_s, const do
       break;
     case KERNEL_MOD_HELMHOLTZ:
       FMMB_CHECK(!a.dvx, ERR_UNSUPPORTED, "dipole sources: Laplace kernel only");
-      evaluate_split_impl<ModHelmholtzF64, false>(a, tau_s, loc, check, out, s, se);
+      evaluate_split_impl<ModHelmholtzF64T, false>(a, tau_s, loc, check, out, s, se);
       break;
     case KERNEL_RADIAL_TABLE:
       FMMB_CHECK(!a.dvx, ERR_UNSUPPORTED, "dipole sources: Laplace kernel only");
@@ -1194,7 +1194,7 @@ void run_local_evaluate(const PassArgs &a, const double *tau_s, const double *tx
       local_impl<LaplaceF64T>(a, tau_s, txs, tys, tkeys, tperm, m, check, scat, tcat, out, s);
       break;
     case KERNEL_MOD_HELMHOLTZ:
-      local_impl<ModHelmholtzF64>(a, tau_s, txs, tys, tkeys, tperm, m, check, scat, tcat, out, s);
+      local_impl<ModHelmholtzF64T>(a, tau_s, txs, tys, tkeys, tperm, m, check, scat, tcat, out, s);
       break;
     case KERNEL_RADIAL_TABLE:
       local_impl<RadialTableF64>(a, tau_s, txs, tys, tkeys, tperm, m, check, scat, tcat, out, s);
@@ -1264,7 +1264,7 @@ void run_evaluate_scratch(const PassArgs &a, const double *tau_s, const double *
   };
   switch (a.kernel_id) {
     case KERNEL_LAPLACE: launch(TypeOf<LaplaceF64T>{}); break;
-    case KERNEL_MOD_HELMHOLTZ: launch(TypeOf<ModHelmholtzF64>{}); break;
+    case KERNEL_MOD_HELMHOLTZ: launch(TypeOf<ModHelmholtzF64T>{}); break;
     case KERNEL_RADIAL_TABLE: launch(TypeOf<RadialTableF64>{}); break;
     default: throw Error(ERR_UNSUPPORTED, "unknown kernel id");
   }

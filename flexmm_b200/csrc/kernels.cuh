@@ -133,6 +133,7 @@ struct LaplaceF64 {
 // at() of an argument inside the table path, and raw_rare() for the others.
 struct LaplaceF64T {
   static constexpr bool kLogTable = true;
+  static constexpr unsigned kRare = LOG2_RARE;  // arguments with this key or above: raw_rare
   static constexpr double kFold = -0.69314718055994530942 / (4.0 * M_PI);  // -ln2 / (4 pi)
   const double2 *lt = nullptr;  // the block's table (FunctorSmem::bind)
   __host__ __device__ explicit LaplaceF64T(const KernelParams &) {}
@@ -153,8 +154,8 @@ struct LaplaceF64T {
   }
   // raw value and raw gradient factor of a pair inside the table path: the
   // potential is kFold * v, its gradient in the target position
-  // kGradFold * w * (dx, dy) (Gradient_Eval, examples/pure_kifmm_laplace_gradient.py:32-55)
-  static constexpr double kGradFold = -1.0 / (2.0 * M_PI);
+  // grad_fold * w * (dx, dy) (Gradient_Eval, examples/pure_kifmm_laplace_gradient.py:32-55)
+  static __host__ __device__ double grad_fold(const KernelParams &) { return -1.0 / (2.0 * M_PI); }
   __device__ __forceinline__ void at_grad(double s, double &v, double &w) const {
     v = at(s);
     w = rcp_newton(s);
@@ -181,27 +182,75 @@ struct FunctorSmem<KF, true> {
 
 struct ModHelmholtzF64 {
   static constexpr bool kLogTable = false;
-  double k;
+  double k, k2;
   const double *tab;
-  __host__ __device__ explicit ModHelmholtzF64(const KernelParams &kp) : k(kp.p[0]), tab(kp.table) {}
+  __host__ __device__ explicit ModHelmholtzF64(const KernelParams &kp)
+      : k(kp.p[0]), k2(kp.p[0] * kp.p[0]), tab(kp.table) {}
   __device__ __forceinline__ double operator()(double sx, double sy, double tx, double ty) const {
-    const double dx = tx - sx, dy = ty - sy;
-    double k0, k1;
-    bessel_k01<false>(k * sqrt(dx * dx + dy * dy), tab, k0, k1);
-    return k0 * (1.0 / (2.0 * M_PI));
+    const double dx = tx - sx, dy = ty - sy, d2 = dx * dx + dy * dy;
+    return bessel_any<false>(k, d2, k2 * d2, tab).x * (1.0 / (2.0 * M_PI));
   }
   // potential and its gradient in the target position, times q:
   // d/dt K0(k r) = -k K1(k r) (t - s) / r
   // (examples/pure_kifmm_modified_helmholtz_gradient.py:45-70)
   __device__ __forceinline__ void grad(double sx, double sy, double tx, double ty, double q,
                                        double &u, double &ux, double &uy) const {
-    const double dx = tx - sx, dy = ty - sy, r = sqrt(dx * dx + dy * dy);
-    double k0, k1;
-    bessel_k01<true>(k * r, tab, k0, k1);
-    const double s = -k * k1 / r * (1.0 / (2.0 * M_PI)) * q;
-    u += k0 * (1.0 / (2.0 * M_PI)) * q;
+    const double dx = tx - sx, dy = ty - sy, d2 = dx * dx + dy * dy;
+    const double2 b = bessel_any<true>(k, d2, k2 * d2, tab);
+    const double s = -k2 * b.y * (1.0 / (2.0 * M_PI)) * q;
+    u += b.x * (1.0 / (2.0 * M_PI)) * q;
     ux += s * dx;
     uy += s * dy;
+  }
+};
+
+// The modified Helmholtz kernel of the FP64 passes: ModHelmholtzF64 in the
+// form of a table functor (see LaplaceF64T), its table path the small
+// arguments x < 1 with the table-driven log2.  The line lies at the series'
+// end: near-field distances are at most about 2.8 leaf widths, so a sweep is
+// on this path unless k is above 1/3 of a reciprocal leaf width.
+struct ModHelmholtzF64T {
+  static constexpr bool kLogTable = true;
+  static constexpr unsigned kRare = 0x3FE00000u;  // log2_rare_key(1.0)
+  static constexpr double kFold = 1.0 / (2.0 * M_PI);
+  double k, k2;
+  const double *tab;
+  const double2 *lt = nullptr;
+  __host__ __device__ explicit ModHelmholtzF64T(const KernelParams &kp)
+      : k(kp.p[0]), k2(kp.p[0] * kp.p[0]), tab(kp.table) {}
+  static __host__ __device__ double grad_fold(const KernelParams &kp) {
+    return -(1.0 / (2.0 * M_PI)) * (kp.p[0] * kp.p[0]);
+  }
+  __device__ __forceinline__ double arg(double d2) const { return k2 * d2; }
+  __device__ __forceinline__ double at(double s) const {
+    double k0, k1x;
+    bessel_small<false>(s, log2_tab(s, lt), k0, k1x);
+    return k0;
+  }
+  __device__ __forceinline__ double raw_rare(double dx, double dy, int check) const {
+    if (check && dx == 0.0 && dy == 0.0) return 0.0;
+    const double d2 = dx * dx + dy * dy;
+    return bessel_any<false>(k, d2, k2 * d2, tab).x;
+  }
+  __device__ __forceinline__ double raw_checked(double dx, double dy, int check) const {
+    const double s = arg(fma(dy, dy, dx * dx));
+    return log2_rare_key(s) >= kRare ? raw_rare(dx, dy, check) : at(s);
+  }
+  __device__ __forceinline__ double raw(double dx, double dy) const { return raw_checked(dx, dy, 0); }
+  __device__ __forceinline__ double operator()(double sx, double sy, double tx, double ty) const {
+    return kFold * raw(tx - sx, ty - sy);
+  }
+  __device__ __forceinline__ void at_grad(double s, double &v, double &w) const {
+    bessel_small<true>(s, log2_tab(s, lt), v, w);
+  }
+  __device__ __forceinline__ void grad_rare(double dx, double dy, int check, double &v,
+                                            double &w) const {
+    v = w = 0.0;
+    if (check && dx == 0.0 && dy == 0.0) return;
+    const double d2 = dx * dx + dy * dy;
+    const double2 b = bessel_any<true>(k, d2, k2 * d2, tab);
+    v = b.x;
+    w = b.y;
   }
 };
 

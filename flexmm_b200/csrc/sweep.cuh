@@ -48,7 +48,7 @@ __device__ __forceinline__ void pot_batch(const KF &K, const double2 *xy, const 
       }
     }
   }
-  if (key < (DIP ? RCP_RARE : LOG2_RARE)) {
+  if (key < (DIP ? min(RCP_RARE, KF::kRare) : KF::kRare)) {
 #pragma unroll
     for (int i = 0; i < U; ++i) {
       const double c = q[j + i * G];
@@ -133,7 +133,7 @@ __device__ __forceinline__ void pot_sweep(const KF &K, const double2 *xy, const 
 }
 
 // v[r] = (u, gx, gy) sums of potential and target gradient; table functors
-// sum raw values (factors kFold, kGradFold applied at the end)
+// sum raw values (factors kFold, grad_fold applied at the end)
 template <class KF, int R>
 __device__ __forceinline__ void grad_sweep(const KF &K, const double2 *xy, const double *q,
                                            const double (&x)[R], const double (&y)[R], int lo,
@@ -154,7 +154,7 @@ __device__ __forceinline__ void grad_sweep(const KF &K, const double2 *xy, const
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         double a, w;
-        if (key < RCP_RARE)
+        if (key < min(RCP_RARE, KF::kRare))
           K.at_grad(s[r], a, w);
         else
           K.grad_rare(dx[r], dy[r], check, a, w);
@@ -239,8 +239,8 @@ struct ChargePolicy {
       o[0] = v[0] + v[1];
     } else if constexpr (KF::kLogTable) {
       o[0] = KF::kFold * v[0];
-      o[1] = KF::kGradFold * v[1];
-      o[2] = KF::kGradFold * v[2];
+      o[1] = KF::grad_fold(kp) * v[1];
+      o[2] = KF::grad_fold(kp) * v[2];
     } else {
       o[0] = v[0];
       o[1] = v[1];
