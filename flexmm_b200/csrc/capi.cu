@@ -10,10 +10,12 @@
 
 #include <memory>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "../../include/flexmm_b200.h"
 #include "fmm.cuh"
+#include "gemm.cuh"
 #include "timing.cuh"
 
 using namespace fmmb;
@@ -74,6 +76,30 @@ void fmmb::smem_limit_impl(const void *kernel, size_t bytes) {
   if (have >= bytes) return;
   FMMB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
   have = bytes;
+}
+
+size_t fmmb::smem_optin() {
+  int dev = 0, v = 0;
+  FMMB_CUDA(cudaGetDevice(&dev));
+  FMMB_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  return size_t(v);
+}
+
+int fmmb::coop_blocks(const void *kernel, int threads, size_t smem, int per_sm) {
+  static std::mutex mu;
+  static std::map<std::tuple<const void *, int, size_t>, int> known;
+  int dev = 0;
+  FMMB_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> g(mu);
+  int &n = known[{kernel, dev, smem}];
+  if (n == 0) {
+    int fit = 0, sms = 0;
+    FMMB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, threads, smem));
+    FMMB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    FMMB_CHECK(fit >= 1, ERR_CUDA, "cooperative kernel does not fit on an SM");
+    n = sms * std::min(fit, per_sm);
+  }
+  return n;
 }
 
 namespace {
@@ -266,6 +292,7 @@ struct fmm_plan {
   DevBuf<float> mult_tc;        // ... multipoles split TF32 hi / lo ...
   DevBuf<double> msum, lsum;    // ... and their FP64 component sums
   DevBuf<double> tsum;          // per node: FP64 sum of its charges
+  DevBuf<RadixSync> sync;       // barriers of the level passes (upward, downward)
   DevBuf<int> err;              // set by kernels whose bounded waits ran out
   int precision = PREC_FP64;
   bool have_expansions = false;
@@ -279,6 +306,9 @@ struct fmm_plan {
   bool has_st_dipoles = false;
   cudaStream_t side = nullptr;  // from the device's pool, not owned
   cudaStream_t pass = nullptr;  // the pair's high-priority stream (PassStream)
+  // whether the expansions built last were evaluated split (assumed of a new
+  // plan): where they were not, the next build stays on the caller's stream
+  bool split_used = true;
   cudaEvent_t ev_ready = nullptr, ev_near = nullptr, ev_far = nullptr, ev_pass = nullptr;
   bool ready_recorded = false;
   // mixed form: the split near field pauses during the M2L (SplitEval::hold)
@@ -354,13 +384,18 @@ void split_prepare(fmm_plan *p) {
 // The stream of a plan's FP64 level passes: the high-priority one of its pair,
 // which waits for ev_ready and which the caller's stream waits for at join()
 // (at the latest when this object ends, so that buffers freed in the caller's
-// stream order are no longer read).  A stream that is being captured keeps
-// its passes: the pool's streams are shared with plans outside the capture.
+// stream order are no longer read).  The passes stay on the caller's stream
+// where no near field is expected beside them (a plan that evaluates gradients
+// or other points only: a batch of 12 on 8 streams of its own takes 7.9 ms that
+// way, 8.8 ms through the pairs), and where that stream is being captured (the
+// pool's streams are shared with plans outside the capture).
 class PassStream {
  public:
   PassStream(fmm_plan *p, cudaStream_t s) : p_(p), s_(s), ps_(s) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (!split_enabled(PREC_FP64) || cudaStreamIsCapturing(s, &st) != cudaSuccess ||
+    const bool near_beside = split_enabled(PREC_FP64) && p->split_used;
+    p->split_used = false;
+    if (!near_beside || cudaStreamIsCapturing(s, &st) != cudaSuccess ||
         st != cudaStreamCaptureStatusNone) {
       cudaGetLastError();
       return;
@@ -474,8 +509,9 @@ int fmm_ops_add(fmm_ops *ops, const fmm_level_ops *lv, int *level_id) {
       return at;
     };
     const size_t o_lx = take(np), o_ly = take(np), o_u = take(size_t(np) * np), o_s = take(np),
-                 o_vh = take(size_t(np) * np), o_m2mct = take(size_t(4) * np * np),
-                 o_m2mc = take(size_t(4) * np * np);
+                 o_vh = take(size_t(np) * np), o_uf = take(size_t(np) * np),
+                 o_vhf = take(size_t(np) * np), o_m2mf = take(size_t(4) * np * np),
+                 o_l2lf = take(size_t(4) * np * np);
     for (int k = 0; k < n; ++k) {
       h[o_lx + k] = lv->large_x[k];
       h[o_ly + k] = lv->large_y[k];
@@ -486,13 +522,17 @@ int fmm_ops_add(fmm_ops *ops, const fmm_level_ops *lv, int *level_id) {
         h[o_u + size_t(i) * np + k] = lv->c2e_u[size_t(i) * n + k];
         h[o_vh + size_t(i) * np + k] = lv->c2e_vh[size_t(i) * n + k];
       }
-    for (int i = 0; i < n; ++i)
-      for (int c = 0; c < 4; ++c)
-        for (int k = 0; k < n; ++k) {
-          const double v = lv->m2mc[size_t(i) * 4 * n + c * n + k];
-          h[o_m2mct + size_t(c * np + k) * np + i] = v;   // [4np x np]
-          h[o_m2mc + size_t(i) * 4 * np + c * np + k] = v;  // [np x 4np]
-        }
+    auto u_at = [&](int i, int k) { return h[o_u + size_t(i) * np + k]; };
+    auto vh_at = [&](int i, int k) { return h[o_vh + size_t(i) * np + k]; };
+    // M2MC[i][c Neq + k] at (row i, child c, k), 0 in the padding
+    auto m2mc_at = [&](int i, int ck) {
+      const int c = ck / np, k = ck % np;
+      return i < n && k < n ? lv->m2mc[size_t(i) * 4 * n + c * n + k] : 0.0;
+    };
+    pack_fragments(np, np, u_at, h.data() + o_uf);
+    pack_fragments(np, np, vh_at, h.data() + o_vhf);
+    pack_fragments(4 * np, np, [&](int ck, int i) { return m2mc_at(i, ck); }, h.data() + o_m2mf);
+    pack_fragments(np, 4 * np, m2mc_at, h.data() + o_l2lf);
     size_t o_m2l[FMM_N_OFFSETS];
     int kind[FMM_N_OFFSETS], rp[FMM_N_OFFSETS];
     for (int o = 0; o < FMM_N_OFFSETS; ++o) {
@@ -622,8 +662,10 @@ int fmm_ops_add(fmm_ops *ops, const fmm_level_ops *lv, int *level_id) {
     e->dev.u = b + o_u;
     e->dev.sinv = b + o_s;
     e->dev.vh = b + o_vh;
-    e->dev.m2mct = b + o_m2mct;
-    e->dev.m2mc = b + o_m2mc;
+    e->dev.u_f = reinterpret_cast<const double2 *>(b + o_uf);
+    e->dev.vh_f = reinterpret_cast<const double2 *>(b + o_vhf);
+    e->dev.m2m_f = reinterpret_cast<const double2 *>(b + o_m2mf);
+    e->dev.l2l_f = reinterpret_cast<const double2 *>(b + o_l2lf);
     for (int o = 0; o < FMM_N_OFFSETS; ++o) {
       e->dev.m2l[o] = kind[o] == M2L_NULL ? nullptr : b + o_m2l[o];
       e->dev.kind[o] = kind[o];
@@ -887,6 +929,7 @@ static PassArgs pass_args(fmm_plan *p) {
   a.td = &p->td;
   a.th = &p->th;
   a.ops_dev = p->ops_dev.get();
+  a.sync = p->sync.get();
   if (p->has_dipoles) {
     a.dvx = p->dvx.get();
     a.dvy = p->dvy.get();
@@ -1032,6 +1075,8 @@ int fmm_build_expansions_multi(fmm_plan *p, const double *tau, int n_rhs, int64_
     const int64_t total = th.n_total(), n = th.n_points, cs = total * np;
     upload_level_ops(p, s);
     p->has_dipoles = false;
+    p->sync.alloc(2, s);
+    p->sync.zero(s);
     PassArgs a = pass_args(p);
     p->tau_s.alloc((size_t)n_rhs * n, s);
     p->mult.alloc((size_t)n_rhs * cs, s);
@@ -1227,6 +1272,7 @@ static void build_expansions_impl(fmm_plan *p, const double *tau, void *stream) 
     upload_level_ops(p, s);
     split_prepare(p);
     p->ready_recorded = false;
+    p->sync.alloc(2, s);
     PassArgs a = pass_args(p);
     p->tau_s.alloc(th.n_points, s);
     if (tau)
@@ -1266,7 +1312,7 @@ static void build_expansions_impl(fmm_plan *p, const double *tau, void *stream) 
     } else {
       p->mult.alloc(total * np, s);
       p->loc.alloc(total * np, s);
-      ZeroBatch(s).add(p->ple).add(p->mult).add(p->loc).run();
+      ZeroBatch(s).add(p->ple).add(p->mult).add(p->loc).add(p->sync).run();
       FMMB_CUDA(cudaEventRecord(p->ev_ready, s));  // sorted charges: all the near field reads
       p->ready_recorded = true;
       t_prep.reset();
@@ -1372,6 +1418,7 @@ void evaluate_own_sources(fmm_plan *p, int nout, int check, double *out, int64_t
                     td.pkeys.get(), td.ordv.get(), m, check, nout, out, ld_out, s);
   else if (nout == 1 && p->ready_recorded && p->n_rhs == 1 && split_enabled(p->precision)) {
     // near field on the side stream, started when the charges were sorted
+    p->split_used = true;
     SplitEval se{p->side, p->ev_ready, p->ev_near, p->ev_far};
     if (p->precision == PREC_MIXED && p->hold_armed) {
       se.hold = p->near_hold.get();

@@ -136,6 +136,30 @@ inline void smem_limit(F *kernel, size_t bytes) {
   smem_limit_impl(reinterpret_cast<const void *>(kernel), bytes);
 }
 
+// State of a cooperative launch's grid barriers (grid_barrier, radix.cuh); zero
+// before the launch
+struct RadixSync {
+  unsigned int count;  // barrier arrivals so far
+  int timeout, pad0, pad1;
+};
+
+// largest dynamic shared memory a block may request on the current device
+size_t smem_optin();
+
+// Blocks of a cooperative launch that are resident at once on the current
+// device, at most per_sm on each SM (looked up once per kernel, device and size)
+int coop_blocks(const void *kernel, int threads, size_t smem, int per_sm);
+
+// cooperative launch; a single block has no barrier to wait at and is launched
+// as any other kernel
+inline void launch_coop(const void *kernel, int grid, int threads, void **args, size_t smem,
+                        cudaStream_t s) {
+  if (grid > 1)
+    FMMB_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, smem, s));
+  else
+    FMMB_CUDA(cudaLaunchKernel(kernel, dim3(1), dim3(threads), args, smem, s));
+}
+
 // blocks for a persistent or grid-stride kernel over `units` work units (at
 // most one block per unit): per_sm blocks per SM on a large problem, fewer
 // on a small one (a batch of small problems then does not launch thousands

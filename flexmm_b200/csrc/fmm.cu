@@ -12,8 +12,8 @@
 //    source multipoles of one offset and multiplies them by that offset's
 //    dense or SVD-factored operator, accumulating all offsets in registers
 //    (the reference multiplies every multipole by every offset, then gathers);
-//  * L2L is parent-centric: one GEMM per tile of 8 parents produces the
-//    partial locals of their 32 children;
+//  * the level passes run as one cooperative launch each, tiles of 8 or 16
+//    rows of a level against operators held in shared memory;
 //  * fake leaves (source-only boxes) get no local expansions: they are never
 //    evaluated and never pass anything down;
 //  * the GEMMs run on the FP64 tensor cores (mma.sync m8n8k4 f64); the
@@ -26,8 +26,10 @@
 
 #include "fmm.cuh"
 #include "gemm.cuh"
+#include "radix.cuh"
 #include "scan.cuh"
 #include "sweep.cuh"
+#include "tcgen05.cuh"
 #include "timing.cuh"
 
 namespace fmmb {
@@ -85,7 +87,7 @@ __device__ __forceinline__ double kernel_at(const KF &K, double ax, double ay) {
 // points, the node's sources staged 32 at a time, four independent sums
 // per lane); C2E runs once for each level the tile holds.
 template <class KF, bool DIP = false>
-__global__ void __launch_bounds__(NT) k_s2m(KernelParams kp, int neq, int np, int L,
+__global__ void __launch_bounds__(NT, 3) k_s2m(KernelParams kp, int neq, int np, int L,
                                             const int *__restrict__ off,
                                             const int *__restrict__ uplist,
                                             const int *__restrict__ n_up_ptr,
@@ -104,11 +106,11 @@ __global__ void __launch_bounds__(NT) k_s2m(KernelParams kp, int neq, int np, in
   // charge column blockIdx.y (multi-RHS: column strides tstride / cstride)
   tau += blockIdx.y * tstride;
   mult += blockIdx.y * cstride;
-  extern __shared__ double smem[];
+  extern __shared__ __align__(16) double smem[];
   const int ldp = pad_ld(np);
   double *P = smem;          // [TN][ldp] check potentials
   double *T = P + TN * ldp;  // [TN][ldp] C2E scratch
-  double *Bs = T + TN * ldp;  // C2E operators streamed through (gemm_stage_doubles(np))
+  __shared__ __align__(16) double part[FG_PART];
   __shared__ double srcx[NT / 32][32], srcy[NT / 32][32], srct[NT / 32][32];
   __shared__ double srcdx[DIP ? NT / 32 : 1][32], srcdy[DIP ? NT / 32 : 1][32];
   __shared__ int node[TN], nlev[TN];
@@ -186,59 +188,196 @@ __global__ void __launch_bounds__(NT) k_s2m(KernelParams kp, int neq, int np, in
       if (threadIdx.x < TN)
         orow[threadIdx.x] = nlev[threadIdx.x] == m ? mult + (size_t)node[threadIdx.x] * np : nullptr;
       __syncthreads();
-      c2e_tile_staged(ops[m], np, P, T, orow, Bs);
+      c2e_rows<TN / 8>(ops[m], np, P, T, part, orow);
     }
     __syncthreads();
   }
 }
 
-// M2M + C2E of the parent boxes of level m (flexmm/flexmm2d/fmm.py:91-98):
-// TN parent groups per tile; their children are the contiguous node rows
-// c_first + 4e .. c_first + 4e + 3 of level m+1.  P[t] = M2MC . children.
-__global__ void __launch_bounds__(NT) k_m2m(int m, int np, int c_first, int n_groups,
-                                            const int *__restrict__ parent,
-                                            const LevelOpsDev *__restrict__ ops,
-                                            double *__restrict__ mult, int64_t cstride) {
-  mult += blockIdx.y * cstride;  // charge column blockIdx.y
-  extern __shared__ double smem[];
-  const int ldp = pad_ld(np), lda = pad_ld(4 * np);
-  double *P = smem;           // [TN][ldp] check potentials
-  double *T = P + TN * ldp;   // [TN][ldp] C2E scratch
-  double *A = T + TN * ldp;   // [TN][lda] children multipoles
-  double *Bs = A + TN * lda;  // operators streamed through (gemm_stage_doubles(np))
-  __shared__ double *orow[TN];
-  const LevelOpsDev &op = ops[m];
-  const int e0 = blockIdx.x * TN, nloc = min(TN, n_groups - e0);
-  for (int i = threadIdx.x; i < TN * ldp; i += NT) P[i] = T[i] = 0.0;
-  for (int i = threadIdx.x + nloc * lda; i < TN * lda; i += NT) A[i] = 0.0;
-  pdl_wait();  // the children's multipoles come from the kernels before
-  pdl_trigger();
-  stage_rows(A, lda, mult + (size_t)(c_first + 4 * e0) * np, nloc, 4 * np);
-  if (threadIdx.x < TN) {
-    const int t = threadIdx.x;
-    orow[t] = t < nloc ? mult + (size_t)parent[c_first + 4 * (e0 + t)] * np : nullptr;
+// The level passes run as one cooperative launch each (upward, downward), one
+// block per SM, the levels in turn with a grid barrier between them.  A level
+// is a short chain (its inputs from L2, three GEMMs on the FP64 tensor cores,
+// its outputs), bound by latency: as a launch of its own it took 26 us at 250k
+// ring points, Nequiv 40 (operators copied through shared memory 16 rows at a
+// time), and with the operators read from L2 as fragments 11 us (one SM reads
+// 13 bytes a clock with four loads in flight per warp, and a new
+// launch fetches its instructions again).  So a block keeps a
+// level's operators in shared memory, copied while it is still busy with the
+// level before (the translation's as soon as its last tile is through it, U
+// and VH at the level's end); between levels it waits for the grid barrier
+// (2,500 clocks) and its first inputs only.  Both passes: 470 -> 195 us at 250k
+// ring points (19 levels), 838 -> 304 us at 1M clustered points, Nequiv 60.
+struct LevelSpan {
+  int first, count;  // first child node (upward) or real group (downward); groups
+  int rb, tiles;     // row blocks (of 8 groups) per tile; tiles per charge column
+};
+struct LevelSpans {
+  int m0, n;  // levels m0, m0 + step, ... (n of them)
+  LevelSpan lv[FMM_MAX_LEVELS_DEV];
+};
+
+// Row blocks per tile of a level of `units` 8-group row blocks on `grid`
+// blocks.  A tile takes about as long with two row blocks as with one (its
+// chain of DMMAs waits on itself): two where that saves a round.
+int level_rows(int64_t units, int64_t grid, int rb_max) {
+  const int64_t one = (units + grid - 1) / grid, two = (units + 2 * grid - 1) / (2 * grid);
+  return rb_max >= 2 && 1.15 * double(two) < double(one) ? 2 : 1;
+}
+
+// A level's operators in shared memory, filled by bulk copies (one thread
+// starts them: copied by all threads in 16-byte pieces they held the block up
+// for 3,400 clocks a level at Nequiv 40) that two mbarriers count: M by
+// bar[0], U, VH and 1/S by bar[1].
+struct LevelStage {
+  double2 *M, *U, *V;  // translation (M2M, or L2L of one class), U, VH fragments
+  double *sinv;        // [np] 1/S
+  int np;
+  uint64_t *bar;
+  // called by one thread, after a block barrier behind the last read
+  __device__ void load_uv(const LevelOpsDev &op) const {
+    const uint32_t sq = 8u * np * np;
+    bulk_expect(bar + 1, 2 * sq + 8u * np);
+    bulk_copy(U, op.u_f, sq, bar + 1);
+    bulk_copy(V, op.vh_f, sq, bar + 1);
+    bulk_copy(sinv, op.sinv, 8u * np, bar + 1);
   }
-  cp_async_wait_all();
+  // wait for the k-th filling of both; false when the wait ran out
+  __device__ bool wait(uint32_t k) const {
+    return tc::mbar_wait(tc::smem_u32(bar), k & 1u, LEVEL_WAIT_TRIES) &&
+           tc::mbar_wait(tc::smem_u32(bar + 1), k & 1u, LEVEL_WAIT_TRIES);
+  }
+  static constexpr uint32_t LEVEL_WAIT_TRIES = 1u << 20;
+};
+// doubles of a stage whose translation has m_blocks np x np blocks
+__host__ __device__ inline size_t level_ops_doubles(int np, int m_blocks) {
+  return (size_t)(2 + m_blocks) * np * np + 64;
+}
+__device__ inline LevelStage level_stage(double *smem, int np, int m_blocks, uint64_t *bar) {
+  double2 *p = reinterpret_cast<double2 *>(smem);
+  LevelStage st;
+  st.np = np;
+  st.M = p;
+  st.U = p + m_blocks * np * np / 2;
+  st.V = st.U + np * np / 2;
+  st.sinv = reinterpret_cast<double *>(st.V + np * np / 2);
+  st.bar = bar;
+  if (threadIdx.x == 0) {
+    tc::mbar_init(tc::smem_u32(bar), 1);
+    tc::mbar_init(tc::smem_u32(bar + 1), 1);
+    tc::fence_mbar_init();
+  }
   __syncthreads();
-  {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = lane >> 2, q = lane & 3;
-    const int r0 = 8 * (warp & 3), c0 = 8 * (warp >> 2);
-    double acc[1][4][2];
-    zero_acc(acc);
-    warp_gemm_staged<1, 4>(A, lda, op.m2mct, np, 4 * np, r0, c0, 2, np, acc, Bs);
-    const int t = r0 + g;
-#pragma unroll
-    for (int cb = 0; cb < 4; ++cb) {
-      const int col = c0 + 16 * cb + 2 * q;
-      if (col < np) {
-        P[t * ldp + col] = acc[0][cb][0];
-        P[t * ldp + col + 1] = acc[0][cb][1];
+  return st;
+}
+
+constexpr int LEVEL_RB = 2;  // most row blocks per tile (4: 649 us for 609 at 100k uniform points)
+struct LevelSmem {           // static shared memory of a level kernel
+  double part[FG_PART];
+  double *orow[2][8 * LEVEL_RB];
+  uint64_t bar[2];
+};
+
+size_t up_smem(int np, int rb) {
+  return sizeof(double) *
+         (level_ops_doubles(np, 4) + (size_t)8 * rb * (2 * (size_t)pad_ld(np) + pad_ld(4 * np)));
+}
+
+// M2M + C2E of one level (flexmm/flexmm2d/fmm.py:91-98): a tile is 8 RB parent
+// groups, whose children are the contiguous node rows first + 4e ..
+// first + 4e + 3 of the level below.  P[t] = M2MC . children.  The next tile's
+// children are copied while the tile is in its check-to-equivalent solve;
+// next_ops() starts the copies of the operators of the block's next level.
+template <int RB, class F>
+__device__ __forceinline__ void up_level(const LevelStage &st, const LevelSpan &lv, int n_rhs,
+                                         const int *__restrict__ parent, double *mult,
+                                         int64_t cstride, double *rows, LevelSmem &sm, F &&next_ops) {
+  constexpr int ROWS = 8 * RB;
+  const int np = st.np, ldp = pad_ld(np), lda = pad_ld(4 * np), ncb = np / 8;
+  double *P = rows;           // [ROWS][ldp] check potentials
+  double *T = P + ROWS * ldp;  // [ROWS][ldp] C2E scratch
+  double *A = T + ROWS * ldp;  // [ROWS][lda] children multipoles
+  const UnitSplit<RB> t(ncb);
+  const int64_t total = (int64_t)lv.tiles * n_rhs;
+  auto load_a = [&](int64_t u, int slot) {  // the tile's inputs (one copy group) and outputs
+    const int col = int(u / lv.tiles), e0 = ROWS * int(u - (int64_t)col * lv.tiles);
+    const int nloc = min(ROWS, lv.count - e0);
+    double *mu = mult + col * cstride;
+    if (threadIdx.x < ROWS)
+      sm.orow[slot][threadIdx.x] =
+          (int)threadIdx.x < nloc
+              ? mu + (size_t)parent[lv.first + 4 * (e0 + (int)threadIdx.x)] * np
+              : nullptr;
+    for (int j = threadIdx.x + nloc * lda; j < ROWS * lda; j += NT) A[j] = 0.0;
+    stage_rows(A, lda, mu + (size_t)(lv.first + 4 * e0) * np, nloc, 4 * np);
+    cp_async_commit_group();
+  };
+  int slot = 0;
+  load_a(blockIdx.x, 0);
+  for (int64_t u = blockIdx.x; u < total; u += gridDim.x, slot ^= 1) {
+    cp_async_wait_all();
+    __syncthreads();
+    double acc[RB][2];
+    unit_gemm(t, A, lda, st.M, ncb, 4 * ncb, acc);
+    unit_sum(t, acc, sm.part);
+    unit_each(t, acc, [&](int r, int c, double a, double b) {
+      *reinterpret_cast<double2 *>(P + r * ldp + c) = make_double2(a, b);
+    });
+    __syncthreads();
+    if (u + gridDim.x < total)
+      load_a(u + gridDim.x, slot ^ 1);
+    else if (threadIdx.x == 0)
+      next_ops();
+    c2e_rows_smem<RB>(st.U, st.V, st.sinv, np, P, T, sm.part, sm.orow[slot]);
+  }
+}
+
+// the first level from i on in which this block has a tile
+__device__ __forceinline__ int next_level(const LevelSpans &sp, int i, int n_rhs) {
+  while (i < sp.n && (int64_t)sp.lv[i].tiles * n_rhs <= blockIdx.x) ++i;
+  return i;
+}
+
+__global__ void __launch_bounds__(NT, 2) k_up_levels(LevelSpans sp, int np, int n_rhs,
+                                                  const int *__restrict__ parent,
+                                                  const LevelOpsDev *__restrict__ ops, double *mult,
+                                                  int64_t cstride, RadixSync *sync, int *fail) {
+  extern __shared__ __align__(16) double smem[];
+  __shared__ __align__(16) LevelSmem sm;
+  const LevelStage st = level_stage(smem, np, 4, sm.bar);
+  double *rows = smem + level_ops_doubles(np, 4);
+  int nxt = next_level(sp, 0, n_rhs);  // the level whose operators are (being) staged
+  uint32_t fills = 0;
+  auto load_m = [&] {
+    if (nxt >= sp.n) return;
+    bulk_expect(sm.bar, 32u * np * np);
+    bulk_copy(st.M, ops[sp.m0 - nxt].m2m_f, 32u * np * np, sm.bar);
+  };
+  if (threadIdx.x == 0 && nxt < sp.n) {
+    load_m();
+    st.load_uv(ops[sp.m0 - nxt]);
+  }
+  for (int i = 0; i < sp.n; ++i) {
+    const LevelSpan lv = sp.lv[i];
+    if (i == nxt) {
+      nxt = next_level(sp, i + 1, n_rhs);
+      if (!__syncthreads_and(st.wait(fills++))) {
+        if (threadIdx.x == 0) atomicExch(fail, 1);
+        return;
+      }
+      if (lv.rb == 1)
+        up_level<1>(st, lv, n_rhs, parent, mult, cstride, rows, sm, load_m);
+      else
+        up_level<2>(st, lv, n_rhs, parent, mult, cstride, rows, sm, load_m);
+      if (nxt < sp.n) {
+        __syncthreads();  // U and VH have been read
+        if (threadIdx.x == 0) st.load_uv(ops[sp.m0 - nxt]);
       }
     }
+    if (i + 1 < sp.n && !grid_barrier(sync, fail)) {
+      if (nxt < sp.n) st.wait(fills);  // the copies in flight
+      return;
+    }
   }
-  __syncthreads();
-  c2e_tile_staged(op, np, P, T, orow, Bs);
 }
 
 // ------------------------------------------------------------------- M2L ----
@@ -271,7 +410,7 @@ __global__ void __launch_bounds__(NT) k_m2l(M2LTiles tiles, int np, const int *_
                                             double *__restrict__ ple, int64_t cstride) {
   mult += blockIdx.y * cstride;  // charge column blockIdx.y
   ple += blockIdx.y * cstride;
-  extern __shared__ double smem[];
+  extern __shared__ __align__(16) double smem[];
   const int ldp = pad_ld(np), ldw = pad_ld(32), ldb = pad_ld(np);
   double *Gb[2] = {smem, smem + TM * ldp};   // [TM][ldp] gathered source multipoles
   double *W = smem + 2 * TM * ldp;           // [TM][ldw] SVD intermediate (rank <= 32)
@@ -407,67 +546,143 @@ __global__ void __launch_bounds__(NT) k_m2l(M2LTiles tiles, int np, const int *_
 }
 
 // -------------------------------------------------------------- downward ----
-// One tile = 8 real sibling groups of level m (32 nodes): L2L from their
-// parents (m >= 3), plus the M2L partial locals, then check-to-equivalent.
-__global__ void __launch_bounds__(NT) k_downward(int m, int np, int rg_lo, int rg_cnt,
-                                                 const int *__restrict__ rg,
-                                                 const int *__restrict__ parent,
-                                                 const LevelOpsDev *__restrict__ ops,
-                                                 const double *__restrict__ ple,
-                                                 double *__restrict__ loc, int64_t cstride) {
-  ple += blockIdx.y * cstride;  // charge column blockIdx.y
-  loc += blockIdx.y * cstride;
-  extern __shared__ double smem[];
-  const int ldp = pad_ld(np);
-  double *P = smem;           // [32][ldp] partial locals
-  double *T = P + TN * ldp;   // [32][ldp] parent locals, then C2E scratch
-  double *Bs = T + TN * ldp;  // operators streamed through (gemm_stage_doubles(4 np))
-  __shared__ int node[TN];
-  __shared__ double *orow[TN];
-  const LevelOpsDev &op = ops[m];
-  const int q0 = 8 * blockIdx.x;
-  const int ngrp = min(8, rg_cnt - q0);
-  if (threadIdx.x < TN) {
-    const int grp = threadIdx.x >> 2;
-    const int n = (grp < ngrp) ? rg[rg_lo + q0 + grp] + int(threadIdx.x & 3) : -1;
-    node[threadIdx.x] = n;
-    orow[threadIdx.x] = n >= 0 ? loc + (size_t)n * np : nullptr;
-  }
-  pdl_wait();  // partial locals (M2L) and the parents' locals come from the kernels before
-  pdl_trigger();
-  __syncthreads();
-  for (int i = threadIdx.x; i < TN * np; i += NT) {
-    const int t = i / np, k = i % np;
-    P[t * ldp + k] = (node[t] >= 0) ? ple[(size_t)node[t] * np + k] : 0.0;
-    T[t * ldp + k] = 0.0;
-  }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-  if (m >= 3) {
-    const LevelOpsDev &opp = ops[m - 1];
-    for (int i = threadIdx.x; i < 8 * np; i += NT) {
-      const int grp = i / np, k = i % np;
-      const int n0 = node[4 * grp];
-      T[grp * ldp + k] = (n0 >= 0) ? loc[(size_t)parent[n0] * np + k] : 0.0;
-    }
-    __syncthreads();
-    // L2L: [8 parents][4np] = Lp . M2MC (flexmm/flexmm2d/fmm.py:140-147);
-    // warp -> column blocks warp + 8*cb of the 4np columns
-    double acc[1][4][2];
-    zero_acc(acc);
-    warp_gemm_staged<1, 4>(T, ldp, opp.m2mc, 4 * np, np, 0, 8 * warp, 8, 4 * np, acc, Bs);
-#pragma unroll
-    for (int cb = 0; cb < 4; ++cb) {
-      const int col = 8 * warp + 64 * cb + 2 * q;  // column of the 4np-wide parent row
-      if (col < 4 * np) {
-        const int c = col / np, i = col % np;
-        P[(4 * g + c) * ldp + i] += acc[0][cb][0];
-        P[(4 * g + c) * ldp + i + 1] += acc[0][cb][1];
+size_t down_smem(int np, int rb) {
+  return sizeof(double) * (level_ops_doubles(np, 1) + (size_t)8 * rb * 5 * pad_ld(np));
+}
+
+// One level: a tile is class c (child c) of 8 RB real sibling groups: L2L from
+// their parents (has_l2l; flexmm/flexmm2d/fmm.py:140-147), plus the M2L partial
+// locals, then check-to-equivalent.  Block b takes class b mod 4 in every
+// level (the grid is a multiple of 4), so it stages a quarter of the L2L
+// operator only.
+template <int RB, class F>
+__device__ __forceinline__ void down_level(const LevelStage &st, const LevelSpan &lv, int n_rhs,
+                                           bool has_l2l, const int *__restrict__ rg,
+                                           const int *__restrict__ parent,
+                                           const double *__restrict__ ple, double *loc,
+                                           int64_t cstride, double *rows, LevelSmem &sm,
+                                           F &&next_ops) {
+  constexpr int ROWS = 8 * RB;
+  const int np = st.np, ldp = pad_ld(np), ncb = np / 8, c = blockIdx.x & 3;
+  double *T = rows;                                            // [ROWS][ldp] C2E scratch
+  double *PL[2] = {T + ROWS * ldp, T + 3 * ROWS * ldp};  // per slot: partial locals, parents' locals
+  const UnitSplit<RB> t(ncb);
+  const int64_t total = (int64_t)lv.tiles * n_rhs;  // tiles of this class
+  const int64_t step = gridDim.x / 4, u0 = blockIdx.x / 4;
+  auto load_rows = [&](int64_t u, int slot) {
+    const int col = int(u / lv.tiles), q0 = ROWS * int(u - (int64_t)col * lv.tiles);
+    const int ngrp = min(ROWS, lv.count - q0);
+    double *lo = loc + col * cstride, *P = PL[slot], *Lp = P + ROWS * ldp;
+    const double *pl = ple + col * cstride;
+    for (int j = threadIdx.x; j < ROWS * (np / 2); j += NT) {
+      const int r = j / (np / 2), k = 2 * (j - r * (np / 2));
+      if (r < ngrp) {
+        const int n = rg[lv.first + q0 + r] + c;
+        cp_async16(P + r * ldp + k, pl + (size_t)n * np + k);
+        if (has_l2l) cp_async16(Lp + r * ldp + k, lo + (size_t)parent[n] * np + k);
+        if (k == 0) sm.orow[slot][r] = lo + (size_t)n * np;
+      } else {
+        P[r * ldp + k] = P[r * ldp + k + 1] = 0.0;
+        Lp[r * ldp + k] = Lp[r * ldp + k + 1] = 0.0;
+        if (k == 0) sm.orow[slot][r] = nullptr;
       }
     }
+    cp_async_commit_group();
+  };
+  int slot = 0;
+  load_rows(u0, 0);
+  for (int64_t u = u0; u < total; u += step, slot ^= 1) {
+    const bool last = u + step >= total;
+    double *P = PL[slot], *Lp = P + ROWS * ldp;
+    cp_async_wait_all();
     __syncthreads();
+    if (!last) load_rows(u + step, slot ^ 1);
+    if (has_l2l) {
+      double acc[RB][2];
+      unit_gemm(t, Lp, ldp, st.M, ncb, ncb, acc);
+      unit_sum(t, acc, sm.part);
+      unit_each(t, acc, [&](int r, int c, double a, double b) {
+        double2 *o = reinterpret_cast<double2 *>(P + r * ldp + c);
+        const double2 w = *o;
+        *o = make_double2(w.x + a, w.y + b);
+      });
+      __syncthreads();
+    }
+    if (last && threadIdx.x == 0) next_ops();
+    c2e_rows_smem<RB>(st.U, st.V, st.sinv, np, P, T, sm.part, sm.orow[slot]);
   }
-  c2e_tile_staged(op, np, P, T, orow, Bs);
+}
+
+__global__ void __launch_bounds__(NT, 2) k_down_levels(LevelSpans sp, int np, int n_rhs,
+                                                    const int *__restrict__ rg,
+                                                    const int *__restrict__ parent,
+                                                    const LevelOpsDev *__restrict__ ops,
+                                                    const double *__restrict__ ple, double *loc,
+                                                    int64_t cstride, RadixSync *sync, int *fail) {
+  extern __shared__ __align__(16) double smem[];
+  __shared__ __align__(16) LevelSmem sm;
+  const LevelStage st = level_stage(smem, np, 1, sm.bar);
+  double *rows = smem + level_ops_doubles(np, 1);
+  auto next_of = [&](int i) {  // the first level from i on in which this block has a tile
+    while (i < sp.n && (int64_t)sp.lv[i].tiles * n_rhs <= blockIdx.x / 4) ++i;
+    return i;
+  };
+  int nxt = next_of(0);
+  uint32_t fills = 0;
+  auto load_m = [&] {  // class c of the parents' L2L operator: its column blocks of each k pair
+    if (nxt >= sp.n) return;
+    const bool has = sp.m0 + nxt >= 3;
+    const uint32_t seg = 64u * np;  // bytes of a k pair's class block
+    bulk_expect(sm.bar, has ? seg * (np / 8) : 0u);
+    if (!has) return;
+    const double2 *src = ops[sp.m0 + nxt - 1].l2l_f + (blockIdx.x & 3) * 4 * np;
+    for (int kp = 0; kp < np / 8; ++kp)
+      bulk_copy(st.M + kp * 4 * np, src + (size_t)kp * 16 * np, seg, sm.bar);
+  };
+  if (threadIdx.x == 0 && nxt < sp.n) {
+    load_m();
+    st.load_uv(ops[sp.m0 + nxt]);
+  }
+  for (int i = 0; i < sp.n; ++i) {
+    const LevelSpan lv = sp.lv[i];
+    if (i == nxt) {
+      const bool has_l2l = sp.m0 + i >= 3;
+      nxt = next_of(i + 1);
+      if (!__syncthreads_and(st.wait(fills++))) {
+        if (threadIdx.x == 0) atomicExch(fail, 1);
+        return;
+      }
+      if (lv.rb == 1)
+        down_level<1>(st, lv, n_rhs, has_l2l, rg, parent, ple, loc, cstride, rows, sm, load_m);
+      else
+        down_level<2>(st, lv, n_rhs, has_l2l, rg, parent, ple, loc, cstride, rows, sm, load_m);
+      if (nxt < sp.n) {
+        __syncthreads();  // U and VH have been read
+        if (threadIdx.x == 0) st.load_uv(ops[sp.m0 + nxt]);
+      }
+    }
+    if (i + 1 < sp.n && !grid_barrier(sync, fail)) {
+      if (nxt < sp.n) st.wait(fills);  // the copies in flight
+      return;
+    }
+  }
+}
+
+// Blocks per SM of a level kernel and its most row blocks per tile.  Several
+// charge columns fill the SMs by themselves: two blocks where their buffers
+// fit with two row blocks each (np <= 40; 16 columns on a ring of 100k: 5319 ->
+// 4883 us a step).  A single column's levels run beside the near field, which
+// wants the rest of the SM (two blocks there: 779 -> 819 us a product at 250k).
+struct LevelFit {
+  int per_sm, rb_max;
+};
+template <class F>
+LevelFit level_fit(F &&bytes, int n_rhs) {
+  const size_t extra = sizeof(LevelSmem) + 1024 + 64, all = smem_optin() + 1024;
+  if (n_rhs > 1 && 2 * (bytes(2) + extra) <= all) return {2, 2};
+  int rb = LEVEL_RB;
+  while (rb > 1 && bytes(rb) + extra > all) rb /= 2;
+  return {1, rb};
 }
 
 // ------------------------------------------------------------ evaluation ----
@@ -818,7 +1033,7 @@ void upward_impl(const PassArgs &a, const double *tau_s, double *mult, cudaStrea
   const TreeDev &td = *a.td;
   const int np = a.np;
   if (th.L < 3) return;
-  const size_t s2m_bytes = sizeof(double) * ((size_t)TN * pad_ld(np) * 2 + gemm_stage_doubles(np));
+  const size_t s2m_bytes = sizeof(double) * ((size_t)TN * pad_ld(np) * 2);
   smem_limit(k_s2m<KF>, s2m_bytes);
   // persistent over the S2M nodes; at most one block per TN nodes of the tree
   // (small trees launch small grids)
@@ -841,16 +1056,31 @@ void upward_impl(const PassArgs &a, const double *tau_s, double *mult, cudaStrea
         mult, nullptr, nullptr, tstride, cstride);
   }
   FMMB_CUDA(cudaGetLastError());
-  const size_t m2m_bytes =
-      sizeof(double) * ((size_t)TN * (2 * pad_ld(np) + pad_ld(4 * np)) + gemm_stage_doubles(np));
-  smem_limit(k_m2m, m2m_bytes);
+  LevelSpans sp{};
+  sp.m0 = th.L - 2;
+  const LevelFit fit = level_fit([&](int rb) { return up_smem(np, rb); }, n_rhs);
+  const int rb_max = fit.rb_max;
+  const size_t up_bytes = up_smem(np, rb_max);
+  smem_limit(k_up_levels, up_bytes);
+  const int64_t cap = coop_blocks((const void *)k_up_levels, NT, up_bytes, fit.per_sm);
+  int64_t widest = 0;
   for (int m = th.L - 2; m >= 2; --m) {
-    const int c_first = th.off[m + 1];
     const int n_groups = (th.off[m + 2] - th.off[m + 1]) / 4;
-    if (n_groups == 0) continue;
-    launch_pdl(k_m2m, dim3((n_groups + TN - 1) / TN, n_rhs), dim3(NT), m2m_bytes, s, m, np,
-               c_first, n_groups, td.parent.get(), a.ops_dev, mult, cstride);
+    const int64_t units = (int64_t)((n_groups + 7) / 8) * n_rhs;
+    const int rb = level_rows(units, cap, rb_max);
+    LevelSpan &lv = sp.lv[sp.n++];
+    lv = LevelSpan{th.off[m + 1], n_groups, rb, (n_groups + 8 * rb - 1) / (8 * rb)};
+    widest = std::max<int64_t>(widest, (int64_t)lv.tiles * n_rhs);
   }
+  if (widest == 0) return;
+  const int grid = int(std::min(widest, cap));
+  int n_rhs_ = n_rhs, np_ = np;
+  const int *parent = td.parent.get();
+  const LevelOpsDev *ops = a.ops_dev;
+  RadixSync *sync = a.sync;
+  int *fail = td.sort_fail.get();
+  void *args[] = {&sp, &np_, &n_rhs_, &parent, &ops, &mult, &cstride, &sync, &fail};
+  launch_coop(reinterpret_cast<const void *>(k_up_levels), grid, NT, args, up_bytes, s);
 }
 
 }  // namespace
@@ -1010,18 +1240,33 @@ void run_downward(const PassArgs &a, const double *ple, double *loc, cudaStream_
                   int64_t cstride) {
   const TreeHost &th = *a.th;
   const TreeDev &td = *a.td;
-  const size_t sm =
-      sizeof(double) * ((size_t)TN * pad_ld(a.np) * 2 + gemm_stage_doubles(4 * a.np));
-  smem_limit(k_downward, sm);
+  LevelSpans sp{};
+  sp.m0 = 2;
+  const LevelFit fit = level_fit([&](int rb) { return down_smem(a.np, rb); }, n_rhs);
+  const int rb_max = fit.rb_max;
+  const size_t bytes = down_smem(a.np, rb_max);
+  smem_limit(k_down_levels, bytes);
+  const int64_t cap = coop_blocks((const void *)k_down_levels, NT, bytes, fit.per_sm) / 4 * 4;
+  FMMB_CHECK(cap >= 4, ERR_UNSUPPORTED, "the downward pass needs four SMs");
+  int64_t widest = 0;
   for (int m = 2; m < th.L; ++m) {
-    const int lo = th.rg_lo[m], cnt = th.rg_hi[m] - th.rg_lo[m];
-    if (cnt <= 0) continue;
-    const int tiles = (cnt + 7) / 8;
-    PhaseTimer timer(PH_DOWNWARD, s);
-    launch_pdl(k_downward, dim3(tiles, n_rhs), dim3(NT), sm, s, m, a.np, lo, cnt, td.rg.get(),
-               td.parent.get(), a.ops_dev, ple, loc, cstride);
-    FMMB_CUDA(cudaGetLastError());
+    const int lo = th.rg_lo[m], cnt = std::max(0, th.rg_hi[m] - th.rg_lo[m]);
+    const int64_t units = (int64_t)((cnt + 7) / 8) * n_rhs;
+    const int rb = level_rows(units, cap / 4, rb_max);
+    LevelSpan &lv = sp.lv[sp.n++];
+    lv = LevelSpan{lo, cnt, rb, (cnt + 8 * rb - 1) / (8 * rb)};
+    widest = std::max<int64_t>(widest, 4 * (int64_t)lv.tiles * n_rhs);
   }
+  if (widest == 0) return;
+  const int grid = int(std::min(widest, cap));
+  PhaseTimer timer(PH_DOWNWARD, s);
+  int n_rhs_ = n_rhs, np_ = a.np;
+  const int *rg = td.rg.get(), *parent = td.parent.get();
+  const LevelOpsDev *ops = a.ops_dev;
+  RadixSync *sync = a.sync + 1;
+  int *fail = td.sort_fail.get();
+  void *args[] = {&sp, &np_, &n_rhs_, &rg, &parent, &ops, &ple, &loc, &cstride, &sync, &fail};
+  launch_coop(reinterpret_cast<const void *>(k_down_levels), grid, NT, args, bytes, s);
 }
 
 void run_evaluate(const PassArgs &a, const double *tau_s, const double *loc, const double *txs,

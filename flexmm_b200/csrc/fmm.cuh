@@ -18,8 +18,9 @@ struct LevelOpsDev {
   const double *u;        // [NP x NP]  S2L = U diag(S) VH
   const double *sinv;     // [NP]       1/S (0 where S <= tol, and in padding)
   const double *vh;       // [NP x NP]
-  const double *m2mct;    // [4NP x NP] m2mct[c*NP+k][i] = M2MC[i][c*Neq+k]
-  const double *m2mc;     // [NP x 4NP] m2mc[k][c*NP+i] = M2MC[k][c*Neq+i]
+  // operators in fragment order (gemm.cuh): U, VH; M2M [4NP x NP], row
+  // c NP + k, column i: M2MC[i][c Neq + k]; L2L [NP x 4NP], its transpose
+  const double2 *u_f, *vh_f, *m2m_f, *l2l_f;
   const double *m2l[N_OFFSETS];  // dense: D^T [NP x NP]; svd: M1^T [NP x RP] then M2^T [RP x NP]
   int kind[N_OFFSETS];
   int rp[N_OFFSETS];
@@ -48,6 +49,7 @@ struct PassArgs {
   const TreeDev *td;
   const TreeHost *th;
   const LevelOpsDev *ops_dev;   // device array indexed by level
+  RadixSync *sync = nullptr;  // two zeroed grid barriers (upward, downward passes)
   // dipole sources (Laplace double layer): per sorted source the dipole
   // vector strength * normal; null when the sources carry charges only
   const double *dvx = nullptr, *dvy = nullptr;

@@ -316,14 +316,6 @@ size_t m2m_mx_smem(int np, bool stage_b) {
          sizeof(float) * ((size_t)TN * pad_f(4 * np) + (stage_b ? (size_t)2 * 4 * np * ldb_f(np) : 0));
 }
 
-// largest dynamic shared memory a block may request on this device
-size_t smem_optin() {
-  int dev = 0, v = 0;
-  FMMB_CUDA(cudaGetDevice(&dev));
-  FMMB_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  return size_t(v);
-}
-
 // ------------------------------------------------------------------- M2L ----
 struct M2LTilesMx {
   int n_levels;

@@ -144,18 +144,6 @@ __device__ inline void c2e_tile(const LevelOpsDev &op, int np, const double *P, 
   c2e_tile<false>(c2e_global(op, np), np, P, T, out_row);
 }
 
-// ---- GEMMs with the B operand streamed through shared memory ----
-// B (row-major [K][ldb] in global memory, first ncols columns) is copied in
-// chunks of GS_KC rows into a double buffer Bs of gemm_stage_doubles(ncols)
-// doubles (row stride pad_ld(ncols)), the next chunk in flight while the
-// warps multiply the current one: the k-loop reads shared memory only,
-// where reading B from L2 inside it left each warp waiting on one L2 round
-// trip per few k-steps.  Called by every thread of the block (barriers
-// inside); ncols even, ldb and B 16-byte aligned, K a multiple of 4; no
-// copies of the caller may be in flight (they would join the first group).
-constexpr int GS_KC = 16;
-__host__ __device__ inline int gemm_stage_doubles(int ncols) { return 2 * GS_KC * pad_ld(ncols); }
-
 __device__ __forceinline__ void cp_async_commit_group() {
   asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
@@ -164,79 +152,299 @@ __device__ __forceinline__ void cp_async_wait_group() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-template <int RB, int CB>
-__device__ void warp_gemm_staged(const double *A, int lda, const double *__restrict__ B, int ldb,
-                                 int K, int r0, int c0, int cstride, int ncols,
-                                 double (&acc)[RB][CB][2], double *Bs) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-  const int ldbs = pad_ld(ncols), per_row = ncols / 2;
-  const int nch = (K + GS_KC - 1) / GS_KC;
-  auto stage = [&](int c) {
-    const int k0 = c * GS_KC, rows = min(GS_KC, K - k0);
-    double *dst = Bs + (c & 1) * GS_KC * ldbs;
-    for (int i = threadIdx.x; i < rows * per_row; i += blockDim.x) {
-      const int r = i / per_row, c2 = 2 * (i - r * per_row);
-      cp_async16(dst + r * ldbs + c2, B + (size_t)(k0 + r) * ldb + c2);
-    }
-    cp_async_commit_group();
-  };
-  stage(0);
-  const double *Ap = A + (r0 + g) * lda + q;
-  for (int c = 0; c < nch; ++c) {
-    if (c + 1 < nch) {
-      stage(c + 1);
-      cp_async_wait_group<1>();
+// ---- GEMMs with the operator in fragment order ----
+// An operator B [K][N] (K, N multiples of 8) is stored as the mma.m8n8k4
+// fragments its readers need: element (kp N/8 + cb) 32 + lane of an array of
+// pairs holds B[8 kp + q][8 cb + g] and B[8 kp + 4 + q][8 cb + g] (g = lane/4,
+// q = lane%4), so a warp reads two k-steps of a column block in one coalesced
+// 512-byte load.  A DMMA takes an SM sub-partition about 16 clocks: at these
+// sizes the loads (from L2, or L1 where several warps read the same column
+// block) keep up with a few in flight, and no shared memory, copies or
+// barriers are spent on operators.
+template <class F>
+inline void pack_fragments(int K, int N, F &&at, double *dst) {
+  for (int kp = 0; kp < K / 8; ++kp)
+    for (int cb = 0; cb < N / 8; ++cb)
+      for (int lane = 0; lane < 32; ++lane)
+        for (int h = 0; h < 2; ++h)
+          dst[((size_t(kp) * (N / 8) + cb) * 32 + lane) * 2 + h] =
+              at(8 * kp + 4 * h + (lane & 3), 8 * cb + (lane >> 2));
+}
+
+// (volatile: the load stays where it is written, ahead of the DMMAs of the
+// pairs before it; left to itself the compiler sinks it to its use)
+__device__ __forceinline__ double2 load_pair(const double2 *p) {
+  double2 v;
+  asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];\n" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
+
+constexpr int FG_WARPS = 8;  // warps of a block that runs these tiles
+constexpr int FG_AHEAD = 4;  // fragment pairs in flight per warp
+
+// How the 8 warps share an output tile of RB row blocks (of 8) x ncb column
+// blocks: a warp keeps to one column block (its fragments are read once); the
+// warps of a column block split its row blocks, and where they outnumber them
+// the k range (KS parts, summed through shared memory afterwards).
+template <int RB>
+struct TileSplit {
+  int cb, rb, rstep, kpart, ks;
+  bool active;
+  __device__ TileSplit(int ncb) {
+    const int warp = threadIdx.x >> 5, wpc = max(1, FG_WARPS / ncb), w = warp / ncb;
+    cb = warp % ncb;
+    if (wpc >= RB) {
+      ks = wpc / RB;
+      rb = w % RB;
+      kpart = w / RB;
+      rstep = RB;
+      active = kpart < ks;
     } else {
-      cp_async_wait_group<0>();
+      ks = 1;
+      rb = w;
+      kpart = 0;
+      rstep = wpc;
+      active = w < wpc;
     }
-    __syncthreads();
-    const double *Bp = Bs + (c & 1) * GS_KC * ldbs + q * ldbs + c0 + g;
-    const int k0 = c * GS_KC, kn = min(GS_KC, K - k0);
-#pragma unroll 4
-    for (int k = 0; k < kn; k += 4) {
-      double a[RB], b[CB];
+  }
+};
+
+// the first fragment pairs of a warp's share (issued before the block waits
+// for its inputs)
+struct FragAhead {
+  double2 b[FG_AHEAD];
+};
+template <int RB>
+__device__ __forceinline__ void frag_ahead(const TileSplit<RB> &t, const double2 *__restrict__ B,
+                                           int ncb, int npairs, FragAhead &f) {
+  const int lane = threadIdx.x & 31;
+  const int k0 = npairs * t.kpart / t.ks, k1 = npairs * (t.kpart + 1) / t.ks;
 #pragma unroll
-      for (int rb = 0; rb < RB; ++rb) a[rb] = Ap[8 * rb * lda + k0 + k];
+  for (int i = 0; i < FG_AHEAD; ++i)
+    if (k0 + i < k1) f.b[i] = load_pair(B + ((size_t)(k0 + i) * ncb + t.cb) * 32 + lane);
+}
+
+// acc[i] (row block t.rb + i t.rstep) += A[rows][8 k0 ..] . B over the warp's
+// k range; A in shared memory, row stride lda (4 mod 16: conflict-free)
+template <int RB>
+__device__ __forceinline__ void frag_gemm(const TileSplit<RB> &t, const double *A, int lda,
+                                          const double2 *__restrict__ B, int ncb, int npairs,
+                                          FragAhead &f, double (&acc)[RB][2]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const int k0 = npairs * t.kpart / t.ks, k1 = npairs * (t.kpart + 1) / t.ks;
+  const double *Ap = A + (8 * t.rb + g) * lda + q;
+  for (int kb = k0; kb < k1; kb += FG_AHEAD) {
 #pragma unroll
-      for (int cb = 0; cb < CB; ++cb)
-        b[cb] = (c0 + 8 * cb * cstride < ncols) ? Bp[k * ldbs + 8 * cb * cstride] : 0.0;
+    for (int i = 0; i < FG_AHEAD; ++i) {
+      const int kp = kb + i;
+      if (kp < k1) {
+        const double2 b = f.b[i];
+        if (kp + FG_AHEAD < k1)
+          f.b[i] = load_pair(B + ((size_t)(kp + FG_AHEAD) * ncb + t.cb) * 32 + lane);
 #pragma unroll
-      for (int rb = 0; rb < RB; ++rb)
-#pragma unroll
-        for (int cb = 0; cb < CB; ++cb)
-          if (c0 + 8 * cb * cstride < ncols) dmma(acc[rb][cb], a[rb], b[cb]);
+        for (int r = 0; r < RB; ++r)
+          if (t.rb + r * t.rstep < RB) {
+            const double *a = Ap + 8 * r * t.rstep * lda + 8 * kp;
+            dmma(acc[r], a[0], b.x);
+            dmma(acc[r], a[4], b.y);
+          }
+      }
     }
-    __syncthreads();  // buffer c & 1 is refilled by the next iteration's copies
   }
 }
 
-// c2e_tile with U and VH streamed through Bs (gemm_stage_doubles(np))
-__device__ inline void c2e_tile_staged(const LevelOpsDev &op, int np, const double *P, double *T,
-                                       double *const *out_row, double *Bs) {
-  const int ldp = pad_ld(np);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-  const int r0 = 8 * (warp & 3), c0 = 8 * (warp >> 2);
-  double acc[1][4][2];
-  zero_acc(acc);
-  warp_gemm_staged<1, 4>(P, ldp, op.u, np, np, r0, c0, 2, np, acc, Bs);
+template <int RB>
+__device__ __forceinline__ void zero_rows(double (&acc)[RB][2]) {
 #pragma unroll
-  for (int cb = 0; cb < 4; ++cb) {
-    const int col = c0 + 16 * cb + 2 * q;
-    if (col < np) {
-      T[(r0 + g) * ldp + col] = acc[0][cb][0] * __ldg(op.sinv + col);
-      T[(r0 + g) * ldp + col + 1] = acc[0][cb][1] * __ldg(op.sinv + col + 1);
+  for (int r = 0; r < RB; ++r) acc[r][0] = acc[r][1] = 0.0;
+}
+
+// doubles of the k-part exchange
+constexpr int FG_PART = FG_WARPS * 64;
+
+// sum the k parts (one row block per warp then) into the warps of part 0
+// through part (FG_PART doubles); a barrier inside when there are several
+template <int RB>
+__device__ __forceinline__ void sum_parts(const TileSplit<RB> &t, double (&acc)[RB][2], double *part) {
+  if (t.ks == 1) return;
+  const int lane = threadIdx.x & 31, slot = (t.cb * RB + t.rb) * (t.ks - 1);
+  if (t.active && t.kpart > 0)
+    *reinterpret_cast<double2 *>(part + (slot + t.kpart - 1) * 64 + 2 * lane) =
+        make_double2(acc[0][0], acc[0][1]);
+  __syncthreads();
+  if (t.active && t.kpart == 0)
+    for (int k = 0; k < t.ks - 1; ++k) {
+      const double2 v = *reinterpret_cast<const double2 *>(part + (slot + k) * 64 + 2 * lane);
+      acc[0][0] += v.x;
+      acc[0][1] += v.y;
     }
+}
+
+// ---- the same with the operator's fragments in shared memory ----
+// The tile's units (row block, column block) are dealt out to the 8 warps, at
+// most RB each; where there are no more than 4 of them the warps split the k
+// range too (KS parts, summed through shared memory).
+template <int RB>
+struct UnitSplit {
+  int ncb, n_units, u0, kpart, ks;
+  __device__ explicit UnitSplit(int ncb_) : ncb(ncb_), n_units(RB * ncb_) {
+    const int warp = threadIdx.x >> 5;
+    ks = n_units <= FG_WARPS / 2 ? FG_WARPS / n_units : 1;
+    u0 = ks > 1 ? warp % n_units : warp;
+    kpart = ks > 1 ? warp / n_units : 0;
+    if (kpart >= ks) u0 = n_units;  // no share
+  }
+  __device__ bool has(int i) const { return u0 + FG_WARPS * i < n_units && (i == 0 || ks == 1); }
+  __device__ int rb(int i) const { return (u0 + FG_WARPS * i) / ncb; }
+  __device__ int cb(int i) const { return (u0 + FG_WARPS * i) % ncb; }
+};
+
+// acc[i] += A[rows of unit i][8 k0 ..] . B; B's k pairs bstride column blocks
+// apart.  A single unit alternates between two accumulators: one chain of
+// dependent DMMAs (32 clocks each) would leave the pipe (18) half idle.
+template <int RB>
+__device__ __forceinline__ void unit_gemm(const UnitSplit<RB> &t, const double *A, int lda,
+                                          const double2 *B, int bstride, int npairs,
+                                          double (&acc)[RB][2]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const int k0 = npairs * t.kpart / t.ks, k1 = npairs * (t.kpart + 1) / t.ks;
+  const double *Ap[RB];
+  const double2 *Bp[RB];
+#pragma unroll
+  for (int i = 0; i < RB; ++i) {
+    acc[i][0] = acc[i][1] = 0.0;
+    const int j = t.has(i) ? i : 0;
+    Ap[i] = A + (8 * t.rb(j) + g) * lda + q;
+    Bp[i] = B + t.cb(j) * 32 + lane;
+  }
+  if (!t.has(0)) return;
+  double odd[2] = {0.0, 0.0};
+#pragma unroll 4
+  for (int kp = k0; kp < k1; ++kp) {
+#pragma unroll
+    for (int i = 0; i < RB; ++i)
+      if (i == 0 || t.has(i)) {
+        const double2 b = Bp[i][kp * bstride * 32];
+        const double a0 = Ap[i][8 * kp], a1 = Ap[i][8 * kp + 4];
+        dmma(acc[i], a0, b.x);
+        if (RB == 1)
+          dmma(odd, a1, b.y);
+        else
+          dmma(acc[i], a1, b.y);
+      }
+  }
+  if (RB == 1) {
+    acc[0][0] += odd[0];
+    acc[0][1] += odd[1];
+  }
+}
+
+// sum the k parts into the warps of part 0 through part (FG_PART doubles); a
+// barrier inside when there are several
+template <int RB>
+__device__ __forceinline__ void unit_sum(const UnitSplit<RB> &t, double (&acc)[RB][2], double *part) {
+  if (t.ks == 1) return;
+  const int lane = threadIdx.x & 31;
+  if (t.has(0) && t.kpart > 0)
+    *reinterpret_cast<double2 *>(part + (t.u0 * (t.ks - 1) + t.kpart - 1) * 64 + 2 * lane) =
+        make_double2(acc[0][0], acc[0][1]);
+  __syncthreads();
+  if (t.has(0) && t.kpart == 0)
+    for (int k = 0; k < t.ks - 1; ++k) {
+      const double2 v =
+          *reinterpret_cast<const double2 *>(part + (t.u0 * (t.ks - 1) + k) * 64 + 2 * lane);
+      acc[0][0] += v.x;
+      acc[0][1] += v.y;
+    }
+}
+
+// f(row, column, accumulator pair) for the tile's summed results
+template <int RB, class F>
+__device__ __forceinline__ void unit_each(const UnitSplit<RB> &t, const double (&acc)[RB][2], F &&f) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  if (t.kpart == 0) {
+#pragma unroll
+    for (int i = 0; i < RB; ++i)
+      if (t.has(i)) f(8 * t.rb(i) + g, 8 * t.cb(i) + 2 * q, acc[i][0], acc[i][1]);
+  }
+}
+
+// c2e_rows with U, VH and 1/S in shared memory
+template <int RB>
+__device__ __forceinline__ void c2e_rows_smem(const double2 *U, const double2 *VH, const double *sinv,
+                                              int np, const double *P, double *T, double *part,
+                                              double *const *out_row) {
+  const int ldp = pad_ld(np), ncb = np / 8;
+  const UnitSplit<RB> t(ncb);
+  double acc[RB][2];
+  unit_gemm(t, P, ldp, U, ncb, ncb, acc);
+  unit_sum(t, acc, part);
+  unit_each(t, acc, [&](int r, int c, double a, double b) {
+    *reinterpret_cast<double2 *>(T + r * ldp + c) = make_double2(a * sinv[c], b * sinv[c + 1]);
+  });
+  __syncthreads();
+  unit_gemm(t, T, ldp, VH, ncb, ncb, acc);
+  unit_sum(t, acc, part);
+  unit_each(t, acc, [&](int r, int c, double a, double b) {
+    double *o = out_row[r];
+    if (o) *reinterpret_cast<double2 *>(o + c) = make_double2(a, b);
+  });
+}
+
+// ---- bulk copies (one thread): global -> shared, counted by an mbarrier ----
+__device__ __forceinline__ void bulk_expect(uint64_t *bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                   static_cast<uint32_t>(__cvta_generic_to_shared(bar))),
+               "r"(bytes)
+               : "memory");
+}
+// dst, src 16-byte aligned, bytes a multiple of 16
+__device__ __forceinline__ void bulk_copy(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+          static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+      "l"(src), "r"(bytes), "r"(static_cast<uint32_t>(__cvta_generic_to_shared(bar)))
+      : "memory");
+}
+
+// Check-to-equivalent of a tile of 8 RB rows: ((P . U) diag(1/S)) . VH, P and T
+// [8 RB][pad_ld(np)] in shared memory; row t goes to out_row[t] (np doubles)
+// where that is not null.  The caller synchronises before.
+template <int RB>
+__device__ inline void c2e_rows(const LevelOpsDev &op, int np, const double *P, double *T,
+                                double *part, double *const *out_row) {
+  const int ldp = pad_ld(np), ncb = np / 8;
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const TileSplit<RB> t(ncb);
+  double acc[RB][2];
+  FragAhead f;
+  zero_rows(acc);
+  if (t.active) {
+    frag_ahead(t, op.u_f, ncb, ncb, f);
+    frag_gemm(t, P, ldp, op.u_f, ncb, ncb, f, acc);
+    frag_ahead(t, op.vh_f, ncb, ncb, f);
+  }
+  sum_parts(t, acc, part);
+  if (t.active && t.kpart == 0) {
+    const double s0 = __ldg(op.sinv + 8 * t.cb + 2 * q), s1 = __ldg(op.sinv + 8 * t.cb + 2 * q + 1);
+#pragma unroll
+    for (int r = 0; r < RB; ++r)
+      if (t.rb + r * t.rstep < RB)
+        *reinterpret_cast<double2 *>(T + (8 * (t.rb + r * t.rstep) + g) * ldp + 8 * t.cb + 2 * q) =
+            make_double2(acc[r][0] * s0, acc[r][1] * s1);
   }
   __syncthreads();
-  zero_acc(acc);
-  warp_gemm_staged<1, 4>(T, ldp, op.vh, np, np, r0, c0, 2, np, acc, Bs);
-  double *o = out_row[r0 + g];
-  if (o) {
+  zero_rows(acc);
+  if (t.active) frag_gemm(t, T, ldp, op.vh_f, ncb, ncb, f, acc);
+  sum_parts(t, acc, part);
+  if (t.active && t.kpart == 0) {
 #pragma unroll
-    for (int cb = 0; cb < 4; ++cb) {
-      const int col = c0 + 16 * cb + 2 * q;
-      if (col < np) *reinterpret_cast<double2 *>(o + col) = make_double2(acc[0][cb][0], acc[0][cb][1]);
-    }
+    for (int r = 0; r < RB; ++r)
+      if (t.rb + r * t.rstep < RB) {
+        double *o = out_row[8 * (t.rb + r * t.rstep) + g];
+        if (o)
+          *reinterpret_cast<double2 *>(o + 8 * t.cb + 2 * q) = make_double2(acc[r][0], acc[r][1]);
+      }
   }
 }
 

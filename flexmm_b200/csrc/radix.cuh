@@ -55,11 +55,6 @@ constexpr unsigned int RS_LOOKBACK_TRIES = 1u << 22;
 constexpr int RS_LB = 16;                          // look-back reads in flight
 constexpr unsigned int RS_AGG = 1u << 30, RS_INC = 2u << 30, RS_VAL = RS_AGG - 1;
 
-struct RadixSync {  // zero before the launch
-  unsigned int count;  // barrier arrivals so far
-  int timeout, pad0, pad1;
-};
-
 struct RadixWork {
   RadixSync *sync;   // zero before the launch
   int *ghist;        // [passes][256], zero before the launch (follows sync)
