@@ -534,34 +534,6 @@ int fmm_ops_add(fmm_ops *ops, const fmm_level_ops *lv, int *level_id) {
     pack_fragments(4 * np, np, [&](int ck, int i) { return m2mc_at(i, ck); }, h.data() + o_m2mf);
     pack_fragments(np, 4 * np, m2mc_at, h.data() + o_l2lf);
     size_t o_m2l[FMM_N_OFFSETS];
-    int kind[FMM_N_OFFSETS], rp[FMM_N_OFFSETS];
-    for (int o = 0; o < FMM_N_OFFSETS; ++o) {
-      const int r = lv->m2l_rank[o];
-      o_m2l[o] = 0;
-      rp[o] = 0;
-      if (r == 0) {
-        kind[o] = M2L_NULL;
-      } else if (r < 0) {
-        kind[o] = M2L_DENSE;
-        o_m2l[o] = take(size_t(np) * np);
-        const double *a = lv->m2l_a[o];  // [n x n] (out i, in k); store D^T [k][i]
-        for (int i = 0; i < n; ++i)
-          for (int k = 0; k < n; ++k) h[o_m2l[o] + size_t(k) * np + i] = a[size_t(i) * n + k];
-      } else {
-        FMMB_CHECK(r <= n, ERR_INVALID_ARGUMENT, "M2L rank exceeds nequiv");
-        kind[o] = M2L_SVD;
-        const int p = pad8(r);
-        rp[o] = p;
-        o_m2l[o] = take(size_t(np) * p + size_t(p) * np);
-        const double *m2 = lv->m2l_a[o];  // [n x r]
-        const double *m1 = lv->m2l_b[o];  // [r x n]
-        for (int q = 0; q < r; ++q)
-          for (int k = 0; k < n; ++k) h[o_m2l[o] + size_t(k) * p + q] = m1[size_t(q) * n + k];
-        const size_t base2 = o_m2l[o] + size_t(np) * p;
-        for (int i = 0; i < n; ++i)
-          for (int q = 0; q < r; ++q) h[base2 + size_t(q) * np + i] = m2[size_t(i) * r + q];
-      }
-    }
     // mixed precision: dense operators minus their mean, as TF32 hi + lo
     std::vector<float> f;
     auto takef = [&](size_t count) {
@@ -604,11 +576,13 @@ int fmm_ops_add(fmm_ops *ops, const fmm_level_ops *lv, int *level_id) {
     for (int o = 0; o < FMM_N_OFFSETS; ++o) {
       const int r = lv->m2l_rank[o];
       c_m2l[o] = 0.0;
+      o_m2l[o] = 0;
       f_m2l_h[o] = f_m2l_l[o] = f_tc_h[o] = f_tc_l[o] = 0;
       if (r == 0) continue;
       if (r < 0) {
         for (size_t i = 0; i < size_t(n) * n; ++i) dense[i] = lv->m2l_a[o][i];
       } else {  // the truncated operator M2 . M1, as the reference applies it
+        FMMB_CHECK(r <= n, ERR_INVALID_ARGUMENT, "M2L rank exceeds nequiv");
         for (int i = 0; i < n; ++i)
           for (int k = 0; k < n; ++k) {
             double acc = 0.0;
@@ -616,6 +590,10 @@ int fmm_ops_add(fmm_ops *ops, const fmm_level_ops *lv, int *level_id) {
             dense[size_t(i) * n + k] = acc;
           }
       }
+      o_m2l[o] = take(size_t(np) * np);  // D^T: row k (source), column i (target)
+      pack_fragments(np, np, [&](int k, int i) {
+        return i < n && k < n ? dense[size_t(i) * n + k] : 0.0;
+      }, h.data() + o_m2l[o]);
       double c = 0.0;
       for (size_t i = 0; i < size_t(n) * n; ++i) c += dense[i];
       c /= double(n) * n;
@@ -667,9 +645,9 @@ int fmm_ops_add(fmm_ops *ops, const fmm_level_ops *lv, int *level_id) {
     e->dev.m2m_f = reinterpret_cast<const double2 *>(b + o_m2mf);
     e->dev.l2l_f = reinterpret_cast<const double2 *>(b + o_l2lf);
     for (int o = 0; o < FMM_N_OFFSETS; ++o) {
-      e->dev.m2l[o] = kind[o] == M2L_NULL ? nullptr : b + o_m2l[o];
-      e->dev.kind[o] = kind[o];
-      e->dev.rp[o] = rp[o];
+      const bool null = lv->m2l_rank[o] == 0;
+      e->dev.m2l_f[o] = null ? nullptr : reinterpret_cast<const double2 *>(b + o_m2l[o]);
+      e->dev.kind[o] = null ? M2L_NULL : M2L_DENSE;
     }
     e->dev_copy.alloc(1, 0);
     FMMB_CUDA(cudaMemcpy(e->dev_copy.get(), &e->dev, sizeof(LevelOpsDev), cudaMemcpyHostToDevice));

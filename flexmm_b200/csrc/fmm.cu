@@ -7,19 +7,19 @@
 //  * check-to-equivalent is applied as VH^T diag(1/S) U^T, the factored SVD
 //    solve (flexmm/kifmm2d/scalar/helpers.py:240-248), never an explicit
 //    inverse; it agrees with the reference's LU solve to ~1e-15;
-//  * M2L is target-centric: a tile of 64 target boxes of one parity class
+//  * M2L is target-centric: a tile of 16 to 64 target boxes of one parity class
 //    (position inside the parent: 27 of the 40 offsets can occur) gathers the
-//    source multipoles of one offset and multiplies them by that offset's
-//    dense or SVD-factored operator, accumulating all offsets in registers
-//    (the reference multiplies every multipole by every offset, then gathers);
+//    source multipoles that exist at one offset and multiplies them by that
+//    offset's operator, accumulating all offsets in shared memory (the
+//    reference multiplies every multipole by every offset, then gathers);
 //  * the level passes run as one cooperative launch each, tiles of 8 or 16
 //    rows of a level against operators held in shared memory;
 //  * fake leaves (source-only boxes) get no local expansions: they are never
 //    evaluated and never pass anything down;
 //  * the GEMMs run on the FP64 tensor cores (mma.sync m8n8k4 f64); the
 //    activations sit in shared memory with padded rows (stride 4 mod 16
-//    doubles: conflict-free fragment loads), the operators are read through
-//    the read-only cache.
+//    doubles: conflict-free fragment loads), the operators are stored in the
+//    order of the fragments their readers need.
 
 #include <algorithm>
 #include <type_traits>
@@ -36,7 +36,6 @@ namespace fmmb {
 namespace {
 
 constexpr int TN = 32;      // nodes per upward / downward tile
-constexpr int TM = 64;      // targets per M2L tile
 constexpr int NT = 256;     // threads per tile CTA
 constexpr int TCH = EVAL_CHUNK;  // targets per evaluation work item
 
@@ -47,6 +46,13 @@ __constant__ int8_t c_class_off[4][27] = {
     {7, 8, 9, 10, 11, 12, 14, 15, 16, 18, 19, 20, 22, 23, 24, 26, 27, 28, 29, 30, 31, 33, 34, 35, 36, 37, 38},
     {1, 2, 3, 4, 5, 6, 8, 9, 10, 11, 12, 13, 15, 16, 17, 19, 20, 21, 23, 24, 25, 27, 28, 29, 30, 31, 32},
     {0, 1, 2, 3, 4, 5, 7, 8, 9, 10, 11, 12, 14, 15, 16, 18, 19, 20, 22, 23, 24, 26, 27, 28, 29, 30, 31}};
+
+// the inverse: class position of offset o in class cls, or -1
+__constant__ int8_t c_oi_of[4][40] = {
+    {-1, -1, -1, -1, -1, -1, -1, -1, 0, 1, 2, 3, 4, 5, -1, 6, 7, 8, -1, 9, 10, 11, -1, 12, 13, 14, -1, 15, 16, 17, 18, 19, 20, -1, 21, 22, 23, 24, 25, 26},
+    {-1, -1, -1, -1, -1, -1, -1, 0, 1, 2, 3, 4, 5, -1, 6, 7, 8, -1, 9, 10, 11, -1, 12, 13, 14, -1, 15, 16, 17, 18, 19, 20, -1, 21, 22, 23, 24, 25, 26, -1},
+    {-1, 0, 1, 2, 3, 4, 5, -1, 6, 7, 8, 9, 10, 11, -1, 12, 13, 14, -1, 15, 16, 17, -1, 18, 19, 20, -1, 21, 22, 23, 24, 25, 26, -1, -1, -1, -1, -1, -1, -1},
+    {0, 1, 2, 3, 4, 5, -1, 6, 7, 8, 9, 10, 11, -1, 12, 13, 14, -1, 15, 16, 17, -1, 18, 19, 20, -1, 21, 22, 23, 24, 25, 26, -1, -1, -1, -1, -1, -1, -1, -1}};
 
 // the factor a kernel's loops fold into their staged charges and locals
 template <class KF, bool kFolded>
@@ -388,160 +394,179 @@ struct M2LTiles {
   int rg_cnt[FMM_MAX_LEVELS_DEV];
 };
 
-// One tile = 64 targets of one parity class of one level (the 27 offsets
-// that class can see).  The active offsets (an operator, and a source for
-// some target) are pipelined: the gathered source multipoles and the
-// offset's operators of offset a + 1 are copied into the second of two
-// shared buffers (cp.async) while the DMMA GEMMs of offset a run, so
-// neither the gather nor the operator reads wait on L2 inside the GEMM.
-// Dense offsets: acc += G . D^T; SVD offsets: W = G . M1^T, acc += W . M2^T.
-__host__ __device__ inline int m2l_op_doubles(int np) {
-  const int dense = np * pad_ld(np), svd = np * pad_ld(32) + 32 * pad_ld(np);
-  return dense > svd ? dense : svd;
-}
-__host__ __device__ inline size_t m2l_smem_doubles(int np) {
-  return (size_t)2 * TM * pad_ld(np) + (size_t)TM * pad_ld(32) + 2 * (size_t)m2l_op_doubles(np);
-}
+// One tile = up to tt targets of one parity class of one level (the 27 offsets
+// that class can see).  Per offset, the targets that have a source there are
+// listed; their source multipoles are gathered next to one another and
+// multiplied by the offset's operator 8 rows at a time, and each product row is
+// added to its target's row of partial locals in shared memory.  So the
+// tensor cores see the interactions that exist, rounded up to 8 per offset and
+// tile: on a ring of points a target has a fraction of its 27 sources, and a
+// tile that multiplies every target's row for every offset (as this kernel did)
+// works on zeros.  250k ring points, Nequiv 40: 370 -> 110 us; 16 columns there
+// 2,910 -> 500; 1M clustered, Nequiv 60: 735 -> 437; 100k uniform, Nequiv 32:
+// 70 -> 34; 3k, Nequiv 16: 45 -> 24.  The row order of a list does not matter: a row's sum runs over the
+// offsets in order.
+// Warp w owns column block w (8 columns) of every row, so rows are updated
+// without conflicts and one barrier per offset (its gather has arrived, the
+// buffer before is free) is all there is.  The operator is read as fragments:
+// into registers, one offset ahead; at np <= 16, where an offset is over before
+// an L2 read returns, through the gather's ring of buffers, three ahead.
+// Factored (SVD) operators are multiplied out on the host: at the ranks the
+// reference's rule factors (below Nequiv / 2, rounded up to 8) two thin products
+// cost as much as the full one.
+template <int NCB>
+struct M2LShape {
+  static constexpr int np = 8 * NCB, ldp = np + 4;
+  static constexpr bool kOpInRing = NCB <= 2;
+  static constexpr int kStages = NCB <= 2 ? 4 : NCB <= 4 ? 3 : 2;
+  static constexpr int kTargets = NCB <= 4 ? 32 : 64;  // targets per tile
+  static constexpr int kBlocks = NCB > 6 ? 2 : NCB > 4 ? 3 : NCB > 2 ? 6 : 8;  // resident per SM
+  static __host__ __device__ size_t stage_doubles(int tt) {
+    return (size_t)tt * ldp + (kOpInRing ? np * np : 0);
+  }
+  static __host__ __device__ size_t smem(int tt) {
+    return 8 * (tt * ldp + kStages * stage_doubles(tt)) + 27 * tt * (sizeof(int) + 1);
+  }
+};
 
-__global__ void __launch_bounds__(NT) k_m2l(M2LTiles tiles, int np, const int *__restrict__ rg,
-                                            const int *__restrict__ il,
-                                            const LevelOpsDev *__restrict__ ops,
-                                            const double *__restrict__ mult,
-                                            double *__restrict__ ple, int64_t cstride) {
+template <int NCB>
+__global__ void __launch_bounds__(32 * NCB, M2LShape<NCB>::kBlocks)
+    k_m2l(M2LTiles tiles, int tt, const int *__restrict__ rg, const int *__restrict__ il,
+          const LevelOpsDev *__restrict__ ops, const double *__restrict__ mult,
+          double *__restrict__ ple, int64_t cstride) {
+  using Sh = M2LShape<NCB>;
+  constexpr int np = Sh::np, ldp = Sh::ldp, S = Sh::kStages, nthr = 32 * NCB;
   mult += blockIdx.y * cstride;  // charge column blockIdx.y
   ple += blockIdx.y * cstride;
   extern __shared__ __align__(16) double smem[];
-  const int ldp = pad_ld(np), ldw = pad_ld(32), ldb = pad_ld(np);
-  double *Gb[2] = {smem, smem + TM * ldp};   // [TM][ldp] gathered source multipoles
-  double *W = smem + 2 * TM * ldp;           // [TM][ldw] SVD intermediate (rank <= 32)
-  double *Ob[2] = {W + TM * ldw, W + TM * ldw + m2l_op_doubles(np)};  // the offset's operators
-  __shared__ int tgt[TM];
-  __shared__ int s_src[27][TM];  // source node per class offset and target row
-  __shared__ int s_act[27];      // active class offsets, in order
-  __shared__ int s_nact;
-  __shared__ unsigned int s_mask;
+  double *acc = smem;                 // [tt][ldp] partial locals
+  double *ring = acc + tt * ldp;      // stages: [tt][ldp] gathered multipoles (, operator)
+  const size_t stage = Sh::stage_doubles(tt);
+  int *l_src = reinterpret_cast<int *>(ring + S * stage);      // [27][tt] source nodes
+  uint8_t *l_row = reinterpret_cast<uint8_t *>(l_src + 27 * tt);  // [27][tt] target rows
+  __shared__ int l_n[27], s_act[27], s_nact;
+  __shared__ const double2 *s_op[27];  // the active offsets' operators
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
   // this block's (level, parity class, range of real groups)
   int slot = 0;
   while (slot + 1 < 4 * tiles.n_levels && tiles.tile_start[slot + 1] <= (int)blockIdx.x) ++slot;
   const int m = slot >> 2, cls = slot & 3;
-  const int q0 = TM * (blockIdx.x - tiles.tile_start[slot]);
-  const int nloc = min(TM, tiles.rg_cnt[m] - q0);
+  const int q0 = tt * (blockIdx.x - tiles.tile_start[slot]);
+  const int nloc = min(tt, tiles.rg_cnt[m] - q0);
+  const int *tgt = rg + tiles.rg_lo[m] + q0;  // target t: node tgt[t] + cls
   const LevelOpsDev &op = ops[m];
-  if (threadIdx.x == 0) s_mask = 0u;
+  if (tid < 27) l_n[tid] = 0;
+  for (int i = tid; i < tt * ldp; i += nthr) acc[i] = 0.0;
   __syncthreads();
-  if (threadIdx.x < TM) {
-    const int tg = (threadIdx.x < nloc) ? rg[tiles.rg_lo[m] + q0 + threadIdx.x] + cls : -1;
-    tgt[threadIdx.x] = tg;
-    int sidx[27];  // all loads issued together
+  for (int t0 = 32 * warp; t0 < nloc; t0 += nthr) {  // lists: a warp lists 32 targets
+    const int t = t0 + lane;
+    int row[N_OFFSETS];
+    const int4 *ilr =
+        reinterpret_cast<const int4 *>(il + (size_t)(t < nloc ? tgt[t] + cls : 0) * N_OFFSETS);
 #pragma unroll
-    for (int oi = 0; oi < 27; ++oi) {
-      const int o = c_class_off[cls][oi];
-      sidx[oi] = (tg >= 0 && op.kind[o] != M2L_NULL) ? __ldg(il + (size_t)tg * N_OFFSETS + o) : -1;
+    for (int i = 0; i < N_OFFSETS / 4; ++i) {
+      const int4 v = t < nloc ? __ldg(ilr + i) : make_int4(-1, -1, -1, -1);
+      row[4 * i] = v.x;
+      row[4 * i + 1] = v.y;
+      row[4 * i + 2] = v.z;
+      row[4 * i + 3] = v.w;
     }
-    unsigned int mask = 0;
 #pragma unroll
-    for (int oi = 0; oi < 27; ++oi) {
-      s_src[oi][threadIdx.x] = sidx[oi];
-      if (sidx[oi] >= 0) mask |= 1u << oi;
+    for (int o = 0; o < N_OFFSETS; ++o) {
+      const int oi = c_oi_of[cls][o];
+      if (oi < 0 || op.kind[o] == M2L_NULL) continue;  // the same for all lanes
+      const unsigned has = __ballot_sync(0xffffffffu, row[o] >= 0);
+      if (!has) continue;
+      int at = 0;
+      if (lane == 0) at = atomicAdd(&l_n[oi], __popc(has));
+      at = __shfl_sync(0xffffffffu, at, 0) + __popc(has & ((1u << lane) - 1u));
+      if (row[o] >= 0) {
+        l_src[oi * tt + at] = row[o];
+        l_row[oi * tt + at] = (uint8_t)t;
+      }
     }
-    mask = __reduce_or_sync(0xffffffffu, mask);
-    if ((threadIdx.x & 31) == 0) atomicOr(&s_mask, mask);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int n = 0;
-    for (int oi = 0; oi < 27; ++oi)
-      if ((s_mask >> oi) & 1u) s_act[n++] = oi;
-    s_nact = n;
+  if (warp == 0) {
+    const unsigned act = __ballot_sync(0xffffffffu, lane < 27 && l_n[lane < 27 ? lane : 0] > 0);
+    if (lane < 27 && (act >> lane & 1u)) {
+      const int at = __popc(act & ((1u << lane) - 1u));
+      s_act[at] = lane;
+      s_op[at] = op.m2l_f[c_class_off[cls][lane]];
+    }
+    if (lane == 0) s_nact = __popc(act);
   }
   __syncthreads();
   const int nact = s_nact;
-  // copies of active offset a into buffer set b (one cp.async group)
-  auto prefetch = [&](int a, int b) {
-    const int oi = s_act[a], o = c_class_off[cls][oi];
-    double *G = Gb[b], *O = Ob[b];
-    const int h = np / 2;
-    for (int i = threadIdx.x; i < TM * h; i += NT) {
-      const int t = i / h, k2 = 2 * (i - t * h);
-      const int src = s_src[oi][t];
-      if (src >= 0) {
-        cp_async16(G + t * ldp + k2, mult + (size_t)src * np + k2);
-      } else {
-        G[t * ldp + k2] = 0.0;
-        G[t * ldp + k2 + 1] = 0.0;
+  auto gather = [&](int a) {  // active offset a into its ring stage (one copy group)
+    if (a < nact) {
+      const int oi = s_act[a], n = l_n[oi];
+      double *G = ring + (a % S) * stage;
+      for (int i = tid; i < n * (np / 2); i += nthr) {
+        const int r = i / (np / 2), k = 2 * (i - r * (np / 2));
+        cp_async16(G + r * ldp + k, mult + (size_t)l_src[oi * tt + r] * np + k);
       }
-    }
-    const double *B = op.m2l[o];
-    if (op.kind[o] == M2L_DENSE) {
-      for (int i = threadIdx.x; i < np * h; i += NT) {
-        const int r = i / h, c2 = 2 * (i - r * h);
-        cp_async16(O + r * ldb + c2, B + (size_t)r * np + c2);
-      }
-    } else {
-      const int rp = op.rp[o], hr = rp / 2, ld1 = pad_ld(rp);
-      for (int i = threadIdx.x; i < np * hr; i += NT) {  // M1^T [np][rp]
-        const int r = i / hr, c2 = 2 * (i - r * hr);
-        cp_async16(O + r * ld1 + c2, B + (size_t)r * rp + c2);
-      }
-      const double *B2 = B + (size_t)np * rp;
-      double *O2 = O + np * ld1;
-      for (int i = threadIdx.x; i < rp * h; i += NT) {  // M2^T [rp][np]
-        const int r = i / h, c2 = 2 * (i - r * h);
-        cp_async16(O2 + r * ldb + c2, B2 + (size_t)r * np + c2);
+      if (Sh::kOpInRing) {
+        const double2 *B = s_op[a];
+        double2 *D = reinterpret_cast<double2 *>(G + tt * ldp);
+        for (int i = tid; i < np * np / 2; i += nthr) cp_async16(D + i, B + i);
       }
     }
     cp_async_commit_group();
   };
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-  // dense / stage-2 mapping: rows 16*(warp&3) + [0,16), column blocks 8*(warp>>2) + 16*cb
-  const int r0 = 16 * (warp & 3), c0 = 8 * (warp >> 2);
-  double acc[2][4][2];
-  zero_acc(acc);
-  if (nact > 0) prefetch(0, 0);
+  double2 b[NCB], bn[Sh::kOpInRing ? 1 : NCB];  // this warp's operator fragments, and the next ones
+  auto load_op = [&](int a, double2 (&v)[Sh::kOpInRing ? 1 : NCB]) {
+    if constexpr (!Sh::kOpInRing) {
+      const double2 *B = s_op[a] + warp * 32 + lane;
+#pragma unroll
+      for (int kp = 0; kp < NCB; ++kp) v[kp] = load_pair(B + kp * NCB * 32);
+    }
+  };
+#pragma unroll
+  for (int a = 0; a < S - 1; ++a) gather(a);
+  if (nact > 0) load_op(0, bn);
   for (int a = 0; a < nact; ++a) {
-    const int b = a & 1;
-    if (a + 1 < nact) {
-      prefetch(a + 1, b ^ 1);
-      cp_async_wait_group<1>();
-    } else {
-      cp_async_wait_group<0>();
-    }
-    __syncthreads();
-    const int o = c_class_off[cls][s_act[a]];
-    if (op.kind[o] == M2L_DENSE) {
-      warp_gemm<2, 4, true>(Gb[b], ldp, Ob[b], ldb, np, r0, c0, 2, np, acc);
-    } else {
-      const int rp = op.rp[o], ld1 = pad_ld(rp);
-      // stage 1: W[64][rp] = G . M1^T ; warp -> rows 8*warp + [0,8), column blocks 0..3
-      double w[1][4][2];
-      zero_acc(w);
-      warp_gemm<1, 4, true>(Gb[b], ldp, Ob[b], ld1, np, 8 * warp, 0, 1, rp, w);
+    cp_async_wait_group<S - 2>();
+    __syncthreads();  // offset a is there, and the stage of offset a - 1 has been read
+    gather(a + S - 1);
+    const int oi = s_act[a], n = l_n[oi];
+    const double *G = ring + (a % S) * stage;
+    if constexpr (Sh::kOpInRing) {
+      const double2 *D = reinterpret_cast<const double2 *>(G + tt * ldp) + warp * 32 + lane;
 #pragma unroll
-      for (int cb = 0; cb < 4; ++cb) {
-        const int col = 8 * cb + 2 * q;
-        if (col < rp) {
-          W[(8 * warp + g) * ldw + col] = w[0][cb][0];
-          W[(8 * warp + g) * ldw + col + 1] = w[0][cb][1];
-        }
-      }
-      __syncthreads();
-      // stage 2: acc += W . M2^T
-      warp_gemm<2, 4, true>(W, ldw, Ob[b] + np * ld1, ldb, rp, r0, c0, 2, np, acc);
+      for (int kp = 0; kp < NCB; ++kp) b[kp] = D[kp * NCB * 32];
+    } else {
+#pragma unroll
+      for (int kp = 0; kp < NCB; ++kp) b[kp] = bn[kp];
+      if (a + 1 < nact) load_op(a + 1, bn);
     }
-    __syncthreads();  // buffer set b is refilled by the next iteration's copies
+    for (int r0 = 0; r0 < n; r0 += 16) {  // two row blocks: two chains of DMMAs
+      const bool two = r0 + 8 < n;
+      const int ra = r0 + g, rb = r0 + 8 + g;
+      double *oa = acc + l_row[oi * tt + min(ra, n - 1)] * ldp + 8 * warp + 2 * q;
+      double *ob = acc + l_row[oi * tt + min(rb, n - 1)] * ldp + 8 * warp + 2 * q;
+      const double *A0 = G + ra * ldp + q, *A1 = two ? A0 + 8 * ldp : A0;
+      double2 va = *reinterpret_cast<const double2 *>(oa);
+      double2 vb = *reinterpret_cast<const double2 *>(ob);
+      double c0[2] = {va.x, va.y}, c1[2] = {vb.x, vb.y};
+#pragma unroll
+      for (int kp = 0; kp < NCB; ++kp) {
+        dmma(c0, A0[8 * kp], b[kp].x);
+        if (two) dmma(c1, A1[8 * kp], b[kp].x);
+        dmma(c0, A0[8 * kp + 4], b[kp].y);
+        if (two) dmma(c1, A1[8 * kp + 4], b[kp].y);
+      }
+      // (rows past the list hold leftovers: a product row depends on its own
+      // row only, and these are not stored)
+      if (ra < n) *reinterpret_cast<double2 *>(oa) = make_double2(c0[0], c0[1]);
+      if (rb < n) *reinterpret_cast<double2 *>(ob) = make_double2(c1[0], c1[1]);
+    }
   }
-#pragma unroll
-  for (int rb = 0; rb < 2; ++rb) {
-    const int t = r0 + 8 * rb + g;
-    if (t < nloc) {
-#pragma unroll
-      for (int cb = 0; cb < 4; ++cb) {
-        const int col = c0 + 16 * cb + 2 * q;
-        if (col < np)
-          *reinterpret_cast<double2 *>(ple + (size_t)tgt[t] * np + col) =
-              make_double2(acc[rb][cb][0], acc[rb][cb][1]);
-      }
-    }
+  __syncthreads();
+  for (int i = tid; i < nloc * (np / 2); i += nthr) {
+    const int t = i / (np / 2), k = 2 * (i - t * (np / 2));
+    *reinterpret_cast<double2 *>(ple + (size_t)(tgt[t] + cls) * np + k) =
+        *reinterpret_cast<const double2 *>(acc + t * ldp + k);
   }
 }
 
@@ -1210,11 +1235,19 @@ void run_upward(const PassArgs &a, const double *tau_s, double *mult, cudaStream
   }
 }
 
+// targets (times charge columns) below which M2L tiles hold 16 targets: fewer
+// would leave SMs without one of 64 (3k points: 45 us with tiles of 64, 24 now)
+constexpr int64_t M2L_FEW_TARGETS = 148 * 64;
+
 void run_m2l(const PassArgs &a, const double *mult, double *ple, cudaStream_t s, int n_rhs,
              int64_t cstride) {
   const TreeHost &th = *a.th;
   if (th.L < 3) return;
   FMMB_CHECK(th.L <= FMM_MAX_LEVELS_DEV, ERR_INVALID_ARGUMENT, "too many levels");
+  int64_t targets = 0;
+  for (int m = 2; m < th.L; ++m) targets += 4 * (int64_t)(th.rg_hi[m] - th.rg_lo[m]);
+  // few targets: smaller tiles, for more blocks and a shorter chain in each
+  const int tt = targets * n_rhs < M2L_FEW_TARGETS ? 16 : a.np <= 32 ? 32 : 64;
   M2LTiles tl{};
   tl.n_levels = th.L;
   int tiles = 0;
@@ -1223,17 +1256,32 @@ void run_m2l(const PassArgs &a, const double *mult, double *ple, cudaStream_t s,
     tl.rg_cnt[m] = th.rg_hi[m] - th.rg_lo[m];
     for (int c = 0; c < 4; ++c) {
       tl.tile_start[4 * m + c] = tiles;
-      if (m >= 2) tiles += (tl.rg_cnt[m] + TM - 1) / TM;
+      if (m >= 2) tiles += (tl.rg_cnt[m] + tt - 1) / tt;
     }
   }
   tl.tile_start[4 * th.L] = tiles;
   if (tiles == 0) return;
-  const size_t sm = sizeof(double) * m2l_smem_doubles(a.np);
-  smem_limit(k_m2l, sizeof(double) * m2l_smem_doubles(64));
   PhaseTimer timer(PH_M2L, s);
-  k_m2l<<<dim3(tiles, n_rhs), NT, sm, s>>>(tl, a.np, a.td->rg.get(), a.td->il.get(), a.ops_dev,
-                                           mult, ple, cstride);
-  FMMB_CUDA(cudaGetLastError());
+  auto launch = [&](auto ncb) {
+    constexpr int NCB = decltype(ncb)::value;
+    const size_t sm = M2LShape<NCB>::smem(tt);
+    static_assert(M2LShape<NCB>::kTargets == (NCB <= 4 ? 32 : 64), "tiles are counted for this size");
+    smem_limit(k_m2l<NCB>, M2LShape<NCB>::smem(M2LShape<NCB>::kTargets));
+    k_m2l<NCB><<<dim3(tiles, n_rhs), 32 * NCB, sm, s>>>(tl, tt, a.td->rg.get(), a.td->il.get(),
+                                                        a.ops_dev, mult, ple, cstride);
+    FMMB_CUDA(cudaGetLastError());
+  };
+  switch (a.np / 8) {
+    case 1: launch(std::integral_constant<int, 1>{}); break;
+    case 2: launch(std::integral_constant<int, 2>{}); break;
+    case 3: launch(std::integral_constant<int, 3>{}); break;
+    case 4: launch(std::integral_constant<int, 4>{}); break;
+    case 5: launch(std::integral_constant<int, 5>{}); break;
+    case 6: launch(std::integral_constant<int, 6>{}); break;
+    case 7: launch(std::integral_constant<int, 7>{}); break;
+    case 8: launch(std::integral_constant<int, 8>{}); break;
+    default: throw Error(ERR_UNSUPPORTED, "unexpected operator size");
+  }
 }
 
 void run_downward(const PassArgs &a, const double *ple, double *loc, cudaStream_t s, int n_rhs,

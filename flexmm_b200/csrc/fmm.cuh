@@ -9,7 +9,7 @@
 
 namespace fmmb {
 
-constexpr int M2L_NULL = 0, M2L_DENSE = 1, M2L_SVD = 2;
+constexpr int M2L_NULL = 0, M2L_DENSE = 1;
 constexpr int FMM_MAX_LEVELS_DEV = 30;  // levels 0..29 (keys hold 29 digits)
 
 // Device view of one width's operators (all arrays zero padded to NP).
@@ -21,9 +21,8 @@ struct LevelOpsDev {
   // operators in fragment order (gemm.cuh): U, VH; M2M [4NP x NP], row
   // c NP + k, column i: M2MC[i][c Neq + k]; L2L [NP x 4NP], its transpose
   const double2 *u_f, *vh_f, *m2m_f, *l2l_f;
-  const double *m2l[N_OFFSETS];  // dense: D^T [NP x NP]; svd: M1^T [NP x RP] then M2^T [RP x NP]
-  int kind[N_OFFSETS];
-  int rp[N_OFFSETS];
+  const double2 *m2l_f[N_OFFSETS];  // D^T [NP x NP] in fragment order (factored ones multiplied out)
+  int kind[N_OFFSETS];              // M2L_NULL or M2L_DENSE
   // mixed precision: operators minus their mean c (the mean enters exactly as
   // c * sum(input), in FP64), rounded to TF32 as hi + lo pairs, B layout [K][N]
   const float *lx32, *ly32;             // [NP]

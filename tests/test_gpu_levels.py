@@ -19,7 +19,7 @@ def test_level_passes_match_oracle(built_lib, neq):
     n = 2300 + neq
     x = np.concatenate([rng.uniform(-1, 1, n - 600), 0.3 + 0.004 * rng.standard_normal(600)])
     y = np.concatenate([rng.uniform(-1, 1, n - 600), -0.2 + 0.004 * rng.standard_normal(600)])
-    tau = rng.standard_normal((3, n))
+    tau = rng.standard_normal((6, n))  # six columns: the larger M2L tiles
     bbox = [-1.0, 1.0, -1.0, 1.0]
     F = KI_FMM(x, y, "Laplace_Eval", 12, neq, bbox=bbox, helper=KI_Helper())
     O = KIFMM(x, y, laplace, 12, neq, bbox=bbox)
@@ -32,5 +32,5 @@ def test_level_passes_match_oracle(built_lib, neq):
     F.build_expansions(tau)
     got = F.source_evaluation(x, y)
     F.status()
-    for k in range(3):
+    for k in range(6):
         assert rel_l2(got[k], want[k]) < 1e-12
