@@ -51,6 +51,7 @@ class BBLevelOps(ctypes.Structure):
 
 
 BB_MAX_P = 16
+BB_MAX_RANK = 64   # columns of a common M2L basis (FMM_BB_MAX_RANK)
 
 
 class StokesLevelOps(ctypes.Structure):
@@ -80,6 +81,8 @@ SIGNATURES = [
     ("fmm_kernel_table_create", ctypes.c_int, [_dp, ctypes.c_int, ctypes.c_int, ctypes.c_int, _ip]),
     ("fmm_bb_ops_create", ctypes.c_int, [ctypes.c_int, _dp, ctypes.c_int, _dp, ctypes.POINTER(_vp)]),
     ("fmm_bb_ops_add", ctypes.c_int, [_vp, ctypes.POINTER(BBLevelOps), _ip]),
+    ("fmm_bb_ops_set_basis", ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, _dp,
+                                            ctypes.POINTER(_dp)]),
     ("fmm_plan_create", ctypes.c_int,
      [_vp, _vp, _vp, ctypes.c_int64, ctypes.c_int, _dp, _vp, ctypes.POINTER(_vp)]),
     ("fmm_plan_info", ctypes.c_int, [_vp, _ip, _dp, _ip]),

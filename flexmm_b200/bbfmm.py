@@ -12,7 +12,11 @@ the reference forms them, are:
   level independent;
 * per box width and offset, M2L = VI . K(nodes + offset w, nodes) . VI^T,
   compressed by the same SVD rule as the KIFMM operators (bbfmm.py:101-122,
-  flexmm/flexmm2d/helpers.py:5-33).
+  flexmm/flexmm2d/helpers.py:5-33);
+* a common orthonormal basis Q of a width's 40 M2L operators (the kernel is
+  radial, so their row and column spaces agree as a set): M2L_o = Q core_o Q^T
+  to the last bit of its largest singular value, in which the device
+  translates.
 
 The device runs S2M (Chebyshev moments), M2M, M2L, L2L (FP64 tensor-core
 row GEMMs with fused gathers, ``csrc/rowgemm.cuh``), L2T (2-D Chebyshev
@@ -63,6 +67,7 @@ class BBPrecomputation:
 
         self.m2l_rank = np.zeros(len(offsets()), dtype=np.int32)
         self.m2l_a, self.m2l_b = [], []
+        self.q, self.core = None, None
         for o, (ox, oy) in enumerate(offsets()):
             m = VI.dot(form(snx + ox * width, sny + oy * width, snx, sny)).dot(VI.T)
             Um, Sm, VHm = np.linalg.svd(m)
@@ -81,6 +86,27 @@ class BBPrecomputation:
                 self.m2l_a.append(np.ascontiguousarray(m))
                 self.m2l_b.append(None)
 
+        self._find_basis(n)
+
+    def _find_basis(self, n):
+        """Q and core_o, where the operators share a small enough space: the
+        right singular vectors of all row-space factors stacked, cut at 4e-16
+        of the largest singular value (the operators' own rounding)."""
+        if n <= _lib.BB_MAX_RANK or not np.all(self.m2l_rank >= 0):
+            return  # small enough as they are, or an operator without a low rank
+        rows = [b for b in self.m2l_b if b is not None]
+        rows += [(a * np.linalg.norm(b, axis=1)).T for a, b in zip(self.m2l_a, self.m2l_b)
+                 if a is not None]
+        if not rows:
+            return
+        _, S, VH = np.linalg.svd(np.linalg.qr(np.vstack(rows), mode="r"))
+        r = int(np.count_nonzero(S > 4e-16 * S[0]))
+        if r > _lib.BB_MAX_RANK:
+            return
+        self.q = np.ascontiguousarray(VH[:r].T)
+        self.core = [None if a is None else np.ascontiguousarray(self.q.T.dot(a).dot(b.dot(self.q)))
+                     for a, b in zip(self.m2l_a, self.m2l_b)]
+
     def upload(self, ops_handle):
         dp = ctypes.POINTER(ctypes.c_double)
 
@@ -94,6 +120,10 @@ class BBPrecomputation:
                              m2l_a=arr_a, m2l_b=arr_b)
         lid = ctypes.c_int(-1)
         _lib.call("fmm_bb_ops_add", ops_handle, ctypes.byref(lv), ctypes.byref(lid))
+        if self.q is not None:
+            arr_c = (dp * len(self.core))(*[ptr(c) for c in self.core])
+            _lib.call("fmm_bb_ops_set_basis", ops_handle, lid.value, self.q.shape[1], ptr(self.q),
+                      arr_c)
         return lid.value
 
 

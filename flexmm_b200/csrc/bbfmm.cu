@@ -7,11 +7,14 @@
 //    source2pMs, bbfmm.py:186-196); no check-to-equivalent step;
 //  * M2M / L2L: the level-independent M2MC [NQ x 4NQ] and its transpose
 //    (bbfmm.py:145-161) on the contiguous child rows of each parent group;
-//  * M2L: per level and offset VI K VI^T (bbfmm.py:101-122), the 40 offsets
-//    of a level applied in one row-GEMM launch (rowgemm.cuh) over the
-//    stacked operators: each tile of 64 target boxes of one parity class
-//    reads the source multipole of each offset it meets, and skips the
-//    offsets absent for the whole tile;
+//  * M2L: per level and offset VI K VI^T (bbfmm.py:101-122).  A width's 40
+//    operators share a space of at most 64 columns for the smooth kernels
+//    (fmm_bb_ops_set_basis): multipoles go into that basis, the KIFMM's M2L
+//    kernel translates rows of 64 there, all levels in one launch, and the
+//    results come back, a sixteenth of the work at p = 16.  Levels without
+//    such a basis apply their operators in a row-GEMM launch
+//    (rowgemm.cuh) over the stacked operators, each tile of 64 target boxes
+//    of one parity class skipping the offsets absent for the whole tile;
 //  * L2T: the local coefficients evaluated as a 2-D Chebyshev series
 //    (chebeval2d1, bbfmm.py:25-31, L2targets, bbfmm.py:198-210);
 //  * P2P: the same colleague sweep as the KIFMM evaluation.
@@ -287,11 +290,37 @@ void run_bb_upward(const BBArgs &b, const double *tau_s, double *mult, cudaStrea
   }
 }
 
-void run_bb_downward(const BBArgs &b, const double *mult, double *ple, cudaStream_t s) {
+void run_bb_downward(const BBArgs &b, const double *mult, double *ple, double *z, double *zl,
+                     cudaStream_t s) {
   const TreeHost &th = *b.th;
   const TreeDev &td = *b.td;
   if (th.L < 3) return;
   const int np = b.np;
+  static_assert(BB_RANK <= 64, "the KIFMM's M2L takes rows of at most 64");
+  if (b.any_fast) {
+    // M2L of these levels in one launch of the KIFMM's kernel, on rows of at most
+    // 64: the coefficients themselves (p <= 8), or those in the common basis
+    const bool basis = np > BB_RANK;
+    for (int m = 2; basis && m < th.L; ++m) {
+      const int r0 = th.off[m], n = th.off[m + 1] - th.off[m];
+      if (!b.fast[m]) continue;
+      rowgemm(RowsContig{mult + (size_t)r0 * np, np, n, np}, StoreRows{z + (size_t)r0 * BB_RANK, BB_RANK},
+              row_tiles(n), b.q[m], BB_RANK, BB_RANK, np, s);
+    }
+    PassArgs a{};
+    a.np = basis ? BB_RANK : np;
+    a.th = b.th;
+    a.td = b.td;
+    a.ops_dev = b.ops_dev;
+    run_m2l(a, basis ? z : mult, basis ? zl : ple, s);
+    for (int m = 2; basis && m < th.L; ++m) {
+      const int r0 = th.off[m], n = th.off[m + 1] - th.off[m];
+      if (!b.fast[m]) continue;
+      rowgemm(RowsContig{zl + (size_t)r0 * BB_RANK, BB_RANK, n, BB_RANK},
+              StoreRows{ple + (size_t)r0 * np, np}, row_tiles(n), b.q[m] + (size_t)np * BB_RANK, np,
+              np, BB_RANK, s);
+    }
+  }
   for (int m = 2; m < th.L; ++m) {
     const int lo = th.rg_lo[m], n_groups = th.rg_hi[m] - th.rg_lo[m];
     if (n_groups == 0) continue;
@@ -301,7 +330,7 @@ void run_bb_downward(const BBArgs &b, const double *mult, double *ple, cudaStrea
               AddChildRows{td.rg.get(), ple, lo, np}, row_tiles(n_groups), b.m2mc, 4 * np, 4 * np,
               np, s);
     }
-    {  // M2L of level m: tiles of one parity class, absent offsets skipped (fmm.py:118-131)
+    if (!b.fast[m]) {  // M2L of level m: tiles of one parity class, absent offsets skipped (fmm.py:118-131)
       PhaseTimer timer(PH_M2L, s);
       const int tpc = row_tiles(n_groups);
       rowgemm(M2LRows{td.rg.get(), td.il.get(), mult, lo, n_groups, np, tpc},

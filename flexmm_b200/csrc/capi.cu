@@ -46,7 +46,12 @@ struct LevelEntry {
   DevBuf<float> buf32;
   LevelOpsDev dev;
   DevBuf<LevelOpsDev> dev_copy;  // `dev` in device memory, gathered per plan by a kernel
-  DevBuf<double> bb_m2l;  // black-box FMM: [np x 40 np], offset blocks side by side
+  DevBuf<double> bb_m2l;  // black-box FMM: [40 np x np], the operators stacked, each transposed
+  // black-box FMM: the common basis Q [np x 64] and its transpose [64 x np],
+  // with the operators in it as M2L fragments (dev.m2l_f); or, at np <= 64, the
+  // operators themselves as fragments (bb_fast without bb_q)
+  DevBuf<double> bb_q, bb_frag;
+  bool bb_fast = false;
   DevBuf<double> st;      // Stokes FMM: this width's operators (StokesArgs::Level layout)
   StokesArgs::Level st_lev{};
 };
@@ -264,6 +269,24 @@ void retain_pool_memory() {
     }
   }
   done_for = dev;
+}
+
+// the 40 M2L operators of a black-box width as fragments: at(o, k, i) = column
+// k (source), row i (target) of offset o's operator; present[o] = 0: none
+template <class F>
+void bb_fragments(LevelEntry &e, int np, const int *present, F &&at) {
+  const size_t sq = size_t(np) * np;
+  std::vector<double> f(sq * N_OFFSETS, 0.0);
+  for (int o = 0; o < N_OFFSETS; ++o)
+    if (present[o]) pack_fragments(np, np, [&](int k, int i) { return at(o, k, i); }, f.data() + o * sq);
+  e.bb_frag.alloc(f.size(), 0);
+  FMMB_CUDA(cudaMemcpy(e.bb_frag.get(), f.data(), f.size() * sizeof(double), cudaMemcpyHostToDevice));
+  for (int o = 0; o < N_OFFSETS; ++o) {
+    e.dev.kind[o] = present[o] ? M2L_DENSE : M2L_NULL;
+    e.dev.m2l_f[o] =
+        present[o] ? reinterpret_cast<const double2 *>(e.bb_frag.get() + o * sq) : nullptr;
+  }
+  e.bb_fast = true;
 }
 }  // namespace
 
@@ -715,11 +738,49 @@ int fmm_bb_ops_add(fmm_ops *ops, const fmm_bb_level_ops *lv, int *level_id) {
       }
     }
     auto e = std::make_unique<LevelEntry>();
+    e->dev = LevelOpsDev{};
     e->dev.inv_w = 1.0 / lv->width;
     e->bb_m2l.alloc(h.size(), 0);
     FMMB_CUDA(cudaMemcpy(e->bb_m2l.get(), h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice));
+    if (np <= FMM_BB_MAX_RANK)  // the KIFMM's M2L takes the operators as they are
+      bb_fragments(*e, np, lv->m2l_rank, [&](int o, int k, int i) {
+        return h[(size_t(o) * np + k) * np + i];
+      });
+    e->dev_copy.alloc(1, 0);
+    FMMB_CUDA(cudaMemcpy(e->dev_copy.get(), &e->dev, sizeof(LevelOpsDev), cudaMemcpyHostToDevice));
     ops->levels.push_back(std::move(e));
     *level_id = int(ops->levels.size()) - 1;
+  });
+}
+
+int fmm_bb_ops_set_basis(fmm_ops *ops, int level_id, int rank, const double *q,
+                         const double *const *core) {
+  return guarded([&] {
+    FMMB_CHECK(ops && q && core, ERR_INVALID_ARGUMENT, "NULL argument");
+    FMMB_CHECK(ops->method == METHOD_BBFMM, ERR_INVALID_ARGUMENT,
+               "fmm_bb_ops_set_basis needs a black-box operator set");
+    FMMB_CHECK(level_id >= 0 && level_id < (int)ops->levels.size(), ERR_INVALID_ARGUMENT,
+               "unknown operator entry");
+    FMMB_CHECK(rank >= 1 && rank <= FMM_BB_MAX_RANK, ERR_INVALID_ARGUMENT,
+               "basis rank must be in [1, 64]");
+    const int n = ops->neq, np = ops->np, R = FMM_BB_MAX_RANK;
+    FMMB_CHECK(np > R, ERR_INVALID_ARGUMENT, "operators this small need no basis");
+    LevelEntry &e = *ops->levels[level_id];
+    FMMB_CHECK(!e.bb_fast, ERR_INVALID_ARGUMENT, "this width has a basis already");
+    std::vector<double> h(size_t(2) * np * R, 0.0);
+    for (int i = 0; i < n; ++i)
+      for (int k = 0; k < rank; ++k) {
+        h[size_t(i) * R + k] = q[size_t(i) * rank + k];
+        h[size_t(np) * R + size_t(k) * np + i] = q[size_t(i) * rank + k];
+      }
+    e.bb_q.alloc(h.size(), 0);
+    FMMB_CUDA(cudaMemcpy(e.bb_q.get(), h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice));
+    int present[N_OFFSETS];
+    for (int o = 0; o < N_OFFSETS; ++o) present[o] = core[o] ? 1 : 0;
+    bb_fragments(e, R, present, [&](int o, int k, int i) {
+      return i < rank && k < rank ? core[o][size_t(i) * rank + k] : 0.0;
+    });
+    FMMB_CUDA(cudaMemcpy(e.dev_copy.get(), &e.dev, sizeof(LevelOpsDev), cudaMemcpyHostToDevice));
   });
 }
 
@@ -981,8 +1042,15 @@ static BBArgs bb_args(fmm_plan *p, cudaStream_t) {
   b.th = &p->th;
   b.m2mc = p->ops->bb_m2mc.get();
   b.m2mct = p->ops->bb_m2mct.get();
-  for (int m = 0; m < p->th.L && m < FMM_MAX_LEVELS_DEV; ++m)
-    b.m2l_cat[m] = p->bound[m] >= 0 ? p->ops->levels[p->bound[m]]->bb_m2l.get() : nullptr;
+  b.any_fast = false;
+  for (int m = 0; m < p->th.L && m < FMM_MAX_LEVELS_DEV; ++m) {
+    const LevelEntry *e = p->bound[m] >= 0 ? p->ops->levels[p->bound[m]].get() : nullptr;
+    b.m2l_cat[m] = e ? e->bb_m2l.get() : nullptr;
+    b.q[m] = e ? e->bb_q.get() : nullptr;
+    b.fast[m] = m >= 2 && e && e->bb_fast;
+    b.any_fast = b.any_fast || b.fast[m];
+  }
+  b.ops_dev = p->ops_dev.get();
   return b;
 }
 
@@ -1234,15 +1302,24 @@ static void build_expansions_impl(fmm_plan *p, const double *tau, void *stream) 
     const int np = p->ops->np;
     const int64_t total = th.n_total();
     if (p->ops->method == METHOD_BBFMM) {
+      upload_level_ops(p, s);
       BBArgs b = bb_args(p, s);
       p->tau_s.alloc(th.n_points, s);
       gather_sorted(tau, p->td.ordv.get(), th.n_points, p->tau_s.get(), s);
       p->mult.alloc(total * np, s);
       p->ple.alloc(total * np, s);
-      p->mult.zero(s);
-      p->ple.zero(s);
+      const bool basis = b.any_fast && np > FMM_BB_MAX_RANK;
+      if (basis) {
+        p->partial.alloc(total * FMM_BB_MAX_RANK, s);
+        p->loc.alloc(total * FMM_BB_MAX_RANK, s);
+      }
+      ZeroBatch zb(s);
+      zb.add(p->mult).add(p->ple);
+      if (basis) zb.add(p->loc);  // (the M2L writes the rows of real groups only)
+      zb.run();
       run_bb_upward(b, p->tau_s.get(), p->mult.get(), s);
-      run_bb_downward(b, p->mult.get(), p->ple.get(), s);
+      run_bb_downward(b, p->mult.get(), p->ple.get(), basis ? p->partial.get() : nullptr,
+                      basis ? p->loc.get() : nullptr, s);
       p->have_expansions = true;
       return;
     }

@@ -67,10 +67,19 @@ struct BBArgs {
   const TreeHost *th;
   const double *m2mc, *m2mct;
   const double *m2l_cat[FMM_MAX_LEVELS_DEV];
+  // fast[m]: the level has its M2L operators as fragments (ops_dev), either as
+  // they are (np <= 64) or in its common basis q[m]: Q [np x 64], then
+  // Q^T [64 x np], zero padded; any_fast: one of the levels >= 2 has
+  bool fast[FMM_MAX_LEVELS_DEV], any_fast;
+  const LevelOpsDev *ops_dev;
+  const double *q[FMM_MAX_LEVELS_DEV];
 };
+constexpr int BB_RANK = 64;  // columns of a common basis
 void run_bb_upward(const BBArgs &b, const double *tau_sorted, double *mult, cudaStream_t s);
-// M2L and L2L, level by level; the locals are the partial locals (no solve)
-void run_bb_downward(const BBArgs &b, const double *mult, double *ple, cudaStream_t s);
+// M2L and L2L; the locals are the partial locals (no solve).  z, zl: multipoles
+// and partial locals in the common bases, [nodes x 64], where there are any
+void run_bb_downward(const BBArgs &b, const double *mult, double *ple, double *z, double *zl,
+                     cudaStream_t s);
 // nout = 1 potential, 3 potential and target gradient (rows, stride ld_out)
 void run_bb_evaluate(const BBArgs &b, const double *tau_sorted, const double *loc,
                      const double *txs, const double *tys, const uint64_t *tkeys, const int *tperm,

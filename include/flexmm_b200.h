@@ -141,6 +141,14 @@ typedef struct fmm_bb_level_ops {
   const double *const *m2l_b;
 } fmm_bb_level_ops;
 int fmm_bb_ops_add(fmm_ops *ops, const fmm_bb_level_ops *lv, int *level_id);
+/* Optional: a common basis of that width's M2L operators, M2L_o = Q core_o Q^T
+ * with Q [NQ x rank] orthonormal and core_o [rank x rank] (NULL where m2l_rank
+ * is 0), row-major, rank <= FMM_BB_MAX_RANK.  A smooth kernel's 40 operators
+ * share a column space far smaller than NQ = p^2 (62 of 256 to 1e-16 for the
+ * log kernel, p = 16); a plan whose levels all have one translates in it. */
+#define FMM_BB_MAX_RANK 64
+int fmm_bb_ops_set_basis(fmm_ops *ops, int level_id, int rank, const double *q,
+                         const double *const *core);
 
 int fmm_ops_create(int kernel_id, const double *kernel_params /* [4] or NULL */, int nequiv,
                    fmm_ops **out);
