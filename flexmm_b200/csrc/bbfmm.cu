@@ -28,14 +28,13 @@
 #include "dense.cuh"
 #include "rowgemm.cuh"
 #include "fmm.cuh"
+#include "sweep.cuh"
 #include "timing.cuh"
 
 namespace fmmb {
 namespace {
 
 constexpr int BB_MAX_P = 16;
-constexpr int TCH_BB = 128;   // evaluation threads per work item
-constexpr int SMAX_BB = 1024;  // sources staged per evaluation pass
 
 // 2 / width per level: maps a box to [-1, 1]^2 (width_adj, bbfmm.py:122)
 struct BBScale {
@@ -108,78 +107,64 @@ __global__ void __launch_bounds__(128) k_bb_s2m(int p, int np, int L, BBScale sc
   }
 }
 
-// Evaluation: L2T as a 2-D Chebyshev series of the leaf's local coefficients,
-// P2P over the colleagues (as k_evaluate).  One work item = (leaf, up to 128
-// of its targets); G threads share a target.  NOUT = 3 adds the gradient in
-// the target position: the series' derivative (T_n' by its recurrence,
-// chebeval2d_dx / _dy, bbfmm.py:32-45) and the kernel's gradient.
+// Evaluation of an item (items.cuh): L2T as a 2-D Chebyshev series of the
+// leaf's local coefficients, sum_a T_a(x) sum_b c[a p + b] T_b(y), the rows a
+// split over the warps and the lanes of a target; P2P as in the KIFMM.
+// NOUT = 3 adds the gradient in the target position: the series' derivative
+// (T_n' by its recurrence, chebeval2d_dx / _dy, bbfmm.py:32-45) and the
+// kernel's gradient.  500k sources, 250k targets, p = 16: potentials 0.85 ->
+// 0.27 ms, the two gradient evaluations 2.55 -> 1.14 ms.
 template <class KF, int NOUT>
-__global__ void __launch_bounds__(TCH_BB) k_bb_evaluate(KernelParams kp, int p, int np, BBScale sc,
-                                                        const int4 *__restrict__ items,
-                                                        const int *__restrict__ n_items_ptr,
-                                                        const int *__restrict__ coll,
-                                                        const int *__restrict__ bot,
-                                                        const int *__restrict__ top,
-                                                        const double *__restrict__ xmid,
-                                                        const double *__restrict__ ymid,
-                                                        const double *__restrict__ sx,
-                                                        const double *__restrict__ sy,
-                                                        const double *__restrict__ tau,
-                                                        const double *__restrict__ loc,
-                                                        const double *__restrict__ txs,
-                                                        const double *__restrict__ tys,
-                                                        const int *__restrict__ tperm, int check,
-                                                        double *__restrict__ out, int64_t ld_out) {
-  __shared__ double ssx[SMAX_BB], ssy[SMAX_BB], stau[SMAX_BB];
-  __shared__ int rb[9], rs[10];
-  __shared__ double red[NOUT][TCH_BB / 32];
-  const KF K(kp);
-  const int n_items = *n_items_ptr;
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const int4 it = items[item];
-    const int g = it.x, lev = it.y, t0 = it.z, cnt = it.w;
-    int G = 1;
-    while (2 * G * cnt <= TCH_BB) G *= 2;
-    const int t = threadIdx.x / G, sub = threadIdx.x % G;
-    const bool valid = t < cnt;
-    const double x = valid ? txs[t0 + t] : 0.0, y = valid ? tys[t0 + t] : 0.0;
-    if (threadIdx.x < 9) {
-      const int cg = coll[(size_t)g * 9 + threadIdx.x];
-      rb[threadIdx.x] = cg >= 0 ? bot[cg] : 0;
-      rs[threadIdx.x + 1] = cg >= 0 ? top[cg] - bot[cg] : 0;
+struct BBPolicy : ChargePolicy<KF, NOUT, false, false> {
+  using Base = ChargePolicy<KF, NOUT, false, false>;
+  static constexpr bool kNear = true, kFar = true;
+  using Smem = typename Base::Smem;
+  int p, np;
+  BBScale sc;
+  const double *xmid, *ymid, *loc;
+
+  __device__ __forceinline__ void stage_far(Smem &, int, int) const {}
+  template <int R>
+  __device__ __forceinline__ void far_field(const KF &, const Smem &, int g, int lev,
+                                            const double (&x)[R], const double (&y)[R], int warp,
+                                            int sub, int G, double (&v)[R][Base::NV]) const {
+    const double a = sc.inv_hw[lev], cx = xmid[g], cy = ymid[g];
+    const double *cr = loc + (size_t)g * np;
+    // raw sums of a table functor are scaled at the end: divide that out here
+    double su = 1.0, sg = a;  // d/dx = (2 / w) d/dxh
+    if constexpr (KF::kLogTable) {
+      su = 1.0 / KF::kFold;
+      sg = a / KF::grad_fold(this->kp);
     }
-    if (threadIdx.x == 0) rs[0] = 0;
-    __syncthreads();
-    if (threadIdx.x == 0)
-      for (int c = 1; c <= 9; ++c) rs[c] += rs[c - 1];
-    double u = 0.0, gx = 0.0, gy = 0.0;
-    if (lev >= 2 && valid) {
-      // sum_a T_a(x) sum_b c[a p + b] T_b(y), rows a split over the G threads
-      const double a = sc.inv_hw[lev];
-      const double xh = (x - xmid[g]) * a, yh = (y - ymid[g]) * a;
-      double ty[BB_MAX_P], dty[BB_MAX_P];
+#pragma unroll 1
+    for (int r = 0; r < R; ++r) {
+      const double xh = ((r == 0 ? x[0] : x[R - 1]) - cx) * a;
+      const double yh = ((r == 0 ? y[0] : y[R - 1]) - cy) * a;
+      double ty[BB_MAX_P], dty[NOUT == 3 ? BB_MAX_P : 1];
       ty[0] = 1.0;
       ty[1] = yh;
-      dty[0] = 0.0;
-      dty[1] = 1.0;
+      if (NOUT == 3) {
+        dty[0] = 0.0;
+        dty[NOUT == 3 ? 1 : 0] = 1.0;
+      }
 #pragma unroll
       for (int b = 2; b < BB_MAX_P; ++b) {
         ty[b] = 2.0 * yh * ty[b - 1] - ty[b - 2];
-        if (NOUT == 3) dty[b] = 2.0 * ty[b - 1] + 2.0 * yh * dty[b - 1] - dty[b - 2];
+        if constexpr (NOUT == 3) dty[b] = 2.0 * ty[b - 1] + 2.0 * yh * dty[b - 1] - dty[b - 2];
       }
-      const double *cr = loc + (size_t)g * np;
-      double tp = 1.0, tc = xh;    // T_{ar-1}, T_ar as ar advances
+      double u = 0.0, gx = 0.0, gy = 0.0;
+      double tp = 1.0, tc = xh;     // T_{ar-1}, T_ar as ar advances
       double dtp = 0.0, dtc = 1.0;  // their derivatives
       for (int ar = 0; ar < p; ++ar) {
         const double tx = ar == 0 ? 1.0 : tc, dtx = ar == 0 ? 0.0 : dtc;
-        if (ar % G == sub) {
+        if ((ar & (EV_WARPS - 1)) == warp && ((ar / EV_WARPS) & (G - 1)) == sub) {
           double s = 0.0, sd = 0.0;
 #pragma unroll
           for (int b = 0; b < BB_MAX_P; ++b)
             if (b < p) {
               const double c = __ldg(cr + ar * p + b);
               s = fma(c, ty[b], s);
-              if (NOUT == 3) sd = fma(c, dty[b], sd);
+              if constexpr (NOUT == 3) sd = fma(c, dty[b], sd);
             }
           u = fma(tx, s, u);
           if (NOUT == 3) {
@@ -198,66 +183,20 @@ __global__ void __launch_bounds__(TCH_BB) k_bb_evaluate(KernelParams kp, int p, 
           tc = tn;
         }
       }
-      gx *= a;  // d/dx = (2 / w) d/dxh
-      gy *= a;
-    }
-    __syncthreads();
-    auto pair = [&](int j) -> double {
-      const double qx = ssx[j], qy = ssy[j];
-      const double v = K(qx, qy, x, y) * stau[j];
-      return (check && x - qx == 0.0 && y - qy == 0.0) ? 0.0 : v;
-    };
-    const int ns = rs[9];
-    double u1 = 0.0, u2 = 0.0, u3 = 0.0;
-    for (int base = 0; base < ns; base += SMAX_BB) {
-      const int nb = min(SMAX_BB, ns - base);
-      for (int i = threadIdx.x; i < nb; i += TCH_BB) {
-        const int idx = base + i;
-        int c = 0;
-        while (idx >= rs[c + 1]) ++c;
-        const int j = rb[c] + (idx - rs[c]);
-        ssx[i] = sx[j];
-        ssy[i] = sy[j];
-        stau[i] = tau[j];
-      }
-      __syncthreads();
-      if (valid) {
-        if constexpr (NOUT == 1) {
-          int j = sub;
-          for (; j + 3 * G < nb; j += 4 * G) {
-            u += pair(j);
-            u1 += pair(j + G);
-            u2 += pair(j + 2 * G);
-            u3 += pair(j + 3 * G);
-          }
-          for (; j < nb; j += G) u += pair(j);
-        } else {
-          for (int j = sub; j < nb; j += G) {
-            const double qx = ssx[j], qy = ssy[j];
-            if (!(check && x - qx == 0.0 && y - qy == 0.0)) K.grad(qx, qy, x, y, stau[j], u, gx, gy);
-          }
-        }
-      }
-      __syncthreads();
-    }
-    double r[3] = {(u + u1) + (u2 + u3), gx, gy};
 #pragma unroll
-    for (int o = 0; o < NOUT; ++o) {
-      double w = r[o];
-      for (int q = min(G, 32) >> 1; q >= 1; q >>= 1) w += __shfl_xor_sync(0xffffffffu, w, q);
-      if (G > 32) {
-        if ((threadIdx.x & 31) == 0) red[o][threadIdx.x >> 5] = w;
-        __syncthreads();
-        if (sub == 0) {
-          w = 0.0;
-          for (int q = 0; q < G / 32; ++q) w += red[o][(threadIdx.x >> 5) + q];
+      for (int k = 0; k < R; ++k)
+        if (k == r) {
+          if constexpr (NOUT == 1) {
+            v[k][0] += u;
+          } else {
+            v[k][0] += u * su;
+            v[k][1] += gx * sg;
+            v[k][2] += gy * sg;
+          }
         }
-      }
-      if (valid && sub == 0) out[o * ld_out + tperm[t0 + t]] = w;
     }
-    __syncthreads();
   }
-}
+};
 
 BBScale bb_scale(const TreeHost &th) {
   BBScale sc{};
@@ -351,23 +290,46 @@ void run_bb_evaluate(const BBArgs &b, const double *tau_s, const double *loc, co
   eval_items(a, tkeys, m, it, s);
   const BBScale sc = bb_scale(*b.th);
   PhaseTimer timer(PH_EVAL, s);
-  auto launch = [&](auto kern) {
-    kern<<<work_grid(b.th->n_total() + m / TCH_BB + 1, 8), TCH_BB, 0, s>>>(
-        b.kp, b.p, b.np, sc, it.items.get(), it.n_items.get(),
-                                    td.coll.get(), td.bot.get(), td.top.get(), td.xmid.get(),
-                                    td.ymid.get(), td.sx.get(), td.sy.get(), tau_s, loc, txs, tys,
-                                    tperm, check, out, ld_out);
+  const ItemArgs ia{it.items.get(), it.n_items.get(), it.n_items.get() + 1, td.coll.get(),
+                    td.bot.get(),   td.top.get(),     txs,                 tys, tperm};
+  auto launch = [&](auto pt, auto blocks) {
+    using Pol = typename decltype(pt)::type;
+    Pol pol{};
+    pol.kp = b.kp;
+    pol.sx = td.sx.get();
+    pol.sy = td.sy.get();
+    pol.tau = tau_s;
+    pol.check = check;
+    pol.out = out;
+    pol.ld_out = ld_out;
+    pol.p = b.p;
+    pol.np = b.np;
+    pol.sc = sc;
+    pol.xmid = td.xmid.get();
+    pol.ymid = td.ymid.get();
+    pol.loc = loc;
+    constexpr int B = decltype(blocks)::value;
+    k_items<Pol, B><<<work_grid(b.th->n_total() + m / EVAL_CHUNK + 1, B), EV_THREADS, 0, s>>>(pol, ia);
   };
+  // resident blocks: the Chebyshev values of a target are held in registers
+  using P1 = std::integral_constant<int, 6>;
+  using P3 = std::integral_constant<int, 4>;
   switch (b.kernel_id) {
     case KERNEL_LAPLACE:
-      nout == 3 ? launch(k_bb_evaluate<LaplaceF64, 3>) : launch(k_bb_evaluate<LaplaceF64, 1>);
+      if (nout == 3)
+        launch(TypeOf<BBPolicy<LaplaceF64T, 3>>{}, P3{});
+      else
+        launch(TypeOf<BBPolicy<LaplaceF64T, 1>>{}, P1{});
       break;
     case KERNEL_MOD_HELMHOLTZ:
-      nout == 3 ? launch(k_bb_evaluate<ModHelmholtzF64, 3>) : launch(k_bb_evaluate<ModHelmholtzF64, 1>);
+      if (nout == 3)
+        launch(TypeOf<BBPolicy<ModHelmholtzF64T, 3>>{}, P3{});
+      else
+        launch(TypeOf<BBPolicy<ModHelmholtzF64T, 1>>{}, P1{});
       break;
     case KERNEL_RADIAL_TABLE:
       FMMB_CHECK(nout == 1, ERR_UNSUPPORTED, "tabulated kernels evaluate potentials only");
-      launch(k_bb_evaluate<RadialTableF64, 1>);
+      launch(TypeOf<BBPolicy<RadialTableF64, 1>>{}, P1{});
       break;
     default: throw Error(ERR_UNSUPPORTED, "unknown kernel id");
   }

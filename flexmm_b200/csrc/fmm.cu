@@ -889,11 +889,6 @@ ItemArgs item_args(const PassArgs &a, const int4 *items, int *n_items, int count
                   td.top.get(), txs, tys, tperm};
 }
 
-template <class T>
-struct TypeOf {
-  using type = T;
-};
-
 // resident blocks per SM the potential and gradient evaluations are built for
 constexpr int EVAL_BLOCKS = 8, EVAL_BLOCKS_GRAD = 6;
 

@@ -32,6 +32,11 @@ namespace {
 constexpr int EV_WARPS = 4, EV_THREADS = 32 * EV_WARPS;
 static_assert(EV_THREADS == EVAL_CHUNK, "an item's targets fit the block's threads");
 
+template <class T>
+struct TypeOf {
+  using type = T;
+};
+
 struct ItemArgs {
   const int4 *items;
   const int *n_items;  // device count

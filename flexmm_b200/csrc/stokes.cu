@@ -24,44 +24,60 @@
 #include "dense.cuh"
 #include "rowgemm.cuh"
 #include "fmm.cuh"
+#include "items.cuh"
 #include "timing.cuh"
 
 namespace fmmb {
 namespace {
 
-constexpr int TCH_ST = 128;
-constexpr int SMAX_ST = 1024;
-
 struct StokesCircles {
   const double *lx[FMM_MAX_LEVELS_DEV], *ly[FMM_MAX_LEVELS_DEV];  // large circle, per level
 };
 
-// one Stokeslet pair, unscaled: u, v times 1/(4 pi), p times 1/(2 pi) later
-// (kernel_apply_single, stokes_fmm.py:166-187)
-__device__ __forceinline__ void stokeslet(double dx, double dy, double fx, double fy, double &u,
-                                          double &v, double &p) {
-  const double id2 = 1.0 / (dx * dx + dy * dy);
-  const double logid = 0.5 * log(id2);
-  const double dxdy = dx * dy * id2;
-  u += (logid + dx * dx * id2) * fx + dxdy * fy;
-  v += dxdy * fx + (logid + dy * dy * id2) * fy;
-  p += (fx * dx + fy * dy) * id2;
-}
+// Sums of Stokeslet (and stresslet) pairs at a target, unscaled (u, v times
+// 1/(4 pi), p times 1/(2 pi) later).  With d = (dx, dy) = target - source,
+// r2 = |d|^2 (kernel_apply_single, stokes_fmm.py:166-187):
+//   u += -log(r2)/2 fx + dx s,  v += -log(r2)/2 fy + dy s,  p += s,
+//   s = (d . f) / r2;
+// a stresslet (kernel_apply_single_with_dipole, stokes_fmm.py:187-235) of
+// strength sigma along the normal n adds, with c = 4 (d . n)(d . sigma) / r2^2,
+//   u += c dx,  v += c dy,  p += c - 2 (n . sigma) / r2.
+// The logarithms are summed as raw log2 values (lx, ly), from the passes'
+// table, and the reciprocal is rcp_newton: about 24 FP64 instructions a pair
+// where the library's logarithm and division took about 60 (a batch of 560k
+// points, forward and adjoint: evaluation kernels 4.4 -> 1.9 ms, S2M 0.75 ->
+// 0.45).
+struct StokesSum {
+  double lx = 0.0, ly = 0.0, u = 0.0, v = 0.0, p = 0.0;
+  __device__ __forceinline__ void add(double dx, double dy, double fx, double fy, double l2, double i2) {
+    const double s = fma(dx, fx, dy * fy) * i2;
+    lx = fma(l2, fx, lx);
+    ly = fma(l2, fy, ly);
+    u = fma(dx, s, u);
+    v = fma(dy, s, v);
+    p += s;
+  }
+  __device__ __forceinline__ void add_dipole(double dx, double dy, double2 sg, double2 n, double i2) {
+    const double c = 4.0 * fma(dx, n.x, dy * n.y) * i2 * (fma(dx, sg.x, dy * sg.y) * i2);
+    u = fma(c, dx, u);
+    v = fma(c, dy, v);
+    p += fma(-2.0 * i2, fma(n.x, sg.x, n.y * sg.y), c);
+  }
+  static constexpr double kLog = -0.5 * 0.69314718055994530942;  // log2(r2) -> -log(r2)/2
+};
 
-// one stresslet (double-layer) pair, unscaled like stokeslet: strength
-// (sgx, sgy) along the normal (nx, ny), d = (dx, dy) target - source
-// (kernel_apply_single_with_dipole, stokes_fmm.py:187-235):
-//   u_a += 4 (d.n) d_a d_b / r^4 sigma_b,
-//   p   += 2 (-n_b / r^2 + 2 d_b (d.n) / r^4) sigma_b
-__device__ __forceinline__ void stresslet(double dx, double dy, double sgx, double sgy, double nx,
-                                          double ny, double &u, double &v, double &p) {
-  const double id2 = 1.0 / (dx * dx + dy * dy);
-  const double dn = dx * nx + dy * ny;
-  const double c = 4.0 * dn * id2 * id2;
-  const double gxy = c * dx * dy;
-  u += c * dx * dx * sgx + gxy * sgy;
-  v += gxy * sgx + c * dy * dy * sgy;
-  p += 2.0 * (-nx * id2 + 0.5 * dx * c) * sgx + 2.0 * (-ny * id2 + 0.5 * dy * c) * sgy;
+// log2(r2) and 1 / r2 of a pair; false for a coincident pair when check is set
+__device__ __forceinline__ bool stokes_radial(const LaplaceF64T &K, double r2, int check, double &l2,
+                                              double &i2) {
+  if (log2_rare_key(r2) < RCP_RARE) {
+    l2 = K.at(r2);
+    i2 = rcp_newton(r2);
+    return true;
+  }
+  if (check && r2 == 0.0) return false;
+  l2 = log2(r2);
+  i2 = 1.0 / r2;
+  return true;
 }
 
 // S2M: velocities at the large circle's points from the box's sources; one
@@ -86,15 +102,18 @@ __global__ void __launch_bounds__(128) k_stokes_s2m(int neq, int np, int L, Stok
                                                     const double *__restrict__ dnx,
                                                     const double *__restrict__ dny) {
   __shared__ double qx[4][32], qy[4][32], qf[4][32], qg[4][32];
-  __shared__ double qs[DIP ? 4 : 1][32], qt[DIP ? 4 : 1][32], qn[DIP ? 4 : 1][32],
-      qm[DIP ? 4 : 1][32];
+  __shared__ double2 qs[DIP ? 4 : 1][32], qn[DIP ? 4 : 1][32];
+  __shared__ FunctorSmem<LaplaceF64T> fsm;
+  LaplaceF64T K(KernelParams{});
+  fsm.bind(K);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_up = *n_up_ptr;
   for (int i = blockIdx.x * 4 + warp; i < n_up; i += gridDim.x * 4) {
     const int g = uplist[i];
     const int m = node_level_of(off, L, g);
     const double cx = xmid[g], cy = ymid[g];
-    double ex[2], ey[2], u[2] = {0.0, 0.0}, v[2] = {0.0, 0.0}, p[2] = {0.0, 0.0};
+    double ex[2], ey[2];
+    StokesSum sum[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int k = lane + 32 * h;
@@ -110,22 +129,21 @@ __global__ void __launch_bounds__(128) k_stokes_s2m(int neq, int np, int L, Stok
         qf[warp][lane] = fx[j0 + lane];
         qg[warp][lane] = fy[j0 + lane];
         if constexpr (DIP) {
-          qs[warp][lane] = sgx[j0 + lane];
-          qt[warp][lane] = sgy[j0 + lane];
-          qn[warp][lane] = dnx[j0 + lane];
-          qm[warp][lane] = dny[j0 + lane];
+          qs[warp][lane] = make_double2(sgx[j0 + lane], sgy[j0 + lane]);
+          qn[warp][lane] = make_double2(dnx[j0 + lane], dny[j0 + lane]);
         }
       }
       __syncwarp();
 #pragma unroll
       for (int h = 0; h < 2; ++h)
         if (lane + 32 * h < neq)
+#pragma unroll 2
           for (int j = 0; j < nj; ++j) {
             const double dx = ex[h] - qx[warp][j], dy = ey[h] - qy[warp][j];
-            stokeslet(dx, dy, qf[warp][j], qg[warp][j], u[h], v[h], p[h]);
-            if constexpr (DIP)
-              stresslet(dx, dy, qs[warp][j], qt[warp][j], qn[warp][j], qm[warp][j], u[h], v[h],
-                        p[h]);
+            double l2, i2;
+            stokes_radial(K, fma(dy, dy, dx * dx), 0, l2, i2);
+            sum[h].add(dx, dy, qf[warp][j], qg[warp][j], l2, i2);
+            if constexpr (DIP) sum[h].add_dipole(dx, dy, qs[warp][j], qn[warp][j], i2);
           }
       __syncwarp();
     }
@@ -134,106 +152,140 @@ __global__ void __launch_bounds__(128) k_stokes_s2m(int neq, int np, int L, Stok
     for (int h = 0; h < 2; ++h) {
       const int k = lane + 32 * h;
       if (k < neq) {
-        partial[(size_t)g * np + k] = u[h] * us;
-        partial[(size_t)g * np + neq + k] = v[h] * us;
+        partial[(size_t)g * np + k] = fma(StokesSum::kLog, sum[h].lx, sum[h].u) * us;
+        partial[(size_t)g * np + neq + k] = fma(StokesSum::kLog, sum[h].ly, sum[h].v) * us;
       }
     }
   }
 }
 
-// Evaluation: (u, v, p) rows of out (stride ld_out).  One work item = (leaf,
-// up to 128 of its targets); G threads share a target.  DIP: the near field
-// adds the sources' stresslets (neighbor_evaluation_dipole,
-// stokes_fmm.py:399-441); the far field is the same local expansion.
+// Evaluation of an item (items.cuh): (u, v, p) rows of out (stride ld_out); the
+// far field is the leaf's local forces on the large circle
+// (local_expansion_evaluation, stokes_fmm.py:331-360), the near field its
+// colleagues' sources, DIP with their stresslets (neighbor_evaluation(_dipole),
+// stokes_fmm.py:361-441).
 template <bool DIP>
-__global__ void __launch_bounds__(TCH_ST) k_stokes_evaluate(
-    int neq, int np, StokesCircles cir, const int4 *__restrict__ items,
-    const int *__restrict__ n_items_ptr, const int *__restrict__ coll, const int *__restrict__ bot,
-    const int *__restrict__ top, const double *__restrict__ xmid, const double *__restrict__ ymid,
-    const double *__restrict__ sx, const double *__restrict__ sy, const double *__restrict__ fx,
-    const double *__restrict__ fy, const double *__restrict__ loc, const double *__restrict__ txs,
-    const double *__restrict__ tys, const int *__restrict__ tperm, int check,
-    double *__restrict__ out, int64_t ld_out, const double *__restrict__ sgx,
-    const double *__restrict__ sgy, const double *__restrict__ dnx,
-    const double *__restrict__ dny) {
-  constexpr int SM = DIP ? SMAX_ST / 2 : SMAX_ST;  // 48 KB of static shared memory at most
-  __shared__ double ssx[SM], ssy[SM], sfx[SM], sfy[SM];
-  __shared__ double ssg[DIP ? SM : 1], stg[DIP ? SM : 1], snx[DIP ? SM : 1], sny[DIP ? SM : 1];
-  __shared__ int rb[9], rs[10];
-  __shared__ double red[3][TCH_ST / 32];
-  const int n_items = *n_items_ptr;
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const int4 it = items[item];
-    const int g = it.x, lev = it.y, t0 = it.z, cnt = it.w;
-    int G = 1;
-    while (2 * G * cnt <= TCH_ST) G *= 2;
-    const int t = threadIdx.x / G, sub = threadIdx.x % G;
-    const bool valid = t < cnt;
-    const double x = valid ? txs[t0 + t] : 0.0, y = valid ? tys[t0 + t] : 0.0;
-    if (threadIdx.x < 9) {
-      const int cg = coll[(size_t)g * 9 + threadIdx.x];
-      rb[threadIdx.x] = cg >= 0 ? bot[cg] : 0;
-      rs[threadIdx.x + 1] = cg >= 0 ? top[cg] - bot[cg] : 0;
-    }
-    if (threadIdx.x == 0) rs[0] = 0;
-    __syncthreads();
-    if (threadIdx.x == 0)
-      for (int c = 1; c <= 9; ++c) rs[c] += rs[c - 1];
-    double u = 0.0, v = 0.0, p = 0.0;
-    if (lev >= 2 && valid) {  // L2T: local forces on the large circle
-      const double dx0 = x - xmid[g], dy0 = y - ymid[g];
-      const double *lf = loc + (size_t)g * np;
-      for (int k = sub; k < neq; k += G)
-        stokeslet(dx0 - cir.lx[lev][k], dy0 - cir.ly[lev][k], lf[k], lf[neq + k], u, v, p);
-    }
-    __syncthreads();
-    const int ns = rs[9];
-    for (int base = 0; base < ns; base += SM) {
-      const int nb = min(SM, ns - base);
-      for (int i = threadIdx.x; i < nb; i += TCH_ST) {
-        const int idx = base + i;
-        int c = 0;
-        while (idx >= rs[c + 1]) ++c;
-        const int j = rb[c] + (idx - rs[c]);
-        ssx[i] = sx[j];
-        ssy[i] = sy[j];
-        sfx[i] = fx[j];
-        sfy[i] = fy[j];
-        if constexpr (DIP) {
-          ssg[i] = sgx[j];
-          stg[i] = sgy[j];
-          snx[i] = dnx[j];
-          sny[i] = dny[j];
-        }
-      }
-      __syncthreads();
-      if (valid)
-        for (int j = sub; j < nb; j += G) {
-          const double dx = x - ssx[j], dy = y - ssy[j];
-          if (check && dx == 0.0 && dy == 0.0) continue;
-          stokeslet(dx, dy, sfx[j], sfy[j], u, v, p);
-          if constexpr (DIP) stresslet(dx, dy, ssg[j], stg[j], snx[j], sny[j], u, v, p);
-        }
-      __syncthreads();
-    }
-    double r[3] = {u * (0.25 / M_PI), v * (0.25 / M_PI), p * (0.5 / M_PI)};
-#pragma unroll
-    for (int o = 0; o < 3; ++o) {
-      double w = r[o];
-      for (int s = min(G, 32) >> 1; s >= 1; s >>= 1) w += __shfl_xor_sync(0xffffffffu, w, s);
-      if (G > 32) {
-        if ((threadIdx.x & 31) == 0) red[o][threadIdx.x >> 5] = w;
-        __syncthreads();
-        if (sub == 0) {
-          w = 0.0;
-          for (int q = 0; q < G / 32; ++q) w += red[o][(threadIdx.x >> 5) + q];
-        }
-      }
-      if (valid && sub == 0) out[o * ld_out + tperm[t0 + t]] = w;
-    }
-    __syncthreads();
+struct StokesPolicy {
+  using Kernel = LaplaceF64T;
+  static constexpr int NOUT = 3, NV = 5;
+  static constexpr int SMAX = DIP ? 384 : 512;  // 48 KB of static shared memory at most
+  static constexpr bool kNear = true, kFar = true;
+  struct Smem {
+    double2 xy[SMAX], f[SMAX];
+    double2 sg[DIP ? SMAX : 1], n[DIP ? SMAX : 1];
+    double2 fxy[64], ff[64];  // the circle's points and forces
+    double cx, cy;
+    FunctorSmem<LaplaceF64T> fs;
+  };
+  template <int R>
+  struct Tgt {};
+  int neq, np, check;
+  StokesCircles cir;
+  const double *xmid, *ymid, *sx, *sy, *fx, *fy, *loc, *sgx, *sgy, *dnx, *dny;
+  double *out;
+  int64_t ld_out;
+
+  __device__ __forceinline__ LaplaceF64T bind(Smem &sm) const {
+    LaplaceF64T K(KernelParams{});
+    sm.fs.bind(K);
+    return K;
   }
-}
+  __device__ __forceinline__ void stage_far(Smem &sm, int g, int lev) const {
+    const double *lf = loc + (size_t)g * np;
+    for (int k = threadIdx.x; k < neq; k += EV_THREADS) {
+      sm.fxy[k] = make_double2(cir.lx[lev][k], cir.ly[lev][k]);
+      sm.ff[k] = make_double2(lf[k], lf[neq + k]);
+    }
+    if (threadIdx.x == 64) {
+      sm.cx = xmid[g];
+      sm.cy = ymid[g];
+    }
+  }
+  __device__ __forceinline__ void stage(Smem &sm, int i, int j) const {
+    sm.xy[i] = make_double2(sx[j], sy[j]);
+    sm.f[i] = make_double2(fx[j], fy[j]);
+    if constexpr (DIP) {
+      sm.sg[i] = make_double2(sgx[j], sgy[j]);
+      sm.n[i] = make_double2(dnx[j], dny[j]);
+    }
+  }
+  template <class T>
+  __device__ __forceinline__ void load_target(T &, int, const int *, int) const {}
+  template <int R, bool D>
+  __device__ __forceinline__ void pairs(const LaplaceF64T &K, const Smem &sm, const double2 *xy,
+                                        const double2 *f, const double (&x)[R], const double (&y)[R],
+                                        int lo, int hi, int G, int chk, double (&v)[R][NV]) const {
+    StokesSum sum[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) sum[r] = {v[r][0], v[r][1], v[r][2], v[r][3], v[r][4]};
+    auto one = [&](double dx, double dy, double2 q, int j, StokesSum &s, double l2, double i2) {
+      s.add(dx, dy, q.x, q.y, l2, i2);
+      if constexpr (D) s.add_dipole(dx, dy, sm.sg[j], sm.n[j], i2);
+    };
+    for (int j = lo; j < hi; j += G) {
+      const double2 p = xy[j], q = f[j];
+      double dx[R], dy[R], r2[R];
+      unsigned key = 0;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        dx[r] = x[r] - p.x;
+        dy[r] = y[r] - p.y;
+        r2[r] = fma(dy[r], dy[r], dx[r] * dx[r]);
+        key = max(key, log2_rare_key(r2[r]));
+      }
+      if (key < RCP_RARE) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          one(dx[r], dy[r], q, j, sum[r], K.at(r2[r]), rcp_newton(r2[r]));
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          double l2, i2;
+          // a pair is left out where it coincides, not where r2 underflows
+          if (chk && dx[r] == 0.0 && dy[r] == 0.0) continue;
+          stokes_radial(K, r2[r], 0, l2, i2);
+          one(dx[r], dy[r], q, j, sum[r], l2, i2);
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      v[r][0] = sum[r].lx;
+      v[r][1] = sum[r].ly;
+      v[r][2] = sum[r].u;
+      v[r][3] = sum[r].v;
+      v[r][4] = sum[r].p;
+    }
+  }
+  template <int R>
+  __device__ __forceinline__ void far_field(const LaplaceF64T &K, const Smem &sm, int, int,
+                                            const double (&x)[R], const double (&y)[R], int warp,
+                                            int sub, int G, double (&v)[R][NV]) const {
+    double dx[R], dy[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      dx[r] = x[r] - sm.cx;
+      dy[r] = y[r] - sm.cy;
+    }
+    pairs<R, false>(K, sm, sm.fxy, sm.ff, dx, dy, (neq * warp) / EV_WARPS + sub,
+                    (neq * (warp + 1)) / EV_WARPS, G, 0, v);
+  }
+  template <int R>
+  __device__ __forceinline__ void sweep(const LaplaceF64T &K, const Smem &sm, const double (&x)[R],
+                                        const double (&y)[R], const Tgt<R> &, int lo, int hi, int G,
+                                        double (&v)[R][NV]) const {
+    pairs<R, DIP>(K, sm, sm.xy, sm.f, x, y, lo, hi, G, check, v);
+  }
+  __device__ __forceinline__ void finish(const double (&v)[NV], double (&o)[NOUT]) const {
+    o[0] = fma(StokesSum::kLog, v[0], v[2]) * (0.25 / M_PI);
+    o[1] = fma(StokesSum::kLog, v[1], v[3]) * (0.25 / M_PI);
+    o[2] = v[4] * (0.5 / M_PI);
+  }
+  __device__ __forceinline__ void store(int i, const double (&o)[NOUT]) const {
+#pragma unroll
+    for (int k = 0; k < NOUT; ++k) out[k * ld_out + i] = o[k];
+  }
+};
 
 StokesCircles circles(const StokesArgs &a) {
   StokesCircles c{};
@@ -336,11 +388,35 @@ void run_stokes_evaluate(const StokesArgs &a, const double *fx, const double *fy
   EvalItems it;
   eval_items(pa, tkeys, m, it, s);
   PhaseTimer timer(PH_EVAL, s);
-  auto ev = a.sgx ? k_stokes_evaluate<true> : k_stokes_evaluate<false>;
-  ev<<<work_grid(a.th->n_total() + m / TCH_ST + 1, 8), TCH_ST, 0, s>>>(
-      a.neq, a.np, circles(a), it.items.get(), it.n_items.get(), td.coll.get(), td.bot.get(),
-      td.top.get(), td.xmid.get(), td.ymid.get(), td.sx.get(), td.sy.get(), fx, fy, loc, txs, tys,
-      tperm, check, out, ld_out, a.sgx, a.sgy, a.dnx, a.dny);
+  const ItemArgs ia{it.items.get(), it.n_items.get(), it.n_items.get() + 1, td.coll.get(),
+                    td.bot.get(),   td.top.get(),     txs,                 tys, tperm};
+  auto launch = [&](auto pt, auto blocks) {
+    using Pol = typename decltype(pt)::type;
+    constexpr int B = decltype(blocks)::value;
+    Pol pol{};
+    pol.neq = a.neq;
+    pol.np = a.np;
+    pol.check = check;
+    pol.cir = circles(a);
+    pol.xmid = td.xmid.get();
+    pol.ymid = td.ymid.get();
+    pol.sx = td.sx.get();
+    pol.sy = td.sy.get();
+    pol.fx = fx;
+    pol.fy = fy;
+    pol.loc = loc;
+    pol.sgx = a.sgx;
+    pol.sgy = a.sgy;
+    pol.dnx = a.dnx;
+    pol.dny = a.dny;
+    pol.out = out;
+    pol.ld_out = ld_out;
+    k_items<Pol, B><<<work_grid(a.th->n_total() + m / EVAL_CHUNK + 1, B), EV_THREADS, 0, s>>>(pol, ia);
+  };
+  if (a.sgx)
+    launch(TypeOf<StokesPolicy<true>>{}, std::integral_constant<int, 4>{});
+  else
+    launch(TypeOf<StokesPolicy<false>>{}, std::integral_constant<int, 6>{});
   FMMB_CUDA(cudaGetLastError());
 }
 

@@ -89,3 +89,57 @@ def test_binned_targets_do_not_depend_on_their_place(built_lib, n):
         p = rng.permutation(n)
         got = F.target_evaluation(torch.from_numpy(tx[p]).cuda(), torch.from_numpy(ty[p]).cuda())
         assert np.array_equal(got.cpu().numpy(), ref[p])
+
+
+@pytest.mark.parametrize("n", SIZES)
+def test_one_leaf_black_box(built_lib, n):
+    import torch
+    from flexmm_b200.bbfmm import BB_FMM, BB_Helper
+    x, y, tau = _points(n, n + 50)
+    xd, yd = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+    F = BB_FMM(xd, yd, "Laplace_Eval", n, 4, bbox=[-1, 1, -1, 1], helper=BB_Helper())
+    F.register_evaluator(None, None, "gradient", 3)
+    F.build_expansions(torch.from_numpy(tau).cuda())
+    scale = np.abs(direct_laplace(x, y, np.abs(tau), x, y, check=True)) + np.abs(tau).sum()
+    _within(F.source_evaluation(xd, yd).cpu().numpy(), direct_laplace(x, y, tau, x, y, check=True),
+            scale, n)
+    want = np.asarray(direct_laplace_grad(x, y, tau, x, y, check=True))
+    r = np.hypot(x[:, None] - x, y[:, None] - y)
+    w = np.where(r > 0, 1 / np.where(r > 0, r, 1), 0.0)
+    got = F.evaluate_to_points(xd, yd, "gradient", True).cpu().numpy()
+    for k in range(3):
+        _within(got[k], want[k], (w * (1 + w * EPS) * np.abs(tau)).sum(1) + np.abs(tau).sum(), n)
+
+
+@pytest.mark.parametrize("dipoles", [False, True])
+@pytest.mark.parametrize("n", SIZES + [383, 384, 385])
+def test_one_leaf_stokes(built_lib, n, dipoles):
+    import torch
+    from flexmm_b200.stokes import FMM
+    from oracle.direct import direct_stokes, direct_stokes_dipole
+    x, y, fx = _points(n, n + 90)
+    rng = np.random.default_rng(n)
+    fy, gx, gy = (rng.standard_normal(n) for _ in range(3))
+    th = rng.uniform(0, 2 * np.pi, n)
+    nx, ny = np.cos(th), np.sin(th)
+    xd, yd = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+    F = FMM(xd, yd, 8, max(n, 1), [-1, 1, -1, 1])
+    c = lambda *a: [torch.from_numpy(v).cuda() for v in a]
+    if dipoles:
+        F.build_expansions_dipole(*c(fx, fy, gx, gy, nx, ny))
+        want = direct_stokes_dipole(x, y, fx, fy, gx, gy, nx, ny, x, y, True)
+    else:
+        F.build_expansions(*c(fx, fy))
+        want = direct_stokes(x, y, fx, fy, x, y, True)
+    got = [v.cpu().numpy() for v in F.evaluate_to_points(xd, yd, True)]
+    # a pair's terms are at most (|log r| + 1 + 1/r) |f| and, for stresslets,
+    # (4/r + 4/r^2) |sigma|, over 4 pi (u, v) and 2 pi (p): all within
+    # (2 + 1/r)|f| + (4/r + 4/r^2)|sigma|; the difference of two coordinates
+    # carries their rounding / r, up to four times over
+    r = np.hypot(x[:, None] - x, y[:, None] - y)
+    w = np.where(r > 0, 1 / np.where(r > 0, r, 1), 0.0)
+    s = (2 + w) * (1 + 4 * w * EPS) * (np.abs(fx) + np.abs(fy))
+    if dipoles:
+        s = s + (4 * w + 4 * w * w) * (1 + 4 * w * EPS) * (np.abs(gx) + np.abs(gy))
+    for k in range(3):
+        _within(got[k], want[k], s.sum(1), n)
