@@ -831,7 +831,7 @@ int fmm_stokes_ops_add(fmm_ops *ops, const fmm_stokes_level_ops *lv, int *level_
     };
     const size_t o_lx = take(neq), o_ly = take(neq);
     const size_t o_eu = take(sq), o_ev = take(sq), o_cu = take(sq), o_cv = take(sq);
-    const size_t o_mm = take(4 * sq), o_ll = take(4 * sq), o_cat = take(size_t(np) * ld);
+    const size_t o_mm = take(4 * sq), o_ll = take(4 * sq), o_m2l = take(size_t(np) * ld);
     for (int k = 0; k < neq; ++k) {
       h[o_lx + k] = lv->large_x[k];
       h[o_ly + k] = lv->large_y[k];
@@ -839,44 +839,62 @@ int fmm_stokes_ops_add(fmm_ops *ops, const fmm_stokes_level_ops *lv, int *level_
     // x = (b . U) . (diag(1/S) VH); the C2E solve drops the extra unknown (column n2)
     auto solve = [&](const double *u, const double *sinv, const double *vh, size_t ou, size_t ov,
                      bool drop_extra) {
-      for (int i = 0; i < n1; ++i)
-        for (int j = 0; j < n1; ++j) {
-          h[ou + size_t(i) * np + j] = u[size_t(i) * n1 + j];
-          if (!(drop_extra && j == n2)) h[ov + size_t(i) * np + j] = sinv[i] * vh[size_t(i) * n1 + j];
-        }
+      pack_fragments(np, np, [&](int i, int j) {
+        return i < n1 && j < n1 ? u[size_t(i) * n1 + j] : 0.0;
+      }, h.data() + ou);
+      pack_fragments(np, np, [&](int i, int j) {
+        return i < n1 && j < n1 && !(drop_extra && j == n2) ? sinv[i] * vh[size_t(i) * n1 + j] : 0.0;
+      }, h.data() + ov);
     };
     solve(lv->e2c_u, lv->e2c_sinv, lv->e2c_vh, o_eu, o_ev, false);
     solve(lv->c2e_u, lv->c2e_sinv, lv->c2e_vh, o_cu, o_cv, true);
-    for (int i = 0; i < n1; ++i)
-      for (int c = 0; c < 4; ++c)
-        for (int k = 0; k < n2; ++k) {
-          h[o_mm + size_t(c * np + k) * np + i] = lv->m2mc[size_t(i) * 4 * n2 + c * n2 + k];
-          h[o_ll + size_t(k) * 4 * np + c * np + i] = lv->l2lc[size_t(c * n1 + i) * n2 + k];
-        }
+    pack_fragments(4 * np, np, [&](int ck, int i) {
+      const int c = ck / np, k = ck % np;
+      return i < n1 && k < n2 ? lv->m2mc[size_t(i) * 4 * n2 + c * n2 + k] : 0.0;
+    }, h.data() + o_mm);
+    pack_fragments(np, 4 * np, [&](int k, int ci) {
+      const int c = ci / np, i = ci % np;
+      return i < n1 && k < n2 ? lv->l2lc[size_t(c * n1 + i) * n2 + k] : 0.0;
+    }, h.data() + o_ll);
+    const bool frag = np <= ST_M2L_NP;
+    auto e = std::make_unique<LevelEntry>();
+    e->dev = LevelOpsDev{};
+    std::vector<double> dense(sq);  // one operator, transposed [np x np]
     for (int o = 0; o < N_OFFSETS; ++o) {
       const int r = lv->m2l_rank[o];
       if (r == 0) continue;
       FMMB_CHECK(lv->m2l_a[o], ERR_INVALID_ARGUMENT, "missing M2L operator");
+      FMMB_CHECK(r < 0 || lv->m2l_b[o], ERR_INVALID_ARGUMENT, "bad M2L factors");
+      std::fill(dense.begin(), dense.end(), 0.0);
       for (int i = 0; i < n1; ++i)
         for (int k = 0; k < n2; ++k) {
           double v;
           if (r < 0) {
             v = lv->m2l_a[o][size_t(i) * n2 + k];
           } else {  // M2 [n1 x r] . M1 [r x n2], the reference's truncated operator
-            FMMB_CHECK(lv->m2l_b[o], ERR_INVALID_ARGUMENT, "bad M2L factors");
             v = 0.0;
             for (int q = 0; q < r; ++q) v += lv->m2l_a[o][size_t(i) * r + q] * lv->m2l_b[o][size_t(q) * n2 + k];
           }
-          h[o_cat + (size_t(o) * np + k) * np + i] = v;  // transposed [40 np x np]
+          dense[size_t(k) * np + i] = v;
         }
+      e->dev.kind[o] = M2L_DENSE;
+      if (frag)
+        pack_fragments(np, np, [&](int k, int i) { return dense[size_t(k) * np + i]; },
+                       h.data() + o_m2l + o * sq);
+      else
+        std::copy(dense.begin(), dense.end(), h.begin() + o_m2l + o * sq);
     }
-    auto e = std::make_unique<LevelEntry>();
     e->st.alloc(h.size(), 0);
     FMMB_CUDA(cudaMemcpy(e->st.get(), h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice));
     double *b = e->st.get();
-    e->st_lev = StokesArgs::Level{b + o_lx, b + o_ly, b + o_eu, b + o_ev, b + o_cu,
-                                  b + o_cv, b + o_mm, b + o_ll, b + o_cat};
+    auto f2 = [&](size_t o) { return reinterpret_cast<const double2 *>(b + o); };
+    e->st_lev = StokesArgs::Level{b + o_lx, b + o_ly, f2(o_eu), f2(o_ev), f2(o_cu), f2(o_cv),
+                                  f2(o_mm), f2(o_ll), b + o_m2l};
+    for (int o = 0; frag && o < N_OFFSETS; ++o)
+      if (e->dev.kind[o] != M2L_NULL) e->dev.m2l_f[o] = f2(o_m2l + o * sq);
     e->dev.inv_w = 1.0 / lv->width;
+    e->dev_copy.alloc(1, 0);
+    FMMB_CUDA(cudaMemcpy(e->dev_copy.get(), &e->dev, sizeof(LevelOpsDev), cudaMemcpyHostToDevice));
     ops->levels.push_back(std::move(e));
     *level_id = int(ops->levels.size()) - 1;
   });
@@ -1019,6 +1037,7 @@ static StokesArgs stokes_args(fmm_plan *p, cudaStream_t) {
   a.np = p->ops->np;
   a.td = &p->td;
   a.th = &p->th;
+  a.ops_dev = p->ops_dev.get();
   for (int m = 0; m < p->th.L && m < FMM_MAX_LEVELS_DEV; ++m)
     if (p->bound[m] >= 0) a.lev[m] = p->ops->levels[p->bound[m]]->st_lev;
   if (p->has_st_dipoles) {
@@ -1090,15 +1109,18 @@ static void build_stokes(fmm_plan *p, const double *fx, const double *fy, const 
       FMMB_CHECK(p->bound[m] >= 0, ERR_NOT_READY, "operators not bound for every level >= 2");
     const int np = p->ops->np;
     const int64_t total = th.n_total();
+    upload_level_ops(p, s);
     StokesArgs a = stokes_args(p, s);
     p->tau_s.alloc(th.n_points, s);
     p->tau2_s.alloc(th.n_points, s);
     gather_sorted(fx, p->td.ordv.get(), th.n_points, p->tau_s.get(), s);
     gather_sorted(fy, p->td.ordv.get(), th.n_points, p->tau2_s.get(), s);
+    ZeroBatch zb(s);
     for (DevBuf<double> *b : {&p->partial, &p->mult, &p->ple, &p->loc}) {
       b->alloc(total * np, s);
-      b->zero(s);
+      zb.add(*b);
     }
+    zb.run();
     run_stokes_upward(a, p->tau_s.get(), p->tau2_s.get(), p->partial.get(), p->mult.get(), s);
     run_stokes_downward(a, p->mult.get(), p->ple.get(), p->loc.get(), s);
     p->have_expansions = true;

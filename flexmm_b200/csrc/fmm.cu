@@ -419,7 +419,7 @@ struct M2LShape {
   static constexpr int np = 8 * NCB, ldp = np + 4;
   static constexpr bool kOpInRing = NCB <= 2;
   static constexpr int kStages = NCB <= 2 ? 4 : NCB <= 4 ? 3 : 2;
-  static constexpr int kTargets = NCB <= 4 ? 32 : 64;  // targets per tile
+  static constexpr int kTargets = NCB <= 4 || NCB > 8 ? 32 : 64;  // targets per tile
   static constexpr int kBlocks = NCB > 6 ? 2 : NCB > 4 ? 3 : NCB > 2 ? 6 : 8;  // resident per SM
   static __host__ __device__ size_t stage_doubles(int tt) {
     return (size_t)tt * ldp + (kOpInRing ? np * np : 0);
@@ -1242,7 +1242,7 @@ void run_m2l(const PassArgs &a, const double *mult, double *ple, cudaStream_t s,
   int64_t targets = 0;
   for (int m = 2; m < th.L; ++m) targets += 4 * (int64_t)(th.rg_hi[m] - th.rg_lo[m]);
   // few targets: smaller tiles, for more blocks and a shorter chain in each
-  const int tt = targets * n_rhs < M2L_FEW_TARGETS ? 16 : a.np <= 32 ? 32 : 64;
+  const int tt = targets * n_rhs < M2L_FEW_TARGETS ? 16 : a.np <= 32 || a.np > 64 ? 32 : 64;
   M2LTiles tl{};
   tl.n_levels = th.L;
   int tiles = 0;
@@ -1260,7 +1260,7 @@ void run_m2l(const PassArgs &a, const double *mult, double *ple, cudaStream_t s,
   auto launch = [&](auto ncb) {
     constexpr int NCB = decltype(ncb)::value;
     const size_t sm = M2LShape<NCB>::smem(tt);
-    static_assert(M2LShape<NCB>::kTargets == (NCB <= 4 ? 32 : 64), "tiles are counted for this size");
+    static_assert(M2LShape<NCB>::kTargets == (NCB <= 4 || NCB > 8 ? 32 : 64), "tiles are counted for this size");
     smem_limit(k_m2l<NCB>, M2LShape<NCB>::smem(M2LShape<NCB>::kTargets));
     k_m2l<NCB><<<dim3(tiles, n_rhs), 32 * NCB, sm, s>>>(tl, tt, a.td->rg.get(), a.td->il.get(),
                                                         a.ops_dev, mult, ple, cstride);
@@ -1275,6 +1275,7 @@ void run_m2l(const PassArgs &a, const double *mult, double *ple, cudaStream_t s,
     case 6: launch(std::integral_constant<int, 6>{}); break;
     case 7: launch(std::integral_constant<int, 7>{}); break;
     case 8: launch(std::integral_constant<int, 8>{}); break;
+    case 9: launch(std::integral_constant<int, 9>{}); break;  // Stokes, Nequiv 28-35
     default: throw Error(ERR_UNSUPPORTED, "unexpected operator size");
   }
 }

@@ -86,25 +86,30 @@ void run_bb_evaluate(const BBArgs &b, const double *tau_sorted, const double *lo
                      int64_t m, int check, int nout, double *out, int64_t ld_out, cudaStream_t s);
 
 // Stokes FMM (stokes.cu): rows of np = pad8(2 Neq + 1) doubles; per level
-// the large circle and the row-major operators of the GEMMs:
+// the large circle and the operators, in fragment order (gemm.cuh):
 //   e2c_u, e2c_vhs [np x np]: E2C solve x = (b . U) . (diag(1/S) VH);
 //   c2e_u, c2e_vhs [np x np]: C2E solve, the extra unknown's column zeroed;
-//   m2mc [4np x np]: parent check row = children rows . m2mc;
-//   l2lc [np x 4np]: children partial-local rows = local row . l2lc;
-//   m2l_cat [40np x np]: the 40 M2L operators stacked, each transposed.
+//   m2m [4np x np]: parent check row = children rows . m2m;
+//   l2l [np x 4np]: children partial-local rows = local row . l2l;
+// and the 40 M2L operators: as fragments in LevelOpsDev (np <= ST_M2L_NP), or
+// m2l_cat [40np x np], stacked, each transposed, row-major.
+constexpr int ST_M2L_NP = 72;  // largest rows the KIFMM's M2L kernel takes
 struct StokesArgs {
   int neq, np;
   const TreeDev *td;
   const TreeHost *th;
+  const LevelOpsDev *ops_dev;
   // double-layer (stresslet) sources: strengths (sigma) and normals, sorted;
   // null when the sources carry forces only (build_expansions_dipole,
   // stokes_fmm.py:738-826)
   const double *sgx = nullptr, *sgy = nullptr, *dnx = nullptr, *dny = nullptr;
   struct Level {
     const double *lx, *ly;
-    const double *e2c_u, *e2c_vhs, *c2e_u, *c2e_vhs, *m2mc, *l2lc, *m2l_cat;
+    const double2 *e2c_u, *e2c_vhs, *c2e_u, *c2e_vhs, *m2m, *l2l;
+    const double *m2l_cat;
   } lev[FMM_MAX_LEVELS_DEV];
 };
+// partial: check rows of the S2M nodes (zeroed); mult, loc zeroed
 void run_stokes_upward(const StokesArgs &a, const double *fx, const double *fy, double *partial,
                        double *mult, cudaStream_t s);
 void run_stokes_downward(const StokesArgs &a, const double *mult, double *ple, double *loc,

@@ -9,15 +9,18 @@
 //    kernel_add's pressure) + M2MC . children (extra unknowns excluded), then
 //    the factored-SVD solve of the corrected equivalent-to-check form
 //    (E2C_SVD, stokes_fmm.py:553-558);
-//  * downward: partial locals += L2LC . parent local (real sibling groups) and
-//    += M2L . source multipoles (the 40 offsets in one row-GEMM launch,
-//    tiles of one parity class skipping absent offsets), then the C2E solve,
-//    extra unknown dropped (stokes_fmm.py:712-733);
+//  * downward: M2L . source multipoles of all levels (the KIFMM's M2L kernel
+//    where a row fits it, np <= 72), then per level += L2LC . parent local
+//    (real sibling groups) and the C2E solve, extra unknown dropped
+//    (stokes_fmm.py:712-733);
 //  * evaluation: (u, v, p) from the leaf's local forces on the large circle
 //    (local_expansion_evaluation, stokes_fmm.py:331-360) plus the colleagues'
 //    sources (neighbor_evaluation, stokes_fmm.py:361-396).
-// Solves and translations are FP64 tensor-core row GEMMs (rowgemm.cuh) on
-// the plan's stream, gathers and scatters fused into their loads and stores.
+// A level is one launch each way: its translation and its solve, on the FP64
+// tensor cores, on tiles of 8 or 16 rows (k_st_up, k_st_down).  As row GEMMs
+// (three launches a level and direction, M2L level by level with 72 columns in
+// two tiles of 64) a batch of 12 problems, forward and adjoint, took 1,058
+// launches and 6.5 ms; 602 and 3.7 ms now.
 
 #include <algorithm>
 
@@ -296,13 +299,189 @@ StokesCircles circles(const StokesArgs &a) {
   return c;
 }
 
-// rows of x := ((b . U) . VHs), row-major np x np operators, n contiguous rows
-void solve_rows(const StokesArgs &a, const double *u, const double *vhs, const double *b, double *x,
-                double *tmp, int n, cudaStream_t s) {
-  const int np = a.np;
-  rowgemm(RowsContig{b, np, n, np}, StoreRows{tmp, np}, row_tiles(n), u, np, np, np, s);
-  rowgemm(RowsContig{tmp, np, n, np}, StoreRows{x, np}, row_tiles(n), vhs, np, np, np, s);
+// ---- level passes: a tile of 8 RB rows, warp w computing column block w ----
+constexpr int ST_AHEAD = 8;  // fragment pairs in flight per warp
+
+// acc[r] += A[8 r ..][.] . B over npairs k pairs of B's column block cb (of nb
+// in a k pair); A in shared memory, operator fragments from L2
+template <int RB>
+__device__ __forceinline__ void st_gemm(const double *A, int lda, const double2 *__restrict__ B,
+                                        int nb, int cb, int npairs, double (&acc)[RB][2]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const double2 *Bp = B + (size_t)cb * 32 + lane;
+  const double *Ap = A + g * lda + q;
+  double2 f[ST_AHEAD];
+#pragma unroll
+  for (int i = 0; i < ST_AHEAD; ++i)
+    if (i < npairs) f[i] = load_pair(Bp + (size_t)i * nb * 32);
+#pragma unroll
+  for (int r = 0; r < RB; ++r) acc[r][0] = acc[r][1] = 0.0;
+  for (int k0 = 0; k0 < npairs; k0 += ST_AHEAD) {
+#pragma unroll
+    for (int i = 0; i < ST_AHEAD; ++i) {
+      const int kp = k0 + i;
+      if (kp < npairs) {
+        const double2 b = f[i];
+        if (kp + ST_AHEAD < npairs) f[i] = load_pair(Bp + (size_t)(kp + ST_AHEAD) * nb * 32);
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+          const double *a = Ap + 8 * r * lda + 8 * kp;
+          dmma(acc[r], a[0], b.x);
+          dmma(acc[r], a[4], b.y);
+        }
+      }
+    }
+  }
 }
+
+// acc to (ADD: onto) shared rows out[8 RB][ldo], this warp's column block
+template <int RB, bool ADD>
+__device__ __forceinline__ void st_put(double *out, int ldo, int cb, const double (&acc)[RB][2]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+#pragma unroll
+  for (int r = 0; r < RB; ++r) {
+    double2 *o = reinterpret_cast<double2 *>(out + (8 * r + g) * ldo + 8 * cb + 2 * q);
+    double2 v = make_double2(acc[r][0], acc[r][1]);
+    if (ADD) {
+      const double2 w = *o;
+      v = make_double2(w.x + v.x, w.y + v.y);
+    }
+    *o = v;
+  }
+}
+
+// x = (P . U) . VHs of the tile's rows, row t to out_row[t] where that is not
+// null; T: scratch rows.  The caller synchronises before.
+template <int RB>
+__device__ __forceinline__ void st_solve(const double2 *U, const double2 *VHs, int np, const double *P,
+                                         double *T, double *const *out_row) {
+  const int ldp = pad_ld(np), ncb = np / 8, cb = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  double acc[RB][2];
+  st_gemm<RB>(P, ldp, U, ncb, cb, ncb, acc);
+  st_put<RB, false>(T, ldp, cb, acc);
+  __syncthreads();
+  st_gemm<RB>(T, ldp, VHs, ncb, cb, ncb, acc);
+#pragma unroll
+  for (int r = 0; r < RB; ++r) {
+    double *o = out_row[8 * r + g];
+    if (o) *reinterpret_cast<double2 *>(o + 8 * cb + 2 * q) = make_double2(acc[r][0], acc[r][1]);
+  }
+}
+
+struct StokesLevels {
+  const double2 *u[FMM_MAX_LEVELS_DEV], *vhs[FMM_MAX_LEVELS_DEV];
+};
+
+// E2C solve of the S2M nodes of all levels: partial check rows -> multipoles
+template <int RB>
+__global__ void k_st_leaves(StokesLevels ops, int np, int L, const int *__restrict__ off,
+                            const int *__restrict__ uplist, const int *__restrict__ n_up_ptr,
+                            const double *__restrict__ partial, double *__restrict__ mult) {
+  constexpr int ROWS = 8 * RB;
+  extern __shared__ __align__(16) double smem[];
+  __shared__ int node[ROWS], lev[ROWS];
+  __shared__ double *orow[ROWS];
+  const int ldp = pad_ld(np), n_up = *n_up_ptr, tid = threadIdx.x;
+  double *P = smem, *T = P + ROWS * ldp;
+  for (int i0 = ROWS * blockIdx.x; i0 < n_up; i0 += ROWS * gridDim.x) {
+    const int nloc = min(ROWS, n_up - i0);
+    __syncthreads();
+    if (tid < ROWS) {
+      const int g = tid < nloc ? uplist[i0 + tid] : -1;
+      node[tid] = g;
+      lev[tid] = g >= 0 ? node_level_of(off, L, g) : -1;
+    }
+    __syncthreads();
+    for (int i = tid; i < ROWS * (np / 2); i += blockDim.x) {
+      const int r = i / (np / 2), k = 2 * (i - r * (np / 2));
+      if (node[r] >= 0)
+        cp_async16(P + r * ldp + k, partial + (size_t)node[r] * np + k);
+      else
+        P[r * ldp + k] = P[r * ldp + k + 1] = 0.0;
+    }
+    cp_async_wait_all();
+    for (int m = lev[0]; m <= lev[nloc - 1]; ++m) {  // the list is level by level
+      __syncthreads();
+      if (tid < ROWS) orow[tid] = lev[tid] == m ? mult + (size_t)node[tid] * np : nullptr;
+      __syncthreads();
+      st_solve<RB>(ops.u[m], ops.vhs[m], np, P, T, orow);
+    }
+  }
+}
+
+// M2M and E2C solve of the parent boxes of one level; their children are the
+// contiguous node rows c_first + 4e .. c_first + 4e + 3
+template <int RB>
+__global__ void k_st_up(StokesArgs::Level op, int np, int c_first, int n_groups,
+                        const int *__restrict__ parent, double *mult) {
+  constexpr int ROWS = 8 * RB;
+  extern __shared__ __align__(16) double smem[];
+  __shared__ double *orow[ROWS];
+  const int ldp = pad_ld(np), lda = pad_ld(4 * np), ncb = np / 8, tid = threadIdx.x;
+  double *P = smem, *T = P + ROWS * ldp, *A = T + ROWS * ldp;
+  const int e0 = ROWS * blockIdx.x, nloc = min(ROWS, n_groups - e0);
+  if (tid < ROWS)
+    orow[tid] = tid < nloc ? mult + (size_t)parent[c_first + 4 * (e0 + tid)] * np : nullptr;
+  for (int i = tid + nloc * lda; i < ROWS * lda; i += blockDim.x) A[i] = 0.0;
+  pdl_wait();  // the children's multipoles come from the kernels before
+  pdl_trigger();
+  stage_rows(A, lda, mult + (size_t)(c_first + 4 * e0) * np, nloc, 4 * np);
+  cp_async_wait_all();
+  __syncthreads();
+  double acc[RB][2];
+  st_gemm<RB>(A, lda, op.m2m, ncb, tid >> 5, 4 * ncb, acc);
+  st_put<RB, false>(P, ldp, tid >> 5, acc);
+  __syncthreads();
+  st_solve<RB>(op.e2c_u, op.e2c_vhs, np, P, T, orow);
+}
+
+// Class c of 8 RB real sibling groups of one level: L2L from their parents
+// (l2l not null; stokes_fmm.py:726-733) onto the M2L partial locals, C2E solve
+template <int RB>
+__global__ void k_st_down(const double2 *c2e_u, const double2 *c2e_vhs, const double2 *l2l, int np,
+                          int rg_lo, int rg_cnt, const int *__restrict__ rg,
+                          const int *__restrict__ parent, const double *__restrict__ ple,
+                          double *loc) {
+  constexpr int ROWS = 8 * RB;
+  extern __shared__ __align__(16) double smem[];
+  __shared__ int node[ROWS], par[ROWS];
+  __shared__ double *orow[ROWS];
+  const int ldp = pad_ld(np), ncb = np / 8, tid = threadIdx.x, cb = tid >> 5;
+  double *P = smem, *T = P + ROWS * ldp, *Lp = T + ROWS * ldp;
+  const int q0 = ROWS * (blockIdx.x >> 2), c = blockIdx.x & 3, ngrp = min(ROWS, rg_cnt - q0);
+  if (tid < ROWS) {
+    const int n = tid < ngrp ? rg[rg_lo + q0 + tid] + c : -1;
+    node[tid] = n;
+    par[tid] = n >= 0 ? parent[n] : -1;
+    orow[tid] = n >= 0 ? loc + (size_t)n * np : nullptr;
+  }
+  __syncthreads();
+  pdl_wait();  // partial locals (M2L) and the parents' locals come from the kernels before
+  pdl_trigger();
+  for (int i = tid; i < ROWS * (np / 2); i += blockDim.x) {
+    const int r = i / (np / 2), k = 2 * (i - r * (np / 2));
+    if (node[r] >= 0) {
+      cp_async16(P + r * ldp + k, ple + (size_t)node[r] * np + k);
+      if (l2l) cp_async16(Lp + r * ldp + k, loc + (size_t)par[r] * np + k);
+    } else {
+      P[r * ldp + k] = P[r * ldp + k + 1] = 0.0;
+      Lp[r * ldp + k] = Lp[r * ldp + k + 1] = 0.0;
+    }
+  }
+  cp_async_wait_all();
+  __syncthreads();
+  if (l2l) {
+    double acc[RB][2];
+    st_gemm<RB>(Lp, ldp, l2l, 4 * ncb, c * ncb + cb, ncb, acc);
+    st_put<RB, true>(P, ldp, cb, acc);
+    __syncthreads();
+  }
+  st_solve<RB>(c2e_u, c2e_vhs, np, P, T, orow);
+}
+
+// two row blocks where one each would fill the SMs more than twice over
+int st_rows(int units) { return units > 2 * 148 ? 2 : 1; }
 
 }  // namespace
 
@@ -312,7 +491,7 @@ void run_stokes_upward(const StokesArgs &a, const double *fx, const double *fy, 
   const TreeDev &td = *a.td;
   if (th.L < 3) return;
   FMMB_CHECK(th.L <= FMM_MAX_LEVELS_DEV, ERR_INVALID_ARGUMENT, "too many levels");
-  const int np = a.np;
+  const int np = a.np, nthr = 4 * np;  // a warp per column block
   PhaseTimer timer(PH_UPWARD, s);
   auto s2m = a.sgx ? k_stokes_s2m<true> : k_stokes_s2m<false>;
   s2m<<<work_grid(th.n_total(), 8), 128, 0, s>>>(a.neq, np, th.L, circles(a), td.dev_off.get(),
@@ -321,23 +500,25 @@ void run_stokes_upward(const StokesArgs &a, const double *fx, const double *fy, 
                                                  td.sx.get(), td.sy.get(), fx, fy, partial, a.sgx,
                                                  a.sgy, a.dnx, a.dny);
   FMMB_CUDA(cudaGetLastError());
-  int max_rows = 0;
-  for (int m = 2; m < th.L; ++m) max_rows = std::max(max_rows, th.off[m + 1] - th.off[m]);
-  DevBuf<double> tmp;
-  tmp.alloc((size_t)max_rows * np, s);
-  for (int m = th.L - 1; m >= 2; --m) {
-    if (m <= th.L - 2) {  // partial of level m's parents = children . M2MC
-      const int c_first = th.off[m + 1];
-      const int n_groups = (th.off[m + 2] - th.off[m + 1]) / 4;
-      if (n_groups > 0)
-        rowgemm(RowsContig{mult + (size_t)c_first * np, 4 * (int64_t)np, n_groups, 4 * np},
-                StoreParents{td.parent.get(), partial, c_first, np}, row_tiles(n_groups),
-                a.lev[m].m2mc, np, np, 4 * np, s);
-    }
-    const int r0 = th.off[m], n = th.off[m + 1] - th.off[m];
-    if (n > 0)
-      solve_rows(a, a.lev[m].e2c_u, a.lev[m].e2c_vhs, partial + (size_t)r0 * np,
-                 mult + (size_t)r0 * np, tmp.get(), n, s);
+  StokesLevels ops{};
+  for (int m = 0; m < th.L; ++m) {
+    ops.u[m] = a.lev[m].e2c_u;
+    ops.vhs[m] = a.lev[m].e2c_vhs;
+  }
+  const size_t leaf_bytes = sizeof(double) * 32 * pad_ld(np);
+  smem_limit(k_st_leaves<2>, leaf_bytes);
+  k_st_leaves<2><<<work_grid((th.n_total() + 15) / 16, 4), nthr, leaf_bytes, s>>>(
+      ops, np, th.L, td.dev_off.get(), td.uplist.get(), td.n_up.get(), partial, mult);
+  FMMB_CUDA(cudaGetLastError());
+  for (int m = th.L - 2; m >= 2; --m) {
+    const int c_first = th.off[m + 1], n_groups = (th.off[m + 2] - th.off[m + 1]) / 4;
+    if (n_groups == 0) continue;
+    const int rb = st_rows((n_groups + 7) / 8);
+    const size_t bytes = sizeof(double) * 8 * rb * (2 * pad_ld(np) + pad_ld(4 * np));
+    auto kern = rb == 1 ? k_st_up<1> : k_st_up<2>;
+    smem_limit(kern, bytes);
+    launch_pdl(kern, dim3((n_groups + 8 * rb - 1) / (8 * rb)), dim3(nthr), bytes, s, a.lev[m], np,
+               c_first, n_groups, td.parent.get(), mult);
   }
 }
 
@@ -346,33 +527,35 @@ void run_stokes_downward(const StokesArgs &a, const double *mult, double *ple, d
   const TreeHost &th = *a.th;
   const TreeDev &td = *a.td;
   if (th.L < 3) return;
-  const int np = a.np;
-  int max_groups = 0, max_rows = 0;
-  for (int m = 2; m < th.L; ++m) {
-    max_groups = std::max(max_groups, th.rg_hi[m] - th.rg_lo[m]);
-    max_rows = std::max(max_rows, th.off[m + 1] - th.off[m]);
-  }
-  DevBuf<double> tmp;
-  tmp.alloc((size_t)std::max(max_rows, 1) * np, s);
-  for (int m = 2; m < th.L; ++m) {
-    const int lo = th.rg_lo[m], n_groups = th.rg_hi[m] - th.rg_lo[m];
-    if (n_groups > 0) {
-      if (m >= 3) {  // L2L from level m-1 (stokes_fmm.py:726-733)
-        PhaseTimer timer(PH_DOWNWARD, s);
-        rowgemm(ParentRows{td.rg.get(), td.parent.get(), loc, lo, n_groups, np},
-                AddChildRows{td.rg.get(), ple, lo, np}, row_tiles(n_groups), a.lev[m - 1].l2lc,
-                4 * np, 4 * np, np, s);
-      }
-      // M2L: tiles of one parity class, absent offsets skipped
-      PhaseTimer timer(PH_M2L, s);
+  const int np = a.np, nthr = 4 * np;
+  if (np <= ST_M2L_NP) {
+    PassArgs pa{};
+    pa.np = np;
+    pa.td = a.td;
+    pa.th = a.th;
+    pa.ops_dev = a.ops_dev;
+    run_m2l(pa, mult, ple, s);
+  } else {  // tiles of one parity class, absent offsets skipped
+    PhaseTimer timer(PH_M2L, s);
+    for (int m = 2; m < th.L; ++m) {
+      const int lo = th.rg_lo[m], n_groups = th.rg_hi[m] - th.rg_lo[m];
+      if (n_groups <= 0) continue;
       const int tpc = row_tiles(n_groups);
       rowgemm(M2LRows{td.rg.get(), td.il.get(), mult, lo, n_groups, np, tpc},
               AddGroupRows{td.rg.get(), ple, lo, np}, 4 * tpc, a.lev[m].m2l_cat, np, np, np, s);
     }
-    const int r0 = th.off[m], nr = th.off[m + 1] - th.off[m];
-    if (nr > 0)
-      solve_rows(a, a.lev[m].c2e_u, a.lev[m].c2e_vhs, ple + (size_t)r0 * np, loc + (size_t)r0 * np,
-                 tmp.get(), nr, s);
+  }
+  for (int m = 2; m < th.L; ++m) {
+    const int lo = th.rg_lo[m], n_groups = th.rg_hi[m] - th.rg_lo[m];
+    if (n_groups <= 0) continue;
+    PhaseTimer timer(PH_DOWNWARD, s);
+    const int rb = st_rows(4 * ((n_groups + 7) / 8));
+    const size_t bytes = sizeof(double) * 8 * rb * 3 * pad_ld(np);
+    auto kern = rb == 1 ? k_st_down<1> : k_st_down<2>;
+    smem_limit(kern, bytes);
+    launch_pdl(kern, dim3(4 * ((n_groups + 8 * rb - 1) / (8 * rb))), dim3(nthr), bytes, s,
+               a.lev[m].c2e_u, a.lev[m].c2e_vhs, m >= 3 ? a.lev[m - 1].l2l : nullptr, np, lo,
+               n_groups, td.rg.get(), td.parent.get(), ple, loc);
   }
 }
 

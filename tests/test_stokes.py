@@ -100,3 +100,24 @@ def test_stresslets_match_reference(built_lib, case):
     for r in range(3):
         assert rel_l2(us[r], g["src_val"][r]) < 1e-11, ("src", r)
         assert rel_l2(ut[r], g["tgt_val"][r]) < 1e-11, ("tgt", r)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("neq", [20, 28, 35, 36, 48])
+def test_stokes_operator_sizes(built_lib, neq):
+    """Operator rows of 48 to 104: the KIFMM's M2L kernel up to 72 (Nequiv 35),
+    row GEMMs above, the level tiles at each.  Against the direct sum; bars a
+    decade above the errors recorded for the reference at Nequiv 16 and 32
+    (1e-2, 1e-5), which larger operators only improve on."""
+    from flexmm_b200.stokes import FMM
+    from oracle.direct import direct_stokes
+    rng = np.random.default_rng(neq)
+    n = 5000
+    x, y, fx, fy = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n), rng.standard_normal(n), rng.standard_normal(n)
+    F = FMM(x, y, neq, 20, [-1, 1, -1, 1])
+    F.build_expansions(fx, fy)
+    got = F.evaluate_to_points(x, y, True)
+    want = direct_stokes(x, y, fx, fy, x, y, True)
+    bar = 1e-4 if neq >= 32 else 1e-1
+    for a, b in zip(got, want):
+        assert np.linalg.norm(a - b) < bar * np.linalg.norm(b)
