@@ -152,6 +152,9 @@ __device__ __forceinline__ int node_level(const int *__restrict__ off, int L, in
   return lo;
 }
 
+// a box's width from its large circle's radius w (4 - sqrt 2) / 2
+__device__ __forceinline__ float box_of_circle(float r) { return r * (2.f / (4.f - 1.41421356f)); }
+
 // S2M + C2E of every S2M node (leaves holding points) of every level, in one
 // launch (flexmm/flexmm2d/kifmm.py:96-105 then fmm.py:86-90).  A tile is TN
 // consecutive entries of the level-major node list; C2E runs once for each
@@ -205,6 +208,19 @@ __global__ void __launch_bounds__(NT) k_s2m_mx(KernelParams kp, int neq, int np,
       const float lx0 = lane < neq ? op.lx32[lane] : 0.f, ly0 = lane < neq ? op.ly32[lane] : 0.f;
       const float lx1 = lane + 32 < neq ? op.lx32[lane + 32] : 0.f;
       const float ly1 = lane + 32 < neq ? op.ly32[lane + 32] : 0.f;
+      // a box's points lie within half a width of its centre, its circle's
+      // within the circle's radius
+      bool near = false;
+      if constexpr (KF32::kNearForm) {
+        const float rc = op.lx32[0], h = rc + 0.51f * box_of_circle(rc);
+        near = K.near_all(h, h);
+      }
+      auto value = [&](float dx, float dy, bool nr) -> float {
+        if constexpr (KF32::kNearForm) {
+          if (nr) return K.radial_near(dx * dx + dy * dy) * KF32::kScale;
+        }
+        return K(dx, dy);
+      };
       for (int j0 = b; j0 < e; j0 += 32) {
         const int nj = min(32, e - j0);
         if (lane < nj) {
@@ -213,10 +229,16 @@ __global__ void __launch_bounds__(NT) k_s2m_mx(KernelParams kp, int neq, int np,
           srct[warp][lane] = (float)tau[j0 + lane];
         }
         __syncwarp();
-        if (lane < neq)
-          for (int j = 0; j < nj; ++j) acc0 = fmaf(K(lx0 - srcx[warp][j], ly0 - srcy[warp][j]), srct[warp][j], acc0);
-        if (lane + 32 < neq)
-          for (int j = 0; j < nj; ++j) acc1 = fmaf(K(lx1 - srcx[warp][j], ly1 - srcy[warp][j]), srct[warp][j], acc1);
+        auto sums = [&](bool nr) {
+          if (lane < neq)
+            for (int j = 0; j < nj; ++j) acc0 = fmaf(value(lx0 - srcx[warp][j], ly0 - srcy[warp][j], nr), srct[warp][j], acc0);
+          if (lane + 32 < neq)
+            for (int j = 0; j < nj; ++j) acc1 = fmaf(value(lx1 - srcx[warp][j], ly1 - srcy[warp][j], nr), srct[warp][j], acc1);
+        };
+        if (near)
+          sums(true);
+        else
+          sums(false);
         __syncwarp();
       }
       const double c0 = op.kofs * tsum[g];  // kernel offset times the box's charge, FP64
@@ -941,18 +963,44 @@ __global__ void __launch_bounds__(TCH, NOUT == 1 ? EvalOcc<KF32>::blocks : 6)
     const float tx = (float)txd, ty = (float)tyd;
     const float tx_lo = (float)(txd - (double)tx), ty_lo = (float)(tyd - (double)ty);
     double acc = 0.0, accx = 0.0, accy = 0.0;  // accx, accy: kScale * (dx, dy) / d2 sums
+    // whether every source of the item (in the leaf's colleagues: within 1.5
+    // widths of its centre, as its circle is) is at a distance of the near form
+    bool near_form = false;
+    if constexpr (KF32::kNearForm) {
+      const float h = 1.501f * box_of_circle(ops[lev].lx32[0]);
+      near_form = K.near_all(fabsf(tx) + h, fabsf(ty) + h);
+    }
+    auto rad = [&](float d2, bool nr) -> float {
+      if constexpr (KF32::kNearForm) {
+        if (nr) return K.radial_near(d2);
+      }
+      return K.radial(d2);
+    };
     if (lev >= 2 && valid && PART != EVAL_NEAR) {  // L2T (flexmm/flexmm2d/kifmm.py:106-120), operands through L1
       const float *Lg = loc32 + (size_t)g * np;
       const float *lx = ops[lev].lx32, *ly = ops[lev].ly32;
       if constexpr (NOUT == 1) {
-        float p0 = 0.f, p1 = 0.f;
-        int k = sub;
-        for (; k + G < neq; k += 2 * G) {
-          p0 = fmaf(K(tx - __ldg(lx + k), ty - __ldg(ly + k)), __ldg(Lg + k), p0);
-          p1 = fmaf(K(tx - __ldg(lx + k + G), ty - __ldg(ly + k + G)), __ldg(Lg + k + G), p1);
-        }
-        if (k < neq) p0 = fmaf(K(tx - __ldg(lx + k), ty - __ldg(ly + k)), __ldg(Lg + k), p0);
-        acc = (double)p0 + (double)p1;
+        auto l2t = [&](bool nr) {
+          auto at = [&](int k) -> float {
+            const float dx = tx - __ldg(lx + k), dy = ty - __ldg(ly + k);
+            if constexpr (KF32::kNearForm) {
+              if (nr) return K.radial_near(dx * dx + dy * dy) * KF32::kScale;
+            }
+            return K(dx, dy);
+          };
+          float p0 = 0.f, p1 = 0.f;
+          int k = sub;
+          for (; k + G < neq; k += 2 * G) {
+            p0 = fmaf(at(k), __ldg(Lg + k), p0);
+            p1 = fmaf(at(k + G), __ldg(Lg + k + G), p1);
+          }
+          if (k < neq) p0 = fmaf(at(k), __ldg(Lg + k), p0);
+          acc = (double)p0 + (double)p1;
+        };
+        if (near_form)
+          l2t(true);
+        else
+          l2t(false);
       } else {
         float p0 = 0.f, px = 0.f, py = 0.f;
         for (int k = sub; k < neq; k += G) {
@@ -1036,10 +1084,11 @@ __global__ void __launch_bounds__(TCH, NOUT == 1 ? EvalOcc<KF32>::blocks : 6)
         const double acc0 = acc, accx0 = accx, accy0 = accy;
         if (fast) {
           if constexpr (NOUT == 1) {
+            auto fast_sweep = [&](bool nr) {
             float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
             auto pair = [&](const float4 q, float &p) {
               const float dx = tx - q.x, dy = ty - q.y;
-              p = fmaf(K.radial(fmaf(dy, dy, dx * dx)), q.z, p);
+              p = fmaf(rad(fmaf(dy, dy, dx * dx), nr), q.z, p);
             };
             auto flush = [&] {
               acc += ((double)p0 + (double)p1) + ((double)p2 + (double)p3);
@@ -1081,6 +1130,11 @@ __global__ void __launch_bounds__(TCH, NOUT == 1 ? EvalOcc<KF32>::blocks : 6)
             } else {
               sweep(0, nb);
             }
+            };
+            if (near_form)
+              fast_sweep(true);
+            else
+              fast_sweep(false);
           } else {
             float p[2] = {0.f, 0.f}, px[2] = {0.f, 0.f}, py[2] = {0.f, 0.f};
             auto pair = [&](int jj, int a) {

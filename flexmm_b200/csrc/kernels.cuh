@@ -311,6 +311,7 @@ __device__ __forceinline__ float lg2_ftz(float x) {
 // apart in FP64).
 struct LaplaceF32 {
   static constexpr bool kScaled = true;
+  static constexpr bool kNearForm = false;
   // radial(d2) is -inf for d2 below FLT_MIN (the flushed log2 of 0)
   static constexpr bool kInfAtZero = true;
   static constexpr float kScale = (float)(-0.69314718055994531 / (4.0 * M_PI));  // -ln2 / (4 pi)
@@ -335,7 +336,9 @@ struct LaplaceF32 {
 //   x > 2:  K0(x) = exp(-x) / sqrt(x) R(2/x) (relative error < 1.9e-7).
 // Both branches are computed and one selected (no divergence within a warp
 // of pairs at mixed distances).  K0(0) = +inf (the flushed log of 0).
-__device__ __forceinline__ float bessel_k0_f32(float x) {
+// bessel_k0_f32_small is the x <= 2 branch alone, for sweeps whose distances
+// are known to lie there (the same bits at 24 instructions for 40).
+__device__ __forceinline__ float bessel_k0_f32_small(float x) {
   const float y = (x * (1.f / 3.75f)) * (x * (1.f / 3.75f));
   const float i0 = fmaf(y, fmaf(y, fmaf(y, fmaf(y, fmaf(y, fmaf(y, 0.0045813f, 0.0360768f), 0.2659732f),
                                                    1.2067492f), 3.0899424f), 3.5156229f), 1.f);
@@ -343,7 +346,10 @@ __device__ __forceinline__ float bessel_k0_f32(float x) {
   const float p = fmaf(t2, fmaf(t2, fmaf(t2, fmaf(t2, fmaf(t2, fmaf(t2, 0.0000074f, 0.0001075f), 0.00262698f),
                                                    0.0348859f), 0.23069756f), 0.4227842f), -0.57721566f);
   // -ln(x/2) = (1 - log2 x) ln 2
-  const float small = fmaf((1.f - lg2_ftz(x)) * 0.69314718f, i0, p);
+  return fmaf((1.f - lg2_ftz(x)) * 0.69314718f, i0, p);
+}
+__device__ __forceinline__ float bessel_k0_f32(float x) {
+  const float small = bessel_k0_f32_small(x);
   const float z = 2.f * __frcp_rn(fmaxf(x, 2.f));
   const float r = fmaf(z, fmaf(z, fmaf(z, fmaf(z, fmaf(z, fmaf(z, 0.00053208f, -0.0025154f), 0.00587872f),
                                                   -0.01062446f), 0.02189568f), -0.07832358f), 1.25331414f);
@@ -358,6 +364,7 @@ __device__ __forceinline__ float bessel_k0_f32(float x) {
 // kernel on width-scaled coordinates.
 struct ModHelmholtzF32 {
   static constexpr bool kScaled = false;
+  static constexpr bool kNearForm = true;  // radial_near
   // radial(d2) is +inf for d2 below FLT_MIN (K0 at a flushed 0)
   static constexpr bool kInfAtZero = true;
   static constexpr float kScale = (float)(1.0 / (2.0 * M_PI));
@@ -366,6 +373,14 @@ struct ModHelmholtzF32 {
   // (squared distances below FLT_MIN flushed to 0: K0 = +inf there)
   __device__ __forceinline__ float radial(float d2) const {
     return bessel_k0_f32(k * (d2 < FLT_MIN ? 0.f : sqrtf(d2)));
+  }
+  // radial() of distances with k r <= 2, which near_all() promises of every
+  // point within (hx, hy) of this one: the rounded products stay below 2
+  __device__ __forceinline__ float radial_near(float d2) const {
+    return bessel_k0_f32_small(k * (d2 < FLT_MIN ? 0.f : sqrtf(d2)));
+  }
+  __device__ __forceinline__ bool near_all(float hx, float hy) const {
+    return k * sqrtf(hx * hx + hy * hy) <= 1.9999f;
   }
   // (dx, dy) = target - source
   __device__ __forceinline__ float operator()(float dx, float dy) const {
