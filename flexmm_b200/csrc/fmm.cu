@@ -35,7 +35,6 @@
 namespace fmmb {
 namespace {
 
-constexpr int TN = 32;      // nodes per upward / downward tile
 constexpr int NT = 256;     // threads per tile CTA
 constexpr int TCH = EVAL_CHUNK;  // targets per evaluation work item
 
@@ -76,127 +75,162 @@ __device__ __forceinline__ int level_of_node(const int *__restrict__ off, int L,
   return lo;
 }
 
-// kernel value at the difference (ax, ay) = target - source; raw log2 for
-// the table-driven Laplace functor (its factor folded into the charges)
-template <class KF>
-__device__ __forceinline__ double kernel_at(const KF &K, double ax, double ay) {
-  if constexpr (KF::kLogTable)
-    return K.raw(ax, ay);
-  else
-    return K(0.0, 0.0, ax, ay);
-}
+// S2M of every S2M node (leaves holding points, levels >= 2) of every level in
+// one launch (flexmm/flexmm2d/kifmm.py:96-105): a warp sums one node's sources
+// into its check potentials, written into the node's multipole row; the
+// check-to-equivalent solve follows in place (k_c2e_leaves), apart from it so
+// that a block needs no room for operators here and many warps hide the loads.
+// The lanes are check points, two each where there are more than 48, one each
+// for the first 32 and G lanes each for up to 16 more; the sweep is the
+// evaluation's (sweep.cuh).  Bound by the FP64 pipe, with the log table's reads.
+// 1M clustered points, Nequiv 60: 120 us and 58 for the solve, where one kernel
+// of 32-node tiles took 250; 250k points on rings, Nequiv 40: 28 + 14 after 64.
+constexpr int S2M_WARPS = 4, S2M_CHUNK = 64;  // sources staged per warp
 
-// S2M + C2E of every S2M node (leaves holding points, levels >= 2) of every
-// level in one launch (flexmm/flexmm2d/kifmm.py:96-105, then fmm.py:86-90):
-// a tile is TN consecutive entries of the level-major S2M node list, a warp
-// sums one node's sources into its check potentials (lanes over check
-// points, the node's sources staged 32 at a time, four independent sums
-// per lane); C2E runs once for each level the tile holds.
-template <class KF, bool DIP = false>
-__global__ void __launch_bounds__(NT, 3) k_s2m(KernelParams kp, int neq, int np, int L,
-                                            const int *__restrict__ off,
-                                            const int *__restrict__ uplist,
-                                            const int *__restrict__ n_up_ptr,
-                                            const int *__restrict__ bot,
-                                            const int *__restrict__ top,
-                                            const double *__restrict__ xmid,
-                                            const double *__restrict__ ymid,
-                                            const double *__restrict__ sx,
-                                            const double *__restrict__ sy,
-                                            const double *__restrict__ tau,
-                                            const LevelOpsDev *__restrict__ ops,
-                                            double *__restrict__ mult,
-                                            const double *__restrict__ dvx = nullptr,
-                                            const double *__restrict__ dvy = nullptr,
-                                            int64_t tstride = 0, int64_t cstride = 0) {
-  // charge column blockIdx.y (multi-RHS: column strides tstride / cstride)
-  tau += blockIdx.y * tstride;
-  mult += blockIdx.y * cstride;
-  extern __shared__ __align__(16) double smem[];
-  const int ldp = pad_ld(np);
-  double *P = smem;          // [TN][ldp] check potentials
-  double *T = P + TN * ldp;  // [TN][ldp] C2E scratch
-  __shared__ __align__(16) double part[FG_PART];
-  __shared__ double srcx[NT / 32][32], srcy[NT / 32][32], srct[NT / 32][32];
-  __shared__ double srcdx[DIP ? NT / 32 : 1][32], srcdy[DIP ? NT / 32 : 1][32];
-  __shared__ int node[TN], nlev[TN];
-  __shared__ double *orow[TN];
+template <class KF, bool DIP>
+__global__ void __launch_bounds__(32 * S2M_WARPS, 8)
+    k_s2m(KernelParams kp, int neq, int np, int L, const int *__restrict__ off,
+          const int *__restrict__ uplist, const int *__restrict__ n_up_ptr,
+          const int *__restrict__ bot, const int *__restrict__ top,
+          const double *__restrict__ xmid, const double *__restrict__ ymid,
+          const double *__restrict__ sx, const double *__restrict__ sy,
+          const double *__restrict__ tau, const LevelOpsDev *__restrict__ ops,
+          double *__restrict__ mult, const double *__restrict__ dvx,
+          const double *__restrict__ dvy) {
+  __shared__ double2 s_xy[S2M_WARPS][S2M_CHUNK], s_dv[DIP ? S2M_WARPS : 1][S2M_CHUNK];
+  __shared__ double s_q[S2M_WARPS][S2M_CHUNK];
   __shared__ FunctorSmem<KF> fsm;
   KF K(kp);
   fsm.bind(K);
   const double fold = fold_of<KF, KF::kLogTable>();
   const int n_up = *n_up_ptr;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int tile = blockIdx.x; tile * TN < n_up; tile += gridDim.x) {
-    const int i0 = tile * TN, nloc = min(TN, n_up - i0);
-    for (int i = threadIdx.x; i < TN * ldp; i += NT) P[i] = 0.0;
-    if (threadIdx.x < TN) {
-      const int g = (int)threadIdx.x < nloc ? uplist[i0 + threadIdx.x] : -1;
-      node[threadIdx.x] = g;
-      nlev[threadIdx.x] = g >= 0 ? level_of_node(off, L, g) : -1;
+  for (int i = blockIdx.x * S2M_WARPS + warp; i < n_up; i += gridDim.x * S2M_WARPS) {
+    const int node = uplist[i];
+    const LevelOpsDev &op = ops[level_of_node(off, L, node)];
+    const int b = bot[node], e = top[node];
+    const double cx = xmid[node], cy = ymid[node];
+    double *row = mult + (size_t)node * np;
+    int staged = -1;
+    auto points = [&](auto rc, int k0, int G) {  // R tiles of check points from k0 on
+      constexpr int R = decltype(rc)::value;
+      const int sub = lane & (G - 1), k = k0 + lane / G;
+      double x[R], y[R], v[R][2];
+      long long none[R] = {};
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        x[r] = op.lx[min(k + 32 * r, neq - 1)];
+        y[r] = op.ly[min(k + 32 * r, neq - 1)];
+        v[r][0] = v[r][1] = 0.0;
+      }
+      for (int j0 = b; j0 < e; j0 += S2M_CHUNK) {
+        const int nj = min(S2M_CHUNK, e - j0);
+        if (staged != j0) {
+          __syncwarp();
+          for (int j = lane; j < nj; j += 32) {
+            s_xy[warp][j] = make_double2(sx[j0 + j] - cx, sy[j0 + j] - cy);
+            s_q[warp][j] = tau[j0 + j] * fold;
+            if constexpr (DIP) s_dv[warp][j] = make_double2(dvx[j0 + j], dvy[j0 + j]);
+          }
+          __syncwarp();
+          staged = j0;
+        }
+        pot_sweep<KF, R, DIP, false>(K, s_xy[warp], s_q[warp], s_dv[DIP ? warp : 0], nullptr, x, y,
+                                     none, sub, nj, G, 0, v);
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        double o = v[r][0] + v[r][1];
+        if (R == 1)
+          for (int w = G >> 1; w >= 1; w >>= 1) o += __shfl_xor_sync(0xffffffffu, o, w);
+        if (sub == 0 && k + 32 * r < neq) row[k + 32 * r] = o;
+      }
+    };
+    if (neq + lane < np) row[neq + lane] = 0.0;  // (np - neq < 8)
+    using One = std::integral_constant<int, 1>;
+    if (neq > 48) {
+      points(std::integral_constant<int, 2>{}, 0, 1);
+    } else {
+      int k = 0;
+      if (neq >= 32) {
+        points(One{}, 0, 1);
+        k = 32;
+      }
+      if (k < neq) {
+        int G = 1;
+        while (2 * G * (neq - k) <= 32) G *= 2;
+        points(One{}, k, G);
+      }
     }
-    __syncthreads();
-    const int mlo = nlev[0], mhi = nlev[nloc - 1];
-    for (int t = warp; t < nloc; t += NT / 32) {
-      const int g = node[t];
-      const LevelOpsDev &op = ops[nlev[t]];
-      const int b = bot[g], e = top[g];
-      const double cx = xmid[g], cy = ymid[g];
-      const bool k0 = lane < neq, k1 = lane + 32 < neq;
-      const double lx0 = k0 ? op.lx[lane] : 0.0, ly0 = k0 ? op.ly[lane] : 0.0;
-      const double lx1 = k1 ? op.lx[lane + 32] : 0.0, ly1 = k1 ? op.ly[lane + 32] : 0.0;
-      double a0 = 0.0, b0 = 0.0, a1 = 0.0, b1 = 0.0;
+  }
+}
+
+// The same for up to S2M_COLS charge columns at a time (column group
+// blockIdx.y): each kernel value is computed once for all of them.  16 columns
+// at 60k points on a ring, K0: 72 us, and 510 us a column at a time.
+constexpr int S2M_COLS = 8;
+template <class KF>
+__global__ void __launch_bounds__(32 * S2M_WARPS, 6)
+    k_s2m_multi(KernelParams kp, int neq, int np, int L, const int *__restrict__ off,
+                const int *__restrict__ uplist, const int *__restrict__ n_up_ptr,
+                const int *__restrict__ bot, const int *__restrict__ top,
+                const double *__restrict__ xmid, const double *__restrict__ ymid,
+                const double *__restrict__ sx, const double *__restrict__ sy,
+                const double *__restrict__ tau, const LevelOpsDev *__restrict__ ops,
+                double *__restrict__ mult, int n_rhs, int64_t tstride, int64_t cstride) {
+  __shared__ double2 s_xy[S2M_WARPS][32];
+  __shared__ double s_q[S2M_WARPS][32][S2M_COLS];
+  __shared__ FunctorSmem<KF> fsm;
+  KF K(kp);
+  fsm.bind(K);
+  const double fold = fold_of<KF, KF::kLogTable>();
+  const int c0 = S2M_COLS * blockIdx.y, ncol = min(S2M_COLS, n_rhs - c0);
+  tau += c0 * tstride;
+  mult += c0 * cstride;
+  const int n_up = *n_up_ptr;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int i = blockIdx.x * S2M_WARPS + warp; i < n_up; i += gridDim.x * S2M_WARPS) {
+    const int node = uplist[i];
+    const LevelOpsDev &op = ops[level_of_node(off, L, node)];
+    const int b = bot[node], e = top[node];
+    const double cx = xmid[node], cy = ymid[node];
+    if (neq + lane < np)
+      for (int c = 0; c < ncol; ++c) mult[c * cstride + (size_t)node * np + neq + lane] = 0.0;
+    for (int k0 = 0; k0 < neq; k0 += 32) {
+      int G = 1;
+      while (2 * G * (neq - k0) <= 32) G *= 2;
+      const int sub = lane & (G - 1), k = k0 + lane / G;
+      const double x = op.lx[min(k, neq - 1)], y = op.ly[min(k, neq - 1)];
+      double v[S2M_COLS] = {};
       for (int j0 = b; j0 < e; j0 += 32) {
         const int nj = min(32, e - j0);
+        __syncwarp();
         if (lane < nj) {
-          srcx[warp][lane] = sx[j0 + lane] - cx;
-          srcy[warp][lane] = sy[j0 + lane] - cy;
-          srct[warp][lane] = tau[j0 + lane] * fold;
-          if constexpr (DIP) {
-            srcdx[warp][lane] = dvx[j0 + lane];
-            srcdy[warp][lane] = dvy[j0 + lane];
-          }
-        } else {  // padding pairs: zero charge at a harmless distance
-          srcx[warp][lane] = 0.0;
-          srcy[warp][lane] = 0.0;
-          srct[warp][lane] = 0.0;
-          if constexpr (DIP) {
-            srcdx[warp][lane] = 0.0;
-            srcdy[warp][lane] = 0.0;
-          }
+          s_xy[warp][lane] = make_double2(sx[j0 + lane] - cx, sy[j0 + lane] - cy);
+#pragma unroll
+          for (int c = 0; c < S2M_COLS; ++c)
+            s_q[warp][lane][c] = c < ncol ? tau[c * tstride + j0 + lane] * fold : 0.0;
         }
         __syncwarp();
-        const int nj2 = (nj + 1) & ~1;
-        // one source's contribution at check point (lx, ly)
-        auto term = [&](double lx, double ly, int j) -> double {
-          const double ax = lx - srcx[warp][j], ay = ly - srcy[warp][j];
-          double v = kernel_at(K, ax, ay) * srct[warp][j];
-          if constexpr (DIP) v += dipole_at(srcdx[warp][j], srcdy[warp][j], ax, ay);
-          return v;
-        };
-        if (k0)
-          for (int j = 0; j < nj2; j += 2) {
-            a0 += term(lx0, ly0, j);
-            b0 += term(lx0, ly0, j + 1);
-          }
-        if (k1)
-          for (int j = 0; j < nj2; j += 2) {
-            a1 += term(lx1, ly1, j);
-            b1 += term(lx1, ly1, j + 1);
-          }
-        __syncwarp();
+#pragma unroll 2
+        for (int j = sub; j < nj; j += G) {
+          const double dx = x - s_xy[warp][j].x, dy = y - s_xy[warp][j].y;
+          double kv;
+          if constexpr (KF::kLogTable)
+            kv = K.raw(dx, dy);
+          else
+            kv = K(0.0, 0.0, dx, dy);
+#pragma unroll
+          for (int c = 0; c < S2M_COLS; ++c) v[c] = fma(kv, s_q[warp][j][c], v[c]);
+        }
       }
-      if (k0) P[t * ldp + lane] = a0 + b0;
-      if (k1) P[t * ldp + lane + 32] = a1 + b1;
+#pragma unroll
+      for (int c = 0; c < S2M_COLS; ++c) {
+        double o = v[c];
+        for (int w = G >> 1; w >= 1; w >>= 1) o += __shfl_xor_sync(0xffffffffu, o, w);
+        if (sub == 0 && k < neq && c < ncol) mult[c * cstride + (size_t)node * np + k] = o;
+      }
     }
-    for (int m = mlo; m <= mhi; ++m) {
-      __syncthreads();
-      if (threadIdx.x < TN)
-        orow[threadIdx.x] = nlev[threadIdx.x] == m ? mult + (size_t)node[threadIdx.x] * np : nullptr;
-      __syncthreads();
-      c2e_rows<TN / 8>(ops[m], np, P, T, part, orow);
-    }
-    __syncthreads();
   }
 }
 
@@ -382,6 +416,76 @@ __global__ void __launch_bounds__(NT, 2) k_up_levels(LevelSpans sp, int np, int 
     if (i + 1 < sp.n && !grid_barrier(sync, fail)) {
       if (nxt < sp.n) st.wait(fills);  // the copies in flight
       return;
+    }
+  }
+}
+
+// Check-to-equivalent of the S2M nodes' rows (check potentials, from S2M) in
+// place, all levels and charge columns in one launch.  A block takes a
+// contiguous run of the level-major list, so it stages a level's operators
+// once or twice, and reads the next tile of 16 rows during the current one.
+// Bound by the DMMA pipe and, at few tiles, by staging the operators.
+constexpr int C2E_RB = 2, C2E_ROWS = 8 * C2E_RB;
+size_t c2e_leaves_smem(int np) {
+  return sizeof(double) * (level_ops_doubles(np, 0) + (size_t)3 * C2E_ROWS * pad_ld(np));
+}
+__global__ void __launch_bounds__(NT, 2) k_c2e_leaves(int np, int L, int n_rhs,
+                                                      const int *__restrict__ off,
+                                                      const int *__restrict__ uplist,
+                                                      const int *__restrict__ n_up_ptr,
+                                                      const LevelOpsDev *__restrict__ ops,
+                                                      double *mult, int64_t cstride) {
+  extern __shared__ __align__(16) double smem[];
+  __shared__ __align__(16) double part[FG_PART];
+  __shared__ double *orow[C2E_ROWS];
+  __shared__ int node[2][C2E_ROWS], lev[2][C2E_ROWS];
+  const int ldp = pad_ld(np), tid = threadIdx.x, n_up = *n_up_ptr;
+  double2 *U = reinterpret_cast<double2 *>(smem), *V = U + np * np / 2;
+  double *sinv = reinterpret_cast<double *>(V + np * np / 2);
+  double *T = smem + level_ops_doubles(np, 0), *P[2] = {T + C2E_ROWS * ldp, T + 2 * C2E_ROWS * ldp};
+  const int tiles = (n_up + C2E_ROWS - 1) / C2E_ROWS;
+  const int64_t total = (int64_t)tiles * n_rhs;
+  const int64_t u0 = total * blockIdx.x / gridDim.x, u1 = total * (blockIdx.x + 1) / gridDim.x;
+  auto load = [&](int64_t u, int slot) {  // the tile's nodes, then their rows (a copy group)
+    const int col = int(u / tiles), i0 = C2E_ROWS * int(u - (int64_t)col * tiles);
+    if (tid < C2E_ROWS) {
+      const int g = i0 + tid < n_up ? uplist[i0 + tid] : -1;
+      node[slot][tid] = g;
+      lev[slot][tid] = g >= 0 ? level_of_node(off, L, g) : -1;
+    }
+    for (int i = tid; i < C2E_ROWS * (np / 2); i += NT) {
+      const int r = i / (np / 2), k = 2 * (i - r * (np / 2));
+      if (i0 + r < n_up)
+        cp_async16(P[slot] + r * ldp + k, mult + col * cstride + (size_t)uplist[i0 + r] * np + k);
+      else
+        P[slot][r * ldp + k] = P[slot][r * ldp + k + 1] = 0.0;
+    }
+    cp_async_commit_group();
+  };
+  int have = -1, slot = 0;  // level whose operators are staged
+  if (u0 < u1) load(u0, 0);
+  for (int64_t u = u0; u < u1; ++u, slot ^= 1) {
+    const int col = int(u / tiles);
+    cp_async_wait_all();
+    __syncthreads();
+    if (u + 1 < u1) load(u + 1, slot ^ 1);
+    const int nloc = min(C2E_ROWS, n_up - C2E_ROWS * int(u - (int64_t)col * tiles));
+    for (int m = lev[slot][0]; m <= lev[slot][nloc - 1]; ++m) {
+      if (tid < C2E_ROWS)
+        orow[tid] = lev[slot][tid] == m ? mult + col * cstride + (size_t)node[slot][tid] * np : nullptr;
+      if (m != have) {
+        for (int j = tid; j < np * np / 2; j += NT) {
+          cp_async16(U + j, ops[m].u_f + j);
+          cp_async16(V + j, ops[m].vh_f + j);
+        }
+        if (tid < np) sinv[tid] = ops[m].sinv[tid];
+        cp_async_commit_group();
+        cp_async_wait_all();
+        have = m;
+      }
+      __syncthreads();
+      c2e_rows_smem<C2E_RB>(U, V, sinv, np, P[slot], T, part, orow);
+      __syncthreads();  // operators, T and orow are free
     }
   }
 }
@@ -1053,28 +1157,36 @@ void upward_impl(const PassArgs &a, const double *tau_s, double *mult, cudaStrea
   const TreeDev &td = *a.td;
   const int np = a.np;
   if (th.L < 3) return;
-  const size_t s2m_bytes = sizeof(double) * ((size_t)TN * pad_ld(np) * 2);
-  smem_limit(k_s2m<KF>, s2m_bytes);
-  // persistent over the S2M nodes; at most one block per TN nodes of the tree
-  // (small trees launch small grids)
-  const int s2m_grid = std::max(1, std::min(148 * 4, (th.n_total() + TN - 1) / TN));
   PhaseTimer timer(PH_UPWARD, s);
-  if (a.dvx) {
-    if constexpr (std::is_same<KF, LaplaceF64T>::value) {
-      smem_limit(k_s2m<KF, true>, s2m_bytes);
-      k_s2m<KF, true><<<dim3(s2m_grid, n_rhs), NT, s2m_bytes, s>>>(
+  const int per_sm = 8;
+  const int64_t warps = std::min<int64_t>(th.n_total(), (int64_t)148 * per_sm * S2M_WARPS);
+  const int s2m_grid = int((warps + S2M_WARPS - 1) / S2M_WARPS);
+  if (n_rhs > 1) {
+    k_s2m_multi<KF><<<dim3(s2m_grid, (n_rhs + S2M_COLS - 1) / S2M_COLS), 32 * S2M_WARPS, 0, s>>>(
+        a.kp, a.neq, np, th.L, td.dev_off.get(), td.uplist.get(), td.n_up.get(), td.bot.get(),
+        td.top.get(), td.xmid.get(), td.ymid.get(), td.sx.get(), td.sy.get(), tau_s, a.ops_dev, mult,
+        n_rhs, tstride, cstride);
+  } else {
+    auto launch = [&](auto kern) {
+      kern<<<s2m_grid, 32 * S2M_WARPS, 0, s>>>(
           a.kp, a.neq, np, th.L, td.dev_off.get(), td.uplist.get(), td.n_up.get(), td.bot.get(),
           td.top.get(), td.xmid.get(), td.ymid.get(), td.sx.get(), td.sy.get(), tau_s, a.ops_dev,
-          mult, a.dvx, a.dvy, tstride, cstride);
-    } else {
+          mult, a.dvx, a.dvy);
+    };
+    if (!a.dvx)
+      launch(k_s2m<KF, false>);
+    else if constexpr (std::is_same<KF, LaplaceF64T>::value)
+      launch(k_s2m<KF, true>);
+    else
       throw Error(ERR_UNSUPPORTED, "dipole sources: Laplace kernel only");
-    }
-  } else {
-    k_s2m<KF><<<dim3(s2m_grid, n_rhs), NT, s2m_bytes, s>>>(
-        a.kp, a.neq, np, th.L, td.dev_off.get(), td.uplist.get(), td.n_up.get(), td.bot.get(),
-        td.top.get(), td.xmid.get(), td.ymid.get(), td.sx.get(), td.sy.get(), tau_s, a.ops_dev,
-        mult, nullptr, nullptr, tstride, cstride);
   }
+  FMMB_CUDA(cudaGetLastError());
+  const size_t c2e_bytes = c2e_leaves_smem(np);
+  smem_limit(k_c2e_leaves, c2e_bytes);
+  // at least two tiles a block: its operators serve 32 rows or more
+  const int64_t c2e_tiles = (int64_t)n_rhs * ((th.n_total() + C2E_ROWS - 1) / C2E_ROWS);
+  k_c2e_leaves<<<work_grid((c2e_tiles + 1) / 2, 2), NT, c2e_bytes, s>>>(
+      np, th.L, n_rhs, td.dev_off.get(), td.uplist.get(), td.n_up.get(), a.ops_dev, mult, cstride);
   FMMB_CUDA(cudaGetLastError());
   LevelSpans sp{};
   sp.m0 = th.L - 2;

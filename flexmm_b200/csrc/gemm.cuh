@@ -157,10 +157,7 @@ __device__ __forceinline__ void cp_async_wait_group() {
 // fragments its readers need: element (kp N/8 + cb) 32 + lane of an array of
 // pairs holds B[8 kp + q][8 cb + g] and B[8 kp + 4 + q][8 cb + g] (g = lane/4,
 // q = lane%4), so a warp reads two k-steps of a column block in one coalesced
-// 512-byte load.  A DMMA takes an SM sub-partition about 16 clocks: at these
-// sizes the loads (from L2, or L1 where several warps read the same column
-// block) keep up with a few in flight, and no shared memory, copies or
-// barriers are spent on operators.
+// 512-byte load (from global memory) or without bank conflicts (from shared).
 template <class F>
 inline void pack_fragments(int K, int N, F &&at, double *dst) {
   for (int kp = 0; kp < K / 8; ++kp)
@@ -180,107 +177,9 @@ __device__ __forceinline__ double2 load_pair(const double2 *p) {
 }
 
 constexpr int FG_WARPS = 8;  // warps of a block that runs these tiles
-constexpr int FG_AHEAD = 4;  // fragment pairs in flight per warp
+constexpr int FG_PART = FG_WARPS * 64;  // doubles of the k-part exchange
 
-// How the 8 warps share an output tile of RB row blocks (of 8) x ncb column
-// blocks: a warp keeps to one column block (its fragments are read once); the
-// warps of a column block split its row blocks, and where they outnumber them
-// the k range (KS parts, summed through shared memory afterwards).
-template <int RB>
-struct TileSplit {
-  int cb, rb, rstep, kpart, ks;
-  bool active;
-  __device__ TileSplit(int ncb) {
-    const int warp = threadIdx.x >> 5, wpc = max(1, FG_WARPS / ncb), w = warp / ncb;
-    cb = warp % ncb;
-    if (wpc >= RB) {
-      ks = wpc / RB;
-      rb = w % RB;
-      kpart = w / RB;
-      rstep = RB;
-      active = kpart < ks;
-    } else {
-      ks = 1;
-      rb = w;
-      kpart = 0;
-      rstep = wpc;
-      active = w < wpc;
-    }
-  }
-};
-
-// the first fragment pairs of a warp's share (issued before the block waits
-// for its inputs)
-struct FragAhead {
-  double2 b[FG_AHEAD];
-};
-template <int RB>
-__device__ __forceinline__ void frag_ahead(const TileSplit<RB> &t, const double2 *__restrict__ B,
-                                           int ncb, int npairs, FragAhead &f) {
-  const int lane = threadIdx.x & 31;
-  const int k0 = npairs * t.kpart / t.ks, k1 = npairs * (t.kpart + 1) / t.ks;
-#pragma unroll
-  for (int i = 0; i < FG_AHEAD; ++i)
-    if (k0 + i < k1) f.b[i] = load_pair(B + ((size_t)(k0 + i) * ncb + t.cb) * 32 + lane);
-}
-
-// acc[i] (row block t.rb + i t.rstep) += A[rows][8 k0 ..] . B over the warp's
-// k range; A in shared memory, row stride lda (4 mod 16: conflict-free)
-template <int RB>
-__device__ __forceinline__ void frag_gemm(const TileSplit<RB> &t, const double *A, int lda,
-                                          const double2 *__restrict__ B, int ncb, int npairs,
-                                          FragAhead &f, double (&acc)[RB][2]) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-  const int k0 = npairs * t.kpart / t.ks, k1 = npairs * (t.kpart + 1) / t.ks;
-  const double *Ap = A + (8 * t.rb + g) * lda + q;
-  for (int kb = k0; kb < k1; kb += FG_AHEAD) {
-#pragma unroll
-    for (int i = 0; i < FG_AHEAD; ++i) {
-      const int kp = kb + i;
-      if (kp < k1) {
-        const double2 b = f.b[i];
-        if (kp + FG_AHEAD < k1)
-          f.b[i] = load_pair(B + ((size_t)(kp + FG_AHEAD) * ncb + t.cb) * 32 + lane);
-#pragma unroll
-        for (int r = 0; r < RB; ++r)
-          if (t.rb + r * t.rstep < RB) {
-            const double *a = Ap + 8 * r * t.rstep * lda + 8 * kp;
-            dmma(acc[r], a[0], b.x);
-            dmma(acc[r], a[4], b.y);
-          }
-      }
-    }
-  }
-}
-
-template <int RB>
-__device__ __forceinline__ void zero_rows(double (&acc)[RB][2]) {
-#pragma unroll
-  for (int r = 0; r < RB; ++r) acc[r][0] = acc[r][1] = 0.0;
-}
-
-// doubles of the k-part exchange
-constexpr int FG_PART = FG_WARPS * 64;
-
-// sum the k parts (one row block per warp then) into the warps of part 0
-// through part (FG_PART doubles); a barrier inside when there are several
-template <int RB>
-__device__ __forceinline__ void sum_parts(const TileSplit<RB> &t, double (&acc)[RB][2], double *part) {
-  if (t.ks == 1) return;
-  const int lane = threadIdx.x & 31, slot = (t.cb * RB + t.rb) * (t.ks - 1);
-  if (t.active && t.kpart > 0)
-    *reinterpret_cast<double2 *>(part + (slot + t.kpart - 1) * 64 + 2 * lane) =
-        make_double2(acc[0][0], acc[0][1]);
-  __syncthreads();
-  if (t.active && t.kpart == 0)
-    for (int k = 0; k < t.ks - 1; ++k) {
-      const double2 v = *reinterpret_cast<const double2 *>(part + (slot + k) * 64 + 2 * lane);
-      acc[0][0] += v.x;
-      acc[0][1] += v.y;
-    }
-}
-
-// ---- the same with the operator's fragments in shared memory ----
+// ---- tiles of 8 RB rows, the operator's fragments in shared memory ----
 // The tile's units (row block, column block) are dealt out to the 8 warps, at
 // most RB each; where there are no more than 4 of them the warps split the k
 // range too (KS parts, summed through shared memory).
@@ -369,7 +268,9 @@ __device__ __forceinline__ void unit_each(const UnitSplit<RB> &t, const double (
   }
 }
 
-// c2e_rows with U, VH and 1/S in shared memory
+// Check-to-equivalent of a tile of 8 RB rows: ((P . U) diag(1/S)) . VH, P and T
+// [8 RB][pad_ld(np)] and the operators in shared memory; row t goes to
+// out_row[t] (np doubles) where that is not null.  The caller synchronises before.
 template <int RB>
 __device__ __forceinline__ void c2e_rows_smem(const double2 *U, const double2 *VH, const double *sinv,
                                               int np, const double *P, double *T, double *part,
@@ -405,47 +306,6 @@ __device__ __forceinline__ void bulk_copy(void *dst, const void *src, uint32_t b
           static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
       "l"(src), "r"(bytes), "r"(static_cast<uint32_t>(__cvta_generic_to_shared(bar)))
       : "memory");
-}
-
-// Check-to-equivalent of a tile of 8 RB rows: ((P . U) diag(1/S)) . VH, P and T
-// [8 RB][pad_ld(np)] in shared memory; row t goes to out_row[t] (np doubles)
-// where that is not null.  The caller synchronises before.
-template <int RB>
-__device__ inline void c2e_rows(const LevelOpsDev &op, int np, const double *P, double *T,
-                                double *part, double *const *out_row) {
-  const int ldp = pad_ld(np), ncb = np / 8;
-  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-  const TileSplit<RB> t(ncb);
-  double acc[RB][2];
-  FragAhead f;
-  zero_rows(acc);
-  if (t.active) {
-    frag_ahead(t, op.u_f, ncb, ncb, f);
-    frag_gemm(t, P, ldp, op.u_f, ncb, ncb, f, acc);
-    frag_ahead(t, op.vh_f, ncb, ncb, f);
-  }
-  sum_parts(t, acc, part);
-  if (t.active && t.kpart == 0) {
-    const double s0 = __ldg(op.sinv + 8 * t.cb + 2 * q), s1 = __ldg(op.sinv + 8 * t.cb + 2 * q + 1);
-#pragma unroll
-    for (int r = 0; r < RB; ++r)
-      if (t.rb + r * t.rstep < RB)
-        *reinterpret_cast<double2 *>(T + (8 * (t.rb + r * t.rstep) + g) * ldp + 8 * t.cb + 2 * q) =
-            make_double2(acc[r][0] * s0, acc[r][1] * s1);
-  }
-  __syncthreads();
-  zero_rows(acc);
-  if (t.active) frag_gemm(t, T, ldp, op.vh_f, ncb, ncb, f, acc);
-  sum_parts(t, acc, part);
-  if (t.active && t.kpart == 0) {
-#pragma unroll
-    for (int r = 0; r < RB; ++r)
-      if (t.rb + r * t.rstep < RB) {
-        double *o = out_row[8 * (t.rb + r * t.rstep) + g];
-        if (o)
-          *reinterpret_cast<double2 *>(o + 8 * t.cb + 2 * q) = make_double2(acc[r][0], acc[r][1]);
-      }
-  }
 }
 
 }  // namespace fmmb
