@@ -1775,7 +1775,6 @@ extern "C" int fmm_evaluate_noalloc(fmm_plan *p, const double *tx, const double 
     // carve the scratch
     const int digits = p->th.L > 1 ? p->th.L - 1 : 1;
     const size_t sort_bytes = round256(sort_points_scratch_bytes(m, digits));
-    const size_t scan_bytes = round256(evaluate_scratch_bytes(total));
     size_t at = 0;
     auto carve = [&](size_t bytes) {
       unsigned char *q = base + at;
@@ -1786,14 +1785,9 @@ extern "C" int fmm_evaluate_noalloc(fmm_plan *p, const double *tx, const double 
     int *tperm = (int *)carve(m * sizeof(int));
     double *txs = (double *)carve(m * sizeof(double));
     double *tys = (double *)carve(m * sizeof(double));
-    int *tb = (int *)carve(total * sizeof(int));
-    int *te = (int *)carve(total * sizeof(int));
-    int *nch = (int *)carve(total * sizeof(int));
-    int *choff = (int *)carve(total * sizeof(int));
     int4 *items = (int4 *)carve((total + m / EVAL_CHUNK + 1) * sizeof(int4));
     int *n_items = (int *)carve((1 + EVAL_COUNTERS) * sizeof(int));
     void *sort_tmp = carve(sort_bytes);
-    void *scan_tmp = carve(scan_bytes);
     FMMB_CHECK(at <= NOALLOC_SCRATCH_BYTES, ERR_CAPACITY,
                "fmm_evaluate_noalloc: scratch needs exceed the static array");
     // the same passes as fmm_evaluate, on the static scratch
@@ -1810,7 +1804,7 @@ extern "C" int fmm_evaluate_noalloc(fmm_plan *p, const double *tx, const double 
       sort_points_scratch(tx, ty, m, p->th, digits, tkeys, tperm, txs, tys, sort_tmp, sort_bytes,
                           p->td.sort_fail.get(), s);
     }
-    run_evaluate_scratch(a, p->tau_s.get(), p->loc.get(), txs, tys, tkeys, tperm, m, check, out, tb,
-                         te, nch, choff, items, n_items, scan_tmp, scan_bytes, s);
+    run_evaluate_scratch(a, p->tau_s.get(), p->loc.get(), txs, tys, tkeys, tperm, m, check, out,
+                         items, n_items, s);
   });
 }

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
+#include <list>
 #include <string>
 #include <vector>
 #include <stdexcept>
@@ -97,6 +98,38 @@ struct DevBuf {
     if (n) FMMB_CUDA(cudaMemsetAsync(p, 0, n * sizeof(T), stream));
   }
   T *get() const { return p; }
+};
+
+// Zeroed device memory for the counters and barriers of a run of launches: one
+// memset of a block serves all of them (a memset of its own costs each about
+// 4 us of device time with the gap around it).  What the block cannot hold is
+// allocated and zeroed apart.  take() hands out each byte once.
+class ZeroPool {
+ public:
+  ZeroPool(void *block, size_t bytes, cudaStream_t stream)
+      : at_(static_cast<unsigned char *>(block)), left_(bytes), s_(stream) {
+    FMMB_CUDA(cudaMemsetAsync(block, 0, bytes, stream));
+  }
+  template <class T>
+  T *take(size_t count) {
+    const size_t bytes = (count * sizeof(T) + 255) & ~size_t(255);
+    if (bytes > left_) {
+      more_.emplace_back();
+      more_.back().alloc(bytes, s_);
+      more_.back().zero(s_);
+      return reinterpret_cast<T *>(more_.back().get());
+    }
+    unsigned char *p = at_;
+    at_ += bytes;
+    left_ -= bytes;
+    return reinterpret_cast<T *>(p);
+  }
+
+ private:
+  unsigned char *at_;
+  size_t left_;
+  cudaStream_t s_;
+  std::list<DevBuf<unsigned char>> more_;
 };
 
 // Programmatic dependent launch: a kernel launched by launch_pdl may start

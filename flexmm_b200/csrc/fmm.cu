@@ -27,7 +27,6 @@
 #include "fmm.cuh"
 #include "gemm.cuh"
 #include "radix.cuh"
-#include "scan.cuh"
 #include "sweep.cuh"
 #include "tcgen05.cuh"
 #include "timing.cuh"
@@ -73,6 +72,21 @@ __device__ __forceinline__ int level_of_node(const int *__restrict__ off, int L,
       hi = mid;
   }
   return lo;
+}
+
+// first of n consecutive places taken from *next for every lane of the warp
+// (one atomic for all; all lanes must call)
+__device__ __forceinline__ int warp_place(int n, int *next) {
+  const int lane = threadIdx.x & 31;
+  int incl = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  int base = 0;
+  if (lane == 31 && incl > 0) base = atomicAdd(next, incl);
+  return __shfl_sync(0xffffffffu, base, 31) + incl - n;
 }
 
 // S2M of every S2M node (leaves holding points, levels >= 2) of every level in
@@ -815,27 +829,37 @@ LevelFit level_fit(F &&bytes, int n_rhs) {
 }
 
 // ------------------------------------------------------------ evaluation ----
-__global__ void k_leaf_targets(int total, int L, const int *__restrict__ off,
+// Work items of a leaf's targets [b, e), for a warp's 32 nodes (any of them
+// empty): their chunk counts are summed over the warp and one atomic finds the
+// place of all its items, so the list needs no scan of its own.  The warps'
+// items follow one another in any order: no item depends on another.
+__device__ __forceinline__ void emit_items(int g, int L, const int *__restrict__ off, int b, int e,
+                                           bool binned, int4 *__restrict__ items, int *n_items) {
+  const int n = (e - b + TCH - 1) / TCH;
+  const int at = warp_place(n, n_items);
+  if (n == 0) return;
+  const int y = level_of_node(off, L, g) | (binned && n > 1 ? EVAL_MULTI : 0) |
+                (binned && e - b > 32 ? EVAL_UNORDERED : 0);
+  for (int c = 0; c < n; ++c) {
+    const int t0 = b + c * TCH;
+    items[at + c] = make_int4(g, y, t0, min(TCH, e - t0));
+  }
+}
+
+// targets sorted by key: each leaf's range by two searches
+__global__ void k_items_sorted(int total, int L, const int *__restrict__ off,
                                const uint64_t *__restrict__ code, const uint8_t *__restrict__ flags,
                                const uint64_t *__restrict__ tkeys, int64_t m,
-                               int *__restrict__ tb, int *__restrict__ te,
-                               int *__restrict__ nchunk) {
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
-    int lo = 0, hi = L;
-    while (hi - lo > 1) {
-      int mid = (lo + hi) >> 1;
-      if (off[mid] <= g)
-        lo = mid;
-      else
-        hi = mid;
-    }
-    const int lev = lo;
+                               int4 *__restrict__ items, int *n_items) {
+  const int stride = gridDim.x * blockDim.x;
+  for (int g0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); g0 < total; g0 += stride) {
+    const int g = g0 + (threadIdx.x & 31);
     int b = 0, e = 0;
-    if ((flags[g] & NF_LEAF) && m > 0) {
+    if (g < total && (flags[g] & NF_LEAF) && m > 0) {
       // both ends of the leaf's key range: two branchless lower-bound
       // searches over [0, m) in step (same length, same step count), so each
       // step's two loads are issued together
-      const int sh = 2 * (MAXD - lev);
+      const int sh = 2 * (MAXD - level_of_node(off, L, g));
       const uint64_t c = code[g];
       const uint64_t vlo = c << sh, vhi = (c + 1) << sh;
       int64_t b0 = 0, b1 = 0, len = m;
@@ -849,35 +873,36 @@ __global__ void k_leaf_targets(int total, int L, const int *__restrict__ off,
       b = int(b0 + (__ldg(tkeys + b0) < vlo ? 1 : 0));
       e = int(b1 + (__ldg(tkeys + b1) < vhi ? 1 : 0));
     }
-    tb[g] = b;
-    te[g] = e;
-    nchunk[g] = (e - b + TCH - 1) / TCH;
+    emit_items(g, L, off, b, e, false, items, n_items);
   }
 }
 
-// expand the per-leaf chunk counts into a flat item list
-__global__ void k_make_items(int total, int L, const int *__restrict__ off, const int *__restrict__ tb,
-                             const int *__restrict__ te, const int *__restrict__ nch,
-                             const int *__restrict__ choff, int4 *__restrict__ items,
-                             int *__restrict__ n_items, int binned) {
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
-    if (g == total - 1) {
-      n_items[0] = choff[g] + nch[g];
-      for (int c = 1; c <= EVAL_COUNTERS; ++c) n_items[c] = 0;
-    }
-    const int n = nch[g];
-    if (n == 0) continue;
-    int lo = 0, hi = L;
-    while (hi - lo > 1) {
-      int mid = (lo + hi) >> 1;
-      if (off[mid] <= g) lo = mid; else hi = mid;
-    }
-    const int y = lo | (binned && n > 1 ? EVAL_MULTI : 0) |
-                  (binned && te[g] - tb[g] > 32 ? EVAL_UNORDERED : 0);
-    for (int c = 0; c < n; ++c) {
-      const int t0 = tb[g] + c * TCH;
-      items[choff[g] + c] = make_int4(g, y, t0, min(TCH, te[g] - t0));
-    }
+// the tree's own sources: each leaf's range is its [bot, top) (the same
+// lower-bound searches of the same sorted keys, done by the node pass)
+__global__ void k_items_sources(int total, int L, const int *__restrict__ off,
+                                const uint8_t *__restrict__ flags, const int *__restrict__ bot,
+                                const int *__restrict__ top, int4 *__restrict__ items,
+                                int *n_items) {
+  const int stride = gridDim.x * blockDim.x;
+  for (int g0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); g0 < total; g0 += stride) {
+    const int g = g0 + (threadIdx.x & 31);
+    const bool leaf = g < total && (flags[g] & NF_LEAF);
+    emit_items(g, L, off, leaf ? bot[g] : 0, leaf ? top[g] : 0, false, items, n_items);
+  }
+}
+
+// binned targets: count[g] of them in leaf g; their places (first[g] on) are
+// given out the same way as the items'
+__global__ void k_items_binned(int total, int L, const int *__restrict__ off,
+                               const int *__restrict__ count, int *__restrict__ first, int *placed,
+                               int4 *__restrict__ items, int *n_items) {
+  const int stride = gridDim.x * blockDim.x;
+  for (int g0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); g0 < total; g0 += stride) {
+    const int g = g0 + (threadIdx.x & 31);
+    const int n = g < total ? count[g] : 0;
+    const int b = warp_place(n, placed);
+    if (g < total) first[g] = b;
+    emit_items(g, L, off, b, b + n, true, items, n_items);
   }
 }
 
@@ -1217,53 +1242,28 @@ void upward_impl(const PassArgs &a, const double *tau_s, double *mult, cudaStrea
 
 }  // namespace
 
-// the tree's own sources: each leaf's range is its [bot, top) (the same
-// lower-bound searches of the same sorted keys, done by the node pass)
-__global__ void k_leaf_sources(int total, const uint8_t *__restrict__ flags,
-                               const int *__restrict__ bot, const int *__restrict__ top,
-                               int *__restrict__ tb, int *__restrict__ te, int *__restrict__ nchunk) {
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
-    const bool leaf = flags[g] & NF_LEAF;
-    const int b = leaf ? bot[g] : 0, e = leaf ? top[g] : 0;
-    tb[g] = b;
-    te[g] = e;
-    nchunk[g] = (e - b + TCH - 1) / TCH;
-  }
-}
-
-void eval_items(const PassArgs &a, const uint64_t *tkeys, int64_t m, EvalItems &it, cudaStream_t s) {
+namespace {
+// the list of targets sorted by key, or of the tree's own sources
+void items_sorted(const PassArgs &a, const uint64_t *tkeys, int64_t m, int4 *items, int *n_items,
+                  cudaStream_t s) {
   const TreeHost &th = *a.th;
   const TreeDev &td = *a.td;
-  const int total = th.n_total();
-  it.tb.alloc(total, s);
-  it.te.alloc(total, s);
-  it.nch.alloc(total, s);
-  it.choff.alloc(total, s);
+  const int total = th.n_total(), grid = grid_for(total, 256);
+  FMMB_CUDA(cudaMemsetAsync(n_items, 0, (1 + EVAL_COUNTERS) * sizeof(int), s));
   if (tkeys == td.pkeys.get() && m == th.n_points)
-    k_leaf_sources<<<grid_for(total, 256), 256, 0, s>>>(total, td.flags.get(), td.bot.get(),
-                                                        td.top.get(), it.tb.get(), it.te.get(),
-                                                        it.nch.get());
+    k_items_sources<<<grid, 256, 0, s>>>(total, th.L, td.dev_off.get(), td.flags.get(),
+                                         td.bot.get(), td.top.get(), items, n_items);
   else
-    k_leaf_targets<<<grid_for(total, 256), 256, 0, s>>>(total, th.L, td.dev_off.get(), td.code.get(),
-                                                        td.flags.get(), tkeys, m, it.tb.get(),
-                                                        it.te.get(), it.nch.get());
-  FMMB_CUDA(cudaGetLastError());
-  prefix_sum<int, false>(it.nch.get(), it.choff.get(), total, td.sort_fail.get(), true, s);
-  it.items.alloc(total + m / TCH + 1, s);
-  it.n_items.alloc(1 + EVAL_COUNTERS, s);
-  k_make_items<<<grid_for(total, 256), 256, 0, s>>>(total, th.L, td.dev_off.get(), it.tb.get(),
-                                                    it.te.get(), it.nch.get(), it.choff.get(),
-                                                    it.items.get(), it.n_items.get(), 0);
+    k_items_sorted<<<grid, 256, 0, s>>>(total, th.L, td.dev_off.get(), td.code.get(),
+                                        td.flags.get(), tkeys, m, items, n_items);
   FMMB_CUDA(cudaGetLastError());
 }
+}  // namespace
 
-// per leaf: end of its target range and its item count (counts from binning)
-__global__ void k_leaf_ranges(int total, const int *__restrict__ count, const int *__restrict__ tb,
-                              int *__restrict__ te, int *__restrict__ nch) {
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
-    te[g] = tb[g] + count[g];
-    nch[g] = (count[g] + TCH - 1) / TCH;
-  }
+void eval_items(const PassArgs &a, const uint64_t *tkeys, int64_t m, EvalItems &it, cudaStream_t s) {
+  it.items.alloc(a.th->n_total() + m / TCH + 1, s);
+  it.n_items.alloc(1 + EVAL_COUNTERS, s);
+  items_sorted(a, tkeys, m, it.items.get(), it.n_items.get(), s);
 }
 
 void eval_items_binned(const PassArgs &a, const double *tx, const double *ty, int64_t m,
@@ -1271,28 +1271,21 @@ void eval_items_binned(const PassArgs &a, const double *tx, const double *ty, in
   const TreeHost &th = *a.th;
   const TreeDev &td = *a.td;
   const int total = th.n_total();
-  DevBuf<int> count, leaf_of, slot;
-  count.alloc(total, s);
-  count.zero(s);
+  DevBuf<int> first, leaf_of, slot;
+  first.alloc(total, s);
   leaf_of.alloc(m, s);
   slot.alloc(m, s);
-  bin_points(tx, ty, m, td, th, count.get(), leaf_of.get(), slot.get(), s);
-  it.tb.alloc(total, s);
-  it.te.alloc(total, s);
-  it.nch.alloc(total, s);
-  it.choff.alloc(total, s);
-  prefix_sum<int, false>(count.get(), it.tb.get(), total, td.sort_fail.get(), true, s);
-  scatter_binned(tx, ty, m, leaf_of.get(), slot.get(), it.tb.get(), txs, tys, tperm, s);
-  k_leaf_ranges<<<grid_for(total, 256), 256, 0, s>>>(total, count.get(), it.tb.get(), it.te.get(),
-                                                     it.nch.get());
-  FMMB_CUDA(cudaGetLastError());
-  prefix_sum<int, false>(it.nch.get(), it.choff.get(), total, td.sort_fail.get(), true, s);
   it.items.alloc(total + m / TCH + 1, s);
-  it.n_items.alloc(1 + EVAL_COUNTERS, s);
-  k_make_items<<<grid_for(total, 256), 256, 0, s>>>(total, th.L, td.dev_off.get(), it.tb.get(),
-                                                    it.te.get(), it.nch.get(), it.choff.get(),
-                                                    it.items.get(), it.n_items.get(), 1);
+  // the list's counters, the targets placed so far and the nodes' counts: one memset
+  it.n_items.alloc(2 + EVAL_COUNTERS + total, s);
+  it.n_items.zero(s);
+  int *placed = it.n_items.get() + 1 + EVAL_COUNTERS, *count = placed + 1;
+  bin_points(tx, ty, m, td, th, count, leaf_of.get(), slot.get(), s);
+  k_items_binned<<<grid_for(total, 256), 256, 0, s>>>(total, th.L, td.dev_off.get(), count,
+                                                      first.get(), placed, it.items.get(),
+                                                      it.n_items.get());
   FMMB_CUDA(cudaGetLastError());
+  scatter_binned(tx, ty, m, leaf_of.get(), slot.get(), first.get(), txs, tys, tperm, s);
 }
 
 namespace {
@@ -1638,24 +1631,13 @@ void run_direct(int kernel_id, const KernelParams &kp, const double *sx, const d
   FMMB_CUDA(cudaGetLastError());
 }
 
-size_t evaluate_scratch_bytes(int total_nodes) { return scan_scratch_bytes<int>(total_nodes); }
-
 void run_evaluate_scratch(const PassArgs &a, const double *tau_s, const double *loc,
                           const double *txs, const double *tys, const uint64_t *tkeys,
-                          const int *tperm, int64_t m, int check, double *out, int *tb, int *te,
-                          int *nch, int *choff, int4 *items, int *n_items, void *temp,
-                          size_t temp_bytes, cudaStream_t s) {
+                          const int *tperm, int64_t m, int check, double *out, int4 *items,
+                          int *n_items, cudaStream_t s) {
   if (m == 0) return;
-  const TreeHost &th = *a.th;
-  const TreeDev &td = *a.td;
-  const int total = th.n_total();
-  k_leaf_targets<<<grid_for(total, 256), 256, 0, s>>>(total, th.L, td.dev_off.get(), td.code.get(),
-                                                      td.flags.get(), tkeys, m, tb, te, nch);
-  FMMB_CUDA(cudaGetLastError());
-  prefix_sum_run<int, false>(nch, choff, total, temp, temp_bytes, td.sort_fail.get(), true, s);
-  k_make_items<<<grid_for(total, 256), 256, 0, s>>>(total, th.L, td.dev_off.get(), tb, te, nch, choff,
-                                                    items, n_items, 0);
-  FMMB_CUDA(cudaGetLastError());
+  const int total = a.th->n_total();
+  items_sorted(a, tkeys, m, items, n_items, s);
   PhaseTimer timer(PH_EVAL, s);
   const ItemArgs ia = item_args(a, items, n_items, 0, txs, tys, tperm);
   auto launch = [&](auto kf) {

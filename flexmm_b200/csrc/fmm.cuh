@@ -194,9 +194,8 @@ void run_evaluate(const PassArgs &a, const double *tau_sorted, const double *loc
                   const EvalItems *pre = nullptr);
 
 // Evaluation work items: per leaf its range of sorted targets, split into
-// chunks of 128 targets; choff = exclusive scan of the chunk counts.
+// chunks of 128 targets, in no particular order of the leaves.
 struct EvalItems {
-  DevBuf<int> tb, te, nch, choff;
   DevBuf<int4> items;   // (leaf, level | flags, first sorted target, count)
   DevBuf<int> n_items;  // [0] device count of items, [1 ..] zeroed hand-out counters
 };
@@ -233,13 +232,11 @@ void run_evaluate_mixed(const PassArgs &a, const double *tau_sorted, const doubl
                         int check, int nout, double *out, int64_t ld_out, cudaStream_t s,
                         const EvalItems *pre = nullptr);
 
-// Evaluation with caller-provided scratch: tb, te, nch, choff hold one int
-// per tree node, temp holds evaluate_scratch_bytes(nodes) bytes.
-size_t evaluate_scratch_bytes(int total_nodes);
+// Evaluation with caller-provided scratch: items [nodes + m / EVAL_CHUNK + 1],
+// n_items [1 + EVAL_COUNTERS]; allocates nothing.
 void run_evaluate_scratch(const PassArgs &a, const double *tau_sorted, const double *loc,
                           const double *txs, const double *tys, const uint64_t *tkeys,
-                          const int *tperm, int64_t m, int check, double *out, int *tb, int *te,
-                          int *nch, int *choff, int4 *items, int *n_items, void *temp,
-                          size_t temp_bytes, cudaStream_t s);
+                          const int *tperm, int64_t m, int check, double *out, int4 *items,
+                          int *n_items, cudaStream_t s);
 
 }  // namespace fmmb

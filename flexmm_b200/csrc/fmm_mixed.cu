@@ -1351,7 +1351,7 @@ void node_charge_sums(const PassArgs &a, const double *tau_s, double *tsum, cuda
   DevBuf<double> pre;
   pre.alloc(n + 1, s);
   FMMB_CUDA(cudaMemsetAsync(pre.get(), 0, sizeof(double), s));
-  prefix_sum<double, true>(tau_s, pre.get() + 1, n, a.td->sort_fail.get(), false, s);
+  prefix_sum<double, true>(tau_s, pre.get() + 1, n, a.td->sort_fail.get(), s);
   k_node_charge_sums<<<grid_for(total, 256), 256, 0, s>>>(total, a.td->bot.get(), a.td->top.get(),
                                                           pre.get(), tsum);
   FMMB_CUDA(cudaGetLastError());

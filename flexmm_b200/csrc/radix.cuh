@@ -385,11 +385,12 @@ size_t radix_scratch_bytes(int64_t n, int passes) {
 }
 
 // Sort n elements on bits [begin_bit, end_bit) with scratch of
-// radix_scratch_bytes<K, VALS>(n, passes) bytes on g = radix_grid(...) blocks.
+// radix_scratch_bytes<K, VALS>(n, passes) bytes on g = radix_grid(...) blocks
+// (zeroed: where the barrier and the digit counts come from, else the scratch).
 template <class K, bool VALS, class Src, class Emit>
 void radix_sort_run(const Src &src, const Emit &emit, int64_t n, int begin_bit, int end_bit,
                     void *scratch, size_t bytes, int g, int *fail, cudaStream_t s,
-                    const unsigned long long *n_dev = nullptr) {
+                    const unsigned long long *n_dev = nullptr, ZeroPool *zeroed = nullptr) {
   if (n <= 0) return;
   FMMB_CHECK(end_bit > begin_bit && end_bit <= int(8 * sizeof(K)) && n < (int64_t(1) << 30),
              ERR_INVALID_ARGUMENT, "radix sort: bad bit range or more than 2^30 elements");
@@ -409,12 +410,14 @@ void radix_sort_run(const Src &src, const Emit &emit, int64_t n, int begin_bit, 
       }
     }
   RadixWork w;
-  w.sync = reinterpret_cast<RadixSync *>(at);
-  w.ghist = reinterpret_cast<int *>(at + sizeof(RadixSync));
-  w.status = reinterpret_cast<unsigned *>(at + sizeof(RadixSync) + sizeof(int) * 256 * passes);
+  const size_t zero_bytes = sizeof(RadixSync) + sizeof(int) * 256 * passes;
+  unsigned char *z = zeroed ? zeroed->take<unsigned char>(zero_bytes) : at;
+  w.sync = reinterpret_cast<RadixSync *>(z);
+  w.ghist = reinterpret_cast<int *>(z + sizeof(RadixSync));
+  w.status = reinterpret_cast<unsigned *>(at + zero_bytes);
   w.fail = fail;
   w.n_dev = n_dev;
-  FMMB_CUDA(cudaMemsetAsync(w.sync, 0, sizeof(RadixSync) + sizeof(int) * 256 * passes, s));
+  if (!zeroed) FMMB_CUDA(cudaMemsetAsync(w.sync, 0, zero_bytes, s));
   auto kern = k_radix_sort<K, Src, Emit, VALS>;
   void *args[] = {(void *)&src, (void *)&emit, (void *)&n, (void *)&begin_bit, (void *)&end_bit,
                   (void *)&kb[0], (void *)&vb[0], (void *)&kb[1], (void *)&vb[1], (void *)&w};
@@ -428,13 +431,15 @@ void radix_sort_run(const Src &src, const Emit &emit, int64_t n, int begin_bit, 
 // The same with scratch from the stream-ordered pool.
 template <class K, bool VALS, class Src, class Emit>
 void radix_sort(const Src &src, const Emit &emit, int64_t n, int begin_bit, int end_bit, int *fail,
-                cudaStream_t s, const unsigned long long *n_dev = nullptr) {
+                cudaStream_t s, const unsigned long long *n_dev = nullptr,
+                ZeroPool *zeroed = nullptr) {
   if (n <= 0) return;
   const int g = radix_grid<K, VALS>(k_radix_sort<K, Src, Emit, VALS>, n);
   const size_t bytes = radix_scratch_bytes<K, VALS>(n, (end_bit - begin_bit + 7) / 8);
   DevBuf<unsigned char> tmp;
   tmp.alloc(bytes, s);
-  radix_sort_run<K, VALS>(src, emit, n, begin_bit, end_bit, tmp.get(), bytes, g, fail, s, n_dev);
+  radix_sort_run<K, VALS>(src, emit, n, begin_bit, end_bit, tmp.get(), bytes, g, fail, s, n_dev,
+                          zeroed);
 }
 
 }  // namespace

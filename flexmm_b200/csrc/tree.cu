@@ -247,59 +247,52 @@ __device__ __forceinline__ void split_range(const uint64_t *__restrict__ keys, i
   if (cnext >= max_split) cnext = max_split - 1;
 }
 
-// number of split boxes each point starts; flags trees too deep for the key
-// or for the partial sort; deepest split level
-__global__ void k_split_counts(const uint64_t *__restrict__ keys, int64_t n, int ppl,
-                               int sorted_digits, unsigned long long *__restrict__ counts,
-                               Counters *cnt, int max_split) {
-  int lmax = -1;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
+// The split boxes, scanned over the points (scan.cuh): the number of boxes
+// point i starts, flags for trees too deep for the key or for the partial sort
+// and the deepest split level; then the boxes at their positions: point-major,
+// so every level's boxes come out in increasing morton order.
+struct SplitScan : ScanHooks {
+  const uint64_t *keys;
+  int64_t n;
+  int ppl, sorted_digits, max_split;
+  uint64_t *out;
+  unsigned long long cap;
+  Counters *cnt;
+  int lmax;  // deepest level this thread has seen
+  __device__ unsigned long long value(int i) {
     int cprev, cnext;
     split_range(keys, n, ppl, i, cprev, cnext, max_split);
-    unsigned long long c = 0;
-    if (cnext > cprev) {
-      if (cnext >= MAXD) {
-        atomicExch(&cnt->too_deep, 1);
-      } else if (sorted_digits < MAXD && cnext >= sorted_digits) {
-        atomicExch(&cnt->need_full_sort, 1);
-      } else {
-        c = (unsigned long long)(cnext - cprev);
-        lmax = max(lmax, cnext);
-      }
+    if (cnext <= cprev) return 0;
+    if (cnext >= MAXD) {
+      atomicExch(&cnt->too_deep, 1);
+      return 0;
     }
-    counts[i] = c;
+    if (sorted_digits < MAXD && cnext >= sorted_digits) {
+      atomicExch(&cnt->need_full_sort, 1);
+      return 0;
+    }
+    lmax = max(lmax, cnext);
+    return (unsigned long long)(cnext - cprev);
   }
-  for (int o = 16; o >= 1; o >>= 1) lmax = max(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
-  if ((threadIdx.x & 31) == 0 && lmax >= 0) atomicMax(&cnt->max_level, lmax);
-}
-
-// writes the split boxes at their scanned positions: point-major, so every
-// level's boxes come out in increasing morton order
-__global__ void k_split_emit(const uint64_t *__restrict__ keys, int64_t n, int ppl,
-                             const unsigned long long *__restrict__ counts,
-                             const unsigned long long *__restrict__ pos, uint64_t *__restrict__ out,
-                             unsigned long long cap, Counters *cnt, int max_split,
-                             const int *__restrict__ sort_fail) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    if (i == n - 1) {
-      cnt->s0_count = pos[i] + counts[i];
-      cnt->sort_fail = *sort_fail;  // the point sort and the scan ran before
-    }
-    if (!counts[i]) continue;
+  __device__ void emit(int i, unsigned long long pos, unsigned long long v) const {
+    if (i == n - 1) cnt->s0_count = pos + v;
+    if (!v) return;
     int cprev, cnext;
     split_range(keys, n, ppl, i, cprev, cnext, max_split);
     const uint64_t k = keys[i];
     for (int m = cprev + 1; m <= cnext; ++m) {
-      const unsigned long long p = pos[i] + (unsigned long long)(m - cprev - 1);
+      const unsigned long long p = pos + (unsigned long long)(m - cprev - 1);
       if (p < cap)
         out[p] = box_code(m, k >> (2 * (MAXD - m)));
       else
         atomicExch(&cnt->overflow, 1);
     }
   }
-}
+  __device__ void end() const {
+    const int l = __reduce_max_sync(0xffffffffu, lmax);
+    if ((threadIdx.x & 31) == 0 && l >= 0) atomicMax(&cnt->max_level, l);
+  }
+};
 
 // split-box count and level count of a tree from its split counters
 // (n0 = 0: the root alone, one level)
@@ -311,9 +304,17 @@ __device__ __forceinline__ int split_levels(const Counters *split, int64_t n0) {
 }
 
 // bounds[l] = first index of a code of level >= l, l = 0..L + 1 (codes sorted
-// by level; n and the tree's L from its split counters, bounds [MAXD + 3])
-__global__ void k_level_starts(const uint64_t *__restrict__ codes, const Counters *split,
-                               unsigned long long cap, int *__restrict__ bounds) {
+// by level; n and the tree's L from its split counters, bounds [MAXD + 3]).
+// The failure flag joins the counters (the point sort, the split scan and the
+// box sort ran before) and the balance's hash table is emptied.
+__global__ void k_level_starts(const uint64_t *__restrict__ codes, Counters *split,
+                               unsigned long long cap, int *__restrict__ bounds,
+                               const int *__restrict__ sort_fail, ulonglong2 *__restrict__ tab,
+                               int64_t tab_pairs) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) split->sort_fail = *sort_fail;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < tab_pairs;
+       i += (int64_t)gridDim.x * blockDim.x)
+    tab[i] = make_ulonglong2(~0ull, ~0ull);
   const int64_t n = split_boxes(split, cap);
   const int L = split_levels(split, n) + 1;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
@@ -447,70 +448,71 @@ __global__ void __launch_bounds__(TPB) k_balance_xlist(
 // --- 6. parent boxes ------------------------------------------------------------
 // Parent boxes (split boxes, then X-list leaves) as compact sort keys:
 // ((level << mb) | morton) << 1 | is_xlist, mb = 2 * (deepest parent level).
-__global__ void k_parent_keys(const uint64_t *__restrict__ s0, int64_t n0,
-                              const uint64_t *__restrict__ f, int64_t nf,
-                              const uint64_t *__restrict__ xl, int64_t nx, int mb,
-                              uint64_t *__restrict__ keys) {
-  const int64_t total = n0 + nf + nx;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t c = (i < n0) ? s0[i] : (i < n0 + nf) ? f[i - n0] : xl[i - n0 - nf];
+struct SrcParents {
+  const uint64_t *s0, *f, *xl;
+  int64_t n0, nf;
+  int mb;
+  __device__ uint64_t key(int i) const {
+    const uint64_t c = i < n0 ? __ldg(s0 + i) : i < n0 + nf ? __ldg(f + (i - n0)) : __ldg(xl + (i - n0 - nf));
     const uint64_t v = (uint64_t(code_level(c)) << mb) | code_morton(c);
-    keys[i] = (v << 1) | uint64_t(i >= n0 + nf);
+    return (v << 1) | uint64_t(i >= n0 + nf);
   }
-}
+  __device__ int val(int) const { return 0; }
+};
 
-// sorted compact keys -> box codes, X-list flags, real flags (children of
-// split boxes form real sibling groups) and level starts pb[0..L]
-__global__ void k_parent_decode(const uint64_t *__restrict__ keys, int64_t n, int mb, int L,
-                                uint64_t *__restrict__ codes, uint8_t *__restrict__ isx,
-                                int *__restrict__ real, int *__restrict__ pb) {
-  const uint64_t mmask = (uint64_t(1) << mb) - 1;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
+// Sorted compact keys -> box codes and X-list flags of the parent boxes, their
+// level starts pb[0..L], and from these directly what the parent boxes fix: the
+// children of parent e are the nodes 1 + 4 e .. 4 + 4 e (the levels follow one
+// another in both orders), so the level offsets are off[l + 1] = 1 + 4 pb[l] and
+// a node's code needs no search.  Scanned over the parents for the real sibling
+// groups (the children of split boxes, not of X-list leaves): their first nodes
+// rg and their bounds by level rgb[0..L]; rgb[L + 1]: the sort failure flag,
+// read back with the bounds.  pb and rgb are zero before.
+struct ParentScan : ScanHooks {
+  const uint64_t *keys;
+  int n, mb, L;
+  uint64_t *codes;
+  uint8_t *isx;
+  int *pb, *rgb, *off, *rg;
+  uint64_t *code;
+  uint8_t *flags;
+  const int *sort_fail;
+  __device__ int level(int i) const { return int((keys[i] >> 1) >> mb); }
+  __device__ void start(int l, int i) const {
+    pb[l] = i;
+    if (l < L) off[l + 1] = 1 + 4 * i;
+  }
+  __device__ int value(int i) const {
     const uint64_t k = keys[i];
-    const int x = int(k & 1);
-    const int lv = int((k >> 1) >> mb);
-    codes[i] = box_code(lv, (k >> 1) & mmask);
+    const int x = int(k & 1), lv = int((k >> 1) >> mb);
+    const uint64_t morton = (k >> 1) & ((uint64_t(1) << mb) - 1);
+    codes[i] = box_code(lv, morton);
     isx[i] = uint8_t(x);
-    real[i] = 1 - x;
-    const int prev = (i == 0) ? -1 : int((keys[i - 1] >> 1) >> mb);
-    for (int l = prev + 1; l <= min(lv, L); ++l) pb[l] = int(i);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      code[1 + 4 * i + j] = (morton << 2) | uint64_t(j);
+      flags[1 + 4 * i + j] = x ? NF_FAKE : 0;
+    }
+    for (int l = (i == 0 ? -1 : level(i - 1)) + 1; l <= min(lv, L); ++l) start(l, i);
     if (i == n - 1)
-      for (int l = lv + 1; l <= L; ++l) pb[l] = int(n);
+      for (int l = lv + 1; l <= L; ++l) start(l, n);
+    if (i == 0) {
+      off[0] = 0;
+      code[0] = 0;
+      flags[0] = 0;
+      if (*sort_fail) failed();
+    }
+    return 1 - x;
   }
-}
-
-// real sibling groups: the children of split boxes (not of X-list leaves)
-// (rgb[L + 1]: the tree's sort failure flag, read back with the bounds;
-// the last thread of the block writes the level offsets, as k_level_offsets)
-__device__ __forceinline__ void level_offsets(const int *__restrict__ pb, int L, int *__restrict__ off) {
-  off[0] = 0;
-  if (L >= 1) off[1] = 1;
-  for (int m = 1; m < L; ++m) off[m + 1] = off[m] + 4 * (pb[m] - pb[m - 1]);
-}
-
-__global__ void k_real_bounds(const int *__restrict__ pos, const int *__restrict__ real, int64_t n,
-                              const int *__restrict__ pb, int L, int *__restrict__ rgb,
-                              const int *__restrict__ sort_fail, int *__restrict__ off) {
-  int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l == (int)blockDim.x - 1) level_offsets(pb, L, off);  // blockDim.x > L + 1
-  if (l == L + 1) rgb[l] = *sort_fail;
-  if (l > L) return;
-  const int total = n ? pos[n - 1] + real[n - 1] : 0;
-  rgb[l] = (pb[l] < n) ? pos[pb[l]] : total;
-}
-
-__global__ void k_real_groups(const uint64_t *__restrict__ pkeys, const int *__restrict__ real,
-                              const int *__restrict__ pos, int64_t n, const int *__restrict__ pb,
-                              const int *__restrict__ off, int *__restrict__ rg) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    if (!real[e]) continue;
-    const int l = code_level(pkeys[e]);
-    rg[pos[e]] = off[l + 1] + 4 * int(e - pb[l]);
+  __device__ void emit(int i, int pos, int real) const {
+    if (real) rg[pos] = 1 + 4 * i;
+    const int lv = level(i);
+    for (int l = (i == 0 ? -1 : level(i - 1)) + 1; l <= min(lv, L); ++l) rgb[l] = pos;
+    if (i == n - 1)
+      for (int l = lv + 1; l <= L; ++l) rgb[l] = pos + real;
   }
-}
+  __device__ void failed() const { atomicExch(rgb + L + 1, 1); }
+};
 
 __device__ __forceinline__ int level_of(const int *__restrict__ off, int L, int g) {
   int lo = 0, hi = L;  // find largest l with off[l] <= g
@@ -525,34 +527,18 @@ __device__ __forceinline__ int level_of(const int *__restrict__ off, int L, int 
 }
 
 // --- 6. node arrays -----------------------------------------------------------
-// level offsets from the per-level parent-box bounds (one thread; a tree
-// without split boxes, else k_real_bounds writes them)
-__global__ void k_level_offsets(const int *__restrict__ pb, int L, int *__restrict__ off) {
+// a tree without split boxes: the root alone (else ParentScan writes these)
+__global__ void k_root(int *off, uint64_t *code, uint8_t *flags) {
   if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  level_offsets(pb, L, off);
+  off[0] = 0;
+  off[1] = 1;
+  code[0] = 0;
+  flags[0] = 0;
 }
 
 // The node kernels are launched for an upper bound of the node count (the
 // host does not wait for it); the count itself is off[L] in device memory.
-__global__ void k_node_codes(const int *__restrict__ off, int L, int total_ub,
-                             const uint64_t *__restrict__ pkeys, const uint8_t *__restrict__ pisx,
-                             const int *__restrict__ pb, uint64_t *__restrict__ code,
-                             uint8_t *__restrict__ flags) {
-  const int total = min(off[L], total_ub);
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
-    const int m = level_of(off, L, g);
-    if (m == 0) {
-      code[g] = 0;
-      flags[g] = 0;
-      continue;
-    }
-    const int j = g - off[m];
-    const int e = pb[m - 1] + (j >> 2);
-    code[g] = (code_morton(pkeys[e]) << 2) | uint64_t(j & 3);
-    flags[g] = pisx[e] ? NF_FAKE : 0;
-  }
-}
-
+//
 // Per node: 12 binary searches (8 colleagues, point range bot / top,
 // parent, children), run as one branchless loop: a search over a range of n
 // keys takes ceil(log2 n) steps whatever it looks for, so the searches of
@@ -725,49 +711,32 @@ __global__ void k_interactions(const int *__restrict__ off, int L, int total_ub,
 }
 
 // S2M nodes: see TreeDev::uplist
-__global__ void k_up_flags(const int *__restrict__ off, int L, int total_ub,
-                           const uint8_t *__restrict__ flags, const int *__restrict__ bot,
-                           const int *__restrict__ top, int *__restrict__ f) {
-  const int total = min(off[L], total_ub);
-  const int g0 = L > 2 ? off[2] : total;
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < total_ub; g += gridDim.x * blockDim.x) {
-    if (g >= total) {
-      f[g] = 0;
-      continue;
-    }
+struct UpScan : ScanHooks {
+  const int *off;
+  int L, total_ub;
+  const uint8_t *flags;
+  const int *bot, *top;
+  int *list, *count;
+  __device__ int value(int g) const {
+    const int total = min(off[L], total_ub);
+    if (g >= total || g < (L > 2 ? off[2] : total)) return 0;
     const uint8_t fl = flags[g];
     const bool up = (((fl & NF_LEAF) && !(fl & NF_XLIST)) || (fl & NF_FAKE)) && top[g] > bot[g];
-    f[g] = (g >= g0 && up) ? 1 : 0;
+    return up ? 1 : 0;
   }
-}
-
-__global__ void k_up_scatter(const int *__restrict__ off, int L, int total_ub,
-                             const int *__restrict__ f, const int *__restrict__ pos,
-                             int *__restrict__ list, int *__restrict__ count) {
-  const int total = min(off[L], total_ub);
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
-    if (f[g]) list[pos[g]] = g;
-    if (g == total - 1) *count = pos[g] + f[g];
+  __device__ void fallback(int g) const {
+    if (g == 0) *count = 0;
   }
-}
+  __device__ void emit(int g, int pos, int v) const {
+    if (v) list[pos] = g;
+    if (g == total_ub - 1) *count = pos + v;
+  }
+};
 
 uint64_t next_pow2(uint64_t v) {
   uint64_t p = 1;
   while (p < v) p <<= 1;
   return p;
-}
-
-// stable sort of keys on bits [begin_bit, end_bit)
-template <class K>
-void sort_keys(const K *kin, K *kout, int64_t n, int begin_bit, int end_bit, int *fail,
-               cudaStream_t s, const unsigned long long *n_dev = nullptr) {
-  radix_sort<K, false>(SrcKeys<K>{kin, nullptr}, EmitPairs<K>{kout, nullptr}, n, begin_bit, end_bit,
-                       fail, s, n_dev);
-}
-
-template <class T>
-void exclusive_sum(const T *in, T *out, int64_t n, int *fail, bool offsets, cudaStream_t s) {
-  prefix_sum<T, false>(in, out, n, fail, offsets, s);
 }
 
 // blocks of a cooperative launch: all co-resident, one per SM (the grid
@@ -889,7 +858,7 @@ size_t point_sort_bytes(int64_t n, int digits) {
 template <class K>
 void point_sort_run(const double *x, const double *y, int64_t n, const TreeHost &th, int digits,
                     uint64_t *keys, int *perm, double *sx, double *sy, void *scratch,
-                    size_t bytes, int *fail, cudaStream_t s) {
+                    size_t bytes, int *fail, cudaStream_t s, ZeroPool *zeroed) {
   double scale, margin;
   key_params(th.x0, th.y0, th.w0, scale, margin);
   int b0, b1;
@@ -897,7 +866,7 @@ void point_sort_run(const double *x, const double *y, int64_t n, const TreeHost 
   const SrcPoints<K> src{x, y, th.x0, th.y0, th.w0, scale, margin};
   const EmitPoints<K> emit{x, y, th.x0, th.y0, th.w0, scale, margin, keys, perm, sx, sy};
   radix_sort_run<K, true>(src, emit, n, b0, b1, scratch, bytes,
-                          radix_grid<K, true>(point_sort_kernel<K>(), n), fail, s);
+                          radix_grid<K, true>(point_sort_kernel<K>(), n), fail, s, nullptr, zeroed);
 }
 }  // namespace
 
@@ -910,20 +879,21 @@ size_t sort_points_scratch_bytes(int64_t n, int sorted_digits) {
 
 void sort_points_scratch(const double *x, const double *y, int64_t n, const TreeHost &th,
                          int sorted_digits, uint64_t *keys, int *perm, double *sx, double *sy,
-                         void *scratch, size_t scratch_bytes, int *fail, cudaStream_t s) {
+                         void *scratch, size_t scratch_bytes, int *fail, cudaStream_t s,
+                         ZeroPool *zeroed) {
   if (n <= 0) return;
   const int digits = clamp_digits(sorted_digits);
   if (digits <= KEY32_DIGITS)
     point_sort_run<uint32_t>(x, y, n, th, digits, keys, perm, sx, sy, scratch, scratch_bytes, fail,
-                             s);
+                             s, zeroed);
   else
     point_sort_run<uint64_t>(x, y, n, th, digits, keys, perm, sx, sy, scratch, scratch_bytes, fail,
-                             s);
+                             s, zeroed);
 }
 
 void sort_points(const double *x, const double *y, int64_t n, const TreeHost &th,
                  DevBuf<uint64_t> &keys, DevBuf<int> &perm, cudaStream_t s, int sorted_digits,
-                 double *sx, double *sy, int *fail) {
+                 double *sx, double *sy, int *fail, ZeroPool *zeroed) {
   keys.alloc(n, s);
   perm.alloc(n, s);
   if (n == 0) return;
@@ -931,7 +901,7 @@ void sort_points(const double *x, const double *y, int64_t n, const TreeHost &th
   DevBuf<unsigned char> tmp;
   tmp.alloc(bytes, s);
   sort_points_scratch(x, y, n, th, sorted_digits, keys.get(), perm.get(), sx, sy, tmp.get(), bytes,
-                      fail, s);
+                      fail, s, zeroed);
 }
 
 // --- targets into leaves without a sort ---------------------------------------
@@ -1029,24 +999,22 @@ void build_tree(TreeDev &td, TreeHost &th, const double *x, const double *y, int
   // balance kernel's; both come back through a pinned block in one copy, at
   // the tree build's one host wait (after the balance kernel: the level sort
   // and the balance kernel read the split counts on the device)
-  DevBuf<Counters> cnt;
-  cnt.alloc(2, s);
-  Counters *csplit = cnt.get(), *cbal = cnt.get() + 1;
+  td.sort_fail.alloc(TREE_ZEROED_INTS, s);
+  ZeroPool zeroed(td.sort_fail.get(), TREE_ZEROED_INTS * sizeof(int), s);
+  int *sort_fail = zeroed.take<int>(1);  // (the block's first element)
+  Counters *cnt = zeroed.take<Counters>(2), *csplit = cnt, *cbal = cnt + 1;
   static_assert(2 * sizeof(Counters) <= PINNED_INTS * sizeof(int), "pinned block too small");
   std::unique_ptr<int, void (*)(int *)> hblk(pinned_acquire(), pinned_release);
   Counters *hcs = reinterpret_cast<Counters *>(hblk.get());
   const Counters &hc = hcs[0], &hb = hcs[1];
   auto read_counters = [&] {
-    FMMB_CUDA(cudaMemcpyAsync(hcs, cnt.get(), 2 * sizeof(Counters), cudaMemcpyDeviceToHost, s));
+    FMMB_CUDA(cudaMemcpyAsync(hcs, cnt, 2 * sizeof(Counters), cudaMemcpyDeviceToHost, s));
     FMMB_CUDA(cudaStreamSynchronize(s));
   };
   const unsigned long long cap0 = (unsigned long long)MAXD * (n / (ppl + 1) + 1) + 64;
   DevBuf<uint64_t> s0raw, s0;
-  DevBuf<unsigned long long> scount, spos;
   s0raw.alloc(cap0, s);
   s0.alloc(cap0, s);
-  scount.alloc(n, s);
-  spos.alloc(n, s);
   DevBuf<int> s0b;            // split boxes' level starts
   s0b.alloc(MAXD + 3, s);
   // balance buffers: first sized from an estimate of the split-box count
@@ -1055,25 +1023,22 @@ void build_tree(TreeDev &td, TreeHost &th, const double *x, const double *y, int
   const unsigned long long n0_est = 2ull * (unsigned long long)(n / (ppl + 1)) + 64;
   unsigned long long capf = 8ull * n0_est + 4096, capx = 8ull * n0_est + 4096;
   DevBuf<uint64_t> tab, forced, xl;
-  DevBuf<unsigned long long> fb;
   uint64_t hcap = 0;
-  auto launch_balance = [&] {
+  auto alloc_balance = [&] {
     hcap = next_pow2(2 * (n0_est + capf + capx));
     tab.alloc(hcap, s);
-    FMMB_CUDA(cudaMemsetAsync(tab.get(), 0xff, hcap * sizeof(uint64_t), s));
     forced.alloc(capf, s);
     xl.alloc(capx, s);
-    fb.alloc(MAXD + 2, s);
-    fb.zero(s);
-    FMMB_CUDA(cudaMemsetAsync(cbal, 0, sizeof(Counters), s));
+  };
+  auto launch_balance = [&] {  // (its table empty, its counters zero)
+    unsigned long long *fbp = zeroed.take<unsigned long long>(MAXD + 2);
     const uint64_t *s0p = s0.get();
     const int *s0bp = s0b.get();
     uint64_t *fp = forced.get(), *xp = xl.get(), *tp = tab.get();
-    unsigned long long *fbp = fb.get();
     uint64_t mask = hcap - 1;
     Counters *cp = cbal;
     const Counters *sp = csplit;
-    const int *sfp = td.sort_fail.get();
+    const int *sfp = sort_fail;
     unsigned long long c0 = cap0;
     void *args[] = {&s0p, &s0bp, &fp, &fbp, &capf, &xp, &capx, &tp, &mask, &cp, &sfp, &sp, &c0};
     FMMB_CUDA(cudaLaunchCooperativeKernel((const void *)k_balance_xlist,
@@ -1088,26 +1053,22 @@ void build_tree(TreeDev &td, TreeHost &th, const double *x, const double *y, int
   std::unique_ptr<PhaseTimer> t_bal;
   td.sx.alloc(n, s);
   td.sy.alloc(n, s);
-  td.sort_fail.alloc(1, s);
-  td.sort_fail.zero(s);
+  alloc_balance();
   for (int digits = SORT_DIGITS;; digits = MAXD) {
-    sort_points(x, y, n, th, td.pkeys, td.ordv, s, digits, td.sx.get(), td.sy.get(),
-                td.sort_fail.get());
-    FMMB_CUDA(cudaMemsetAsync(csplit, 0, sizeof(Counters), s));
-    k_split_counts<<<grid_for(n, TPB), TPB, 0, s>>>(td.pkeys.get(), n, ppl, digits, scount.get(),
-                                                     csplit, max_split);
-    FMMB_CUDA(cudaGetLastError());
-    // (k_split_emit checks its writes against the capacity)
-    exclusive_sum(scount.get(), spos.get(), n, td.sort_fail.get(), false, s);
-    k_split_emit<<<grid_for(n, TPB), TPB, 0, s>>>(td.pkeys.get(), n, ppl, scount.get(), spos.get(),
-                                                   s0raw.get(), cap0, csplit, max_split,
-                                                   td.sort_fail.get());
-    FMMB_CUDA(cudaGetLastError());
+    sort_points(x, y, n, th, td.pkeys, td.ordv, s, digits, td.sx.get(), td.sy.get(), sort_fail,
+                &zeroed);
+    // (it checks its writes against the capacity)
+    scan_each<unsigned long long, false>(
+        SplitScan{{}, td.pkeys.get(), n, ppl, digits, max_split, s0raw.get(), cap0, csplit, -1}, n,
+        sort_fail, zeroed, s);
     t_split.reset();
     t_bal.reset(new PhaseTimer(PH_TREE_BALANCE, s));
-    sort_keys(s0raw.get(), s0.get(), (int64_t)cap0, LEVEL_SHIFT, LEVEL_SHIFT + 5,
-              td.sort_fail.get(), s, &csplit->s0_count);
-    k_level_starts<<<grid_for((int64_t)cap0, TPB), TPB, 0, s>>>(s0.get(), csplit, cap0, s0b.get());
+    radix_sort<uint64_t, false>(SrcKeys<uint64_t>{s0raw.get(), nullptr},
+                                EmitPairs<uint64_t>{s0.get(), nullptr}, (int64_t)cap0, LEVEL_SHIFT,
+                                LEVEL_SHIFT + 5, sort_fail, s, &csplit->s0_count, &zeroed);
+    k_level_starts<<<grid_for(std::max<int64_t>(cap0, hcap / 2), TPB), TPB, 0, s>>>(
+        s0.get(), csplit, cap0, s0b.get(), sort_fail, reinterpret_cast<ulonglong2 *>(tab.get()),
+        (int64_t)(hcap / 2));
     FMMB_CUDA(cudaGetLastError());
     launch_balance();
     read_counters();
@@ -1118,17 +1079,15 @@ void build_tree(TreeDev &td, TreeHost &th, const double *x, const double *y, int
     if (!hc.need_full_sort || digits == MAXD) break;
     t_bal.reset();
     t_split.reset(new PhaseTimer(PH_TREE_SPLITS, s));
+    FMMB_CUDA(cudaMemsetAsync(cnt, 0, 2 * sizeof(Counters), s));
   }
-  scount.release();
-  spos.release();
   const int64_t n0 = (int64_t)hc.s0_count;
   const int L = (n0 > 0) ? hc.max_level + 2 : 1;
   th.L = L;
 
-  DevBuf<uint64_t> pk, pkc, pks;  // parent boxes: compact keys (unsorted, sorted), codes
+  DevBuf<uint64_t> pkc, pks;  // parent boxes: sorted compact keys, codes
   DevBuf<uint8_t> pxs;
-  DevBuf<int> pb, preal, ppos;
-  int64_t np = 0;
+  int64_t np = 0, nf = 0;
   const int mb = 2 * (L - 2);  // morton bits of the deepest parent level
   if (n0 > 0) {
     for (int attempt = 0;; ++attempt) {
@@ -1139,40 +1098,41 @@ void build_tree(TreeDev &td, TreeHost &th, const double *x, const double *y, int
       FMMB_CHECK(attempt < 6, ERR_CAPACITY, "tree balance buffers overflow");
       capf = std::max(4 * capf, 8ull * n0 + 4096);
       capx = std::max(4 * capx, 8ull * n0 + 4096);
+      alloc_balance();
+      FMMB_CUDA(cudaMemsetAsync(tab.get(), 0xff, hcap * sizeof(uint64_t), s));
+      FMMB_CUDA(cudaMemsetAsync(cbal, 0, sizeof(Counters), s));
       launch_balance();
       read_counters();
     }
-    const int64_t nf = (int64_t)hb.f_count, nx = (int64_t)hb.x_count;
-    np = n0 + nf + nx;
-    pk.alloc(np, s);
-    k_parent_keys<<<grid_for(np, TPB), TPB, 0, s>>>(s0.get(), n0, forced.get(), nf, xl.get(), nx,
-                                                     mb, pk.get());
-    FMMB_CUDA(cudaGetLastError());
-    // 6: sorted parent boxes, per-level bounds, real sibling groups
+    nf = (int64_t)hb.f_count;
+    np = n0 + nf + (int64_t)hb.x_count;
+  }
+  // every parent box has 4 children: 1 + 4 np nodes, at most np real groups
+  const int total_ub = 1 + 4 * int(np);
+  td.rg.alloc(np > 0 ? np : 1, s);
+  td.dev_off.alloc(L + 1, s);
+  td.code.alloc(total_ub, s);
+  td.flags.alloc(total_ub, s);
+  // pb[0..L], the real-group bounds rgb[0..L] and the sort failure flag share
+  // one buffer: one copy back
+  int *pb = zeroed.take<int>(2 * (L + 1) + 1);
+  pks.alloc(np > 0 ? np : 1, s);
+  pxs.alloc(np > 0 ? np : 1, s);
+  if (np > 0) {
+    // 6: sorted parent boxes, per-level bounds, node codes, real sibling groups
     t_bal.reset();
     pkc.alloc(np, s);
-    sort_keys(pk.get(), pkc.get(), np, 0, 1 + mb + 5, td.sort_fail.get(), s);
-    pks.alloc(np, s);
-    pxs.alloc(np, s);
-    preal.alloc(np, s);
-    ppos.alloc(np, s);
-    // pb[0..L], the real-group bounds rgb[0..L] and the sort failure flag
-    // share one buffer: one copy back
-    pb.alloc(2 * (L + 1) + 1, s);
-    k_parent_decode<<<grid_for(np, TPB), TPB, 0, s>>>(pkc.get(), np, mb, L, pks.get(), pxs.get(),
-                                                       preal.get(), pb.get());
-    FMMB_CUDA(cudaGetLastError());
-    exclusive_sum(preal.get(), ppos.get(), np, td.sort_fail.get(), true, s);
-    td.dev_off.alloc(L + 1, s);
-    k_real_bounds<<<1, 64, 0, s>>>(ppos.get(), preal.get(), np, pb.get(), L, pb.get() + L + 1,
-                                   td.sort_fail.get(), td.dev_off.get());
-    FMMB_CUDA(cudaGetLastError());
+    radix_sort<uint64_t, false>(SrcParents{s0.get(), forced.get(), xl.get(), n0, nf, mb},
+                                EmitPairs<uint64_t>{pkc.get(), nullptr}, np, 0, 1 + mb + 5,
+                                sort_fail, s, nullptr, &zeroed);
+    scan_each<int, false>(
+        ParentScan{{}, pkc.get(), int(np), mb, L, pks.get(), pxs.get(), pb, pb + L + 1,
+                   td.dev_off.get(), td.rg.get(), td.code.get(), td.flags.get(), sort_fail},
+        np, sort_fail, zeroed, s);
   } else {
-    pb.alloc(2 * (L + 1) + 1, s);
-    pb.zero(s);
-    pks.alloc(1, s);
-    pxs.alloc(1, s);
+    k_root<<<1, 1, 0, s>>>(td.dev_off.get(), td.code.get(), td.flags.get());
   }
+  FMMB_CUDA(cudaGetLastError());
 
   t_bal.reset();
   PhaseTimer t_nodes(PH_TREE_NODES, s);
@@ -1184,22 +1144,7 @@ void build_tree(TreeDev &td, TreeHost &th, const double *x, const double *y, int
   }
   // level offsets on the device; their host copy (with the real-group
   // bounds) travels back without a wait (finalize_tree)
-  if (n0 == 0) {  // (otherwise k_real_bounds wrote them)
-    td.dev_off.alloc(L + 1, s);
-    k_level_offsets<<<1, 1, 0, s>>>(pb.get(), L, td.dev_off.get());
-    FMMB_CUDA(cudaGetLastError());
-  }
-  begin_pending_counts(th, pb.get(), 2 * (L + 1), s);
-  // every parent box has 4 children: at most 1 + 4 np nodes, np real groups
-  const int total_ub = 1 + 4 * int(np);
-  td.rg.alloc(np > 0 ? np : 1, s);
-  if (np > 0) {
-    k_real_groups<<<grid_for(np, TPB), TPB, 0, s>>>(pks.get(), preal.get(), ppos.get(), np, pb.get(),
-                                                     td.dev_off.get(), td.rg.get());
-    FMMB_CUDA(cudaGetLastError());
-  }
-  td.code.alloc(total_ub, s);
-  td.flags.alloc(total_ub, s);
+  begin_pending_counts(th, pb, 2 * (L + 1), s);
   td.xmin.alloc(total_ub, s);
   td.ymin.alloc(total_ub, s);
   td.xmid.alloc(total_ub, s);
@@ -1212,13 +1157,9 @@ void build_tree(TreeDev &td, TreeHost &th, const double *x, const double *y, int
   td.il.alloc(int64_t(total_ub) * N_OFFSETS, s);
   td.ix.alloc(total_ub, s);
   td.iy.alloc(total_ub, s);
-  k_node_codes<<<grid_for(total_ub, TPB), TPB, 0, s>>>(td.dev_off.get(), L, total_ub, pks.get(),
-                                                         pxs.get(), pb.get(), td.code.get(),
-                                                         td.flags.get());
-  FMMB_CUDA(cudaGetLastError());
   k_node_attrs<<<grid_for(total_ub, TPB), TPB, 0, s>>>(
       td.dev_off.get(), L, total_ub, th.x0, th.y0, th.w0, td.pkeys.get(), n, pks.get(), pxs.get(),
-      pb.get(), td.code.get(), td.flags.get(), td.xmin.get(), td.ymin.get(), td.xmid.get(),
+      pb, td.code.get(), td.flags.get(), td.xmin.get(), td.ymin.get(), td.xmid.get(),
       td.ymid.get(), td.bot.get(), td.top.get(), td.parent.get(), td.child.get(), td.coll.get(),
       td.ix.get(), td.iy.get());
   FMMB_CUDA(cudaGetLastError());
@@ -1227,22 +1168,11 @@ void build_tree(TreeDev &td, TreeHost &th, const double *x, const double *y, int
       td.ix.get(), td.iy.get(), td.bot.get(), td.top.get(), td.il.get());
   FMMB_CUDA(cudaGetLastError());
   // S2M node list
-  {
-    DevBuf<int> f, pos;
-    f.alloc(total_ub, s);
-    pos.alloc(total_ub, s);
-    td.uplist.alloc(total_ub, s);
-    td.n_up.alloc(1, s);
-    k_up_flags<<<grid_for(total_ub, TPB), TPB, 0, s>>>(td.dev_off.get(), L, total_ub,
-                                                         td.flags.get(), td.bot.get(), td.top.get(),
-                                                         f.get());
-    FMMB_CUDA(cudaGetLastError());
-    exclusive_sum(f.get(), pos.get(), total_ub, td.sort_fail.get(), true, s);
-    k_up_scatter<<<grid_for(total_ub, TPB), TPB, 0, s>>>(td.dev_off.get(), L, total_ub, f.get(),
-                                                           pos.get(), td.uplist.get(),
-                                                           td.n_up.get());
-    FMMB_CUDA(cudaGetLastError());
-  }
+  td.uplist.alloc(total_ub, s);
+  td.n_up.alloc(1, s);
+  scan_each<int, false>(UpScan{{}, td.dev_off.get(), L, total_ub, td.flags.get(), td.bot.get(),
+                               td.top.get(), td.uplist.get(), td.n_up.get()},
+                        total_ub, sort_fail, zeroed, s);
 }
 
 }  // namespace fmmb

@@ -31,6 +31,7 @@ __host__ __device__ inline void offset_of(int id, int &ox, int &oy) {
   ox = oy = 0;
 }
 
+constexpr int TREE_ZEROED_INTS = 4096;  // see TreeDev::sort_fail
 struct TreeDev {
   // points (sorted by key)
   DevBuf<uint64_t> pkeys;
@@ -50,8 +51,9 @@ struct TreeDev {
   // real leaves that are not X-list leaves, and fake leaves, holding points;
   // in node order (so level-major).  Count on the device.
   DevBuf<int> uplist, n_up;
-  // set to 1 by a radix sort of this tree (the build's or a target sort)
-  // whose grid barrier wait ran out; the sorted outputs are then invalid
+  // [0] is set to 1 by a radix sort or scan of this tree (the build's or a
+  // target sort) whose grid barrier wait ran out; the sorted outputs are then
+  // invalid.  The rest holds the build's own counters (ZeroPool).
   DevBuf<int> sort_fail;
 };
 
@@ -96,7 +98,7 @@ void build_tree(TreeDev &td, TreeHost &th, const double *x, const double *y, int
 void sort_points(const double *x, const double *y, int64_t n, const TreeHost &th,
                  DevBuf<uint64_t> &keys, DevBuf<int> &perm, cudaStream_t stream,
                  int sorted_digits = MAXD, double *sx = nullptr, double *sy = nullptr,
-                 int *fail = nullptr);
+                 int *fail = nullptr, ZeroPool *zeroed = nullptr);
 
 // The same into caller-provided memory: keys [n], perm [n], optional sx, sy
 // [n], and scratch of sort_points_scratch_bytes(n, sorted_digits) bytes.
@@ -106,7 +108,7 @@ size_t sort_points_scratch_bytes(int64_t n, int sorted_digits);
 // holding point i, -1 for none) and slot[i] (its place among the leaf's
 // points, in no particular order); count[node] (zeroed by the caller) gets
 // the points per leaf.  scatter_binned then writes the points leaf by leaf
-// (first[node]: the exclusive scan of count) with perm (position -> point).
+// (first[node]: the place of the leaf's first) with perm (position -> point).
 void bin_points(const double *x, const double *y, int64_t m, const TreeDev &td, const TreeHost &th,
                 int *count, int *leaf_of, int *slot, cudaStream_t s);
 void scatter_binned(const double *x, const double *y, int64_t m, const int *leaf_of,
@@ -114,6 +116,7 @@ void scatter_binned(const double *x, const double *y, int64_t m, const int *leaf
                     cudaStream_t s);
 void sort_points_scratch(const double *x, const double *y, int64_t n, const TreeHost &th,
                          int sorted_digits, uint64_t *keys, int *perm, double *sx, double *sy,
-                         void *scratch, size_t scratch_bytes, int *fail, cudaStream_t stream);
+                         void *scratch, size_t scratch_bytes, int *fail, cudaStream_t stream,
+                         ZeroPool *zeroed = nullptr);
 
 }  // namespace fmmb
