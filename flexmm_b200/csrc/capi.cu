@@ -211,9 +211,14 @@ KernelParams kernel_params(int kernel_id, const double *kparams) {
     int dev = 0;
     FMMB_CUDA(cudaGetDevice(&dev));
     if (!t.dev.count(dev)) {
+      // rows of coefficient pairs: an odd count is filled up with a zero
+      const int row = (t.ncheb + 1) / 2 * 2;
+      std::vector<double> h((size_t)t.noct * row, 0.0);
+      for (int o = 0; o < t.noct; ++o)
+        std::copy_n(t.coef.data() + (size_t)o * t.ncheb, t.ncheb, h.data() + (size_t)o * row);
       double *d = nullptr;
-      FMMB_CUDA(cudaMalloc((void **)&d, t.coef.size() * sizeof(double)));
-      FMMB_CUDA(cudaMemcpy(d, t.coef.data(), t.coef.size() * sizeof(double), cudaMemcpyHostToDevice));
+      FMMB_CUDA(cudaMalloc((void **)&d, h.size() * sizeof(double)));
+      FMMB_CUDA(cudaMemcpy(d, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice));
       t.dev[dev] = d;
     }
     kp.table = t.dev[dev];
