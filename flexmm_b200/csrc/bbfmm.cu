@@ -6,7 +6,11 @@
 //    M[a p + b] = sum_j T_a(x_j) T_b(y_j) tau_j (anterpolate2, bbfmm.py:11-24,
 //    source2pMs, bbfmm.py:186-196); no check-to-equivalent step;
 //  * M2M / L2L: the level-independent M2MC [NQ x 4NQ] and its transpose
-//    (bbfmm.py:145-161) on the contiguous child rows of each parent group;
+//    (bbfmm.py:145-161) on the contiguous child rows of each parent group.  A
+//    child's block of M2MC is the tensor product X (x) Y of two p x p matrices:
+//    a row as a p x p matrix C goes to X C Y^T, 4 p^3 operations a child instead
+//    of 2 p^4 (k_bb_shift).  Operators that are no such product (the entry point
+//    takes any) go through the row GEMM;
 //  * M2L: per level and offset VI K VI^T (bbfmm.py:101-122).  A width's 40
 //    operators share a space of at most 64 columns for the smooth kernels
 //    (fmm_bb_ops_set_basis): multipoles go into that basis, the KIFMM's M2L
@@ -198,6 +202,99 @@ struct BBPolicy : ChargePolicy<KF, NOUT, false, false> {
   }
 };
 
+// M2M (UP: the children's rows into their parent's, overwritten) or L2L (the
+// parent's row added to the children's) of one level by the operators' tensor
+// factors, a warp a parent or a child.  With D = X C Y^T as D^T = (Y C^T) X^T
+// the first product's accumulators are the second's operand as they lie (the k
+// index of a DMMA is free: 2 q and 2 q + 1 of the two steps), C is read from
+// global memory in the operand's own layout, and only the factors (fragments,
+// sep: Y then X, bb_shift_fragments in capi.cu) are staged.  Bound by latency
+// and the launches on coarse levels.  500k sources, p = 16, three passes of five
+// levels: M2M 1051 -> 176 us, L2L 477 -> 214 us (row GEMMs before).
+constexpr int SHIFT_WARPS = 4;
+template <int P, bool UP>
+__global__ void __launch_bounds__(32 * SHIFT_WARPS)
+    k_bb_shift(int p, int np, const double *__restrict__ sep, const int *__restrict__ parent,
+               const int *__restrict__ rg, int first, int units, double *rows) {
+  constexpr int NB = P / 8, KS = P / 4, F = 4 * P * P;
+  __shared__ double fy[F], fx[F];
+  for (int i = threadIdx.x; i < F; i += 32 * SHIFT_WARPS) {
+    fy[i] = __ldg(sep + i);
+    fx[i] = __ldg(sep + F + i);
+  }
+  __syncthreads();
+  pdl_wait();
+  pdl_trigger();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  for (int u = blockIdx.x * SHIFT_WARPS + warp; u < units; u += gridDim.x * SHIFT_WARPS) {
+    double out[NB][NB][2];
+#pragma unroll
+    for (int i = 0; i < NB; ++i)
+#pragma unroll
+      for (int j = 0; j < NB; ++j) out[i][j][0] = out[i][j][1] = 0.0;
+    auto load = [&](const double *row, double (&b)[NB][KS]) {
+#pragma unroll
+      for (int cb = 0; cb < NB; ++cb)
+#pragma unroll
+        for (int ks = 0; ks < KS; ++ks)
+          b[cb][ks] = 8 * cb + g < p && 4 * ks + q < p ? row[(8 * cb + g) * p + 4 * ks + q] : 0.0;
+    };
+    auto shift = [&](int c, const double (&b)[NB][KS]) {
+#pragma unroll
+      for (int rb = 0; rb < NB; ++rb) {
+        double v[NB][2];
+#pragma unroll
+        for (int cb = 0; cb < NB; ++cb) {
+          v[cb][0] = v[cb][1] = 0.0;
+#pragma unroll
+          for (int ks = 0; ks < KS; ++ks)
+            dmma(v[cb], fy[((c * NB + rb) * KS + ks) * 32 + lane], b[cb][ks]);
+        }
+#pragma unroll
+        for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+          for (int cb = 0; cb < NB; ++cb)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+              dmma(out[rb][nb], v[cb][h], fx[(((c * NB + nb) * NB + cb) * 2 + h) * 32 + lane]);
+      }
+    };
+    double *dst;
+    if (UP) {
+      const double *src = rows + (size_t)(first + 4 * u) * np;
+      dst = rows + (size_t)parent[first + 4 * u] * np;
+      double b[4][NB][KS];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) load(src + (size_t)c * np, b[c]);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) shift(c, b[c]);
+    } else {
+      const int node = rg[first + (u >> 2)] + (u & 3);
+      dst = rows + (size_t)node * np;
+      double b[NB][KS];
+      load(rows + (size_t)parent[node] * np, b);
+      shift(u & 3, b);
+    }
+#pragma unroll
+    for (int rb = 0; rb < NB; ++rb)
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int a = 8 * nb + 2 * q + j, b = 8 * rb + g;
+          if (a < p && b < p) dst[a * p + b] = UP ? out[rb][nb][j] : dst[a * p + b] + out[rb][nb][j];
+        }
+  }
+}
+
+template <bool UP>
+void bb_shift(const BBArgs &b, int first, int units, double *rows, cudaStream_t s) {
+  const dim3 grid(work_grid((units + SHIFT_WARPS - 1) / SHIFT_WARPS, 4));
+  launch_pdl(b.p <= 8 ? k_bb_shift<8, UP> : k_bb_shift<16, UP>, grid, dim3(32 * SHIFT_WARPS), 0, s,
+             b.p, b.np, UP ? b.m2m_sep : b.l2l_sep, b.td->parent.get(), b.td->rg.get(), first, units,
+             rows);
+}
+
 BBScale bb_scale(const TreeHost &th) {
   BBScale sc{};
   for (int m = 0; m < th.L && m < FMM_MAX_LEVELS_DEV; ++m) sc.inv_hw[m] = 2.0 / th.width[m];
@@ -222,6 +319,10 @@ void run_bb_upward(const BBArgs &b, const double *tau_s, double *mult, cudaStrea
     const int c_first = th.off[m + 1];
     const int n_groups = (th.off[m + 2] - th.off[m + 1]) / 4;
     if (n_groups == 0) continue;
+    if (b.m2m_sep) {
+      bb_shift<true>(b, c_first, n_groups, mult, s);
+      continue;
+    }
     // parent rows = children rows (contiguous, 4np wide) . M2MC^T (fmm.py:93-96)
     rowgemm(RowsContig{mult + (size_t)c_first * np, 4 * (int64_t)np, n_groups, 4 * np},
             StoreParents{td.parent.get(), mult, c_first, np}, row_tiles(n_groups), b.m2mct, np, np,
@@ -240,34 +341,38 @@ void run_bb_downward(const BBArgs &b, const double *mult, double *ple, double *z
     // M2L of these levels in one launch of the KIFMM's kernel, on rows of at most
     // 64: the coefficients themselves (p <= 8), or those in the common basis
     const bool basis = np > BB_RANK;
-    for (int m = 2; basis && m < th.L; ++m) {
-      const int r0 = th.off[m], n = th.off[m + 1] - th.off[m];
-      if (!b.fast[m]) continue;
-      rowgemm(RowsContig{mult + (size_t)r0 * np, np, n, np}, StoreRows{z + (size_t)r0 * BB_RANK, BB_RANK},
-              row_tiles(n), b.q[m], BB_RANK, BB_RANK, np, s);
-    }
+    // into the basis and back, all these levels in one launch each
+    RowsLevels in{}, back{};
+    for (int m = 2; basis && m < th.L; ++m)
+      if (b.fast[m]) {
+        in.add(th.off[m], th.off[m + 1] - th.off[m], b.q[m]);
+        back.add(th.off[m], th.off[m + 1] - th.off[m], b.q[m] + (size_t)np * BB_RANK);
+      }
+    in.base = mult;
+    in.ld = np;
+    back.base = zl;
+    back.ld = BB_RANK;
+    if (basis)
+      rowgemm(in, StoreRows{z, BB_RANK}, in.tile0[in.n], b.q[2], BB_RANK, BB_RANK, np, s);
     PassArgs a{};
     a.np = basis ? BB_RANK : np;
     a.th = b.th;
     a.td = b.td;
     a.ops_dev = b.ops_dev;
     run_m2l(a, basis ? z : mult, basis ? zl : ple, s);
-    for (int m = 2; basis && m < th.L; ++m) {
-      const int r0 = th.off[m], n = th.off[m + 1] - th.off[m];
-      if (!b.fast[m]) continue;
-      rowgemm(RowsContig{zl + (size_t)r0 * BB_RANK, BB_RANK, n, BB_RANK},
-              StoreRows{ple + (size_t)r0 * np, np}, row_tiles(n), b.q[m] + (size_t)np * BB_RANK, np,
-              np, BB_RANK, s);
-    }
+    if (basis) rowgemm(back, StoreRows{ple, np}, back.tile0[back.n], b.q[2], np, np, BB_RANK, s);
   }
   for (int m = 2; m < th.L; ++m) {
     const int lo = th.rg_lo[m], n_groups = th.rg_hi[m] - th.rg_lo[m];
     if (n_groups == 0) continue;
     if (m >= 3) {  // L2L from level m-1: children += parent local . M2MC (bbfmm.py:161, fmm.py:140-147)
       PhaseTimer timer(PH_DOWNWARD, s);
-      rowgemm(ParentRows{td.rg.get(), td.parent.get(), ple, lo, n_groups, np},
-              AddChildRows{td.rg.get(), ple, lo, np}, row_tiles(n_groups), b.m2mc, 4 * np, 4 * np,
-              np, s);
+      if (b.l2l_sep)
+        bb_shift<false>(b, lo, 4 * n_groups, ple, s);
+      else
+        rowgemm(ParentRows{td.rg.get(), td.parent.get(), ple, lo, n_groups, np},
+                AddChildRows{td.rg.get(), ple, lo, np}, row_tiles(n_groups), b.m2mc, 4 * np,
+                4 * np, np, s);
     }
     if (!b.fast[m]) {  // M2L of level m: tiles of one parity class, absent offsets skipped (fmm.py:118-131)
       PhaseTimer timer(PH_M2L, s);

@@ -276,6 +276,53 @@ void retain_pool_memory() {
   done_for = dev;
 }
 
+// The black-box M2M operator [p^2 x 4 p^2] as tensor factors: child c's block is
+// X_c (x) Y_c, read off its first rows and columns (T_0 = 1 keeps its value under
+// a shift, so X_c[0][0] = Y_c[0][0] = 1).  False where that is not the operator to
+// 2e-14 of its largest element (the factors of the Chebyshev shift reproduce it
+// to 5e-15 at most, p = 2 .. 16; any other is applied as it is).  Fragments for k_bb_shift
+// (bbfmm.cu): M2M's Y and X, then L2L's, Y^T and X^T, each [4][P x P], P = 8 or 16.
+bool bb_shift_fragments(int p, const double *m2mc, std::vector<double> &out) {
+  const int n = p * p, P = p <= 8 ? 8 : 16;
+  auto at = [&](int c, int a, int b, int a1, int b1) {
+    return m2mc[size_t(a * p + b) * 4 * n + c * n + a1 * p + b1];
+  };
+  auto X = [&](int c, int a, int a1) { return a < p && a1 < p ? at(c, a, 0, a1, 0) : 0.0; };
+  auto Y = [&](int c, int b, int b1) { return b < p && b1 < p ? at(c, 0, b, 0, b1) : 0.0; };
+  double big = 0.0, off = 0.0;
+  for (int c = 0; c < 4; ++c)
+    for (int a = 0; a < p; ++a)
+      for (int b = 0; b < p; ++b)
+        for (int a1 = 0; a1 < p; ++a1)
+          for (int b1 = 0; b1 < p; ++b1) {
+            const double v = at(c, a, b, a1, b1);
+            big = std::max(big, std::fabs(v));
+            const double d = std::fabs(v - X(c, a, a1) * Y(c, b, b1));
+            if (!(d <= off)) off = d;  // (NaN stays)
+          }
+  if (!(off <= 2e-14 * big)) return false;
+  const size_t F = size_t(4) * P * P;
+  out.assign(4 * F, 0.0);
+  const int NB = P / 8, KS = P / 4;
+  for (int t = 0; t < 2; ++t)  // M2M, L2L
+    for (int c = 0; c < 4; ++c)
+      for (int i = 0; i < NB; ++i)
+        for (int lane = 0; lane < 32; ++lane) {
+          const int g = lane >> 2, q = lane & 3;
+          for (int ks = 0; ks < KS; ++ks) {
+            const int r = 8 * i + g, k = 4 * ks + q;
+            out[2 * t * F + ((size_t(c) * NB + i) * KS + ks) * 32 + lane] = t ? Y(c, k, r) : Y(c, r, k);
+          }
+          for (int cb = 0; cb < NB; ++cb)
+            for (int h = 0; h < 2; ++h) {
+              const int r = 8 * i + g, k = 8 * cb + 2 * q + h;
+              out[(2 * t + 1) * F + (((size_t(c) * NB + i) * NB + cb) * 2 + h) * 32 + lane] =
+                  t ? X(c, k, r) : X(c, r, k);
+            }
+        }
+  return true;
+}
+
 // the 40 M2L operators of a black-box width as fragments: at(o, k, i) = column
 // k (source), row i (target) of offset o's operator; present[o] = 0: none
 template <class F>
@@ -305,6 +352,7 @@ struct fmm_ops {
   int p = 0;                  // black-box FMM: Chebyshev order
   DevBuf<double> bb_m2mc;     // black-box FMM: M2MC [np x 4np]
   DevBuf<double> bb_m2mct;    // and its transpose [4np x np]
+  DevBuf<double> bb_sep;      // tensor factors of both (bb_shift_fragments); empty: none
   std::vector<std::unique_ptr<LevelEntry>> levels;
 };
 
@@ -711,6 +759,12 @@ int fmm_bb_ops_create(int kernel_id, const double *kparams, int p, const double 
     o->bb_m2mct.alloc(ht.size(), 0);
     FMMB_CUDA(cudaMemcpy(o->bb_m2mct.get(), ht.data(), ht.size() * sizeof(double),
                          cudaMemcpyHostToDevice));
+    std::vector<double> sep;
+    if (bb_shift_fragments(p, m2mc, sep)) {
+      o->bb_sep.alloc(sep.size(), 0);
+      FMMB_CUDA(cudaMemcpy(o->bb_sep.get(), sep.data(), sep.size() * sizeof(double),
+                           cudaMemcpyHostToDevice));
+    }
     *out = o.release();
   });
 }
@@ -1066,6 +1120,10 @@ static BBArgs bb_args(fmm_plan *p, cudaStream_t) {
   b.th = &p->th;
   b.m2mc = p->ops->bb_m2mc.get();
   b.m2mct = p->ops->bb_m2mct.get();
+  if (const double *sep = p->ops->bb_sep.get()) {
+    b.m2m_sep = sep;
+    b.l2l_sep = sep + p->ops->bb_sep.n / 2;
+  }
   b.any_fast = false;
   for (int m = 0; m < p->th.L && m < FMM_MAX_LEVELS_DEV; ++m) {
     const LevelEntry *e = p->bound[m] >= 0 ? p->ops->levels[p->bound[m]].get() : nullptr;

@@ -66,6 +66,8 @@ struct BBArgs {
   const TreeDev *td;
   const TreeHost *th;
   const double *m2mc, *m2mct;
+  // M2M and L2L as tensor factors (fragments), where the operator is a product
+  const double *m2m_sep, *l2l_sep;
   const double *m2l_cat[FMM_MAX_LEVELS_DEV];
   // fast[m]: the level has its M2L operators as fragments (ops_dev), either as
   // they are (np <= 64) or in its common basis q[m]: Q [np x 64], then

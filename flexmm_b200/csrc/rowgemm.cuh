@@ -77,6 +77,48 @@ struct M2LRows {
   }
 };
 
+// Rows of several levels, each level with an operator of its own: level i's
+// rows r0[i] .. r0[i] + n_rows[i] - 1 of base (row stride ld) are the tiles
+// tile0[i] on, with W w[i].  (Six basis changes of a pass on 500k sources, one
+// launch a level: 36 launches, 501 us; so: 6, 206.)
+struct RowsLevels {
+  const double *base;
+  int64_t ld;
+  int n;
+  int tile0[FMM_MAX_LEVELS_DEV + 1], r0[FMM_MAX_LEVELS_DEV], n_rows[FMM_MAX_LEVELS_DEV];
+  const double *w[FMM_MAX_LEVELS_DEV];
+  void add(int first, int rows, const double *op) {
+    r0[n] = first;
+    n_rows[n] = rows;
+    w[n] = op;
+    tile0[n + 1] = tile0[n] + (rows + RG_TM - 1) / RG_TM;
+    ++n;
+  }
+  __device__ int level(int tile) const {
+    int i = 0;
+    while (i + 1 < n && tile0[i + 1] <= tile) ++i;
+    return i;
+  }
+  __device__ const double *op(int tile) const { return w[level(tile)]; }
+  __device__ int nblk() const { return 1; }
+  __device__ int row(int tile, int i) const {
+    const int l = level(tile), r = (tile - tile0[l]) * RG_TM + i;
+    return r < n_rows[l] ? r0[l] + r : -1;
+  }
+  __device__ const double *src(int r, int) const { return base + r * ld; }
+};
+
+// the operator of a tile: the load's own where it has one, else the launch's
+template <class Load>
+__device__ __forceinline__ auto tile_op(const Load &ld, int tile, const double *, int)
+    -> decltype(ld.op(tile)) {
+  return ld.op(tile);
+}
+template <class Load>
+__device__ __forceinline__ const double *tile_op(const Load &, int, const double *W, long) {
+  return W;
+}
+
 // ---- stores (two consecutive columns) ----
 struct StoreRows {  // Y row r at base + r * ld, overwritten
   double *base;
@@ -121,7 +163,7 @@ struct AddGroupRows {  // row 4 g + c -> ple[rg[lo+g] + c], added (M2L)
 
 template <class Load, class Store>
 __global__ void __launch_bounds__(RG_THREADS) k_rowgemm(Load ld, Store st,
-                                                       const double *__restrict__ W, int ldw,
+                                                       const double *__restrict__ W0, int ldw,
                                                        int M, int kb) {
   // two buffers of each chunk: chunk c + 1 of an input block is copied while
   // chunk c is multiplied
@@ -130,6 +172,7 @@ __global__ void __launch_bounds__(RG_THREADS) k_rowgemm(Load ld, Store st,
   __shared__ int rid[RG_TM];
   __shared__ const double *rsrc[RG_TM];
   const int tile = blockIdx.x, c0 = blockIdx.y * RG_TN;
+  const double *__restrict__ W = tile_op(ld, tile, W0, 0);
   if (threadIdx.x < RG_TM) rid[threadIdx.x] = ld.row(tile, threadIdx.x);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   const int r0 = 16 * (warp & 3), cw = 32 * (warp >> 2);
