@@ -1207,17 +1207,15 @@ int fmm_build_expansions_multi(fmm_plan *p, const double *tau, int n_rhs, int64_
     upload_level_ops(p, s);
     p->has_dipoles = false;
     p->sync.alloc(2, s);
-    p->sync.zero(s);
     PassArgs a = pass_args(p);
     p->tau_s.alloc((size_t)n_rhs * n, s);
     p->mult.alloc((size_t)n_rhs * cs, s);
     p->ple.alloc((size_t)n_rhs * cs, s);
     p->loc.alloc((size_t)n_rhs * cs, s);
-    p->mult.zero(s);
-    p->ple.zero(s);
-    p->loc.zero(s);
-    for (int r = 0; r < n_rhs; ++r)
-      gather_sorted(tau + (size_t)r * ld_tau, p->td.ordv.get(), n, p->tau_s.get() + (size_t)r * n, s);
+    ZeroBatch zb(s);
+    zb.add(p->mult).add(p->ple).add(p->loc).add(p->sync);
+    zb.run();
+    gather_sorted(tau, p->td.ordv.get(), n, p->tau_s.get(), s, n_rhs, ld_tau);
     // every pass once per level for all columns (column = blockIdx.y)
     run_upward(a, p->tau_s.get(), p->mult.get(), s, n_rhs, n, cs);
     run_m2l(a, p->mult.get(), p->ple.get(), s, n_rhs, cs);

@@ -1027,13 +1027,15 @@ void launch_items(const Pol &pol, const ItemArgs &ia, int64_t units, int per_sm,
   FMMB_CUDA(cudaGetLastError());
 }
 
-// FP64 direct sum (kernel_apply / kernel_apply_single_check,
-// flexmm/flexmm2d/helpers.py:91-116): all sources, one target per thread,
 // Several charge columns on one tree (multi-RHS): columns r0 .. r0 + R - 1
 // of the charges (stride n_src) and locals (stride col_stride); each kernel
 // value (L2T and P2P) is computed once and applied to the R columns.  Output
-// row r of out (stride ld_out).  One work item = (leaf, up to 128 targets).
-constexpr int SMAX_MR = 256;
+// row r of out (stride ld_out).  One work item = (leaf, up to 128 targets);
+// the leaf's equivalent sources are staged and swept as its neighbours are.
+// Bound by the kernel values and the columns' FMAs, whose charges are read from
+// shared memory two at a time.  16 columns of K0 at 60k points on a ring:
+// 541 us in two launches of 8 columns before, 312 in one.
+constexpr int SMAX_MR = 192;
 template <class KF, int R>
 __global__ void __launch_bounds__(TCH) k_evaluate_multi(KernelParams kp, int neq, int np, int ncol,
                                                         const int4 *__restrict__ items,
@@ -1053,7 +1055,8 @@ __global__ void __launch_bounds__(TCH) k_evaluate_multi(KernelParams kp, int neq
                                                         const double *__restrict__ tys,
                                                         const int *__restrict__ tperm, int check,
                                                         double *__restrict__ out, int64_t ld_out) {
-  __shared__ double ssx[SMAX_MR], ssy[SMAX_MR], stau[R][SMAX_MR];
+  __shared__ double2 sxy[SMAX_MR];
+  __shared__ __align__(16) double stau[SMAX_MR][R + 2];  // (padded: fewer bank conflicts)
   __shared__ int rb[9], rs[10];
   __shared__ double red[R][TCH / 32];
   __shared__ FunctorSmem<KF> fsm;
@@ -1081,15 +1084,30 @@ __global__ void __launch_bounds__(TCH) k_evaluate_multi(KernelParams kp, int neq
     double u[R];
 #pragma unroll
     for (int c = 0; c < R; ++c) u[c] = 0.0;
-    if (lev >= 2 && valid) {  // L2T, one kernel value per circle point for all columns
-      const double dx = x - xmid[g], dy = y - ymid[g];
-      const double *lx = ops[lev].lx, *ly = ops[lev].ly;
-      for (int k = sub; k < neq; k += G) {
-        const double kv = K(lx[k], ly[k], dx, dy);
+    auto sweep = [&](int n, double px, double py, bool chk) {  // the staged sources
+      if (!valid) return;
+#pragma unroll 2
+      for (int j = sub; j < n; j += G) {
+        const double2 q = sxy[j];
+        if (chk && px - q.x == 0.0 && py - q.y == 0.0) continue;
+        const double kv = K(q.x, q.y, px, py);
+        const double2 *tq = reinterpret_cast<const double2 *>(stau[j]);
 #pragma unroll
-        for (int c = 0; c < R; ++c)
-          if (c < ncol) u[c] = fma(kv, loc[c * col_stride + (size_t)g * np + k], u[c]);
+        for (int c = 0; c < R / 2; ++c) {
+          const double2 w = tq[c];
+          u[2 * c] = fma(kv, w.x, u[2 * c]);
+          u[2 * c + 1] = fma(kv, w.y, u[2 * c + 1]);
+        }
       }
+    };
+    if (lev >= 2) {  // L2T
+      for (int k = threadIdx.x; k < neq; k += TCH) sxy[k] = make_double2(ops[lev].lx[k], ops[lev].ly[k]);
+      for (int i = threadIdx.x; i < neq * R; i += TCH) {
+        const int c = i / neq, k = i - c * neq;
+        stau[k][c] = c < ncol ? loc[c * col_stride + (size_t)g * np + k] : 0.0;
+      }
+      __syncthreads();
+      sweep(neq, x - xmid[g], y - ymid[g], false);
     }
     __syncthreads();
     const int ns = rs[9];
@@ -1100,20 +1118,12 @@ __global__ void __launch_bounds__(TCH) k_evaluate_multi(KernelParams kp, int neq
         int c = 0;
         while (idx >= rs[c + 1]) ++c;
         const int j = rb[c] + (idx - rs[c]);
-        ssx[i] = sx[j];
-        ssy[i] = sy[j];
+        sxy[i] = make_double2(sx[j], sy[j]);
 #pragma unroll
-        for (int q = 0; q < R; ++q) stau[q][i] = q < ncol ? tau[q * n_src + j] : 0.0;
+        for (int q = 0; q < R; ++q) stau[i][q] = q < ncol ? tau[q * n_src + j] : 0.0;
       }
       __syncthreads();
-      if (valid)
-        for (int j = sub; j < nb; j += G) {
-          const double qx = ssx[j], qy = ssy[j];
-          if (check && x - qx == 0.0 && y - qy == 0.0) continue;
-          const double kv = K(qx, qy, x, y);
-#pragma unroll
-          for (int c = 0; c < R; ++c) u[c] = fma(kv, stau[c][j], u[c]);
-        }
+      sweep(nb, x, y, check);
       __syncthreads();
     }
 #pragma unroll
@@ -1134,6 +1144,8 @@ __global__ void __launch_bounds__(TCH) k_evaluate_multi(KernelParams kp, int neq
   }
 }
 
+// FP64 direct sum (kernel_apply / kernel_apply_single_check,
+// flexmm/flexmm2d/helpers.py:91-116): all sources, one target per thread,
 // sources staged through shared memory
 template <class KF>
 __global__ void __launch_bounds__(256) k_direct(KernelParams kp, const double *__restrict__ sx,
@@ -1169,7 +1181,9 @@ __global__ void __launch_bounds__(256) k_direct(KernelParams kp, const double *_
 }
 
 __global__ void k_gather_sorted(const double *__restrict__ v, const int *__restrict__ perm,
-                                int64_t n, double *__restrict__ o) {
+                                int64_t n, double *__restrict__ o, int64_t ld_v) {
+  v += blockIdx.y * ld_v;  // column blockIdx.y
+  o += blockIdx.y * n;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     o[i] = v[perm[i]];
@@ -1497,15 +1511,24 @@ void evaluate_multi_impl(const PassArgs &a, const double *tau_s, int64_t n_src, 
   EvalItems it;
   eval_items(a, tkeys, m, it, s);
   PhaseTimer timer(PH_EVAL, s);
-  constexpr int R = 8;
-  for (int r0 = 0; r0 < n_rhs; r0 += R) {
-    const int ncol = std::min(R, n_rhs - r0);
-    k_evaluate_multi<KF, R><<<work_grid(a.th->n_total() + m / TCH + 1, 8), TCH, 0, s>>>(
-        a.kp, a.neq, a.np, ncol, it.items.get(), it.n_items.get(), td.coll.get(), td.bot.get(),
-        td.top.get(), td.xmid.get(), td.ymid.get(), td.sx.get(), td.sy.get(), tau_s + r0 * n_src,
-        n_src, a.ops_dev, loc + r0 * col_stride, col_stride, txs, tys, tperm, check,
-        out + r0 * ld_out, ld_out);
-    FMMB_CUDA(cudaGetLastError());
+  // columns at a time: 16 where there are more than 8 (the kernel values of a
+  // second launch cost more than the smaller occupancy)
+  for (int r0 = 0; r0 < n_rhs;) {
+    auto launch = [&](auto rc) {
+      constexpr int R = decltype(rc)::value;
+      const int ncol = std::min(R, n_rhs - r0);
+      k_evaluate_multi<KF, R><<<work_grid(a.th->n_total() + m / TCH + 1, 8), TCH, 0, s>>>(
+          a.kp, a.neq, a.np, ncol, it.items.get(), it.n_items.get(), td.coll.get(), td.bot.get(),
+          td.top.get(), td.xmid.get(), td.ymid.get(), td.sx.get(), td.sy.get(), tau_s + r0 * n_src,
+          n_src, a.ops_dev, loc + r0 * col_stride, col_stride, txs, tys, tperm, check,
+          out + r0 * ld_out, ld_out);
+      FMMB_CUDA(cudaGetLastError());
+      r0 += R;
+    };
+    if (n_rhs - r0 > 8)
+      launch(std::integral_constant<int, 16>{});
+    else
+      launch(std::integral_constant<int, 8>{});
   }
 }
 }  // namespace
@@ -1674,9 +1697,12 @@ void run_diag_log2(const double *x, int64_t n, double *out_tab, double *out_lib,
   FMMB_CUDA(cudaGetLastError());
 }
 
-void gather_sorted(const double *v, const int *perm, int64_t n, double *o, cudaStream_t s) {
+void gather_sorted(const double *v, const int *perm, int64_t n, double *o, cudaStream_t s,
+                   int columns, int64_t ld_v) {
   if (n == 0) return;
-  k_gather_sorted<<<grid_for(n, 256), 256, 0, s>>>(v, perm, n, o);
+  for (int c = 0; c < columns; c += 65535)
+    k_gather_sorted<<<dim3(grid_for(n, 256), std::min(columns - c, 65535)), 256, 0, s>>>(
+        v + c * ld_v, perm, n, o + c * n, ld_v);
   FMMB_CUDA(cudaGetLastError());
 }
 

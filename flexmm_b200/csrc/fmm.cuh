@@ -176,7 +176,9 @@ void run_downward(const PassArgs &a, const double *ple, double *loc, cudaStream_
 void run_direct(int kernel_id, const KernelParams &kp, const double *sx, const double *sy,
                 const double *tau, int64_t ns, const double *tx, const double *ty, int64_t nt,
                 int check, double *out, cudaStream_t s);
-void gather_sorted(const double *v, const int *perm, int64_t n, double *o, cudaStream_t s);
+// o[c n + i] = v[c ld_v + perm[i]], c < columns
+void gather_sorted(const double *v, const int *perm, int64_t n, double *o, cudaStream_t s,
+                   int columns = 1, int64_t ld_v = 0);
 void gather_sorted_i64(const int64_t *v, const int *perm, int64_t n, int64_t *o, cudaStream_t s);
 // near field only (local evaluator): out[i] = sum over the target's
 // colleagues' sources; scat (sorted) / tcat (caller's order) categories, or null
