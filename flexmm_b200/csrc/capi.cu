@@ -385,11 +385,13 @@ struct fmm_plan {
   // whether the expansions built last were evaluated split (assumed of a new
   // plan): where they were not, the next build stays on the caller's stream
   bool split_used = true;
+  bool split_scratch_ready = false;  // allocated for this tree, before its ev_ready
   cudaEvent_t ev_ready = nullptr, ev_near = nullptr, ev_far = nullptr, ev_pass = nullptr;
   bool ready_recorded = false;
   // mixed form: the split near field pauses during the M2L (SplitEval::hold)
   cudaEvent_t ev_m2l = nullptr;
   DevBuf<int> near_hold;
+  SplitScratch split_scratch;  // see split_scratch_prepare
   bool hold_armed = false;
   ~fmm_plan() {
     for (cudaEvent_t e : {ev_ready, ev_near, ev_far, ev_m2l, ev_pass})
@@ -431,10 +433,10 @@ cudaStream_t side_stream(cudaStream_t *pass) {
 }
 
 // Whether own-source evaluation runs split (near field beside the level
-// passes).  Measured at 1M clustered sources: the FP64 form gains ~0.3 ms
-// (2.72 ms with its passes at high priority, 2.89 without); the mixed form,
-// whose near field pauses while the persistent tcgen05 M2L runs, gains
-// ~0.03 ms (1.39 -> 1.36 ms).  On for both by default;
+// passes).  Measured, off and on: a step of 1M clustered sources 2.34 and 2.27
+// ms, of 200k with K0 0.97 and 0.86, a product on 250k ring points 0.58 and 0.49;
+// the mixed form, whose near field pauses while the persistent tcgen05 M2L
+// runs, 1.18 and 1.14 ms at 1M.  On for both by default;
 // FLEXMM_B200_SPLIT_EVAL=0 turns it off, =1 on.
 std::atomic<int> g_split_mode{-2};  // -2: not yet read from the environment
 
@@ -457,6 +459,23 @@ void split_prepare(fmm_plan *p) {
     if (!*e) FMMB_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
 }
 
+bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return st != cudaStreamCaptureStatusNone;
+}
+
+// the scratch of the split evaluation that is expected, ahead of ev_ready
+void split_scratch_prepare(fmm_plan *p, cudaStream_t s) {
+  if (p->split_used && split_enabled(p->precision) && !capturing(s)) {
+    p->split_scratch.alloc(p->th.n_total(), p->th.n_points, p->precision == PREC_MIXED, s);
+    p->split_scratch_ready = true;
+  }
+}
+
 // The stream of a plan's FP64 level passes: the high-priority one of its pair,
 // which waits for ev_ready and which the caller's stream waits for at join()
 // (at the latest when this object ends, so that buffers freed in the caller's
@@ -468,14 +487,9 @@ void split_prepare(fmm_plan *p) {
 class PassStream {
  public:
   PassStream(fmm_plan *p, cudaStream_t s) : p_(p), s_(s), ps_(s) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     const bool near_beside = split_enabled(PREC_FP64) && p->split_used;
     p->split_used = false;
-    if (!near_beside || cudaStreamIsCapturing(s, &st) != cudaSuccess ||
-        st != cudaStreamCaptureStatusNone) {
-      cudaGetLastError();
-      return;
-    }
+    if (!near_beside || capturing(s)) return;
     FMMB_CUDA(cudaStreamWaitEvent(p->pass, p->ev_ready, 0));
     ps_ = p->pass;
   }
@@ -1410,6 +1424,8 @@ static void build_expansions_impl(fmm_plan *p, const double *tau, void *stream) 
     upload_level_ops(p, s);
     split_prepare(p);
     p->ready_recorded = false;
+    p->split_scratch_ready = false;
+    split_scratch_prepare(p, s);
     p->sync.alloc(2, s);
     PassArgs a = pass_args(p);
     p->tau_s.alloc(th.n_points, s);
@@ -1558,6 +1574,7 @@ void evaluate_own_sources(fmm_plan *p, int nout, int check, double *out, int64_t
     // near field on the side stream, started when the charges were sorted
     p->split_used = true;
     SplitEval se{p->side, p->ev_ready, p->ev_near, p->ev_far};
+    if (p->split_scratch_ready && !capturing(s)) se.scratch = &p->split_scratch;
     if (p->precision == PREC_MIXED && p->hold_armed) {
       se.hold = p->near_hold.get();
       se.m2l_done = p->ev_m2l;
@@ -1654,6 +1671,8 @@ int fmm_plan_drop_expansions(fmm_plan *p) {
     p->has_dipoles = false;
     p->st_dip.release();
     p->has_st_dipoles = false;
+    p->split_scratch.release();
+    p->split_scratch_ready = false;
     p->have_expansions = false;
     p->ready_recorded = false;
   });

@@ -1461,10 +1461,11 @@ void evaluate_split_impl(const PassArgs &a, const double *tau_s, const double *l
   const TreeDev &td = *a.td;
   const int64_t m = a.th->n_points;
   FMMB_CUDA(cudaStreamWaitEvent(se.side, se.ready, 0));
-  EvalItems it;
+  SplitScratch own, &w = se.scratch ? *se.scratch : own;
+  if (!se.scratch) w.alloc(a.th->n_total(), m, false, se.side);
+  EvalItems &it = w.it;
+  DevBuf<double> &near = w.near;
   eval_items(a, td.pkeys.get(), m, it, se.side);
-  DevBuf<double> near;
-  near.alloc(m, se.side);
   const int64_t units = a.th->n_total() + m / TCH + 1;  // work items, upper bound
   {
     // the SMs keep their largest shared-memory carveout while near-field
@@ -1496,7 +1497,7 @@ void evaluate_split_impl(const PassArgs &a, const double *tau_s, const double *l
         item_args(a, it.items.get(), it.n_items.get(), 1, td.sx.get(), td.sy.get(), td.ordv.get()),
         units, EVAL_BLOCKS, s);
   }
-  // the scratch (allocated on the side stream) is freed there once the plan
+  // the scratch is used again (or freed) on the side stream once the plan
   // stream is done with it
   FMMB_CUDA(cudaEventRecord(se.far_done, s));
   FMMB_CUDA(cudaStreamWaitEvent(se.side, se.far_done, 0));

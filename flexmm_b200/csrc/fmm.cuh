@@ -122,6 +122,34 @@ void run_stokes_evaluate(const StokesArgs &a, const double *fx, const double *fy
                          const int *tperm, int64_t m, int check, double *out, int64_t ld_out,
                          cudaStream_t s);
 
+// Evaluation work items: per leaf its range of sorted targets, split into
+// chunks of 128 targets, in no particular order of the leaves.
+struct EvalItems {
+  DevBuf<int4> items;   // (leaf, level | flags, first sorted target, count)
+  DevBuf<int> n_items;  // [0] device count of items, [1 ..] zeroed hand-out counters
+};
+
+// Scratch of a split evaluation, the plan's: allocated on the plan's stream
+// before `ready` is recorded, kept, and used by one evaluation at a time (each
+// leaves the side stream waiting for its end).  Allocated on the side stream by
+// each call, its memory changed streams at every step, which the allocator has
+// to order: a step of 100k points took 668 us of the host, 383 so; the mixed step
+// of 1M 1.177 -> 1.140 ms in a row, 1.55 -> 1.20 from a new state.
+struct SplitScratch {
+  EvalItems it;
+  DevBuf<double> near;         // near-field potentials
+  DevBuf<unsigned char> desc;  // mixed form: the items' descriptors ...
+  DevBuf<int> next_item;       // ... and the near- and far-field hand-out counters
+  void alloc(int64_t nodes, int64_t m, bool mixed, cudaStream_t s);
+  void release() {
+    it.items.release();
+    it.n_items.release();
+    near.release();
+    desc.release();
+    next_item.release();
+  }
+};
+
 // n_rhs charge columns (stride n_src, sorted order) and their locals (stride
 // col_stride): out row r (stride ld_out) for column r
 void run_evaluate_multi(const PassArgs &a, const double *tau_sorted, int64_t n_src, int n_rhs,
@@ -143,6 +171,9 @@ struct SplitEval {
   // second launch after m2l_done finishes the rest.  hold NULL: one launch.
   int *hold = nullptr;
   cudaEvent_t m2l_done = nullptr;
+  // NULL (a stream being captured, whose graph may run beside other
+  // evaluations): each call's own, allocated on the side stream
+  SplitScratch *scratch = nullptr;
 };
 // FP64 near field beside the passes: items a block takes before it ends (its
 // place may then go to a level pass, which has the higher priority).  Step in
@@ -190,19 +221,12 @@ void run_local_evaluate(const PassArgs &a, const double *tau_sorted, const doubl
 void run_diag_log2(const double *x, int64_t n, double *out_tab, double *out_lib, cudaStream_t s);
 // nout = 1: potential into out[m]; nout = 3: potential and its gradient in the
 // target position into out[0..2][m] (row stride ld_out)
-struct EvalItems;
 // (pre: work items already built for txs, tys; else built from tkeys)
 void run_evaluate(const PassArgs &a, const double *tau_sorted, const double *loc,
                   const double *txs, const double *tys, const uint64_t *tkeys, const int *tperm,
                   int64_t m, int check, int nout, double *out, int64_t ld_out, cudaStream_t s,
                   const EvalItems *pre = nullptr);
 
-// Evaluation work items: per leaf its range of sorted targets, split into
-// chunks of 128 targets, in no particular order of the leaves.
-struct EvalItems {
-  DevBuf<int4> items;   // (leaf, level | flags, first sorted target, count)
-  DevBuf<int> n_items;  // [0] device count of items, [1 ..] zeroed hand-out counters
-};
 constexpr int EVAL_COUNTERS = 3;  // hand-out counters of an item list (one per launch over it)
 // item .y: the leaf's level, plus EVAL_MULTI when the leaf's targets fill more
 // than one item (targets placed in no particular order inside the leaf): then

@@ -1455,18 +1455,17 @@ void split_mixed_impl(const PassArgs &a, const double *tau_s, const double *tsum
   const int64_t m = th.n_points;
   const int total = th.n_total();
   FMMB_CUDA(cudaStreamWaitEvent(se.side, se.ready, 0));
-  EvalItems it;
+  SplitScratch own, &w = se.scratch ? *se.scratch : own;
+  if (!se.scratch) w.alloc(total, m, true, se.side);
+  EvalItems &it = w.it;
+  DevBuf<double> &near = w.near;
+  DevBuf<int> &next_item = w.next_item;  // [0] near-field, [1] far-field hand-out counters
+  EvalDesc *desc = reinterpret_cast<EvalDesc *>(w.desc.get());
   eval_items(a, td.pkeys.get(), m, it, se.side);
-  DevBuf<EvalDesc> desc;
-  desc.alloc(total + m / TCH + 1, se.side);
-  DevBuf<int> next_item;  // [0] near-field, [1] far-field hand-out counters
-  next_item.alloc(2, se.side);
-  next_item.zero(se.side);
-  DevBuf<double> near;
-  near.alloc(m, se.side);
+  FMMB_CUDA(cudaMemsetAsync(next_item.get(), 0, 2 * sizeof(int), se.side));
   k_eval_desc<<<grid_for(total + m / TCH + 1, 256), 256, 0, se.side>>>(
       it.items.get(), it.n_items.get(), td.coll.get(), td.bot.get(), td.top.get(), td.xmid.get(),
-      td.ymid.get(), tsum, desc.get());
+      td.ymid.get(), tsum, desc);
   FMMB_CUDA(cudaGetLastError());
   {
     // the SMs keep their largest shared-memory carveout while near-field
@@ -1489,7 +1488,7 @@ void split_mixed_impl(const PassArgs &a, const double *tau_s, const double *tsum
       k_evaluate_mx<KF32, KF64, 1, EVAL_NEAR>
           <<<work_grid(total + m / TCH + 1, part == 0 ? NEAR_BLOCKS_PER_SM_MIXED
                                                       : NEAR_BLOCKS_PER_SM_MIXED_RESUME),
-             TCH, 0, se.side>>>(a.kp, a.neq, a.np, desc.get(), it.n_items.get(), td.sx.get(),
+             TCH, 0, se.side>>>(a.kp, a.neq, a.np, desc, it.n_items.get(), td.sx.get(),
                                 td.sy.get(), tau_s, a.ops_dev, loc32, lsum, td.sx.get(),
                                 td.sy.get(), td.ordv.get(), check, 1, out, 0, next_item.get(),
                                 near.get(), se.hold);
@@ -1502,13 +1501,24 @@ void split_mixed_impl(const PassArgs &a, const double *tau_s, const double *tsum
     PhaseTimer timer(PH_EVAL, s);
     k_evaluate_mx<KF32, KF64, 1, EVAL_FAR>
         <<<work_grid(total + m / TCH + 1, EvalOcc<KF32>::blocks), TCH, 0, s>>>(
-        a.kp, a.neq, a.np, desc.get(), it.n_items.get(), td.sx.get(), td.sy.get(), tau_s,
+        a.kp, a.neq, a.np, desc, it.n_items.get(), td.sx.get(), td.sy.get(), tau_s,
         a.ops_dev, loc32, lsum, td.sx.get(), td.sy.get(), td.ordv.get(), check, 1, out, 0,
         next_item.get() + 1, near.get());
     FMMB_CUDA(cudaGetLastError());
   }
   FMMB_CUDA(cudaEventRecord(se.far_done, s));
   FMMB_CUDA(cudaStreamWaitEvent(se.side, se.far_done, 0));
+}
+
+void SplitScratch::alloc(int64_t nodes, int64_t m, bool mixed, cudaStream_t s) {
+  const int64_t items = nodes + m / EVAL_CHUNK + 1;
+  it.items.alloc(items, s);
+  it.n_items.alloc(1 + EVAL_COUNTERS, s);
+  near.alloc(m, s);
+  if (mixed) {
+    desc.alloc(items * sizeof(EvalDesc), s);
+    next_item.alloc(2, s);
+  }
 }
 
 void run_evaluate_sources_split_mixed(const PassArgs &a, const double *tau_s,
