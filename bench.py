@@ -666,8 +666,8 @@ def measure_bb_adjoint(args, world=1, steps=3):
             "metric": "(sources + targets) / s", "unit": "Mpts/s", "dtype": "f64",
             "value": world * pts / (ms_fb * 1e-3) / 1e6, "ms_per_step": ms_fb,
             "forward": {"value": world * pts / (ms_f * 1e-3) / 1e6, "ms": ms_f}, "steps": steps,
-            "note": "trees built inside every step; translations on the FP64 tensor-core row "
-                    "GEMM; accuracy checked by the test suite (1e-8 vs FP64 direct-sum "
+            "note": "trees built inside every step; shifts by tensor factors and M2L in a common "
+                    "basis on the FP64 tensor cores; accuracy checked by the test suite (1e-8 vs FP64 direct-sum "
                     "gradients at N = 20,000)"}
 
 
@@ -676,8 +676,9 @@ def measure_multi_rhs(args, world=1, n=1_000_000, n_rhs=64, steps=3):
     circle of radius 0.5 (radial jitter U(-1e-3, 1e-3)), 64 charge columns
     N(0,1) on one tree, the modified Helmholtz kernel K0(10 r)/(2 pi), Nequiv
     40, Ncutoff 64, bbox from the points, self-evaluation of every column.
-    A step: tree + expansions of all 64 columns (one launch per level for all
-    columns) + source evaluation (each kernel value applied to 8 columns).
+    A step: tree + expansions of all 64 columns (one launch per pass for all
+    columns; each kernel value applied to 8 columns in S2M) + source evaluation
+    (to 16).
     Metric: point-RHS per second, 64 N / T.  Inputs resident; CUDA events.
     With N > 1 ranks the columns are split into blocks over the ranks
     (flexmm_b200.shard, no exchange while computing)."""
@@ -727,8 +728,8 @@ def measure_multi_rhs(args, world=1, n=1_000_000, n_rhs=64, steps=3):
             "value": n * n_rhs / (ms * 1e-3) / 1e6, "ms_per_step": ms, "steps": steps,
             "rel_l2_vs_direct": err,
             "accuracy_sample": "columns 0 and last of this rank, 1000 sources, FP64 direct sum",
-            "note": "one launch per level for all columns (column = blockIdx.y); evaluation "
-                    "shares each kernel value across 8 columns; inputs resident"
+            "note": "one launch per pass for all columns; S2M shares each kernel value across 8 "
+                    "columns, evaluation across 16; inputs resident"
                     + (f"; columns split over {world} ranks, slowest rank's time" if world > 1 else ""),
             "mixed": {"value": n * n_rhs / (ms_mx * 1e-3) / 1e6, "ms_per_step": ms_mx,
                       "rel_l2_vs_direct": err_mx, "dtype": "f32+tf32x3/f64",

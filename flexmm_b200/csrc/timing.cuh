@@ -11,15 +11,15 @@
 namespace fmmb {
 
 enum Phase : int {
-  PH_TREE = 0,      // whole tree build (span, includes its two host waits)
+  PH_TREE = 0,      // whole tree build (span, includes its host wait)
   PH_SORT_TGT = 1,  // targets into leaves: keys, binning (KIFMM) or sort (BB, Stokes), items
-  PH_UPWARD = 2,    // k_upward launches (S2M + M2M + C2E)
+  PH_UPWARD = 2,    // upward pass (S2M + M2M + C2E)
   PH_M2L = 3,       // k_m2l launch
-  PH_DOWNWARD = 4,  // k_downward launches (L2L + C2E)
-  PH_EVAL = 5,      // k_evaluate launch (L2T + P2P)
+  PH_DOWNWARD = 4,  // downward pass (L2L + C2E)
+  PH_EVAL = 5,      // evaluation launches (L2T + P2P)
   PH_DIRECT = 6,    // direct sums
-  PH_TREE_SPLITS = 7,   // tree: point keys, sort, initial splits (to the first host round trip)
-  PH_TREE_BALANCE = 8,  // tree: 2:1 closure and X-list (to the second)
+  PH_TREE_SPLITS = 7,   // tree: point keys, sort, initial splits
+  PH_TREE_BALANCE = 8,  // tree: 2:1 closure and X-list (to the host's wait)
   PH_TREE_NODES = 9,    // tree: parent-box sort, node arrays, colleagues, interaction lists
   PH_PREP = 10,         // expansions: charge gather, buffers, per-node charge sums
   N_PHASES = 12

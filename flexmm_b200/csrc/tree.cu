@@ -27,9 +27,9 @@
 //     (level, morton); each contributes 4 consecutive children, so node
 //     arrays, ranges, colleagues and interaction lists follow from binary
 //     searches in sorted arrays.
-// The host waits twice (for the split-box count and depth, then for the
-// balance closure's size); the per-level node counts come back without a
-// wait (finalize_tree).
+// The host waits once (for the counts of the splits and of the balance
+// closure); the per-level node counts come back without a wait
+// (finalize_tree).
 #include <cmath>
 
 #include <memory>

@@ -341,8 +341,8 @@ int fmm_evaluate_noalloc(fmm_plan *plan, const double *tx, const double *ty, int
                          double *out, void *stream);
 
 /* Diagnostic: the table-driven log2 that the FP64 passes use for the
- * Laplace kernel (exponent split, a 257-entry table of 1/F and log2 F,
- * degree-5 series; Tang, ACM TOMS 16, 1990) and CUDA's log2, at n device
+ * Laplace kernel (exponent split, a table of 129 pairs 1/F and log2 F, a
+ * degree-5 polynomial; Tang, ACM TOMS 16, 1990) and CUDA's log2, at n device
  * points x, into out_table and out_library.  For tests of its accuracy. */
 int fmm_diag_log2(const double *x, int64_t n, double *out_table, double *out_library,
                   void *stream);
