@@ -460,7 +460,7 @@ def work_counts_gemm(F, neq, c):
 # clustered sources + 1000^2 grid): ncu captures of the 200k-source /
 # 450^2-grid case of the same distribution, scaled by the points each
 # launch evaluates, averaged over the source and grid launches
-NCU_TRAFFIC_BYTES = {("mixed", "evaluate"): 46_400_000, ("fp64", "evaluate"): 60_600_000}
+NCU_TRAFFIC_BYTES = {("mixed", "evaluate"): 46_400_000, ("fp64", "evaluate"): 60_900_000}
 
 
 def roofline_of(res, precision, peaks, steps, default_workload):
