@@ -641,9 +641,11 @@ int fmm_ops_add(fmm_ops *ops, const fmm_level_ops *lv, int *level_id) {
     FMMB_CHECK(!scaled || lv->width > 0, ERR_INVALID_ARGUMENT, "level width must be positive");
     const double inv_w = scaled ? 1.0 / lv->width : 1.0;
     const size_t f_lx = takef(np), f_ly = takef(np);
+    float reach = 0.f;
     for (int k = 0; k < n; ++k) {
       f[f_lx + k] = (float)(lv->large_x[k] * inv_w);
       f[f_ly + k] = (float)(lv->large_y[k] * inv_w);
+      reach = std::max({reach, std::fabs(f[f_lx + k]), std::fabs(f[f_ly + k])});
     }
     double c_m2m = 0.0;
     for (size_t i = 0; i < size_t(n) * 4 * n; ++i) c_m2m += lv->m2mc[i];
@@ -713,6 +715,7 @@ int fmm_ops_add(fmm_ops *ops, const fmm_level_ops *lv, int *level_id) {
       e->dev.m2mc_lo = fb + f_m2mc_l;
       e->dev.c_m2m = c_m2m;
       e->dev.inv_w = inv_w;
+    e->dev.reach32 = reach;
       e->dev.kofs = scaled ? kernel_offset(ops->kernel_id, ops->kp, lv->width) : 0.0;
       for (int o = 0; o < FMM_N_OFFSETS; ++o) {
         e->dev.m2l_hi[o] = lv->m2l_rank[o] == 0 ? nullptr : fb + f_m2l_h[o];
@@ -1083,6 +1086,10 @@ __global__ void k_gather_dipoles(const double *__restrict__ str, const double *_
 // entries' addresses)
 struct LevelOpsSrc {
   const LevelOpsDev *p[FMM_MAX_LEVELS_DEV];
+  double width[FMM_MAX_LEVELS_DEV];
+  // scaling of levels without operators (0 and 1 need none: no expansions there,
+  // but the mixed near field of a leaf there does read its scaling)
+  double inv_w[FMM_MAX_LEVELS_DEV], kofs[FMM_MAX_LEVELS_DEV];
 };
 static_assert(sizeof(LevelOpsDev) % sizeof(int) == 0, "LevelOpsDev is copied as words");
 
@@ -1091,6 +1098,15 @@ __global__ void k_gather_level_ops(LevelOpsSrc src, LevelOpsDev *__restrict__ ds
   const int *from = reinterpret_cast<const int *>(src.p[blockIdx.x]);
   int *to = reinterpret_cast<int *>(dst + blockIdx.x);
   for (int i = threadIdx.x; i < NW; i += blockDim.x) to[i] = from ? from[i] : 0;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    LevelOpsDev &d = dst[blockIdx.x];
+    if (!from) {
+      d.inv_w = src.inv_w[blockIdx.x];
+      d.kofs = src.kofs[blockIdx.x];
+    }
+    d.box32 = float(src.width[blockIdx.x] * d.inv_w);
+  }
 }
 
 static void upload_level_ops(fmm_plan *p, cudaStream_t s) {
@@ -1098,8 +1114,16 @@ static void upload_level_ops(fmm_plan *p, cudaStream_t s) {
   FMMB_CHECK(L <= FMM_MAX_LEVELS_DEV, ERR_INVALID_ARGUMENT, "too many levels");
   p->ops_dev.alloc(L, s);
   LevelOpsSrc src{};
-  for (int m = 0; m < L; ++m)
-    if (p->bound[m] >= 0) src.p[m] = p->ops->levels[p->bound[m]]->dev_copy.get();
+  const bool scaled = p->ops->method == METHOD_KIFMM && kernel_scaled(p->ops->kernel_id);
+  for (int m = 0; m < L; ++m) {
+    const double w = src.width[m] = p->th.width[m];
+    if (p->bound[m] >= 0) {
+      src.p[m] = p->ops->levels[p->bound[m]]->dev_copy.get();
+    } else {
+      src.inv_w[m] = scaled ? 1.0 / w : 1.0;
+      src.kofs[m] = scaled ? kernel_offset(p->ops->kernel_id, p->ops->kp, w) : 0.0;
+    }
+  }
   k_gather_level_ops<<<L, 128, 0, s>>>(src, p->ops_dev.get());
   FMMB_CUDA(cudaGetLastError());
 }

@@ -37,6 +37,9 @@ struct LevelOpsDev {
   // kernel's offset(width), else 0) times the charge sum is added in FP64;
   // lx32 / ly32 hold the check circle already scaled
   double inv_w, kofs;
+  // extents in these units: the circle's largest |coordinate| and, from the
+  // plan's tree (upload_level_ops), the box width
+  float reach32, box32;
 };
 
 constexpr int PREC_FP64 = 0, PREC_MIXED = 1;

@@ -152,9 +152,6 @@ __device__ __forceinline__ int node_level(const int *__restrict__ off, int L, in
   return lo;
 }
 
-// a box's width from its large circle's radius w (4 - sqrt 2) / 2
-__device__ __forceinline__ float box_of_circle(float r) { return r * (2.f / (4.f - 1.41421356f)); }
-
 // S2M + C2E of every S2M node (leaves holding points) of every level, in one
 // launch (flexmm/flexmm2d/kifmm.py:96-105 then fmm.py:86-90).  A tile is TN
 // consecutive entries of the level-major node list; C2E runs once for each
@@ -209,10 +206,10 @@ __global__ void __launch_bounds__(NT) k_s2m_mx(KernelParams kp, int neq, int np,
       const float lx1 = lane + 32 < neq ? op.lx32[lane + 32] : 0.f;
       const float ly1 = lane + 32 < neq ? op.ly32[lane + 32] : 0.f;
       // a box's points lie within half a width of its centre, its circle's
-      // within the circle's radius
+      // within the circle's reach
       bool near = false;
       if constexpr (KF32::kNearForm) {
-        const float rc = op.lx32[0], h = rc + 0.51f * box_of_circle(rc);
+        const float h = op.reach32 + 0.51f * op.box32;
         near = K.near_all(h, h);
       }
       auto value = [&](float dx, float dy, bool nr) -> float {
@@ -964,10 +961,10 @@ __global__ void __launch_bounds__(TCH, NOUT == 1 ? EvalOcc<KF32>::blocks : 6)
     const float tx_lo = (float)(txd - (double)tx), ty_lo = (float)(tyd - (double)ty);
     double acc = 0.0, accx = 0.0, accy = 0.0;  // accx, accy: kScale * (dx, dy) / d2 sums
     // whether every source of the item (in the leaf's colleagues: within 1.5
-    // widths of its centre, as its circle is) is at a distance of the near form
+    // widths of its centre) and of its circle is at a distance of the near form
     bool near_form = false;
     if constexpr (KF32::kNearForm) {
-      const float h = 1.501f * box_of_circle(ops[lev].lx32[0]);
+      const float h = fmaxf(1.501f * ops[lev].box32, ops[lev].reach32);
       near_form = K.near_all(fabsf(tx) + h, fabsf(ty) + h);
     }
     auto rad = [&](float d2, bool nr) -> float {
