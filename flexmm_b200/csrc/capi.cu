@@ -371,6 +371,7 @@ struct fmm_plan {
   DevBuf<RadixSync> sync;       // barriers of the level passes (upward, downward)
   DevBuf<int> err;              // set by kernels whose bounded waits ran out
   int precision = PREC_FP64;
+  bool moved = false;  // sources moved on the frozen tree: a box no longer bounds its own
   bool have_expansions = false;
   DevBuf<double> tau2_s, partial;  // Stokes FMM: sorted fy; partial multipoles
   int n_rhs = 1;                   // charge columns of the last build (multi-RHS)
@@ -1086,7 +1087,7 @@ __global__ void k_gather_dipoles(const double *__restrict__ str, const double *_
 // entries' addresses)
 struct LevelOpsSrc {
   const LevelOpsDev *p[FMM_MAX_LEVELS_DEV];
-  double width[FMM_MAX_LEVELS_DEV];
+  double width[FMM_MAX_LEVELS_DEV];  // what a box's sources keep to; infinite once they were moved
   // scaling of levels without operators (0 and 1 need none: no expansions there,
   // but the mixed near field of a leaf there does read its scaling)
   double inv_w[FMM_MAX_LEVELS_DEV], kofs[FMM_MAX_LEVELS_DEV];
@@ -1116,7 +1117,8 @@ static void upload_level_ops(fmm_plan *p, cudaStream_t s) {
   LevelOpsSrc src{};
   const bool scaled = p->ops->method == METHOD_KIFMM && kernel_scaled(p->ops->kernel_id);
   for (int m = 0; m < L; ++m) {
-    const double w = src.width[m] = p->th.width[m];
+    const double w = p->th.width[m];
+    src.width[m] = p->moved ? HUGE_VAL : w;
     if (p->bound[m] >= 0) {
       src.p[m] = p->ops->levels[p->bound[m]]->dev_copy.get();
     } else {
@@ -1713,6 +1715,7 @@ int fmm_plan_move_sources(fmm_plan *p, const double *x, const double *y, void *s
     // the tree's sorted copy, in the tree's own order (sorted -> original)
     gather_sorted(x, p->td.ordv.get(), n, p->td.sx.get(), s);
     gather_sorted(y, p->td.ordv.get(), n, p->td.sy.get(), s);
+    p->moved = true;
     p->have_expansions = false;
     p->ready_recorded = false;
   });

@@ -38,7 +38,8 @@ struct LevelOpsDev {
   // lx32 / ly32 hold the check circle already scaled
   double inv_w, kofs;
   // extents in these units: the circle's largest |coordinate| and, from the
-  // plan's tree (upload_level_ops), the box width
+  // plan's tree (upload_level_ops), the box width (infinite where sources were
+  // moved out of what the tree knows)
   float reach32, box32;
 };
 

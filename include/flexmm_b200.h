@@ -267,7 +267,9 @@ int fmm_evaluate_sources_outputs(fmm_plan *plan, int evaluator, int check, doubl
 int fmm_plan_drop_expansions(fmm_plan *plan);
 /* Move the plan's sources to new coordinates (device x, y in the caller's
  * original order) without rebuilding the tree: every source keeps the leaf
- * the tree gave it ("frozen tree"; points may leave their box slightly).
+ * the tree gave it ("frozen tree"; points may leave their box slightly: the far
+ * field converges for points in their boxes, the near field is exact anywhere,
+ * and from then on no pass takes a distance bound from the boxes).
  * Expansions must be built again afterwards.  For finite-difference checks
  * and optimisation loops over slowly moving points; no counterpart in the
  * reference, whose Tree copies the points once (flexmm/tree.py:459-460). */
