@@ -92,19 +92,19 @@ size_t fmmb::smem_optin() {
 
 int fmmb::coop_blocks(const void *kernel, int threads, size_t smem, int per_sm) {
   static std::mutex mu;
-  static std::map<std::tuple<const void *, int, size_t>, int> known;
+  static std::map<std::tuple<const void *, int, int, size_t>, std::pair<int, int>> known;
   int dev = 0;
   FMMB_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> g(mu);
-  int &n = known[{kernel, dev, smem}];
-  if (n == 0) {
+  std::pair<int, int> &k = known[{kernel, dev, threads, smem}];  // SMs, blocks that fit on one
+  if (k.first == 0) {
     int fit = 0, sms = 0;
     FMMB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, threads, smem));
     FMMB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     FMMB_CHECK(fit >= 1, ERR_CUDA, "cooperative kernel does not fit on an SM");
-    n = sms * std::min(fit, per_sm);
+    k = {sms, fit};
   }
-  return n;
+  return k.first * std::min(k.second, per_sm);
 }
 
 namespace {

@@ -180,7 +180,8 @@ struct RadixSync {
 size_t smem_optin();
 
 // Blocks of a cooperative launch that are resident at once on the current
-// device, at most per_sm on each SM (looked up once per kernel, device and size)
+// device, at most per_sm on each SM (how many fit is looked up once per kernel,
+// device and block size; per_sm is the call's own)
 int coop_blocks(const void *kernel, int threads, size_t smem, int per_sm);
 
 // cooperative launch; a single block has no barrier to wait at and is launched
