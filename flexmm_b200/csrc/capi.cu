@@ -353,6 +353,8 @@ struct fmm_ops {
   DevBuf<double> bb_m2mc;     // black-box FMM: M2MC [np x 4np]
   DevBuf<double> bb_m2mct;    // and its transpose [4np x np]
   DevBuf<double> bb_sep;      // tensor factors of both (bb_shift_fragments); empty: none
+  // what the plans of this set did last (fmm_plan::split_expected): a new plan's guess
+  std::atomic<bool> split_expected{true};
   std::vector<std::unique_ptr<LevelEntry>> levels;
 };
 
@@ -383,9 +385,12 @@ struct fmm_plan {
   bool has_st_dipoles = false;
   cudaStream_t side = nullptr;  // from the device's pool, not owned
   cudaStream_t pass = nullptr;  // the pair's high-priority stream (PassStream)
-  // whether the expansions built last were evaluated split (assumed of a new
-  // plan): where they were not, the next build stays on the caller's stream
-  bool split_used = true;
+  // Whether the expansions will be evaluated split, so that the build takes the
+  // scratch and the high-priority stream for it: as the last ones were (the
+  // first build: as the last of the operator set's were; -1 before it).  A guess
+  // for speed alone: a split evaluation without either gives the same bits.
+  int split_expected = -1;
+  bool split_since_build = false;
   bool split_scratch_ready = false;  // allocated for this tree, before its ev_ready
   cudaEvent_t ev_ready = nullptr, ev_near = nullptr, ev_far = nullptr, ev_pass = nullptr;
   bool ready_recorded = false;
@@ -469,12 +474,28 @@ bool capturing(cudaStream_t s) {
   return st != cudaStreamCaptureStatusNone;
 }
 
-// the scratch of the split evaluation that is expected, ahead of ev_ready
+// The scratch of the split evaluation that is expected, ahead of ev_ready; given
+// back where none is.  (Plans that evaluate gradients or other points only held
+// it for nothing: the first pass of a new batch of 12 Stokes problems, whose
+// adjoint evaluates Laplace gradients, 15.4 -> 13.9 ms.)
 void split_scratch_prepare(fmm_plan *p, cudaStream_t s) {
-  if (p->split_used && split_enabled(p->precision) && !capturing(s)) {
+  p->split_since_build = p->split_scratch_ready = false;
+  if (p->split_expected < 0) p->split_expected = p->ops->split_expected;
+  if (capturing(s)) return;
+  if (!p->split_expected || !split_enabled(p->precision)) {
+    p->split_scratch.release();
+  } else {
     p->split_scratch.alloc(p->th.n_total(), p->th.n_points, p->precision == PREC_MIXED, s);
     p->split_scratch_ready = true;
   }
+}
+
+// what an evaluation of a plan's expansions says about the next ones
+void split_note(fmm_plan *p, bool split) {
+  if (p->split_since_build) return;
+  p->split_since_build = split;
+  p->split_expected = split;
+  p->ops->split_expected = split;
 }
 
 // The stream of a plan's FP64 level passes: the high-priority one of its pair,
@@ -488,8 +509,7 @@ void split_scratch_prepare(fmm_plan *p, cudaStream_t s) {
 class PassStream {
  public:
   PassStream(fmm_plan *p, cudaStream_t s) : p_(p), s_(s), ps_(s) {
-    const bool near_beside = split_enabled(PREC_FP64) && p->split_used;
-    p->split_used = false;
+    const bool near_beside = split_enabled(PREC_FP64) && p->split_expected;
     if (!near_beside || capturing(s)) return;
     FMMB_CUDA(cudaStreamWaitEvent(p->pass, p->ev_ready, 0));
     ps_ = p->pass;
@@ -1450,7 +1470,6 @@ static void build_expansions_impl(fmm_plan *p, const double *tau, void *stream) 
     upload_level_ops(p, s);
     split_prepare(p);
     p->ready_recorded = false;
-    p->split_scratch_ready = false;
     split_scratch_prepare(p, s);
     p->sync.alloc(2, s);
     PassArgs a = pass_args(p);
@@ -1540,6 +1559,7 @@ void evaluate_points(fmm_plan *p, int nout, const double *tx, const double *ty, 
   txs.alloc(m, s);
   tys.alloc(m, s);
   if (p->ops->method == METHOD_KIFMM) {
+    split_note(p, false);
     // targets binned into their leaves (a descent along each key's digits and
     // a count per leaf) instead of sorted
     EvalItems it;
@@ -1598,7 +1618,7 @@ void evaluate_own_sources(fmm_plan *p, int nout, int check, double *out, int64_t
                     td.pkeys.get(), td.ordv.get(), m, check, nout, out, ld_out, s);
   else if (nout == 1 && p->ready_recorded && p->n_rhs == 1 && split_enabled(p->precision)) {
     // near field on the side stream, started when the charges were sorted
-    p->split_used = true;
+    split_note(p, true);
     SplitEval se{p->side, p->ev_ready, p->ev_near, p->ev_far};
     if (p->split_scratch_ready && !capturing(s)) se.scratch = &p->split_scratch;
     if (p->precision == PREC_MIXED && p->hold_armed) {
@@ -1610,13 +1630,16 @@ void evaluate_own_sources(fmm_plan *p, int nout, int check, double *out, int64_t
                                        p->lsum.get(), check, out, s, se);
     else
       run_evaluate_sources_split(a, p->tau_s.get(), p->loc.get(), check, out, s, se);
-  } else if (p->precision == PREC_MIXED)
-    run_evaluate_mixed(a, p->tau_s.get(), p->tsum.get(), p->loc32.get(), p->lsum.get(),
-                       td.sx.get(), td.sy.get(), td.pkeys.get(), td.ordv.get(), m, check, nout,
-                       out, ld_out, s);
-  else
-    run_evaluate(a, p->tau_s.get(), p->loc.get(), td.sx.get(), td.sy.get(), td.pkeys.get(),
-                 td.ordv.get(), m, check, nout, out, ld_out, s);
+  } else {
+    split_note(p, false);
+    if (p->precision == PREC_MIXED)
+      run_evaluate_mixed(a, p->tau_s.get(), p->tsum.get(), p->loc32.get(), p->lsum.get(),
+                         td.sx.get(), td.sy.get(), td.pkeys.get(), td.ordv.get(), m, check, nout,
+                         out, ld_out, s);
+    else
+      run_evaluate(a, p->tau_s.get(), p->loc.get(), td.sx.get(), td.sy.get(), td.pkeys.get(),
+                   td.ordv.get(), m, check, nout, out, ld_out, s);
+  }
 }
 }  // namespace
 
