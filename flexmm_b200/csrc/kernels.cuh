@@ -139,16 +139,14 @@ struct LaplaceF64T {
   __host__ __device__ explicit LaplaceF64T(const KernelParams &) {}
   __device__ __forceinline__ double arg(double d2) const { return d2; }
   __device__ __forceinline__ double at(double s) const { return log2_tab(s, lt); }
-  // a pair whose argument is outside the table path; 0 for a coincident pair
-  // when check is set (flexmm/flexmm2d/helpers.py:99-107)
-  __device__ __forceinline__ double raw_rare(double dx, double dy, int check) const {
-    return (check && dx == 0.0 && dy == 0.0) ? 0.0 : log2(dx * dx + dy * dy);
+  // a pair whose argument is outside the table path
+  __device__ __forceinline__ double raw_rare(double dx, double dy) const {
+    return log2(fma(dy, dy, dx * dx));
   }
-  __device__ __forceinline__ double raw_checked(double dx, double dy, int check) const {
+  __device__ __forceinline__ double raw(double dx, double dy) const {
     const double s = arg(fma(dy, dy, dx * dx));
-    return log2_tab_rare(s) ? raw_rare(dx, dy, check) : at(s);
+    return log2_tab_rare(s) ? raw_rare(dx, dy) : at(s);
   }
-  __device__ __forceinline__ double raw(double dx, double dy) const { return raw_checked(dx, dy, 0); }
   __device__ __forceinline__ double operator()(double sx, double sy, double tx, double ty) const {
     return kFold * raw(tx - sx, ty - sy);
   }
@@ -164,7 +162,7 @@ struct LaplaceF64T {
                                             double &w) const {
     v = w = 0.0;
     if (check && dx == 0.0 && dy == 0.0) return;
-    const double d2 = dx * dx + dy * dy;
+    const double d2 = fma(dy, dy, dx * dx);
     v = log2(d2);
     w = 1.0 / d2;
   }
@@ -227,16 +225,14 @@ struct ModHelmholtzF64T {
     bessel_small<false>(s, log2_tab(s, lt), k0, k1x);
     return k0;
   }
-  __device__ __forceinline__ double raw_rare(double dx, double dy, int check) const {
-    if (check && dx == 0.0 && dy == 0.0) return 0.0;
-    const double d2 = dx * dx + dy * dy;
+  __device__ __forceinline__ double raw_rare(double dx, double dy) const {
+    const double d2 = fma(dy, dy, dx * dx);
     return bessel_any<false>(k, d2, k2 * d2, tab).x;
   }
-  __device__ __forceinline__ double raw_checked(double dx, double dy, int check) const {
+  __device__ __forceinline__ double raw(double dx, double dy) const {
     const double s = arg(fma(dy, dy, dx * dx));
-    return log2_rare_key(s) >= kRare ? raw_rare(dx, dy, check) : at(s);
+    return log2_rare_key(s) >= kRare ? raw_rare(dx, dy) : at(s);
   }
-  __device__ __forceinline__ double raw(double dx, double dy) const { return raw_checked(dx, dy, 0); }
   __device__ __forceinline__ double operator()(double sx, double sy, double tx, double ty) const {
     return kFold * raw(tx - sx, ty - sy);
   }
@@ -247,7 +243,7 @@ struct ModHelmholtzF64T {
                                             double &w) const {
     v = w = 0.0;
     if (check && dx == 0.0 && dy == 0.0) return;
-    const double d2 = dx * dx + dy * dy;
+    const double d2 = fma(dy, dy, dx * dx);
     const double2 b = bessel_any<true>(k, d2, k2 * d2, tab);
     v = b.x;
     w = b.y;

@@ -11,9 +11,10 @@ constexpr double INV_2PI = 1.0 / (2.0 * M_PI);
 
 // double-layer kernel of the Laplace kernel -log(r^2)/(4 pi): the field at
 // offset (ax, ay) = target - source of a dipole (dx, dy) = strength * normal,
-// (d . a) / (2 pi |a|^2) (Laplace_Both_Eval, examples/pure_kifmm_laplace_dipoles.py:31-40)
+// (d . a) / (2 pi |a|^2) (Laplace_Both_Eval, examples/pure_kifmm_laplace_dipoles.py:31-40),
+// times 2 pi
 __device__ __forceinline__ double dipole_at(double dx, double dy, double ax, double ay) {
-  return fma(dx, ax, dy * ay) / fma(ax, ax, ay * ay) * INV_2PI;
+  return fma(dx, ax, dy * ay) / fma(ax, ax, ay * ay);
 }
 
 template <int R, int NV>
@@ -22,9 +23,12 @@ using PairAcc = double[R][NV];
 // Potential sums of a table functor: every charge q is staged times KF::kFold,
 // so a pair adds q * raw.  Batches of U sources and R targets test their
 // arguments together: one pair outside the table path (a coincident pair,
-// as a rule) sends its batch to the pair-by-pair path.  Sources alternate
-// between two chains per target (v[r][0], v[r][1]) by their place in the
-// thread's sequence, whatever U is.
+// as a rule) sends its batch to the pair-by-pair path.  Which targets share a
+// batch is chance where they stand in no particular order, so a pair's
+// arithmetic is its own: both paths add a pair inside the table by the same
+// operations, all written out (fma, __dmul_rn), none left to the compiler to
+// contract.  Sources alternate between two chains per target (v[r][0], v[r][1])
+// by their place in the thread's sequence, whatever U is.
 template <class KF, int R, int U, bool DIP, bool CAT>
 __device__ __forceinline__ void pot_batch(const KF &K, const double2 *xy, const double *q,
                                           const double2 *dv, const long long *cat,
@@ -33,6 +37,15 @@ __device__ __forceinline__ void pot_batch(const KF &K, const double2 *xy, const 
                                           double (&v)[R][2]) {
   double s[R][U];
   double ax[DIP ? R : 1][U], ay[DIP ? R : 1][U];
+  constexpr unsigned LIMIT = DIP && RCP_RARE < KF::kRare ? RCP_RARE : KF::kRare;
+  // a pair inside the table: s its argument, w its charge, (dx, dy) its offset
+  auto table_pair = [&](double s, double w, double dx, double dy, int jj, double &o) {
+    o = fma(K.at(s), w, o);
+    if constexpr (DIP) {
+      const double2 d = dv[jj];
+      o = fma(fma(d.x, dx, d.y * dy) * INV_2PI, rcp_newton(s), o);
+    }
+  };
   unsigned key = 0;
 #pragma unroll
   for (int i = 0; i < U; ++i) {
@@ -48,7 +61,7 @@ __device__ __forceinline__ void pot_batch(const KF &K, const double2 *xy, const 
       }
     }
   }
-  if (key < (DIP ? min(RCP_RARE, KF::kRare) : KF::kRare)) {
+  if (key < LIMIT) {
 #pragma unroll
     for (int i = 0; i < U; ++i) {
       const double c = q[j + i * G];
@@ -56,12 +69,8 @@ __device__ __forceinline__ void pot_batch(const KF &K, const double2 *xy, const 
       for (int r = 0; r < R; ++r) {
         double w = c;
         if constexpr (CAT) w = cat[j + i * G] == tc[r] ? 0.0 : c;
-        v[r][i & 1] = fma(K.at(s[r][i]), w, v[r][i & 1]);
-        if constexpr (DIP) {
-          const double2 d = dv[j + i * G];
-          v[r][i & 1] = fma(fma(d.x, ax[r][i], d.y * ay[r][i]) * INV_2PI, rcp_newton(s[r][i]),
-                            v[r][i & 1]);
-        }
+        table_pair(s[r][i], w, DIP ? ax[DIP ? r : 0][i] : 0.0, DIP ? ay[DIP ? r : 0][i] : 0.0,
+                   j + i * G, v[r][i & 1]);
       }
     }
   } else {
@@ -72,21 +81,24 @@ __device__ __forceinline__ void pot_batch(const KF &K, const double2 *xy, const 
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const double dx = x[r] - p.x, dy = y[r] - p.y;
-        double a = 0.0;
-        if constexpr (CAT) {
-          if (cat[j + i * G] != tc[r]) a = K.raw_checked(dx, dy, check) * c;
-        } else if constexpr (DIP) {
-          if (!(check && dx == 0.0 && dy == 0.0)) {
+        const double t = K.arg(fma(dy, dy, dx * dx));
+        if constexpr (CAT)
+          if (cat[j + i * G] == tc[r]) continue;
+        double o = i & 1 ? v[r][1] : v[r][0];
+        if (log2_rare_key(t) < LIMIT) {
+          table_pair(t, c, dx, dy, j + i * G, o);
+        } else if (!(check && dx == 0.0 && dy == 0.0)) {
+          // (a coincident pair is skipped when check is set, helpers.py:99-107)
+          o = fma(DIP ? K.raw(dx, dy) : K.raw_rare(dx, dy), c, o);
+          if constexpr (DIP) {
             const double2 d = dv[j + i * G];
-            a = K.raw(dx, dy) * c + dipole_at(d.x, d.y, dx, dy);
+            o = fma(dipole_at(d.x, d.y, dx, dy), INV_2PI, o);
           }
-        } else {
-          a = K.raw_checked(dx, dy, check) * c;
         }
         if (i & 1)
-          v[r][1] += a;
+          v[r][1] = o;
         else
-          v[r][0] += a;
+          v[r][0] = o;
       }
     }
   }
@@ -96,7 +108,7 @@ __device__ __forceinline__ void pot_batch(const KF &K, const double2 *xy, const 
 template <class KF>
 __device__ __forceinline__ double pair_value(const KF &K, double2 p, double x, double y, double q,
                                              int check) {
-  const double v = K(p.x, p.y, x, y) * q;
+  const double v = __dmul_rn(K(p.x, p.y, x, y), q);
   return (check && x - p.x == 0.0 && y - p.y == 0.0) ? 0.0 : v;
 }
 
@@ -142,26 +154,40 @@ __device__ __forceinline__ void grad_sweep(const KF &K, const double2 *xy, const
     const double2 p = xy[j];
     const double c = q[j];
     if constexpr (KF::kLogTable) {
+      // (the targets test together for the common case, each decides for itself)
+      constexpr unsigned LIMIT = RCP_RARE < KF::kRare ? RCP_RARE : KF::kRare;
       double dx[R], dy[R], s[R];
-      unsigned key = 0;
+      unsigned key[R], most = 0;
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         dx[r] = x[r] - p.x;
         dy[r] = y[r] - p.y;
         s[r] = K.arg(fma(dy[r], dy[r], dx[r] * dx[r]));
-        key = max(key, log2_rare_key(s[r]));
+        key[r] = log2_rare_key(s[r]);
+        most = max(most, key[r]);
       }
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        double a, w;
-        if (key < min(RCP_RARE, KF::kRare))
-          K.at_grad(s[r], a, w);
-        else
-          K.grad_rare(dx[r], dy[r], check, a, w);
-        w *= c;
+      auto add = [&](int r, double a, double w) {
+        w = __dmul_rn(w, c);
         v[r][0] = fma(a, c, v[r][0]);
         v[r][1] = fma(w, dx[r], v[r][1]);
         v[r][2] = fma(w, dy[r], v[r][2]);
+      };
+      double a, w;
+      if (most < LIMIT) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          K.at_grad(s[r], a, w);
+          add(r, a, w);
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          if (key[r] < LIMIT)
+            K.at_grad(s[r], a, w);
+          else
+            K.grad_rare(dx[r], dy[r], check, a, w);
+          add(r, a, w);
+        }
       }
     } else {
 #pragma unroll
