@@ -109,6 +109,7 @@ SIGNATURES = [
     ("fmm_tree_export", ctypes.c_int, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     ("fmm_direct", ctypes.c_int, [ctypes.c_int, _dp, _vp, _vp, _vp, ctypes.c_int64, _vp, _vp,
                                   ctypes.c_int64, ctypes.c_int, _vp, _vp]),
+    ("fmm_diag_fail_passes", ctypes.c_int, [_vp, _vp]),
     ("fmm_diag_log2", ctypes.c_int, [_vp, ctypes.c_int64, _vp, _vp, _vp]),
     ("fmm_timing_enable", ctypes.c_int, [ctypes.c_int]),
     ("fmm_set_split_evaluation", ctypes.c_int, [ctypes.c_int]),

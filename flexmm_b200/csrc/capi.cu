@@ -370,7 +370,10 @@ struct fmm_plan {
   DevBuf<float> mult_tc;        // ... multipoles split TF32 hi / lo ...
   DevBuf<double> msum, lsum;    // ... and their FP64 component sums
   DevBuf<double> tsum;          // per node: FP64 sum of its charges
-  DevBuf<RadixSync> sync;       // barriers of the level passes (upward, downward)
+  // FP64 level passes: their barriers (upward, downward) and, as the third's
+  // timeout, their failure flag; zeroed by each build
+  DevBuf<RadixSync> sync;
+  int *pass_fail() const { return sync.get() ? &sync.get()[2].timeout : nullptr; }
   DevBuf<int> err;              // set by kernels whose bounded waits ran out
   int precision = PREC_FP64;
   bool moved = false;  // sources moved on the frozen tree: a box no longer bounds its own
@@ -1084,6 +1087,7 @@ static PassArgs pass_args(fmm_plan *p) {
   a.th = &p->th;
   a.ops_dev = p->ops_dev.get();
   a.sync = p->sync.get();
+  if (p->precision == PREC_FP64) a.fail = p->pass_fail();
   if (p->has_dipoles) {
     a.dvx = p->dvx.get();
     a.dvy = p->dvy.get();
@@ -1266,7 +1270,7 @@ int fmm_build_expansions_multi(fmm_plan *p, const double *tau, int n_rhs, int64_
     const int64_t total = th.n_total(), n = th.n_points, cs = total * np;
     upload_level_ops(p, s);
     p->has_dipoles = false;
-    p->sync.alloc(2, s);
+    p->sync.alloc(3, s);
     PassArgs a = pass_args(p);
     p->tau_s.alloc((size_t)n_rhs * n, s);
     p->mult.alloc((size_t)n_rhs * cs, s);
@@ -1471,7 +1475,7 @@ static void build_expansions_impl(fmm_plan *p, const double *tau, void *stream) 
     split_prepare(p);
     p->ready_recorded = false;
     split_scratch_prepare(p, s);
-    p->sync.alloc(2, s);
+    p->sync.alloc(3, s);
     PassArgs a = pass_args(p);
     p->tau_s.alloc(th.n_points, s);
     if (tau)
@@ -1694,8 +1698,25 @@ int fmm_plan_status(fmm_plan *p) {
     if (p->td.sort_fail.get()) {
       int h = 0;
       FMMB_CUDA(cudaMemcpy(&h, p->td.sort_fail.get(), sizeof(int), cudaMemcpyDeviceToHost));
-      FMMB_CHECK(h == 0, ERR_CUDA, "a radix sort's grid barrier wait ran out of time; results are invalid");
+      FMMB_CHECK(h == 0, ERR_CUDA,
+                 "a sort's or scan's grid barrier wait ran out of time; results are invalid");
     }
+    if (p->precision == PREC_FP64 && p->pass_fail()) {
+      int h = 0;
+      FMMB_CUDA(cudaMemcpy(&h, p->pass_fail(), sizeof(int), cudaMemcpyDeviceToHost));
+      FMMB_CHECK(h == 0, ERR_CUDA,
+                 "a level pass's wait (grid barrier or operator copy) ran out of time; results are "
+                 "invalid (NaN)");
+    }
+  });
+}
+
+int fmm_diag_fail_passes(fmm_plan *p, void *stream) {
+  return guarded([&] {
+    FMMB_CHECK(p, ERR_INVALID_ARGUMENT, "plan is NULL");
+    FMMB_CHECK(p->have_expansions && p->precision == PREC_FP64 && p->pass_fail(), ERR_NOT_READY,
+               "no FP64 KIFMM expansions have been built");
+    FMMB_CUDA(cudaMemsetAsync(p->pass_fail(), 1, sizeof(int), (cudaStream_t)stream));
   });
 }
 
@@ -1921,14 +1942,7 @@ extern "C" int fmm_evaluate_noalloc(fmm_plan *p, const double *tx, const double 
     FMMB_CHECK(at <= NOALLOC_SCRATCH_BYTES, ERR_CAPACITY,
                "fmm_evaluate_noalloc: scratch needs exceed the static array");
     // the same passes as fmm_evaluate, on the static scratch
-    PassArgs a;
-    a.kernel_id = p->ops->kernel_id;
-    a.kp = p->ops->kp;
-    a.neq = p->ops->neq;
-    a.np = p->ops->np;
-    a.td = &p->td;
-    a.th = &p->th;
-    a.ops_dev = p->ops_dev.get();
+    const PassArgs a = pass_args(p);
     {
       PhaseTimer timer(PH_SORT_TGT, s);
       sort_points_scratch(tx, ty, m, p->th, digits, tkeys, tperm, txs, tys, sort_tmp, sort_bytes,

@@ -933,7 +933,10 @@ struct KIPolicy : ChargePolicy<KF, NOUT, DIP, CAT> {
   const double *xmid, *ymid, *loc;
   const LevelOpsDev *ops;
   double *near;
+  const int *fail;  // PassArgs::fail
 
+  // (the near field alone reads no expansions, and runs beside the passes)
+  __device__ __forceinline__ bool failed() const { return kFar && fail && *fail; }
   __device__ __forceinline__ void stage_far(Smem &sm, int g, int lev) const {
     if constexpr (kFar) {
       for (int k = threadIdx.x; k < neq; k += EV_THREADS) {
@@ -1008,6 +1011,7 @@ Pol ki_policy(const PassArgs &a, const double *tau_s, const double *loc, int che
   p.loc = loc;
   p.ops = a.ops_dev;
   p.near = near;
+  p.fail = a.fail;
   return p;
 }
 
@@ -1054,7 +1058,8 @@ __global__ void __launch_bounds__(TCH) k_evaluate_multi(KernelParams kp, int neq
                                                         const double *__restrict__ txs,
                                                         const double *__restrict__ tys,
                                                         const int *__restrict__ tperm, int check,
-                                                        double *__restrict__ out, int64_t ld_out) {
+                                                        double *__restrict__ out, int64_t ld_out,
+                                                        const int *__restrict__ fail) {
   __shared__ double2 sxy[SMAX_MR];
   __shared__ __align__(16) double stau[SMAX_MR][R + 2];  // (padded: fewer bank conflicts)
   __shared__ int rb[9], rs[10];
@@ -1063,6 +1068,7 @@ __global__ void __launch_bounds__(TCH) k_evaluate_multi(KernelParams kp, int neq
   KF K(kp);
   fsm.bind(K);
   const int n_items = *n_items_ptr;
+  const bool failed = fail && *fail;
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
     const int4 it = items[item];
     const int g = it.x, lev = it.y & EVAL_LEVEL_MASK, t0 = it.z, cnt = it.w;
@@ -1138,7 +1144,7 @@ __global__ void __launch_bounds__(TCH) k_evaluate_multi(KernelParams kp, int neq
           for (int q = 0; q < G / 32; ++q) w += red[c][(threadIdx.x >> 5) + q];
         }
       }
-      if (valid && sub == 0 && c < ncol) out[c * ld_out + tperm[t0 + t]] = w;
+      if (valid && sub == 0 && c < ncol) out[c * ld_out + tperm[t0 + t]] = failed ? nan("") : w;
     }
     __syncthreads();
   }
@@ -1249,7 +1255,7 @@ void upward_impl(const PassArgs &a, const double *tau_s, double *mult, cudaStrea
   const int *parent = td.parent.get();
   const LevelOpsDev *ops = a.ops_dev;
   RadixSync *sync = a.sync;
-  int *fail = td.sort_fail.get();
+  int *fail = a.fail;
   void *args[] = {&sp, &np_, &n_rhs_, &parent, &ops, &mult, &cstride, &sync, &fail};
   launch_coop(reinterpret_cast<const void *>(k_up_levels), grid, NT, args, up_bytes, s);
 }
@@ -1427,7 +1433,7 @@ void run_downward(const PassArgs &a, const double *ple, double *loc, cudaStream_
   const int *rg = td.rg.get(), *parent = td.parent.get();
   const LevelOpsDev *ops = a.ops_dev;
   RadixSync *sync = a.sync + 1;
-  int *fail = td.sort_fail.get();
+  int *fail = a.fail;
   void *args[] = {&sp, &np_, &n_rhs_, &rg, &parent, &ops, &ple, &loc, &cstride, &sync, &fail};
   launch_coop(reinterpret_cast<const void *>(k_down_levels), grid, NT, args, bytes, s);
 }
@@ -1522,7 +1528,7 @@ void evaluate_multi_impl(const PassArgs &a, const double *tau_s, int64_t n_src, 
           a.kp, a.neq, a.np, ncol, it.items.get(), it.n_items.get(), td.coll.get(), td.bot.get(),
           td.top.get(), td.xmid.get(), td.ymid.get(), td.sx.get(), td.sy.get(), tau_s + r0 * n_src,
           n_src, a.ops_dev, loc + r0 * col_stride, col_stride, txs, tys, tperm, check,
-          out + r0 * ld_out, ld_out);
+          out + r0 * ld_out, ld_out, a.fail);
       FMMB_CUDA(cudaGetLastError());
       r0 += R;
     };

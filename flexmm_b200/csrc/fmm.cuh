@@ -53,6 +53,9 @@ struct PassArgs {
   const TreeHost *th;
   const LevelOpsDev *ops_dev;   // device array indexed by level
   RadixSync *sync = nullptr;  // two zeroed grid barriers (upward, downward passes)
+  // set to 1 by a level pass whose bounded wait ran out (its expansions are then
+  // half formed), 0 before; the FP64 evaluations give NaN where it is set
+  int *fail = nullptr;
   // dipole sources (Laplace double layer): per sorted source the dipole
   // vector strength * normal; null when the sources carry charges only
   const double *dvx = nullptr, *dvy = nullptr;

@@ -21,6 +21,7 @@
 //
 // A policy holds what one form sums: its staged source record, the far field
 // and the pair sweep.  All its members run on every thread of the block.
+// failed(): the expansions are not to be used (the results are NaN then).
 #pragma once
 #include <type_traits>
 
@@ -56,6 +57,7 @@ __global__ void __launch_bounds__(EV_THREADS, BLOCKS) k_items(const Pol pol, con
   __shared__ int s_next;
   typename Pol::Kernel K = pol.bind(sm);
   const int n_items = *a.n_items;
+  const bool failed = pol.failed();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int item = blockIdx.x, left = a.per_block;
   while (item < n_items && left-- > 0) {
@@ -153,7 +155,8 @@ __global__ void __launch_bounds__(EV_THREADS, BLOCKS) k_items(const Pol pol, con
       double o[Pol::NOUT];
 #pragma unroll
       for (int k = 0; k < Pol::NOUT; ++k)
-        o[k] = (red[k][0][tid] + red[k][1][tid]) + (red[k][2][tid] + red[k][3][tid]);
+        o[k] = failed ? nan("")
+                      : (red[k][0][tid] + red[k][1][tid]) + (red[k][2][tid] + red[k][3][tid]);
       pol.store(a.tperm[t0 + tid], o);
     }
     item = next;

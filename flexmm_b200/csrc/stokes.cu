@@ -188,6 +188,7 @@ struct StokesPolicy {
   double *out;
   int64_t ld_out;
 
+  __device__ __forceinline__ bool failed() const { return false; }
   __device__ __forceinline__ LaplaceF64T bind(Smem &sm) const {
     LaplaceF64T K(KernelParams{});
     sm.fs.bind(K);

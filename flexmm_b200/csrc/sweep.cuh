@@ -247,6 +247,7 @@ struct ChargePolicy {
     if constexpr (DIP) sm.dv[i] = make_double2(dvx[j], dvy[j]);
     if constexpr (CAT) sm.cat[i] = (long long)scat[j];
   }
+  __device__ __forceinline__ bool failed() const { return false; }
   template <class T>
   __device__ __forceinline__ void load_target(T &tg, int r, const int *tperm, int t) const {
     if constexpr (CAT) tg.cat[r] = (long long)tcat[tperm[t]];

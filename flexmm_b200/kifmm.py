@@ -486,7 +486,10 @@ class KI_FMM:
         return self._evaluate(x, y, False)
 
     def status(self):
-        """Wait for this object's GPU work and raise if a kernel reported a failure."""
+        """Wait for this object's GPU work and raise if a kernel reported a failure.
+
+        Nothing else waits to ask: FP64 evaluations give NaN where a level pass
+        of the build before them stopped one of its bounded waits."""
         _lib.call("fmm_plan_status", self._plan)
 
     def direct_evaluation(self, x, y, check=False):

@@ -279,7 +279,10 @@ int fmm_plan_move_sources(fmm_plan *plan, const double *x, const double *y, void
  * loop that builds a plan per step keeps the host ahead of the GPU. */
 int fmm_plan_destroy(fmm_plan *plan);
 /* Wait for the plan's work and report failures of it: FMM_ERR_CUDA when a
- * kernel stopped one of its bounded waits (the results are then invalid). */
+ * kernel stopped one of its bounded waits (the results are then invalid).  No
+ * other call waits for the GPU to ask: a tree build whose sorts stopped fails
+ * in fmm_plan_create; the FP64 evaluations give NaN where a level pass of the
+ * build before them stopped (the next build starts afresh). */
 int fmm_plan_status(fmm_plan *plan);
 
 /* Copy the tree to host arrays sized by fmm_plan_info (nodes = sum n_nodes):
@@ -341,6 +344,10 @@ int fmm_set_split_evaluation(int mode);
 #define FMM_NOALLOC_MAX_NODES 262144
 int fmm_evaluate_noalloc(fmm_plan *plan, const double *tx, const double *ty, int64_t m, int check,
                          double *out, void *stream);
+
+/* Diagnostic: leaves the expansions of an FP64 KIFMM plan marked as a level pass
+ * does whose bounded wait ran out, on `stream`.  For tests of how that shows. */
+int fmm_diag_fail_passes(fmm_plan *plan, void *stream);
 
 /* Diagnostic: the table-driven log2 that the FP64 passes use for the
  * Laplace kernel (exponent split, a table of 129 pairs 1/F and log2 F, a
