@@ -279,7 +279,7 @@ void retain_pool_memory() {
 // The black-box M2M operator [p^2 x 4 p^2] as tensor factors: child c's block is
 // X_c (x) Y_c, read off its first rows and columns (T_0 = 1 keeps its value under
 // a shift, so X_c[0][0] = Y_c[0][0] = 1).  False where that is not the operator to
-// 2e-14 of its largest element (the factors of the Chebyshev shift reproduce it
+// 6e-15 of its largest element (the factors of the Chebyshev shift reproduce it
 // to 5e-15 at most, p = 2 .. 16; any other is applied as it is).  Fragments for k_bb_shift
 // (bbfmm.cu): M2M's Y and X, then L2L's, Y^T and X^T, each [4][P x P], P = 8 or 16.
 bool bb_shift_fragments(int p, const double *m2mc, std::vector<double> &out) {
@@ -300,7 +300,7 @@ bool bb_shift_fragments(int p, const double *m2mc, std::vector<double> &out) {
             const double d = std::fabs(v - X(c, a, a1) * Y(c, b, b1));
             if (!(d <= off)) off = d;  // (NaN stays)
           }
-  if (!(off <= 2e-14 * big)) return false;
+  if (!(off <= 6e-15 * big)) return false;
   const size_t F = size_t(4) * P * P;
   out.assign(4 * F, 0.0);
   const int NB = P / 8, KS = P / 4;
