@@ -116,25 +116,38 @@ __device__ __noinline__ double2 bessel_large(double x, const double *__restrict_
   return make_double2(r[0], r[1]);
 }
 
-// K0(x) and K1(x) / x for any x = k r >= 0: r2 = r^2, s = k^2 r2
+// k^2 as the arguments s = k^2 r^2 take it: 0 where the square has lost bits
+// below the normal range (every pair then goes by bessel_any's last branch)
+__host__ __device__ __forceinline__ double bessel_k2(double k) {
+  const double k2 = k * k;
+  return k2 < 0x1p-1022 ? 0.0 : k2;
+}
+
+// K0(x) and, with K1 = true, k^2 K1(x) / x (the gradient's factor, 1 / r^2 for
+// small x), for any x = k r >= 0: r2 = r^2, s = bessel_k2(k) r2
 template <bool K1>
 __device__ __noinline__ double2 bessel_any(double k, double r2, double s,
                                            const double *__restrict__ tab) {
-  if (s >= 1.0 && s < 1048576.0) return bessel_large<K1>(sqrt(s), tab);
-  double2 r;
-  if (s >= 0x1p-1022 && s < 1.0) {
+  double2 r = make_double2(0.0, 0.0);
+  if (s >= 1.0 && s < 1048576.0) {
+    r = bessel_large<K1>(sqrt(s), tab);
+  } else if (s >= 0x1p-1022 && s < 1.0) {
     bessel_small<K1>(s, log2(s), r.x, r.y);
-    return r;
+  } else {
+    // a square leaves the range: the distance itself may not
+    const double x = k * sqrt(r2);
+    if (x < 1.0) {
+      bessel_small<K1>(x * x, 2.0 * log2(x), r.x, r.y);
+      // (x K1(x) = 1 + O(x^2 log x): 1 to the last bit)
+      if (K1 && x < 0x1p-30) return make_double2(r.x, 1.0 / r2);
+    } else if (x < 1024.0) {
+      r = bessel_large<K1>(x, tab);
+    } else {
+      r.x = r.y = x >= 1024.0 ? 0.0 : x;  // NaN stays
+    }
   }
-  // the square leaves the range: the distance itself may not
-  const double x = k * sqrt(r2);
-  if (x < 1.0) {
-    bessel_small<K1>(x * x, 2.0 * log2(x), r.x, r.y);
-    return r;
-  }
-  if (x < 1024.0) return bessel_large<K1>(x, tab);
-  const double v = x >= 1024.0 ? 0.0 : x;  // NaN stays
-  return make_double2(v, v);
+  if (K1) r.y = k * (k * r.y);  // (k^2 may leave the range where this does not)
+  return r;
 }
 
 }  // namespace fmmb

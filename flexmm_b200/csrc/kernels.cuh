@@ -183,7 +183,7 @@ struct ModHelmholtzF64 {
   double k, k2;
   const double *tab;
   __host__ __device__ explicit ModHelmholtzF64(const KernelParams &kp)
-      : k(kp.p[0]), k2(kp.p[0] * kp.p[0]), tab(kp.table) {}
+      : k(kp.p[0]), k2(bessel_k2(kp.p[0])), tab(kp.table) {}
   __device__ __forceinline__ double operator()(double sx, double sy, double tx, double ty) const {
     const double dx = tx - sx, dy = ty - sy, d2 = dx * dx + dy * dy;
     return bessel_any<false>(k, d2, k2 * d2, tab).x * (1.0 / (2.0 * M_PI));
@@ -195,7 +195,7 @@ struct ModHelmholtzF64 {
                                        double &u, double &ux, double &uy) const {
     const double dx = tx - sx, dy = ty - sy, d2 = dx * dx + dy * dy;
     const double2 b = bessel_any<true>(k, d2, k2 * d2, tab);
-    const double s = -k2 * b.y * (1.0 / (2.0 * M_PI)) * q;
+    const double s = -b.y * (1.0 / (2.0 * M_PI)) * q;
     u += b.x * (1.0 / (2.0 * M_PI)) * q;
     ux += s * dx;
     uy += s * dy;
@@ -215,10 +215,8 @@ struct ModHelmholtzF64T {
   const double *tab;
   const double2 *lt = nullptr;
   __host__ __device__ explicit ModHelmholtzF64T(const KernelParams &kp)
-      : k(kp.p[0]), k2(kp.p[0] * kp.p[0]), tab(kp.table) {}
-  static __host__ __device__ double grad_fold(const KernelParams &kp) {
-    return -(1.0 / (2.0 * M_PI)) * (kp.p[0] * kp.p[0]);
-  }
+      : k(kp.p[0]), k2(bessel_k2(kp.p[0])), tab(kp.table) {}
+  static __host__ __device__ double grad_fold(const KernelParams &) { return -1.0 / (2.0 * M_PI); }
   __device__ __forceinline__ double arg(double d2) const { return k2 * d2; }
   __device__ __forceinline__ double at(double s) const {
     double k0, k1x;
@@ -238,6 +236,7 @@ struct ModHelmholtzF64T {
   }
   __device__ __forceinline__ void at_grad(double s, double &v, double &w) const {
     bessel_small<true>(s, log2_tab(s, lt), v, w);
+    w *= k2;  // here and not on the sums: 1 / k^2 and with it K1(x) / x may leave the range
   }
   __device__ __forceinline__ void grad_rare(double dx, double dy, int check, double &v,
                                             double &w) const {
