@@ -6,6 +6,7 @@
 
 #include <map>
 #include <atomic>
+#include <cstddef>
 #include <mutex>
 
 #include <memory>
@@ -1114,23 +1115,28 @@ struct LevelOpsSrc {
   double width[FMM_MAX_LEVELS_DEV];  // what a box's sources keep to; infinite once they were moved
   // scaling of levels without operators (0 and 1 need none: no expansions there,
   // but the mixed near field of a leaf there does read its scaling)
-  double inv_w[FMM_MAX_LEVELS_DEV], kofs[FMM_MAX_LEVELS_DEV];
+  struct Scale {
+    double inv_w, kofs;
+  } scale[FMM_MAX_LEVELS_DEV];
 };
+static_assert(offsetof(LevelOpsDev, kofs) == offsetof(LevelOpsDev, inv_w) + sizeof(double),
+              "LevelOpsSrc::Scale is copied over both");
 static_assert(sizeof(LevelOpsDev) % sizeof(int) == 0, "LevelOpsDev is copied as words");
 
 __global__ void k_gather_level_ops(LevelOpsSrc src, LevelOpsDev *__restrict__ dst) {
   constexpr int NW = int(sizeof(LevelOpsDev) / sizeof(int));
   const int *from = reinterpret_cast<const int *>(src.p[blockIdx.x]);
   int *to = reinterpret_cast<int *>(dst + blockIdx.x);
-  for (int i = threadIdx.x; i < NW; i += blockDim.x) to[i] = from ? from[i] : 0;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    LevelOpsDev &d = dst[blockIdx.x];
-    if (!from) {
-      d.inv_w = src.inv_w[blockIdx.x];
-      d.kofs = src.kofs[blockIdx.x];
-    }
-    d.box32 = float(src.width[blockIdx.x] * d.inv_w);
+  constexpr int SCALE = int(offsetof(LevelOpsDev, inv_w) / sizeof(int));
+  constexpr int BOX = int(offsetof(LevelOpsDev, box32) / sizeof(int));
+  const LevelOpsSrc::Scale &sc = src.scale[blockIdx.x];
+  for (int i = threadIdx.x; i < NW; i += blockDim.x) {
+    int v = from ? from[i] : 0;
+    if (i == BOX)
+      v = __float_as_int(float(src.width[blockIdx.x] * (from ? src.p[blockIdx.x]->inv_w : sc.inv_w)));
+    else if (!from && i >= SCALE && i < SCALE + 4)
+      v = reinterpret_cast<const int *>(&sc)[i - SCALE];
+    to[i] = v;
   }
 }
 
@@ -1146,8 +1152,8 @@ static void upload_level_ops(fmm_plan *p, cudaStream_t s) {
     if (p->bound[m] >= 0) {
       src.p[m] = p->ops->levels[p->bound[m]]->dev_copy.get();
     } else {
-      src.inv_w[m] = scaled ? 1.0 / w : 1.0;
-      src.kofs[m] = scaled ? kernel_offset(p->ops->kernel_id, p->ops->kp, w) : 0.0;
+      src.scale[m] = {scaled ? 1.0 / w : 1.0,
+                      scaled ? kernel_offset(p->ops->kernel_id, p->ops->kp, w) : 0.0};
     }
   }
   k_gather_level_ops<<<L, 128, 0, s>>>(src, p->ops_dev.get());
