@@ -17,6 +17,7 @@
 
 #include "bessel.cuh"
 #include "common.cuh"
+#include "log2_table.cuh"
 
 namespace fmmb {
 
@@ -32,29 +33,26 @@ struct KernelParams {
 // ---------------------------------------------------------------------------
 // Table-driven FP64 log2, after P. T. P. Tang, "Table-driven implementation
 // of the logarithm function in IEEE floating-point arithmetic", ACM TOMS 16
-// (1990): d = 2^e m, m in [1, 2); F = 1 + j/128 is the table point nearest m
-// and c = 1/F rounded, so r = m c - 1 (one fused multiply-add) has
-// |r| <= 2^-8 and
+// (1990): d = 2^e m, m in [1, 2); F = 1 + j/256 is the table point nearest m
+// and c next to 1/F, so r = m c - 1 (one fused multiply-add) has |r| <= 2^-9 and
 //   log2 d = e - log2 c + log2(1 + r),  log2(1 + r) = r q(r),
 // q the degree-4 polynomial that takes log2(1 + r)/r's values at the five
-// Chebyshev nodes of [-2^-8, 2^-8] (error of r q(r): 5.4e-17).  The table
-// holds c (IEEE division) and -log2 c (CUDA's log2) for j = 0..128, filled in
-// shared memory by each block.  Absolute error about one ulp of the result
-// (~1e-16 relative to max(1, |log2 d|)): far inside the 1e-12 parity bar, in
-// 9 FP64 instructions.  Zero, subnormal, infinite and NaN arguments take the
-// library log2 instead.
-// A pair loop over it costs 11.8 clocks per 32 pairs and SM with two targets
-// a thread, 17.2 with the 257-point table and r = (m - F) / F before (the
-// FP64 instructions alone: 7.2); spreading the table over the banks (8
-// copies) gave 11.35 for 14 KB more per block.
-constexpr int LOG2_TAB_N = 128;
+// Chebyshev nodes of [-2^-9, 2^-9] (error of r q(r): 9e-19).  The table holds c
+// and -log2 c for j = 0..256 (log2_table.cuh), copied to shared memory by each
+// block; its values are doubles to 2^-13 of their last place.  So the error is
+// the two roundings of the last sum, half an ulp each: at most 2.2e-16 relative
+// to max(1, |log2 d|), 2e-18 next to d = 1, in 9 FP64 instructions.  Zero,
+// subnormal, infinite and NaN arguments take the library log2 instead.
+// 257 rows and not 129: with these q would have to have one more term (an FP64
+// instruction in 13 of a pair) or be off by 5e-17, more than all else next to
+// d = 1.  Copied and not formed in each block by a division and a logarithm a
+// row: a step of 1M clustered points, near field 1.2 ms of it, takes 2254 us with 129
+// rows copied, 2285 with 129 formed, 2282 with 257 copied, 2319 with 257 formed,
+// 2286 with 129 copied and the longer q.
 struct Log2Table {
   double2 t[LOG2_TAB_N + 1];
   __device__ void fill() {
-    for (int i = threadIdx.x; i <= LOG2_TAB_N; i += blockDim.x) {
-      const double c = 1.0 / (1.0 + i * (1.0 / LOG2_TAB_N));
-      t[i] = make_double2(c, -log2(c));
-    }
+    for (int i = threadIdx.x; i <= LOG2_TAB_N; i += blockDim.x) t[i] = LOG2_ROWS[i];
   }
 };
 
@@ -70,13 +68,13 @@ __device__ __forceinline__ bool log2_tab_rare(double d) { return log2_rare_key(d
 // log2 of a positive normal finite d (callers route log2_tab_rare arguments
 // elsewhere)
 __device__ __forceinline__ double log2_tab(double d, const double2 *__restrict__ tab) {
-  constexpr double Q0 = 0x1.71547652b82fep+0, Q1 = -0x1.7154765291b6fp-1,
-                   Q2 = 0x1.ec709dc35e431p-2, Q3 = -0x1.7155aa1a01b8ap-2,
-                   Q4 = 0x1.2777ccebb940ap-2;
+  constexpr double Q0 = 0x1.71547652b82fep+0, Q1 = -0x1.71547652b5c85p-1,
+                   Q2 = 0x1.ec709dc39c20ap-2, Q3 = -0x1.7154c3445f43cp-2,
+                   Q4 = 0x1.27770702adfd1p-2;
   const int hi = __double2hiint(d), lo = __double2loint(d);
   const int mh = hi & 0x000FFFFF;
   const double m = __hiloint2double(mh | 0x3FF00000, lo);  // [1, 2)
-  const double2 tj = tab[(mh + (1 << 12)) >> 13];          // nearest 1/128 step: 0..128
+  const double2 tj = tab[(mh + (1 << 11)) >> 12];          // nearest 1/256 step: 0..256
   const double r = fma(m, tj.x, -1.0);
   // the exponent as a double without a conversion instruction: the bits
   // (0x43300000, n) are 2^52 + n

@@ -350,7 +350,7 @@ int fmm_evaluate_noalloc(fmm_plan *plan, const double *tx, const double *ty, int
 int fmm_diag_fail_passes(fmm_plan *plan, void *stream);
 
 /* Diagnostic: the table-driven log2 that the FP64 passes use for the
- * Laplace kernel (exponent split, a table of 129 pairs 1/F and log2 F, a
+ * Laplace kernel (exponent split, a table of 257 pairs 1/F and log2 F, a
  * degree-5 polynomial; Tang, ACM TOMS 16, 1990) and CUDA's log2, at n device
  * points x, into out_table and out_library.  For tests of its accuracy. */
 int fmm_diag_log2(const double *x, int64_t n, double *out_table, double *out_library,
