@@ -88,8 +88,9 @@ __device__ __forceinline__ double log2_tab(double d, const double2 *__restrict__
 
 // 1/d for d in [2^-1022, 2^1021): the hardware's approximate reciprocal
 // (rcp.approx.ftz.f64, about 20 bits), refined by the third-order Newton step
-// y (1 + e + e^2), e = 1 - d y: error e^3, below the last bit
-constexpr unsigned RCP_RARE = 0x7FC00000u;  // log2_rare_key from here on: not for rcp_newton
+// y (1 + e + e^2), e = 1 - d y: error e^3, below the last bit.  (Above,
+// 1/d comes down to 2^-1022, below which the approximation is flushed to 0.)
+constexpr unsigned RCP_RARE = 0x7FB00000u;  // log2_rare_key from here on: not for rcp_newton
 __device__ __forceinline__ double rcp_newton(double d) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
