@@ -1286,7 +1286,7 @@ int fmm_build_expansions_multi(fmm_plan *p, const double *tau, int n_rhs, int64_
     zb.add(p->mult).add(p->ple).add(p->loc).add(p->sync);
     zb.run();
     gather_sorted(tau, p->td.ordv.get(), n, p->tau_s.get(), s, n_rhs, ld_tau);
-    // every pass once per level for all columns (column = blockIdx.y)
+    // every pass once for all columns
     run_upward(a, p->tau_s.get(), p->mult.get(), s, n_rhs, n, cs);
     run_m2l(a, p->mult.get(), p->ple.get(), s, n_rhs, cs);
     run_downward(a, p->ple.get(), p->loc.get(), s, n_rhs, cs);

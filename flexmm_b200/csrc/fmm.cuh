@@ -167,8 +167,9 @@ void run_evaluate_multi(const PassArgs &a, const double *tau_sorted, int64_t n_s
 // as `ready` (recorded on the plan stream once the charges are sorted) has
 // passed, beside the level passes still queued on the plan stream; the far
 // field (L2T) runs on the plan stream after them and adds the near field.
-// near_done / far_done are scratch events of the plan.  Scratch lives on the
-// side stream and is released there after the plan stream has used it.
+// near_done / far_done are scratch events of the plan.  Scratch is the plan's
+// (SplitScratch), or the call's own on the side stream, released there after the
+// plan stream has used it.
 struct SplitEval {
   cudaStream_t side;
   cudaEvent_t ready, near_done, far_done;
@@ -203,7 +204,7 @@ void run_evaluate_sources_split_mixed(const PassArgs &a, const double *tau_sorte
                                       int check, double *out, cudaStream_t s, const SplitEval &se);
 // The FP64 passes; n_rhs charge columns at once (multi-RHS: column r's
 // charges at tau_sorted + r * tstride, its expansions at + r * cstride),
-// one launch per level for all columns.
+// one cooperative launch over the levels each way for all columns.
 void run_upward(const PassArgs &a, const double *tau_sorted, double *mult, cudaStream_t s,
                 int n_rhs = 1, int64_t tstride = 0, int64_t cstride = 0);
 void run_m2l(const PassArgs &a, const double *mult, double *ple, cudaStream_t s, int n_rhs = 1,

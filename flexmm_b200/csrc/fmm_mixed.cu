@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(NT) k_s2m_mx(KernelParams kp, int neq, int np,
       if (threadIdx.x < TN) orow[threadIdx.x] = nlev[threadIdx.x] == m ? P + threadIdx.x * ldp : nullptr;
       cp_async_wait_all();
       __syncthreads();
-      c2e_tile<true>(cv, np, P, T, orow);
+      c2e_tile(cv, np, P, T, orow);
     }
     __syncthreads();
     store_mixed(P, ldp, np, neq, node, TN, mult32, msum, mult_tc);
@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(NT) k_m2m_mx(int m, int neq, int np, int c_fir
       }
   }
   __syncthreads();
-  c2e_tile<true>(cv, np, P, T, orow);
+  c2e_tile(cv, np, P, T, orow);
   __syncthreads();
   store_mixed(P, ldp, np, neq, node, TN, mult32, msum, mult_tc);
 }
@@ -811,7 +811,7 @@ __global__ void __launch_bounds__(NT) k_downward_mx(int m, int neq, int np, int 
   }
   cp_async_wait_all();
   __syncthreads();
-  c2e_tile<true>(cv, np, P, T, orow);
+  c2e_tile(cv, np, P, T, orow);
   __syncthreads();
   store_mixed(P, ldp, np, neq, node, TN, loc32, lsum);
 }

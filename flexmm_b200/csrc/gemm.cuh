@@ -16,9 +16,8 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
 // Warp tile: C[r0 + 8*rb + g][c0 + 8*cb*cstride + 2q + i] += sum_k A[.][k] * B[k][.]
 // for rb < RB and the column blocks cb < CB that start below ncols
 // (g = lane/4, q = lane%4; fragment layouts of mma.m8n8k4.f64).
-// A: shared memory, row-major, stride lda.  B: row-major [K][ldb], in global
-// memory (SB = false) or staged in shared memory (SB = true).
-template <int RB, int CB, bool SB = false>
+// A: shared memory, row-major, stride lda.  B: shared memory, row-major [K][ldb].
+template <int RB, int CB>
 __device__ __forceinline__ void warp_gemm(const double *A, int lda, const double *B, int ldb, int K,
                                           int r0, int c0, int cstride, int ncols,
                                           double (&acc)[RB][CB][2]) {
@@ -33,7 +32,7 @@ __device__ __forceinline__ void warp_gemm(const double *A, int lda, const double
 #pragma unroll
     for (int cb = 0; cb < CB; ++cb) {
       const double *bp = Bp + (size_t)k * ldb + 8 * cb * cstride;
-      b[cb] = (c0 + 8 * cb * cstride < ncols) ? (SB ? *bp : __ldg(bp)) : 0.0;
+      b[cb] = (c0 + 8 * cb * cstride < ncols) ? *bp : 0.0;
     }
 #pragma unroll
     for (int rb = 0; rb < RB; ++rb)
@@ -81,15 +80,11 @@ __device__ __forceinline__ void zero_acc(double (&acc)[RB][CB][2]) {
 }
 
 // Check-to-equivalent operators as a GEMM reads them: U and VH row-major
-// with row stride ld, in global memory or staged in shared memory.
+// with row stride ld, staged in shared memory.
 struct C2EView {
   const double *u, *sinv, *vh;
   int ld;
 };
-
-__device__ __forceinline__ C2EView c2e_global(const LevelOpsDev &op, int np) {
-  return {op.u, op.sinv, op.vh, np};
-}
 
 // start staging a level's check-to-equivalent operators (U, 1/S, VH) in
 // shared memory (asynchronous, see stage_rows): dst holds
@@ -109,7 +104,6 @@ __host__ __device__ inline int c2e_stage_doubles(int np) { return 2 * np * pad_l
 // P, T: shared [32][pad_ld(np)].  Row t goes to out_row[t] (np doubles) when
 // out_row[t] is not null.  Starts and ends with a barrier-free read of P; the
 // caller synchronises before.
-template <bool SB>
 __device__ inline void c2e_tile(const C2EView &op, int np, const double *P, double *T,
                                 double *const *out_row) {
   const int ldp = pad_ld(np);
@@ -117,7 +111,7 @@ __device__ inline void c2e_tile(const C2EView &op, int np, const double *P, doub
   const int r0 = 8 * (warp & 3), c0 = 8 * (warp >> 2);
   double acc[1][4][2];
   zero_acc(acc);
-  warp_gemm<1, 4, SB>(P, ldp, op.u, op.ld, np, r0, c0, 2, np, acc);
+  warp_gemm<1, 4>(P, ldp, op.u, op.ld, np, r0, c0, 2, np, acc);
 #pragma unroll
   for (int cb = 0; cb < 4; ++cb) {
     const int col = c0 + 16 * cb + 2 * q;
@@ -128,7 +122,7 @@ __device__ inline void c2e_tile(const C2EView &op, int np, const double *P, doub
   }
   __syncthreads();
   zero_acc(acc);
-  warp_gemm<1, 4, SB>(T, ldp, op.vh, op.ld, np, r0, c0, 2, np, acc);
+  warp_gemm<1, 4>(T, ldp, op.vh, op.ld, np, r0, c0, 2, np, acc);
   double *o = out_row[r0 + g];
   if (o) {
 #pragma unroll
@@ -137,11 +131,6 @@ __device__ inline void c2e_tile(const C2EView &op, int np, const double *P, doub
       if (col < np) *reinterpret_cast<double2 *>(o + col) = make_double2(acc[0][cb][0], acc[0][cb][1]);
     }
   }
-}
-
-__device__ inline void c2e_tile(const LevelOpsDev &op, int np, const double *P, double *T,
-                                double *const *out_row) {
-  c2e_tile<false>(c2e_global(op, np), np, P, T, out_row);
 }
 
 __device__ __forceinline__ void cp_async_commit_group() {

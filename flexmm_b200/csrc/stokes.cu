@@ -69,18 +69,16 @@ struct StokesSum {
   static constexpr double kLog = -0.5 * 0.69314718055994530942;  // log2(r2) -> -log(r2)/2
 };
 
-// log2(r2) and 1 / r2 of a pair; false for a coincident pair when check is set
-__device__ __forceinline__ bool stokes_radial(const LaplaceF64T &K, double r2, int check, double &l2,
+// log2(r2) and 1 / r2 of a pair
+__device__ __forceinline__ void stokes_radial(const LaplaceF64T &K, double r2, double &l2,
                                               double &i2) {
   if (log2_rare_key(r2) < RCP_RARE) {
     l2 = K.at(r2);
     i2 = rcp_newton(r2);
-    return true;
+  } else {
+    l2 = log2(r2);
+    i2 = 1.0 / r2;
   }
-  if (check && r2 == 0.0) return false;
-  l2 = log2(r2);
-  i2 = 1.0 / r2;
-  return true;
 }
 
 // S2M: velocities at the large circle's points from the box's sources; one
@@ -144,7 +142,7 @@ __global__ void __launch_bounds__(128) k_stokes_s2m(int neq, int np, int L, Stok
           for (int j = 0; j < nj; ++j) {
             const double dx = ex[h] - qx[warp][j], dy = ey[h] - qy[warp][j];
             double l2, i2;
-            stokes_radial(K, fma(dy, dy, dx * dx), 0, l2, i2);
+            stokes_radial(K, fma(dy, dy, dx * dx), l2, i2);
             sum[h].add(dx, dy, qf[warp][j], qg[warp][j], l2, i2);
             if constexpr (DIP) sum[h].add_dipole(dx, dy, qs[warp][j], qn[warp][j], i2);
           }
@@ -247,7 +245,7 @@ struct StokesPolicy {
           double l2, i2;
           // a pair is left out where it coincides, not where r2 underflows
           if (chk && dx[r] == 0.0 && dy[r] == 0.0) continue;
-          stokes_radial(K, r2[r], 0, l2, i2);
+          stokes_radial(K, r2[r], l2, i2);
           one(dx[r], dy[r], q, j, sum[r], l2, i2);
         }
       }

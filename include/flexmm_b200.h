@@ -145,7 +145,7 @@ int fmm_bb_ops_add(fmm_ops *ops, const fmm_bb_level_ops *lv, int *level_id);
  * with Q [NQ x rank] orthonormal and core_o [rank x rank] (NULL where m2l_rank
  * is 0), row-major, rank <= FMM_BB_MAX_RANK.  A smooth kernel's 40 operators
  * share a column space far smaller than NQ = p^2 (62 of 256 to 1e-16 for the
- * log kernel, p = 16); a plan whose levels all have one translates in it. */
+ * log kernel, p = 16); a level that has one translates in it. */
 #define FMM_BB_MAX_RANK 64
 int fmm_bb_ops_set_basis(fmm_ops *ops, int level_id, int rank, const double *q,
                          const double *const *core);
@@ -235,7 +235,7 @@ int fmm_build_expansions_dipole(fmm_plan *plan, const double *tau, const double 
 /* Several charge columns on one tree (multi-RHS; the reference's kifmm2d
  * FMM takes tau [k, N], flexmm/kifmm2d/scalar/fmm.py:71-87): column r is
  * tau[r * ld_tau .. + n), caller's source order.  FP64 KIFMM plans.  The
- * evaluation computes each kernel value once for up to 8 columns; result
+ * evaluation computes each kernel value once for up to 16 columns; result
  * row r is out[r * ld_out .. + m).  fmm_evaluate after a multi build uses
  * column 0. */
 int fmm_build_expansions_multi(fmm_plan *plan, const double *tau, int n_rhs, int64_t ld_tau,
