@@ -300,6 +300,10 @@ StokesCircles circles(const StokesArgs &a) {
 
 // ---- level passes: a tile of 8 RB rows, warp w computing column block w ----
 constexpr int ST_AHEAD = 8;  // fragment pairs in flight per warp
+// threads of the widest row's block (Nequiv 64: 136 columns).  17 warps are five on
+// one of the SM's four parts, which holds that many of 96 registers a thread; the
+// level kernels take 64 at most by themselves.
+constexpr int ST_MAX_THREADS = 544;
 
 // acc[r] += A[8 r ..][.] . B over npairs k pairs of B's column block cb (of nb
 // in a k pair); A in shared memory, operator fragments from L2
@@ -374,7 +378,8 @@ struct StokesLevels {
 
 // E2C solve of the S2M nodes of all levels: partial check rows -> multipoles
 template <int RB>
-__global__ void k_st_leaves(StokesLevels ops, int np, int L, const int *__restrict__ off,
+__global__ void __launch_bounds__(ST_MAX_THREADS)
+    k_st_leaves(StokesLevels ops, int np, int L, const int *__restrict__ off,
                             const int *__restrict__ uplist, const int *__restrict__ n_up_ptr,
                             const double *__restrict__ partial, double *__restrict__ mult) {
   constexpr int ROWS = 8 * RB;
