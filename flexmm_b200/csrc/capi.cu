@@ -1115,13 +1115,11 @@ struct LevelOpsSrc {
   double width[FMM_MAX_LEVELS_DEV];  // what a box's sources keep to; infinite once they were moved
   // scaling of levels without operators (0 and 1 need none: no expansions there,
   // but the mixed near field of a leaf there does read its scaling)
-  struct Scale {
-    double inv_w, kofs;
-  } scale[FMM_MAX_LEVELS_DEV];
+  double inv_w[FMM_MAX_LEVELS_DEV], kofs[FMM_MAX_LEVELS_DEV];
 };
-static_assert(offsetof(LevelOpsDev, kofs) == offsetof(LevelOpsDev, inv_w) + sizeof(double),
-              "LevelOpsSrc::Scale is copied over both");
 static_assert(sizeof(LevelOpsDev) % sizeof(int) == 0, "LevelOpsDev is copied as words");
+static_assert(offsetof(LevelOpsDev, kofs) == offsetof(LevelOpsDev, inv_w) + sizeof(double),
+              "k_gather_level_ops fills in both together");
 
 __global__ void k_gather_level_ops(LevelOpsSrc src, LevelOpsDev *__restrict__ dst) {
   constexpr int NW = int(sizeof(LevelOpsDev) / sizeof(int));
@@ -1129,15 +1127,17 @@ __global__ void k_gather_level_ops(LevelOpsSrc src, LevelOpsDev *__restrict__ ds
   int *to = reinterpret_cast<int *>(dst + blockIdx.x);
   constexpr int SCALE = int(offsetof(LevelOpsDev, inv_w) / sizeof(int));
   constexpr int BOX = int(offsetof(LevelOpsDev, box32) / sizeof(int));
-  const LevelOpsSrc::Scale &sc = src.scale[blockIdx.x];
-  for (int i = threadIdx.x; i < NW; i += blockDim.x) {
-    int v = from ? from[i] : 0;
-    if (i == BOX)
-      v = __float_as_int(float(src.width[blockIdx.x] * (from ? src.p[blockIdx.x]->inv_w : sc.inv_w)));
-    else if (!from && i >= SCALE && i < SCALE + 4)
-      v = reinterpret_cast<const int *>(&sc)[i - SCALE];
-    to[i] = v;
-  }
+  const double iw = from ? src.p[blockIdx.x]->inv_w : src.inv_w[blockIdx.x];
+  for (int i = threadIdx.x; i < NW; i += blockDim.x) to[i] = from ? from[i] : 0;
+  // what the tree adds, each word by the thread that has just copied it
+  auto mine = [](int word) { return threadIdx.x == word % blockDim.x; };
+  if (mine(BOX)) to[BOX] = __float_as_int(float(src.width[blockIdx.x] * iw));
+  if (!from)
+    for (int k = 0; k < 4; ++k)
+      if (mine(SCALE + k)) {
+        const double d = k < 2 ? iw : src.kofs[blockIdx.x];
+        to[SCALE + k] = k & 1 ? __double2hiint(d) : __double2loint(d);
+      }
 }
 
 static void upload_level_ops(fmm_plan *p, cudaStream_t s) {
@@ -1152,8 +1152,8 @@ static void upload_level_ops(fmm_plan *p, cudaStream_t s) {
     if (p->bound[m] >= 0) {
       src.p[m] = p->ops->levels[p->bound[m]]->dev_copy.get();
     } else {
-      src.scale[m] = {scaled ? 1.0 / w : 1.0,
-                      scaled ? kernel_offset(p->ops->kernel_id, p->ops->kp, w) : 0.0};
+      src.inv_w[m] = scaled ? 1.0 / w : 1.0;
+      src.kofs[m] = scaled ? kernel_offset(p->ops->kernel_id, p->ops->kp, w) : 0.0;
     }
   }
   k_gather_level_ops<<<L, 128, 0, s>>>(src, p->ops_dev.get());
