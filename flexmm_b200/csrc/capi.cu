@@ -443,10 +443,10 @@ cudaStream_t side_stream(cudaStream_t *pass) {
 }
 
 // Whether own-source evaluation runs split (near field beside the level
-// passes).  Measured, off and on: a step of 1M clustered sources 2.34 and 2.27
-// ms, of 200k with K0 0.97 and 0.86, a product on 250k ring points 0.58 and 0.49;
+// passes).  Measured, off and on: a step of 1M clustered sources 2.35 and 2.28
+// ms, of 200k with K0 0.96 and 0.85, a product on 250k ring points 0.56 and 0.50;
 // the mixed form, whose near field pauses while the persistent tcgen05 M2L
-// runs, 1.18 and 1.14 ms at 1M.  On for both by default;
+// runs, 1.21 and 1.18 ms at 1M.  On for both by default;
 // FLEXMM_B200_SPLIT_EVAL=0 turns it off, =1 on.
 std::atomic<int> g_split_mode{-2};  // -2: not yet read from the environment
 

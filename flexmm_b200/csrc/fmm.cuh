@@ -140,8 +140,9 @@ struct EvalItems {
 // before `ready` is recorded, kept, and used by one evaluation at a time (each
 // leaves the side stream waiting for its end).  Allocated on the side stream by
 // each call, its memory changed streams at every step, which the allocator has
-// to order: a step of 100k points took 668 us of the host, 383 so; the mixed step
-// of 1M 1.177 -> 1.140 ms in a row, 1.55 -> 1.20 from a new state.
+// to order.  One step at a time, each call's own and the plan's: 100k points 0.71
+// and 0.50 ms, 1M 2.54 and 2.31, the mixed 1M 1.52 and 1.23; in a row 476 and 468
+// us, 2.29 and 2.28 ms, 1.184 and 1.180.
 struct SplitScratch {
   EvalItems it;
   DevBuf<double> near;         // near-field potentials
